@@ -122,6 +122,7 @@ add_layernorm_kernel(const uint4* x, const uint4* residual, const uint4* __restr
   const long long warp0 = (long long)blockIdx.x * kWarpsPerBlock + (threadIdx.x >> 5);
   const long long stride = (long long)gridDim.x * kWarpsPerBlock;
   wait_for_predecessor();
+  release_successor();
   for (long long row = warp0; row < rows; row += stride) {
     // an index outside its table reads as a row of zeros and is reported through the status word
     long long x_row = row, res_row = row;
@@ -244,6 +245,7 @@ __global__ void __launch_bounds__(256) copy_rows_kernel(const uint4* __restrict_
   const long long warp0 = (long long)blockIdx.x * 8 + (threadIdx.x >> 5);
   const long long stride = (long long)gridDim.x * 8;
   wait_for_predecessor();
+  release_successor();
   for (long long r = warp0; r < n_rows; r += stride) {
     const long long from = rows[r];
     for (int c = lane; c < vecs_per_row; c += 32)

@@ -75,22 +75,34 @@ inline int configure_kernel(KernelDeviceConfig& cfg, Kernel kernel, int smem_byt
 // This takes the launch latency and the kernel's set-up (barrier initialisation, tensor-memory allocation, descriptor
 // prefetch) off the path between two dependent kernels.
 template <typename... KArgs, typename... Args>
-inline cudaError_t launch_after_predecessor(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
-                                            cudaStream_t stream, Args... args) {
+inline cudaError_t launch_clusters_after_predecessor(void (*kernel)(KArgs...), dim3 grid, dim3 block, int cluster,
+                                                     size_t smem, cudaStream_t stream, Args... args) {
   cudaLaunchConfig_t cfg{};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
+  cudaLaunchAttribute attr[2];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
+  attr[1].id = cudaLaunchAttributeClusterDimension;
+  attr[1].val.clusterDim.x = cluster;
+  attr[1].val.clusterDim.y = attr[1].val.clusterDim.z = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  cfg.numAttrs = cluster > 0 ? 2 : 1;   // 0: no cluster, or the kernel's own __cluster_dims__
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+template <typename... KArgs, typename... Args>
+inline cudaError_t launch_after_predecessor(void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem,
+                                            cudaStream_t stream, Args... args) {
+  return launch_clusters_after_predecessor(kernel, grid, block, 0, smem, stream, args...);
 }
 // Device side of the above: wait for the previous kernel of the stream (no-op for a plain launch).
 __device__ __forceinline__ void wait_for_predecessor() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+// Lets the next kernel of the stream be scheduled as soon as every CTA of this grid has called it (its own
+// wait_for_predecessor() still holds it back until this grid has completed).  Called only after this kernel's own
+// wait: whatever ran before this kernel is then complete when the next kernel starts its set-up.
+__device__ __forceinline__ void release_successor() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 
 inline bool aligned16(const void* p) { return (reinterpret_cast<uintptr_t>(p) & 15u) == 0; }
 
@@ -161,6 +173,9 @@ struct GemmDesc {
   // rows row_groups[g] .. +31 of the [out_seqs * rows_per_seq] output row space.  Null: row m goes to row m.
   const int* row_groups;
   int out_seqs;         // sequences of the output tensors when row_groups is set (else M / rows_per_seq)
+  // 1: the kernel before this one in the stream is one of this library's that waited for its own predecessor and
+  // does not write W or the bias, so that W may be read before that kernel has finished (see release_successor())
+  int weights_early;
 };
 
 // tanh for the GEMM epilogues of 16-bit outputs: 1 - 2 / (1 + e^(2x)) with approximate exp2 and reciprocal

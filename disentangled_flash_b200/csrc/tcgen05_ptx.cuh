@@ -136,6 +136,40 @@ __device__ __forceinline__ void tma_load_3d(void* smem_dst, const CUtensorMap* m
       : "memory");
 }
 
+// Four-dimensional load issued by one elected lane of a converged warp (operands stay warp-uniform, see
+// umma_ss_f16_warp); `bar_cluster_addr` is a shared::cluster address when PAIR.
+template <bool PAIR>
+__device__ __forceinline__ void tma_load_4d_warp(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar, int x, int y,
+                                                 int z, int w) {
+  if (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.4d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+        ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+        "@q cp.async.bulk.tensor.4d.shared::cluster.global.mbarrier::complete_tx::bytes"
+        " [%0], [%1, {%3, %4, %5, %6}], [%2];\n\t}"
+        ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar), "r"(x), "r"(y), "r"(z), "r"(w)
+        : "memory");
+}
+__device__ __forceinline__ void mbar_arrive_expect_tx_warp(uint32_t bar, uint32_t bytes) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;\n\t}" ::"r"(bar), "r"(bytes) : "memory");
+}
+
+// Contiguous copy from this CTA's shared memory to the shared memory of another CTA of the cluster (16-byte aligned
+// addresses and size); the bytes are reported to a barrier of the destination CTA.
+__device__ __forceinline__ void bulk_copy_to_cta(uint32_t dst_cluster, uint32_t src, uint32_t bytes, uint32_t bar_cluster) {
+  asm volatile("cp.async.bulk.shared::cluster.shared::cta.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
+               ::"r"(dst_cluster), "r"(src), "r"(bytes), "r"(bar_cluster)
+               : "memory");
+}
+
 // Tiled store shared -> global (bulk async-group completion).  x is the innermost coordinate and must be a
 // multiple of 16 bytes; coordinates are never negative here.
 __device__ __forceinline__ void tma_store_3d(const CUtensorMap* map, const void* smem_src, int x, int y, int z) {
@@ -235,6 +269,11 @@ __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank
 __device__ __forceinline__ void cluster_sync_all() {
   asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
 }
+// Execution barrier only: nothing this CTA wrote before it has to be visible to the others (a releasing arrive waits
+// for every outstanding global store of the CTA, 0.6 us at the end of a GEMM).
+__device__ __forceinline__ void cluster_sync_all_relaxed() {
+  asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
+}
 __device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
@@ -268,13 +307,57 @@ __device__ __forceinline__ void umma_ss_f16_pair(uint32_t d_tmem, uint64_t a_des
       ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
-// Arrive on the barrier at the same shared-memory offset in both CTAs of the pair when all previously issued MMAs
-// of this thread have completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar) {
-  const uint16_t both = 3;
+// Arrive on the barrier at the same shared-memory offset in both CTAs of the pair (cluster ranks `leader` and
+// leader + 1) when all previously issued MMAs of this thread have completed.
+__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t leader = 0) {
+  const uint16_t both = (uint16_t)(3u << leader);
   asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
                ::"r"(smem_u32(bar)), "h"(both)
                : "memory");
+}
+
+// The same instructions for a whole converged warp: the operands are computed by every lane, hence warp-uniform, and
+// one elected lane issues (the same lane every time, so that a commit covers the MMAs before it).  A branch on the lane
+// around the plain forms keeps the operands out of the uniform registers the instruction reads, and moving them there
+// costs more than a narrow MMA runs: M=128 SS N=32 / 64 / 128 measured 41 / 49 / 65 cycles per MMA in this form, 57 /
+// 57 / 65 in the other; with A in TMEM 18 / 33 / 65 against 54 / 54 / 65.
+__device__ __forceinline__ void umma_ss_f16_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ts_f16_warp(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                                 uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_ss_f16_pair_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
+                                                      uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p, q;\n\telect.sync _|q, 0xffffffff;\n\tsetp.ne.b32 p, %4, 0;\n\t"
+      "@q tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
+      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
+      : "memory");
+}
+__device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar, uint32_t leader = 0) {
+  const uint16_t both = (uint16_t)(3u << leader);
+  asm volatile(
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
+      ::"r"(smem_u32(bar)), "h"(both)
+      : "memory");
 }
 
 // TMEM <-> registers: each thread of a warp owns one lane (row); N consecutive 32-bit columns.
@@ -296,6 +379,27 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
       "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+      : "r"(taddr)
+      : "memory");
+}
+// The same as fp32 values.
+__device__ __forceinline__ void tmem_ld32_f(uint32_t taddr, float (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
+        "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15]), "=f"(r[16]),
+        "=f"(r[17]), "=f"(r[18]), "=f"(r[19]), "=f"(r[20]), "=f"(r[21]), "=f"(r[22]), "=f"(r[23]), "=f"(r[24]),
+        "=f"(r[25]), "=f"(r[26]), "=f"(r[27]), "=f"(r[28]), "=f"(r[29]), "=f"(r[30]), "=f"(r[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tmem_ld16_f(uint32_t taddr, float (&r)[16]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, "
+      "[%16];"
+      : "=f"(r[0]), "=f"(r[1]), "=f"(r[2]), "=f"(r[3]), "=f"(r[4]), "=f"(r[5]), "=f"(r[6]), "=f"(r[7]), "=f"(r[8]),
+        "=f"(r[9]), "=f"(r[10]), "=f"(r[11]), "=f"(r[12]), "=f"(r[13]), "=f"(r[14]), "=f"(r[15])
       : "r"(taddr)
       : "memory");
 }
@@ -367,5 +471,13 @@ __host__ __device__ constexpr uint32_t make_idesc_f16(int is_bf16, int m, int n,
 int encode_tensor_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t batch,
                          uint64_t row_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_inner,
                          uint32_t box_rows, int swizzle_bytes);
+
+// 4-D map of K-major operands for k-blocks of 64 elements, 128-byte swizzle.  box_pieces = 1: {inner, rows, batch, 1},
+// a load at x = 64 * k-block brings one block (zeros beyond `inner`).  box_pieces > 1: {64, rows, batch, inner / 64}, a
+// load at piece k-block brings `box_pieces` consecutive blocks, one 128-byte-swizzle tile behind the other; `inner` must
+// be a multiple of 64 and the rows of a box a multiple of 8.
+int encode_tensor_map_pieces(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t batch,
+                             uint64_t row_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_rows,
+                             uint32_t box_batch, uint32_t box_pieces);
 
 }  // namespace dfl
