@@ -39,6 +39,7 @@ workload; under torchrun only rank 0 runs it.
 from __future__ import annotations
 
 import argparse
+import ctypes
 import json
 import os
 import statistics
@@ -207,6 +208,26 @@ class LaunchObserver:
     def install(self, binding):
         for attr, name in self.KERNELS.items():
             setattr(binding, attr, self._wrap(getattr(binding, attr), name))
+        binding.encoder_fwd = self._wrap_encoder(binding.encoder_fwd)
+
+    def _wrap_encoder(self, fn):
+        """The whole layer loop is one call: it reports how many kernels it launched and records events around the
+        attention of every layer where it is given some."""
+
+        def call(p, device):
+            if not self.enabled:
+                return fn(p, device)
+            events = [torch.cuda.Event(enable_timing=True) for _ in range(2 * p.n_layers)]
+            for event in events:
+                event.record()   # creates the handle; the call records it again at its place
+            p.attention_events = (ctypes.c_void_p * len(events))(*(event.cuda_event for event in events))
+            fn(p, device)
+            self.launches += p.launches
+            first = p.layers[0]
+            self.kernel_name = "dfl_attention_rel_fwd" if first.rel_key or first.rel_query else "dfl_attention_fwd"
+            self.events += list(zip(events[::2], events[1::2]))
+
+        return call
 
     def _wrap(self, fn, name):
         def call(*args, **kwargs):

@@ -53,6 +53,8 @@ EXPORTED_SYMBOLS = (
     "dfl_expand_rel_tables",
     "dfl_attention_rel_supported",
     "dfl_attention_rel_fwd",
+    "dfl_encoder_workspace_bytes",
+    "dfl_encoder_fwd",
 )
 
 
@@ -133,6 +135,27 @@ class DflEmbedLayerNormParams(Structure):
                 ("mask_elem_size", c_int), ("status", c_void_p)]
 
 
+class DflEncoderLayer(Structure):
+    _fields_ = [(name, c_void_p) for name in (
+        "qkv_w", "qkv_b", "attn_out_w", "attn_out_b", "attn_norm_w", "attn_norm_b", "ffn_in_w", "ffn_in_b", "ffn_out_w",
+        "ffn_out_b", "ffn_norm_w", "ffn_norm_b", "rel_key", "rel_query", "pos_key", "pos_query")] + [
+        ("attn_norm_eps", c_float), ("ffn_norm_eps", c_float)]
+
+
+class DflEncoderParams(Structure):
+    _fields_ = [
+        ("layers", POINTER(DflEncoderLayer)), ("outs", POINTER(c_void_p)), ("x", c_void_p), ("mask", c_void_p),
+        ("workspace", c_void_p), ("workspace_bytes", ctypes.c_size_t), ("lut", c_void_p), ("status", c_void_p),
+        ("conv_w", c_void_p), ("conv_b", c_void_p), ("conv_norm_w", c_void_p), ("conv_norm_b", c_void_p),
+        ("conv_taps", c_int32), ("conv_activation", c_int32), ("conv_norm_eps", c_float),
+        ("n_layers", c_int32), ("batch", c_int32), ("seq_len", c_int32), ("hidden", c_int32), ("heads", c_int32),
+        ("head_dim", c_int32), ("ffn", c_int32), ("n_active", c_int32), ("mask_elem_size", c_int32), ("dtype", c_int32),
+        ("scale", c_float), ("attention_events", POINTER(c_void_p)), ("launches", c_int32), ("packed_rows", c_int32),
+        ("pack_rows", c_void_p), ("row_groups", c_void_p), ("row_base", c_void_p), ("row_count", c_void_p),
+        ("qkv", c_void_p * 3),
+    ]
+
+
 class DflError(RuntimeError):
     """A C entry point returned a negative status."""
 
@@ -196,6 +219,10 @@ def load_library() -> ctypes.CDLL:
     lib.dfl_attention_rel_supported.argtypes = [POINTER(DflAttnRelParams)]
     lib.dfl_attention_rel_fwd.restype = c_int
     lib.dfl_attention_rel_fwd.argtypes = [POINTER(DflAttnRelParams), c_void_p]
+    lib.dfl_encoder_workspace_bytes.restype = ctypes.c_size_t
+    lib.dfl_encoder_workspace_bytes.argtypes = [POINTER(DflEncoderParams)]
+    lib.dfl_encoder_fwd.restype = c_int
+    lib.dfl_encoder_fwd.argtypes = [POINTER(DflEncoderParams), c_void_p]
     _lib = lib
     return lib
 
@@ -700,3 +727,15 @@ def attention_rel_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, rel_key
     with _on_device(q.device):
         _check(lib.dfl_attention_rel_fwd(ctypes.byref(p), _stream(q.device)), "dfl_attention_rel_fwd")
     return out
+
+
+def encoder_fwd(p: DflEncoderParams, device: torch.device) -> None:
+    """The whole layer loop (``dfl_encoder_fwd``) on the current stream; every field but the workspace is the caller's."""
+
+    lib = load_library()
+    ref = ctypes.byref(p)
+    size = lib.dfl_encoder_workspace_bytes(ref)
+    with _on_device(device):
+        workspace = torch.empty(size, dtype=torch.uint8, device=device)
+        p.workspace, p.workspace_bytes = workspace.data_ptr(), size
+        _check(lib.dfl_encoder_fwd(ref, _stream(device)), "dfl_encoder_fwd")

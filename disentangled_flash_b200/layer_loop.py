@@ -1,0 +1,192 @@
+"""The prepared layer loop of one bucket as a single native call (``dfl_encoder_fwd``).
+
+Built by ``DebertaV2InferenceEncoder.prepare_for_inference`` for a bucket whose layers all have the Hugging Face shape
+in a 16-bit type; the encoder's Python loop serves everything else.  Holds the pointers of every parameter the loop reads
+and compares them with the modules' current ones before each call, so a parameter that was exchanged or moved after the
+preparation is never read at its old place.
+"""
+
+from __future__ import annotations
+
+import ctypes
+import math
+from typing import Any
+
+import torch
+from torch import nn
+
+from . import _cabi
+
+_LAYER_FIELDS = (
+    ("qkv_w", "attention.self", "_cached_qkv_weight"), ("qkv_b", "attention.self", "_cached_qkv_bias"),
+    ("attn_out_w", "attention.output.dense", "weight"), ("attn_out_b", "attention.output.dense", "bias"),
+    ("attn_norm_w", "attention.output.LayerNorm", "weight"), ("attn_norm_b", "attention.output.LayerNorm", "bias"),
+    ("ffn_in_w", "intermediate.dense", "weight"), ("ffn_in_b", "intermediate.dense", "bias"),
+    ("ffn_out_w", "output.dense", "weight"), ("ffn_out_b", "output.dense", "bias"),
+    ("ffn_norm_w", "output.LayerNorm", "weight"), ("ffn_norm_b", "output.LayerNorm", "bias"),
+)
+_data_ptr = torch.Tensor.data_ptr
+
+
+def _module_at(root: nn.Module, path: str) -> nn.Module:
+    for name in path.split("."):
+        root = getattr(root, name)
+    return root
+
+
+class LayerLoop:
+    """One bucket of one encoder.  ``build`` returns None where the loop does not cover the encoder."""
+
+    def __init__(self) -> None:
+        self.plans: Any = None
+        self.length = 0
+
+    @staticmethod
+    def build(encoder: nn.Module, length: int, plans: Any, conv_covered: bool) -> "LayerLoop | None":
+        first = encoder.layer[0].attention.self
+        weight = first.query_proj.weight
+        dtype, device = weight.dtype, weight.device
+        if device.type != "cuda" or dtype not in (torch.float16, torch.bfloat16):
+            return None
+        if not (all(a and b for a, b in encoder._fused_output_blocks) and all(encoder._fused_intermediates)):
+            return None
+        if encoder.conv is not None and not conv_covered:
+            return None
+        self = LayerLoop()
+        self.plans, self.length, self.device, self.dtype = plans, length, device, dtype
+        self.attention = [layer.attention.self for layer in encoder.layer]
+        hidden, ffn = weight.shape[1], encoder.layer[0].intermediate.dense.weight.shape[0]
+        width = first.all_head_size
+        if hidden % 8 or ffn % 8 or first.attention_head_size not in (32, 64, 128):
+            return None
+        n = len(encoder.layer)
+        self.layers = (_cabi.DflEncoderLayer * n)()
+        # (owner dict, key) of every tensor the loop reads, and where it was
+        self._owners: list[dict] = []
+        self._keys: list[str] = []
+
+        def read(module: nn.Module, key: str) -> torch.Tensor | None:
+            for owner in (module._parameters, module._buffers):
+                tensor = owner.get(key)
+                if tensor is not None:
+                    if tensor.dtype != dtype or tensor.device != device or not tensor.is_contiguous():
+                        raise _NotCovered
+                    self._owners.append(owner)
+                    self._keys.append(key)
+                    return tensor
+            return None
+
+        shapes = {"qkv_w": (3 * width, hidden), "attn_out_w": (hidden, width), "ffn_in_w": (ffn, hidden),
+                  "ffn_out_w": (hidden, ffn), "attn_norm_w": (hidden,), "ffn_norm_w": (hidden,)}
+        try:
+            for index, layer in enumerate(encoder.layer):
+                entry, plan = self.layers[index], plans[index]
+                for field, path, key in _LAYER_FIELDS:
+                    tensor = read(_module_at(layer, path), key)
+                    if field in shapes and (tensor is None or tuple(tensor.shape) != shapes[field]):
+                        return None
+                    setattr(entry, field, None if tensor is None else tensor.data_ptr())
+                entry.attn_norm_eps = float(layer.attention.output.LayerNorm.eps)
+                entry.ffn_norm_eps = float(layer.output.LayerNorm.eps)
+                module = layer.attention.self
+                has_c2p, has_p2c = module.has_c2p, module.has_p2c
+                if has_c2p != first.has_c2p or has_p2c != first.has_p2c or module.pos_att_type != first.pos_att_type:
+                    return None
+                for field, wanted in (("rel_key", has_c2p), ("rel_query", has_p2c), ("pos_key", has_c2p), ("pos_query", has_p2c)):
+                    tensor = getattr(plan, field) if wanted else None
+                    setattr(entry, field, None if tensor is None else tensor.data_ptr())
+            p = _cabi.DflEncoderParams()
+            if encoder.conv is not None:
+                norm = encoder.conv.LayerNorm
+                bias = read(encoder.conv.conv, "bias")
+                gamma, beta = read(norm, "weight"), read(norm, "bias")
+                read(encoder.conv.conv, "weight")
+                self._conv_weight = encoder._conv_weight   # [taps, out, in], permuted at prepare time
+                p.conv_w, p.conv_b = self._conv_weight.data_ptr(), None if bias is None else bias.data_ptr()
+                p.conv_norm_w, p.conv_norm_b = gamma.data_ptr(), None if beta is None else beta.data_ptr()
+                p.conv_taps, p.conv_activation = self._conv_weight.shape[0], encoder._conv_activation_code
+                p.conv_norm_eps = float(norm.eps)
+        except _NotCovered:
+            return None
+        self._pointers = self._current_pointers()
+        lut = plans[0].delta_to_local
+        p.layers, p.n_layers = self.layers, n
+        p.seq_len, p.hidden, p.heads, p.head_dim, p.ffn = length, hidden, first.num_attention_heads, first.attention_head_size, ffn
+        p.lut, p.n_active = lut.data_ptr(), plans[0].active_slots.numel()
+        terms = 1 + int("c2p" in first.pos_att_type) + int("p2c" in first.pos_att_type)
+        p.scale, p.dtype = 1.0 / math.sqrt(first.attention_head_size * terms), _cabi.dtype_code(dtype)
+        self.params, self.n_layers, self.hidden = p, n, hidden
+        return self
+
+    def _current_pointers(self) -> list[int]:
+        return list(map(_data_ptr, map(dict.__getitem__, self._owners, self._keys)))
+
+    def covers(self, encoder: nn.Module, plans: Any, hidden: torch.Tensor, mask: torch.Tensor) -> bool:
+        """Whether this call can take the native loop (the state it was built from still holds)."""
+
+        if plans is not self.plans or hidden.dtype != self.dtype or hidden.device != self.device or hidden.dim() != 3:
+            return False
+        if hidden.shape[1] != self.length or hidden.shape[2] != self.hidden or hidden.shape[0] < 1:
+            return False
+        if mask.shape != hidden.shape[:2] or mask.device != self.device or torch.is_grad_enabled():
+            return False
+        for fused in encoder._fused_output_blocks:
+            if not (fused[0] and fused[1]):
+                return False
+        if not all(encoder._fused_intermediates):
+            return False
+        for module in self.attention:
+            if module.training or module._algo != _cabi.ALGO_AUTO:
+                return False
+        try:
+            return self._current_pointers() == self._pointers
+        except (KeyError, TypeError):   # a parameter was deleted or set to None
+            return False
+
+    def _call(self, hidden: torch.Tensor, mask: torch.Tensor, outs: Any, status: torch.Tensor | None) -> _cabi.DflEncoderParams:
+        if mask.dtype.is_floating_point or mask.element_size() not in (1, 4, 8):
+            mask = mask.bool()
+        hidden, mask = hidden.contiguous(), mask.contiguous()
+        p = _cabi.DflEncoderParams()
+        ctypes.pointer(p)[0] = self.params   # a copy: several threads may run one bucket
+        p.x, p.mask, p.mask_elem_size, p.batch = hidden.data_ptr(), mask.data_ptr(), mask.element_size(), hidden.shape[0]
+        p.status = None if status is None else status.data_ptr()
+        p.outs = outs
+        p._keep = (hidden, mask)
+        return p
+
+    def run(self, hidden: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None,
+            trace: list[torch.Tensor] | None) -> torch.Tensor:
+        outs = (ctypes.c_void_p * self.n_layers)()
+        out = torch.empty(hidden.shape, dtype=self.dtype, device=self.device)
+        outs[self.n_layers - 1] = out.data_ptr()
+        if trace is not None:
+            for layer in range(self.n_layers - 1):
+                state = torch.empty(hidden.shape, dtype=self.dtype, device=self.device)
+                outs[layer] = state.data_ptr()
+                trace.append(state)
+            trace.append(out)
+        _cabi.encoder_fwd(self._call(hidden, mask, outs, status), self.device)
+        return out
+
+    def run_packed(self, hidden: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None, out: torch.Tensor,
+                   tables: tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor],
+                   qkv: tuple[torch.Tensor, ...]) -> None:
+        """``tables`` = (pack_rows, row_groups, row_base, row_count); the result goes to the covered rows of ``out``."""
+
+        outs = (ctypes.c_void_p * self.n_layers)()
+        outs[self.n_layers - 1] = out.data_ptr()
+        p = self._call(hidden, mask, outs, status)
+        pack_rows, row_groups, row_base, row_count = tables
+        p.packed_rows, p.pack_rows, p.row_groups = pack_rows.numel(), pack_rows.data_ptr(), row_groups.data_ptr()
+        p.row_base, p.row_count = row_base.data_ptr(), row_count.data_ptr()
+        for i in range(3):
+            p.qkv[i] = qkv[i].data_ptr()
+        _cabi.encoder_fwd(p, self.device)
+
+
+class _NotCovered(Exception):
+    pass
+
+
+__all__ = ["LayerLoop"]

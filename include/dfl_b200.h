@@ -385,6 +385,61 @@ typedef struct DflEmbedLayerNormParams {
 } DflEmbedLayerNormParams;
 DFL_API int dfl_embed_layernorm(const DflEmbedLayerNormParams* p, void* stream);
 
+/*
+ * The layer loop of a prepared encoder in one call (deberta.py:247-285): per layer the fused QKV projection, the
+ * attention, attention.output (dense, residual, LayerNorm), intermediate (dense + erf GELU) and output (dense, residual,
+ * LayerNorm), and after layer 0 the optional convolution branch.  Every step is one of the functions above; the call
+ * exists because a forward of a small batch is bound by what the host spends per launch, and because a kernel that is
+ * known to follow one of this library's may load its weights before that one has finished.
+ * F16/BF16, hidden == heads * head_dim not required, hidden and ffn multiples of 8, hidden as dfl_add_layernorm takes it.
+ * Attention: rel_key / rel_query where given (dfl_attention_rel_fwd), else pos_key / pos_query (dfl_pos_scores +
+ * dfl_attention_fwd, `lut` required).
+ */
+typedef struct DflEncoderLayer {
+  const void *qkv_w, *qkv_b;              /* [3*heads*head_dim, hidden], [3*heads*head_dim] or NULL */
+  const void *attn_out_w, *attn_out_b;    /* [hidden, heads*head_dim], [hidden] or NULL */
+  const void *attn_norm_w, *attn_norm_b;  /* [hidden], [hidden] or NULL */
+  const void *ffn_in_w, *ffn_in_b;        /* [ffn, hidden], [ffn] or NULL */
+  const void *ffn_out_w, *ffn_out_b;      /* [hidden, ffn], [hidden] or NULL */
+  const void *ffn_norm_w, *ffn_norm_b;    /* [hidden], [hidden] or NULL */
+  const void *rel_key, *rel_query;        /* [heads, 2L-1, head_dim] or NULL */
+  const void *pos_key, *pos_query;        /* [heads, n_active, head_dim] or NULL; used when both rel_* are NULL */
+  float attn_norm_eps, ffn_norm_eps;
+} DflEncoderLayer;
+typedef struct DflEncoderParams {
+  const DflEncoderLayer* layers;   /* host array [n_layers] */
+  void* const* outs;               /* host array [n_layers]: where layer l's result goes, [batch, seq_len, hidden]; NULL
+                                      entries keep it in the workspace.  The last entry must be given. */
+  const void* x;                   /* [batch, seq_len, hidden] */
+  const void* mask;                /* [batch, seq_len], mask_elem_size bytes per element */
+  void* workspace;                 /* dfl_encoder_workspace_bytes() bytes, 16-byte aligned, contents undefined */
+  size_t workspace_bytes;
+  const int32_t* lut;              /* [2L-1], for the pos_* form */
+  int32_t* status;                 /* optional device int32, see dfl_check_status() */
+  /* convolution branch after layer 0, or conv_w NULL: x_1 = keep * LayerNorm(x_1 + act(keep * conv1d(x))) */
+  const void *conv_w, *conv_b, *conv_norm_w, *conv_norm_b;   /* [taps, hidden, hidden], [hidden], [hidden], [hidden] */
+  int32_t conv_taps, conv_activation;
+  float conv_norm_eps;
+  int32_t n_layers, batch, seq_len, hidden, heads, head_dim, ffn, n_active;
+  int32_t mask_elem_size, dtype;
+  float scale;
+  /* Optional timing marks (cudaEvent_t handles, host array [2 * n_layers] or NULL): event 2l is recorded before and
+   * event 2l+1 after the attention of layer l. */
+  void* const* attention_events;
+  int32_t launches;                /* out: kernels this call has launched */
+  /* Packed form (packed_rows > 0, rel_* form only, seq_len a multiple of 32): between the attention kernels the layers
+   * run on the valid positions, packed in groups of 32 rows.  outs[n_layers-1] receives the unpacked result; positions
+   * no group covers are left as they are there.  No other entry of outs may be given. */
+  int32_t packed_rows;             /* T, a multiple of 32 */
+  const int32_t* pack_rows;        /* device [T]: row of [batch*seq_len] each packed row holds */
+  const int32_t* row_groups;       /* device [T/32]: first of them per group */
+  const int32_t* row_base;         /* device [batch]: first packed row of a sequence */
+  const int32_t* row_count;        /* device [batch]: packed rows of a sequence */
+  void* qkv[3];                    /* [batch, heads, seq_len, head_dim] each, finite contents, kept from call to call */
+} DflEncoderParams;
+DFL_API size_t dfl_encoder_workspace_bytes(const DflEncoderParams* p);
+DFL_API int dfl_encoder_fwd(DflEncoderParams* p, void* stream);
+
 #ifdef __cplusplus
 }
 #endif
