@@ -53,6 +53,9 @@ EXPORTED_SYMBOLS = (
     "dfl_expand_rel_tables",
     "dfl_attention_rel_supported",
     "dfl_attention_rel_fwd",
+    "dfl_qkv_proj_planes",
+    "dfl_split_planes",
+    "dfl_f32_planes_supported",
     "dfl_encoder_workspace_bytes",
     "dfl_encoder_fwd",
 )
@@ -150,7 +153,8 @@ class DflEncoderParams(Structure):
         ("conv_taps", c_int32), ("conv_activation", c_int32), ("conv_norm_eps", c_float),
         ("n_layers", c_int32), ("batch", c_int32), ("seq_len", c_int32), ("hidden", c_int32), ("heads", c_int32),
         ("head_dim", c_int32), ("ffn", c_int32), ("n_active", c_int32), ("mask_elem_size", c_int32), ("dtype", c_int32),
-        ("scale", c_float), ("attention_events", POINTER(c_void_p)), ("launches", c_int32), ("packed_rows", c_int32),
+        ("scale", c_float), ("attention_events", POINTER(c_void_p)), ("launches", c_int32), ("attention_only", c_int32),
+        ("packed_rows", c_int32),
         ("pack_rows", c_void_p), ("row_groups", c_void_p), ("row_base", c_void_p), ("row_count", c_void_p),
         ("qkv", c_void_p * 3),
     ]
@@ -219,6 +223,12 @@ def load_library() -> ctypes.CDLL:
     lib.dfl_attention_rel_supported.argtypes = [POINTER(DflAttnRelParams)]
     lib.dfl_attention_rel_fwd.restype = c_int
     lib.dfl_attention_rel_fwd.argtypes = [POINTER(DflAttnRelParams), c_void_p]
+    lib.dfl_qkv_proj_planes.restype = c_int
+    lib.dfl_qkv_proj_planes.argtypes = [POINTER(DflLinearParams), c_void_p]
+    lib.dfl_f32_planes_supported.restype = c_int
+    lib.dfl_f32_planes_supported.argtypes = [c_int, c_int]
+    lib.dfl_split_planes.restype = c_int
+    lib.dfl_split_planes.argtypes = [c_void_p, c_void_p, ctypes.c_int64, c_void_p]
     lib.dfl_encoder_workspace_bytes.restype = ctypes.c_size_t
     lib.dfl_encoder_workspace_bytes.argtypes = [POINTER(DflEncoderParams)]
     lib.dfl_encoder_fwd.restype = c_int
@@ -726,6 +736,42 @@ def attention_rel_fwd(q: torch.Tensor, k: torch.Tensor, v: torch.Tensor, rel_key
     p.mask_elem_size, p.scale, p.dtype, p.algo = mask.element_size(), scale, dtype_code(q.dtype), ALGO_AUTO
     with _on_device(q.device):
         _check(lib.dfl_attention_rel_fwd(ctypes.byref(p), _stream(q.device)), "dfl_attention_rel_fwd")
+    return out
+
+
+def f32_planes_supported(head_dim: int, seq_len: int) -> bool:
+    """Whether the FP32 form of ``encoder_fwd`` covers these sizes."""
+
+    return bool(load_library().dfl_f32_planes_supported(head_dim, seq_len))
+
+
+def split_planes(x: torch.Tensor) -> torch.Tensor:
+    """FP32 ``x`` as bf16 planes ``[3, *x.shape]`` whose sum is ``x`` exactly (prepare-time)."""
+
+    lib = load_library()
+    _require_cuda_contiguous("x", x)
+    if x.dtype != torch.float32:
+        raise TypeError("split_planes takes FP32")
+    planes = torch.empty(3, *x.shape, dtype=torch.bfloat16, device=x.device)
+    with _on_device(x.device):
+        _check(lib.dfl_split_planes(x.data_ptr(), planes.data_ptr(), x.numel(), _stream(x.device)), "dfl_split_planes")
+    return planes
+
+
+def linear_heads_planes(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, *, heads: int, head_dim: int,
+                        status: torch.Tensor | None = None) -> torch.Tensor:
+    """FP32 ``x[M,K] @ weight[heads*head_dim,K]^T + bias`` as ``[heads, M, head_dim]`` over bf16 planes (prepare-time)."""
+
+    lib = load_library()
+    x_planes, w_planes = split_planes(x.contiguous()), split_planes(weight.contiguous())
+    out = torch.empty(heads, x.shape[0], head_dim, dtype=torch.float32, device=x.device)
+    p = DflLinearParams()
+    p.x, p.w, p.bias = x_planes.data_ptr(), w_planes.data_ptr(), _ptr(bias)
+    p.out[0] = out.data_ptr()
+    p.M, p.K, p.n_out, p.heads, p.head_dim, p.rows_per_seq = x.shape[0], x.shape[1], 1, heads, head_dim, x.shape[0]
+    p.dtype, p.algo, p.status = DFL_F32, ALGO_AUTO, _ptr(status)
+    with _on_device(x.device):
+        _check(lib.dfl_qkv_proj_planes(ctypes.byref(p), _stream(x.device)), "dfl_qkv_proj_planes")
     return out
 
 

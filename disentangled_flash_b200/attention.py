@@ -24,6 +24,7 @@ There is no PyTorch, Triton or CPU implementation behind them.
 
 from __future__ import annotations
 
+import ctypes
 import math
 from typing import Any, NamedTuple, Optional
 
@@ -35,6 +36,14 @@ from .config import normalise_pos_att_type
 from .position import SharedPositionPlanCache, canonical_device
 
 SUPPORTED_HEAD_DIMS = (32, 64, 128)
+
+
+def f32_on_tensor_cores(hidden: int) -> bool:
+    """Whether an FP32 layer of this width runs over bf16 planes on the tensor cores.  Below 256 columns an inner product
+    has fewer than four 64-deep k-blocks: the tensor-core GEMM is all set-up and drain there, and the CUDA-core kernels
+    (one pass of 16-deep steps) take as long without the planes."""
+
+    return hidden >= 256 and hidden % 8 == 0
 
 
 class B200PreparedPositionPlan(NamedTuple):
@@ -53,6 +62,9 @@ class B200PreparedPositionPlan(NamedTuple):
     # single-launch attention kernel covers the configuration (else None)
     rel_key: torch.Tensor | None = None
     rel_query: torch.Tensor | None = None
+    # FP32: the pruned tables as bf16 planes [3, H, A, d] for the tensor-core score GEMMs
+    pos_key_planes: torch.Tensor | None = None
+    pos_query_planes: torch.Tensor | None = None
 
 
 # --------------------------------------------------------------------------
@@ -129,6 +141,54 @@ def _require_2d_padding_mask(attention_mask: torch.Tensor, batch_size: int, sequ
     return attention_mask.contiguous()
 
 
+class _LayerCall:
+    """The QKV projection and the attention of one layer and length as one native call (``dfl_encoder_fwd`` with
+    ``attention_only``): less host time per call, and in FP32 the tensor-core GEMMs over bf16 planes."""
+
+    def __init__(self, module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> None:
+        self.plan, self.qkv_weight = plan, module._cached_qkv_weight
+        weight = module._cached_qkv_weight
+        self.layers = (_cabi.DflEncoderLayer * 1)()
+        fill_attention_fields(self.layers[0], module, plan)
+        p = self.params = _cabi.DflEncoderParams()
+        p.layers, p.n_layers, p.attention_only = self.layers, 1, 1
+        p.seq_len, p.hidden, p.heads = plan.sequence_length, weight.shape[1], module.num_attention_heads
+        p.head_dim, p.dtype, p.scale = module.attention_head_size, _cabi.dtype_code(weight.dtype), module._score_scale()
+        p.lut, p.n_active = plan.delta_to_local.data_ptr(), plan.active_slots.numel()
+        self.width = module.all_head_size
+
+    @staticmethod
+    def covers(module: "DisentangledFlashAttention", length: int) -> bool:
+        if module._algo != _cabi.ALGO_AUTO or module._cached_qkv_weight.shape[1] % 8:
+            return False
+        f32 = module._cached_qkv_weight.dtype == torch.float32
+        return not f32 or (module._cached_qkv_planes is not None and _cabi.f32_planes_supported(module.attention_head_size, length))
+
+    def __call__(self, hidden_states: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None) -> torch.Tensor:
+        p = _cabi.DflEncoderParams()
+        ctypes.pointer(p)[0] = self.params   # a copy: several threads may run one module
+        out = torch.empty(*hidden_states.shape[:2], self.width, dtype=hidden_states.dtype, device=hidden_states.device)
+        p.x, p.mask, p.mask_elem_size, p.batch = hidden_states.data_ptr(), mask.data_ptr(), mask.element_size(), hidden_states.shape[0]
+        p.outs = (ctypes.c_void_p * 1)(out.data_ptr())
+        p.status = None if status is None else status.data_ptr()
+        _cabi.encoder_fwd(p, hidden_states.device)
+        return out
+
+
+def fill_attention_fields(entry: "_cabi.DflEncoderLayer", module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> None:
+    """The QKV and position-table entries of one layer of ``dfl_encoder_fwd``."""
+
+    f32 = module._cached_qkv_weight.dtype == torch.float32
+    tensors = {
+        "qkv_w": module._cached_qkv_planes if f32 else module._cached_qkv_weight, "qkv_b": module._cached_qkv_bias,
+        "rel_key": plan.rel_key if module.has_c2p else None, "rel_query": plan.rel_query if module.has_p2c else None,
+        "pos_key": (plan.pos_key_planes if f32 else plan.pos_key) if module.has_c2p else None,
+        "pos_query": (plan.pos_query_planes if f32 else plan.pos_query) if module.has_p2c else None,
+    }
+    for field, tensor in tensors.items():
+        setattr(entry, field, None if tensor is None else tensor.data_ptr())
+
+
 def _invalidate_attention_cache_after_load(module: nn.Module, _incompatible_keys: Any) -> None:
     module.clear_inference_cache()
 
@@ -136,10 +196,11 @@ def _invalidate_attention_cache_after_load(module: nn.Module, _incompatible_keys
 class DisentangledFlashAttention(nn.Module):
     """Forward-only CUDA DeBERTa-v2/v3 self-attention for head dims 32, 64 and 128.
 
-    FP16/BF16 run on the tcgen05 tensor-core kernels.  FP32 always runs the
-    IEEE-fp32 CUDA-core kernels: ``fp32_precision="strict"`` is what they
-    implement, and ``"fast"`` (TF32 in the reference) is accepted and served by
-    the same, more accurate, kernels.
+    FP16/BF16 run on the tcgen05 tensor-core kernels.  FP32 runs at fp32
+    accuracy whatever ``fp32_precision`` says (``"fast"``, TF32 in the
+    reference, is served by the same kernels): on the tensor cores over exact
+    bf16 planes for layers of at least 256 columns (``f32_on_tensor_cores``), on
+    the IEEE-fp32 CUDA-core kernels otherwise.
     """
 
     def __init__(self, config: Any, *, position_plan_cache: SharedPositionPlanCache | None = None,
@@ -185,10 +246,12 @@ class DisentangledFlashAttention(nn.Module):
         self.register_buffer("_cached_pos_query", None, persistent=False)
         self.register_buffer("_cached_qkv_weight", None, persistent=False)
         self.register_buffer("_cached_qkv_bias", None, persistent=False)
+        self.register_buffer("_cached_qkv_planes", None, persistent=False)   # FP32: the weight as bf16 planes
         # device int32 that the kernels of this layer write if one of their bounded waits expires; an encoder
         # shares one word between its layers (set_status_word) and reads it in check_device_status()
         self.register_buffer("_status_word", None, persistent=False)
         self._position_projection_cache: dict[tuple[int, str], B200PreparedPositionPlan] = {}
+        self._layer_calls: dict[int, _LayerCall] = {}   # per sequence length
         self._algo = _cabi.ALGO_AUTO
         self.register_load_state_dict_post_hook(_invalidate_attention_cache_after_load)
 
@@ -201,6 +264,11 @@ class DisentangledFlashAttention(nn.Module):
     def has_p2c(self) -> bool:
         return self.relative_attention and "p2c" in self.pos_att_type
 
+    def _score_scale(self) -> float:
+        # Hugging Face counts the configured position terms in the scale even
+        # when relative attention is switched off (_reference.py:277-286).
+        return 1.0 / self._scale(1 + int("c2p" in self.pos_att_type) + int("p2c" in self.pos_att_type))
+
     def _scale(self, scale_factor: int) -> float:
         return math.sqrt(self.attention_head_size * scale_factor)
 
@@ -208,6 +276,7 @@ class DisentangledFlashAttention(nn.Module):
     def set_position_plan_cache(self, cache: SharedPositionPlanCache) -> "DisentangledFlashAttention":
         self.position_plan_cache = cache
         self._position_projection_cache.clear()
+        self._layer_calls.clear()
         return self
 
     def set_status_word(self, status: torch.Tensor | None) -> "DisentangledFlashAttention":
@@ -232,8 +301,10 @@ class DisentangledFlashAttention(nn.Module):
         self._cached_pos_query = None
         self._cached_qkv_weight = None
         self._cached_qkv_bias = None
+        self._cached_qkv_planes = None
         if hasattr(self, "_position_projection_cache"):
             self._position_projection_cache.clear()
+            self._layer_calls.clear()
 
     def train(self, mode: bool = True) -> "DisentangledFlashAttention":
         if mode:
@@ -263,10 +334,15 @@ class DisentangledFlashAttention(nn.Module):
         self._cached_qkv_bias = (
             torch.cat(biases, dim=0).contiguous() if all(b is not None for b in biases) else None
         )
+        if self._cached_qkv_weight.dtype == torch.float32 and f32_on_tensor_cores(self._cached_qkv_weight.shape[1]):
+            self._cached_qkv_planes = _cabi.split_planes(self._cached_qkv_weight)
 
     def _project_relative(self, relative: torch.Tensor, projection: nn.Linear) -> torch.Tensor:
         """``[2*span, hid] -> [H, 2*span, d]`` through ``dfl_qkv_proj`` with ``n_out=1``."""
 
+        if relative.dtype == torch.float32 and self._algo == _cabi.ALGO_AUTO and f32_on_tensor_cores(relative.shape[1]):
+            return _cabi.linear_heads_planes(relative, projection.weight, projection.bias, heads=self.num_attention_heads,
+                                             head_dim=self.attention_head_size, status=self._status_word)
         (projected,) = _cabi.linear_heads(
             relative, projection.weight.contiguous(), projection.bias, n_out=1, heads=self.num_attention_heads,
             head_dim=self.attention_head_size, rows_per_seq=relative.shape[0], algo=self._algo,
@@ -342,6 +418,7 @@ class DisentangledFlashAttention(nn.Module):
                 rel_key = _cabi.expand_rel_tables(pos_key, indices.delta_to_local, sequence_length)
             if pos_query is not None:
                 rel_query = _cabi.expand_rel_tables(pos_query, indices.delta_to_local, sequence_length)
+        f32 = dtype == torch.float32 and self._cached_qkv_planes is not None
         plan = B200PreparedPositionPlan(
             sequence_length=sequence_length,
             active_slots=indices.active_slots,
@@ -350,6 +427,8 @@ class DisentangledFlashAttention(nn.Module):
             pos_query=pos_query,
             rel_key=rel_key,
             rel_query=rel_query,
+            pos_key_planes=_cabi.split_planes(pos_key) if f32 and pos_key is not None else None,
+            pos_query_planes=_cabi.split_planes(pos_query) if f32 and pos_query is not None else None,
         )
         self._position_projection_cache[key] = plan
         return plan
@@ -398,9 +477,12 @@ class DisentangledFlashAttention(nn.Module):
         if self.has_p2c and plan.pos_query is None:
             raise ValueError("prepared plan has no position-to-content queries")
 
-        # Hugging Face counts the configured position terms in the scale even
-        # when relative attention is switched off (_reference.py:277-286).
-        scale_factor = 1 + int("c2p" in self.pos_att_type) + int("p2c" in self.pos_att_type)
+        if not torch.compiler.is_compiling():
+            call = self._layer_calls.get(sequence_length)
+            if call is None or call.plan is not plan or call.qkv_weight is not self._cached_qkv_weight:
+                call = self._layer_calls[sequence_length] = _LayerCall(self, plan) if _LayerCall.covers(self, sequence_length) else None
+            if call is not None and self._algo == _cabi.ALGO_AUTO:
+                return call(hidden_states.contiguous(), base_mask, self._status_word), None
         uses_lut = self.has_c2p or self.has_p2c
         output = (_attention_forward_op if torch.compiler.is_compiling() else _attention_forward)(
             hidden_states.contiguous(),
@@ -414,7 +496,7 @@ class DisentangledFlashAttention(nn.Module):
             plan.rel_query if self.has_p2c else None,
             self.num_attention_heads,
             self.attention_head_size,
-            1.0 / self._scale(scale_factor),
+            self._score_scale(),
             self._algo,
             self._status_word,
         )
@@ -446,14 +528,13 @@ class DisentangledFlashAttention(nn.Module):
         if rel_key is None and rel_query is None:
             raise NotImplementedError("packed rows need the single-launch attention path (expanded position tables)")
         base_mask = _require_2d_padding_mask(attention_mask, batch_size, sequence_length)
-        scale_factor = 1 + int("c2p" in self.pos_att_type) + int("p2c" in self.pos_att_type)
         row_groups, buffers = packed_input if packed_input is not None else (None, None)
         query, key, value = _cabi.linear_heads(
             hidden_states.contiguous(), self._cached_qkv_weight, self._cached_qkv_bias, n_out=3,
             heads=self.num_attention_heads, head_dim=self.attention_head_size, rows_per_seq=sequence_length,
             algo=self._algo, status=self._status_word, row_groups=row_groups, outs=buffers)
         return _cabi.attention_rel_fwd(query, key, value, rel_key, rel_query, base_mask,
-                                       1.0 / self._scale(scale_factor), status=self._status_word,
+                                       self._score_scale(), status=self._status_word,
                                        packed_rows=packed_rows)
 
     def forward(self, hidden_states: torch.Tensor, attention_mask: torch.Tensor, output_attentions: bool = False,

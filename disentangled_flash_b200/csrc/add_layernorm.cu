@@ -13,7 +13,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
-#include "dfl_common.cuh"
+#include "f32_planes.cuh"
 
 namespace dfl {
 namespace {
@@ -114,7 +114,7 @@ __global__ void __launch_bounds__(kWarpsPerBlock * 32)
 add_layernorm_kernel(const uint4* x, const uint4* residual, const uint4* __restrict__ gamma,
                      const uint4* __restrict__ beta, uint4* out, long long rows, int hidden, float eps,
                      const void* __restrict__ row_mask, int mask_elem, uint4* out2,
-                     const int32_t* __restrict__ out2_rows, const RowSource src) {
+                     const int32_t* __restrict__ out2_rows, const RowSource src, uint2* planes) {
   constexpr int E = Vec16<T>::kElems;
   const int lane = threadIdx.x & 31;
   const int vecs_per_row = hidden / E;
@@ -199,6 +199,14 @@ add_layernorm_kernel(const uint4* x, const uint4* residual, const uint4* __restr
         const uint4 packed = pack<T>(y);
         orow[c] = packed;
         if (orow2) orow2[c] = packed;
+        if constexpr (sizeof(T) == 4) {
+          if (planes) {   // the result once more as bf16 planes [3][rows][hidden], what the FP32 GEMM after this reads
+            uint2 w[kPlanes];
+            split3x4(y, w);
+#pragma unroll
+            for (int q = 0; q < kPlanes; ++q) planes[(q * rows + row) * vecs_per_row + c] = w[q];
+          }
+        }
       }
     }
   }
@@ -207,25 +215,25 @@ add_layernorm_kernel(const uint4* x, const uint4* residual, const uint4* __restr
 template <typename T, int VEC>
 void launch_one(const void* x, const void* residual, const void* gamma, const void* beta, void* out, long long rows,
                 int hidden, float eps, const void* row_mask, int mask_elem, void* out2, const int32_t* out2_rows,
-                const RowSource& src, int sm_count, cudaStream_t stream) {
+                const RowSource& src, void* planes, int sm_count, cudaStream_t stream) {
   const long long wanted = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
   const long long cap = (long long)sm_count * 8;   // 8 CTAs of 8 warps per SM: one wave, grid-stride beyond it
   const int blocks = (int)(wanted < cap ? wanted : cap);
   launch_after_predecessor(add_layernorm_kernel<T, VEC>, dim3(blocks), dim3(kWarpsPerBlock * 32), 0, stream,
                            (const uint4*)x, (const uint4*)residual, (const uint4*)gamma, (const uint4*)beta, (uint4*)out,
-                           rows, hidden, eps, row_mask, mask_elem, (uint4*)out2, out2_rows, src);
+                           rows, hidden, eps, row_mask, mask_elem, (uint4*)out2, out2_rows, src, (uint2*)planes);
 }
 
 template <typename T>
 int launch_typed(const void* x, const void* residual, const void* gamma, const void* beta, void* out, long long rows,
                  int hidden, float eps, const void* row_mask, int mask_elem, void* out2, const int32_t* out2_rows,
-                 const RowSource& src, int sm_count, cudaStream_t stream) {
+                 const RowSource& src, void* planes, int sm_count, cudaStream_t stream) {
   constexpr int E = Vec16<T>::kElems;
   const int vec = (hidden / E + 31) / 32;
 #define DFL_LN_CASE(V)                                                                              \
   if (vec <= V) {                                                                                   \
     launch_one<T, V>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows,   \
-                     src, sm_count, stream);                                                                   \
+                     src, planes, sm_count, stream);                                                           \
     return check_launch("add_layernorm_kernel");                                                    \
   }
   DFL_LN_CASE(1) DFL_LN_CASE(2) DFL_LN_CASE(3) DFL_LN_CASE(4) DFL_LN_CASE(6) DFL_LN_CASE(8) DFL_LN_CASE(12)
@@ -272,24 +280,24 @@ int add_layernorm_max_hidden(size_t elem_size) { return 16 * 32 * (int)(16 / ele
 namespace {
 int launch_rows(const void* x, const void* residual, const void* gamma, const void* beta, void* out, long long rows,
                 int hidden, float eps, int dtype, const void* row_mask, int mask_elem, void* out2,
-                const int32_t* out2_rows, const RowSource& src, cudaStream_t stream) {
+                const int32_t* out2_rows, const RowSource& src, void* planes, cudaStream_t stream) {
   static KernelDeviceConfig config;   // only the SM count of the current device is needed (no shared memory)
   int sm_count = 0;
   if (int rc = configure_kernel(config, add_layernorm_kernel<float, 1>, 0, &sm_count, "add_layernorm_kernel")) return rc;
   switch (dtype) {
-    case DFL_F16: return launch_typed<__half>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, sm_count, stream);
-    case DFL_BF16: return launch_typed<__nv_bfloat16>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, sm_count, stream);
-    default: return launch_typed<float>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, sm_count, stream);
+    case DFL_F16: return launch_typed<__half>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, planes, sm_count, stream);
+    case DFL_BF16: return launch_typed<__nv_bfloat16>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, planes, sm_count, stream);
+    default: return launch_typed<float>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, planes, sm_count, stream);
   }
 }
 }  // namespace
 
 int launch_add_layernorm(const void* x, const void* residual, const void* gamma, const void* beta, void* out,
                          long long rows, int hidden, float eps, int dtype, const void* row_mask, int mask_elem,
-                         void* out2, const int32_t* out2_rows, cudaStream_t stream) {
+                         void* out2, const int32_t* out2_rows, void* planes, cudaStream_t stream) {
   const RowSource plain{nullptr, nullptr, 4, 0, 0, nullptr};
   return launch_rows(x, residual, gamma, beta, out, rows, hidden, eps, dtype, row_mask, mask_elem, out2, out2_rows, plain,
-                     stream);
+                     planes, stream);
 }
 
 // Embedding front-end: out[r] = LayerNorm(table[ids[r]] (+ pos_table[pos_ids[r]])), masked rows zero.
@@ -299,7 +307,7 @@ int launch_embed_layernorm(const void* ids, const void* table, long long vocab, 
                            const void* row_mask, int mask_elem, int* status, cudaStream_t stream) {
   const RowSource src{ids, pos_table ? pos_ids : nullptr, idx_elem, vocab, positions, status};
   return launch_rows(table, pos_table, gamma, beta, out, rows, hidden, eps, dtype, row_mask, mask_elem, nullptr, nullptr,
-                     src, stream);
+                     src, nullptr, stream);
 }
 
 }  // namespace dfl

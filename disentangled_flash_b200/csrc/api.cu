@@ -83,7 +83,8 @@ int dfl_gather_slots(const void* src, const int64_t* active_dev, void* dst, int 
                              (cudaStream_t)stream);
 }
 
-int dfl_qkv_proj(const DflLinearParams* p, void* stream) {
+namespace {
+int head_projection(const DflLinearParams* p, bool planes, void* stream) {
   if (!p) return fail(DFL_ERR_BAD_ARG, "null params");
   if (!valid_dtype(p->dtype)) return fail(DFL_ERR_BAD_ARG, "unknown dtype %d", p->dtype);
   if (p->n_out < 1 || p->n_out > 3) return fail(DFL_ERR_BAD_ARG, "n_out must be 1..3");
@@ -115,8 +116,17 @@ int dfl_qkv_proj(const DflLinearParams* p, void* stream) {
   g.dtype = p->dtype;
   g.status = p->status;
   g.row_groups = p->row_groups; g.out_seqs = p->out_seqs;
+  if (planes) return launch_gemm_f32_planes(g, (cudaStream_t)stream);
   if (use_tensor_cores(p->dtype, p->algo)) return launch_gemm_tc(g, (cudaStream_t)stream);
   return launch_gemm_simt(g, (cudaStream_t)stream);
+}
+}  // namespace
+
+int dfl_qkv_proj(const DflLinearParams* p, void* stream) { return head_projection(p, false, stream); }
+
+int dfl_qkv_proj_planes(const DflLinearParams* p, void* stream) {
+  if (p && (p->dtype != DFL_F32 || p->row_groups)) return fail(DFL_ERR_UNSUPPORTED, "planes are an F32 form without row_groups");
+  return head_projection(p, true, stream);
 }
 
 int dfl_pos_scores(const DflPosScoreParams* p, void* stream) {
@@ -247,6 +257,16 @@ int dfl_conv1d(const DflConv1dParams* p, void* stream) {
   return launch_gemm_tc(g, (cudaStream_t)stream);
 }
 
+int dfl_f32_planes_supported(int head_dim, int seq_len) { return attention_f32_planes_supported(head_dim, seq_len) ? 1 : 0; }
+
+int dfl_split_planes(const void* x, void* planes, int64_t n, void* stream) {
+  if (n < 0 || n % 4) return fail(DFL_ERR_BAD_ARG, "a multiple of 4 elements");
+  if (n == 0) return DFL_OK;
+  if (!x || !planes) return fail(DFL_ERR_BAD_ARG, "null pointer");
+  if (!aligned16(x) || !aligned16(planes)) return fail(DFL_ERR_ALIGNMENT, "pointers must be 16-byte aligned");
+  return launch_split_planes(x, planes, n, (cudaStream_t)stream);
+}
+
 int dfl_copy_rows(const void* src, void* dst, const int32_t* rows_dev, int64_t n_rows, int32_t row_bytes, void* stream) {
   if (n_rows < 0 || row_bytes < 16 || (row_bytes % 16)) return fail(DFL_ERR_BAD_ARG, "rows of a positive multiple of 16 bytes");
   if (n_rows == 0) return DFL_OK;
@@ -278,7 +298,7 @@ int dfl_add_layernorm(const DflAddLayerNormParams* p, void* stream) {
   if ((p->out2 != nullptr) != (p->out2_rows != nullptr)) return fail(DFL_ERR_BAD_ARG, "out2 and out2_rows go together");
   if (!aligned16(p->out2)) return fail(DFL_ERR_ALIGNMENT, "out2 must be 16-byte aligned");
   return launch_add_layernorm(p->x, p->residual, p->gamma, p->beta, p->out, p->rows, p->hidden, p->eps, p->dtype,
-                              p->row_mask, p->mask_elem_size, p->out2, p->out2_rows, (cudaStream_t)stream);
+                              p->row_mask, p->mask_elem_size, p->out2, p->out2_rows, nullptr, (cudaStream_t)stream);
 }
 
 int dfl_embed_layernorm(const DflEmbedLayerNormParams* p, void* stream) {

@@ -176,6 +176,7 @@ struct GemmDesc {
   // 1: the kernel before this one in the stream is one of this library's that waited for its own predecessor and
   // does not write W or the bias, so that W may be read before that kernel has finished (see release_successor())
   int weights_early;
+  int out_planes;       // linear_f32.cu: write the result (batch 1) as bf16 planes [3][...] instead of fp32
 };
 
 // tanh for the GEMM epilogues of 16-bit outputs: 1 - 2 / (1 + e^(2x)) with approximate exp2 and reciprocal
@@ -210,15 +211,21 @@ __device__ __forceinline__ float gelu_erf_fast(float x) {
 }
 int launch_gemm_simt(const GemmDesc& g, cudaStream_t stream);
 int launch_gemm_tc(const GemmDesc& g, cudaStream_t stream);
+// FP32 on the tensor cores: g.x is [3][batch][M][K] and g.w [3][w_mod][N][K] bf16 planes (launch_split_planes).
+int launch_gemm_f32_planes(const GemmDesc& g, cudaStream_t stream);
+int launch_split_planes(const void* x, void* planes, long long n, cudaStream_t stream);   // n a multiple of 4
 
 int launch_attention_simt(const DflAttnParams& p, cudaStream_t stream);
+// FP32 over bf16 planes: p.q, p.k, p.v are [3][B,H,L,d], the scores fp32, the output fp32 or planes [3][B,L,H*d].
+bool attention_f32_planes_supported(int head_dim, int seq_len);
+int launch_attention_f32_planes(const DflAttnParams& p, int out_planes, cudaStream_t stream);
 int launch_attention_tc(const DflAttnParams& p, cudaStream_t stream);
 bool attention_rel_supported(const DflAttnRelParams& p);
 int launch_attention_rel(const DflAttnRelParams& p, cudaStream_t stream);
 int add_layernorm_max_hidden(size_t elem_size);
 int launch_add_layernorm(const void* x, const void* residual, const void* gamma, const void* beta, void* out,
                          long long rows, int hidden, float eps, int dtype, const void* row_mask, int mask_elem,
-                         void* out2, const int32_t* out2_rows, cudaStream_t stream);
+                         void* out2, const int32_t* out2_rows, void* planes, cudaStream_t stream);
 int launch_embed_layernorm(const void* ids, const void* table, long long vocab, const void* pos_ids,
                            const void* pos_table, long long positions, int idx_elem, const void* gamma,
                            const void* beta, void* out, long long rows, int hidden, float eps, int dtype,

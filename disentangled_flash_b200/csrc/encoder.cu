@@ -14,7 +14,12 @@ size_t padded(size_t bytes) { return (bytes + kAlign - 1) / kAlign * kAlign; }
 // Offsets of the activations inside the workspace.
 struct Workspace {
   size_t qkv, context, dense, mixed, inner, state[2], scores[2], total;
+  // F32: bf16 planes of the layer's input, of its first output block, and of the FFN's inside (Q, K, V and the context
+  // are planes there too)
+  size_t state_planes, mixed_planes, inner_planes;
 };
+
+constexpr size_t kPlaneBytes = 6;   // three bf16 planes per element
 
 bool two_call(const DflEncoderParams& p) { return !p.layers[0].rel_key && !p.layers[0].rel_query; }
 
@@ -29,13 +34,23 @@ Workspace plan_workspace(const DflEncoderParams& p) {
     at += padded(bytes);
     return here;
   };
-  w.qkv = take(p.packed_rows > 0 ? 0 : 3 * padded(positions * width * es));
-  w.context = take(rows * width * es);
-  w.dense = take(rows * p.hidden * es);
-  w.mixed = take(rows * p.hidden * es);
-  const size_t inner = rows * (size_t)p.ffn, conv = p.conv_w ? positions * (size_t)p.hidden : 0;
-  w.inner = take((inner > conv ? inner : conv) * es);   // also the convolution's output
-  for (int i = 0; i < 2; ++i) w.state[i] = take(rows * p.hidden * es);
+  const bool f32 = p.dtype == DFL_F32, layers = !p.attention_only;
+  w.qkv = take(p.packed_rows > 0 ? 0 : 3 * padded(positions * width * (f32 ? kPlaneBytes : es)));
+  if (layers) {
+    w.context = take(rows * width * (f32 ? kPlaneBytes : es));
+    w.dense = take(rows * p.hidden * es);
+    w.mixed = take(rows * p.hidden * es);
+    const size_t inner = f32 ? 0 : rows * (size_t)p.ffn, conv = p.conv_w ? positions * (size_t)p.hidden : 0;
+    w.inner = take((inner > conv ? inner : conv) * es);   // also the convolution's output
+    for (int i = 0; i < 2; ++i) w.state[i] = take(rows * p.hidden * es);
+  }
+  if (f32) {
+    w.state_planes = take(rows * p.hidden * kPlaneBytes);
+    if (layers) {
+      w.mixed_planes = take(rows * p.hidden * kPlaneBytes);
+      w.inner_planes = take(rows * (size_t)p.ffn * kPlaneBytes);
+    }
+  }
   if (two_call(p)) {
     const size_t ld = ((size_t)p.n_active + 7) / 8 * 8;
     for (int i = 0; i < 2; ++i) w.scores[i] = take(positions * p.heads * ld * es);
@@ -45,12 +60,12 @@ Workspace plan_workspace(const DflEncoderParams& p) {
 }
 
 int validate(const DflEncoderParams& p) {
-  if (p.dtype != DFL_F16 && p.dtype != DFL_BF16) return fail(DFL_ERR_UNSUPPORTED, "dfl_encoder_fwd takes F16 or BF16");
-  if (p.n_layers < 1 || p.batch < 1 || p.seq_len < 1 || p.hidden < 1 || p.heads < 1 || p.ffn < 1)
+  if (p.dtype != DFL_F16 && p.dtype != DFL_BF16 && p.dtype != DFL_F32) return fail(DFL_ERR_BAD_ARG, "unknown dtype %d", p.dtype);
+  if (p.n_layers < 1 || p.batch < 1 || p.seq_len < 1 || p.hidden < 1 || p.heads < 1 || (p.ffn < 1 && !p.attention_only))
     return fail(DFL_ERR_BAD_ARG, "non-positive size");
   if (p.head_dim != 32 && p.head_dim != 64 && p.head_dim != 128)
     return fail(DFL_ERR_UNSUPPORTED, "head_dim %d not in {32,64,128}", p.head_dim);
-  if (p.hidden % 8 || p.ffn % 8 || !dfl_add_layernorm_supported(p.dtype, p.hidden))
+  if (p.hidden % 8 || (!p.attention_only && (p.ffn % 8 || !dfl_add_layernorm_supported(p.dtype, p.hidden))))
     return fail(DFL_ERR_UNSUPPORTED, "hidden %d / ffn %d not covered", p.hidden, p.ffn);
   if (!p.layers || !p.outs || !p.outs[p.n_layers - 1] || !p.x || !p.mask || !p.workspace)
     return fail(DFL_ERR_BAD_ARG, "null pointer");
@@ -60,7 +75,7 @@ int validate(const DflEncoderParams& p) {
   if (!aligned16(p.x) || !aligned16(p.workspace)) return fail(DFL_ERR_ALIGNMENT, "tensors must be 16-byte aligned");
   for (int l = 0; l < p.n_layers; ++l) {
     const DflEncoderLayer& y = p.layers[l];
-    if (!y.qkv_w || !y.attn_out_w || !y.attn_norm_w || !y.ffn_in_w || !y.ffn_out_w || !y.ffn_norm_w)
+    if (!y.qkv_w || (!p.attention_only && (!y.attn_out_w || !y.attn_norm_w || !y.ffn_in_w || !y.ffn_out_w || !y.ffn_norm_w)))
       return fail(DFL_ERR_BAD_ARG, "layer %d: null weight", l);
     const void* all[16] = {y.qkv_w, y.qkv_b, y.attn_out_w, y.attn_out_b, y.attn_norm_w, y.attn_norm_b, y.ffn_in_w, y.ffn_in_b,
                            y.ffn_out_w, y.ffn_out_b, y.ffn_norm_w, y.ffn_norm_b, y.rel_key, y.rel_query, y.pos_key, y.pos_query};
@@ -70,6 +85,13 @@ int validate(const DflEncoderParams& p) {
     if (!(y.attn_norm_eps >= 0.0f) || !(y.ffn_norm_eps >= 0.0f)) return fail(DFL_ERR_BAD_ARG, "eps must be non-negative");
     if ((!y.rel_key && !y.rel_query) != two_call(p)) return fail(DFL_ERR_BAD_ARG, "layers with and without rel tables");
   }
+  if (p.attention_only && (p.n_layers != 1 || p.packed_rows > 0 || p.conv_w))
+    return fail(DFL_ERR_BAD_ARG, "attention_only takes one layer of padded rows");
+  if (p.dtype == DFL_F32 && (p.conv_w || p.packed_rows > 0 || !two_call(p)))
+    return fail(DFL_ERR_UNSUPPORTED, "F32 has no convolution branch, no packed rows and no rel_key / rel_query form");
+  if (p.dtype == DFL_F32 && !attention_f32_planes_supported(p.head_dim, p.seq_len))
+    return fail(DFL_ERR_UNSUPPORTED, "head_dim %d at seq_len %d in F32", p.head_dim, p.seq_len);
+  if ((long long)p.batch * p.heads > 65535) return fail(DFL_ERR_TOO_LARGE, "batch*heads > 65535");
   if (p.packed_rows > 0) {
     if (two_call(p)) return fail(DFL_ERR_UNSUPPORTED, "packed rows need the rel_key / rel_query form");
     if (p.packed_rows % 32 || p.seq_len % 32) return fail(DFL_ERR_BAD_ARG, "packed rows come in groups of 32");
@@ -89,7 +111,7 @@ struct Loop {
 
   // out[rows, n] = act(x[rows, k] w^T + b), or the three head-major tensors of the QKV projection
   int gemm(const void* x, const void* weight, const void* bias, void* out, int rows, int n, int k, int activation,
-           void* const* heads_out = nullptr) {
+           void* const* heads_out = nullptr, bool out_planes = false) {
     GemmDesc g{};
     g.x = x; g.w = weight; g.bias = bias;
     g.M = rows; g.N = n; g.K = k;
@@ -108,14 +130,36 @@ struct Loop {
       g.out[0] = out;
     }
     ++p.launches;
+    if (p.dtype == DFL_F32) {
+      g.out_planes = out_planes ? 1 : 0;
+      return launch_gemm_f32_planes(g, stream);
+    }
     return launch_gemm_tc(g, stream);
   }
 
+  int split(const void* x, void* planes, size_t elements) {
+    ++p.launches;
+    return launch_split_planes(x, planes, (long long)elements, stream);
+  }
+
+  // scores[b, h, row, slot] = head[b, h, row, :] . table[h, slot, :] in F32 over the planes of both
+  int scores_f32(const void* head, const void* table, void* out, int ld) {
+    GemmDesc g{};
+    g.x = head; g.w = table; g.out[0] = out;
+    g.M = p.seq_len; g.N = p.n_active; g.K = p.head_dim;
+    g.batch = p.batch * p.heads; g.w_mod = p.heads;
+    g.stride_c = (long long)p.seq_len * ld; g.ldc = ld;
+    g.heads = p.heads; g.head_dim = p.head_dim; g.rows_per_seq = p.seq_len;
+    g.dtype = p.dtype; g.status = p.status; g.weights_early = 1;
+    ++p.launches;
+    return launch_gemm_f32_planes(g, stream);
+  }
+
   int norm(const void* x, const void* residual, const void* gamma, const void* beta, void* out, int rows, float eps,
-           const void* row_mask = nullptr, void* out2 = nullptr) {
+           const void* row_mask = nullptr, void* out2 = nullptr, void* planes = nullptr) {
     ++p.launches;
     return launch_add_layernorm(x, residual, gamma, beta, out, rows, p.hidden, eps, p.dtype, row_mask, p.mask_elem_size, out2,
-                                out2 ? p.pack_rows : nullptr, stream);
+                                out2 ? p.pack_rows : nullptr, planes, stream);
   }
 
   int attention(const DflEncoderLayer& y, void* const* qkv, void* out, int layer) {
@@ -137,7 +181,17 @@ struct Loop {
     } else {
       DflAttnParams a{};
       const int ld = (p.n_active + 7) / 8 * 8;
-      if (y.pos_key || y.pos_query) {
+      if ((y.pos_key || y.pos_query) && p.dtype == DFL_F32) {
+        if (y.pos_key) {
+          a.c2p = at(w.scores[0]);
+          if (int rc2 = scores_f32(qkv[0], y.pos_key, at(w.scores[0]), ld)) return rc2;
+        }
+        if (y.pos_query) {
+          a.p2c = at(w.scores[1]);
+          if (int rc2 = scores_f32(qkv[1], y.pos_query, at(w.scores[1]), ld)) return rc2;
+        }
+        a.ld_slots = ld;
+      } else if (y.pos_key || y.pos_query) {
         DflPosScoreParams s{};
         s.q = y.pos_key ? qkv[0] : nullptr; s.k = y.pos_query ? qkv[1] : nullptr;
         s.pos_key = y.pos_key; s.pos_query = y.pos_query;
@@ -153,7 +207,7 @@ struct Loop {
       a.batch = p.batch; a.heads = p.heads; a.seq_len = p.seq_len; a.head_dim = p.head_dim;
       a.mask_elem_size = p.mask_elem_size; a.scale = p.scale; a.dtype = p.dtype; a.algo = DFL_ALGO_AUTO;
       ++p.launches;
-      rc = dfl_attention_fwd(&a, stream);
+      rc = p.dtype == DFL_F32 ? launch_attention_f32_planes(a, p.attention_only ? 0 : 1, stream) : dfl_attention_fwd(&a, stream);
     }
     if (rc == DFL_OK && p.attention_events && cudaEventRecord((cudaEvent_t)p.attention_events[2 * layer + 1], stream) != cudaSuccess)
       return fail(DFL_ERR_LAUNCH, "recording a timing event");
@@ -180,27 +234,37 @@ struct Loop {
     const int rows = packed ? p.packed_rows : p.batch * p.seq_len, width = p.heads * p.head_dim;
     void* qkv[3];
     for (int i = 0; i < 3; ++i)
-      qkv[i] = packed ? p.qkv[i] : at(w.qkv + (size_t)i * padded((size_t)rows * width * dtype_size(p.dtype)));
+      qkv[i] = packed ? p.qkv[i] : at(w.qkv + (size_t)i * padded((size_t)rows * width * (p.dtype == DFL_F32 ? kPlaneBytes : dtype_size(p.dtype))));
     const void* state = p.x;
+    const bool f32 = p.dtype == DFL_F32;
     void* unpacked = p.outs[p.n_layers - 1];
     if (packed) {
       ++p.launches;
       if (int rc = launch_copy_rows(p.x, at(w.state[1]), p.pack_rows, rows, p.hidden * (int)dtype_size(p.dtype), stream)) return rc;
       state = at(w.state[1]);
     }
+    if (f32)
+      if (int rc = split(state, at(w.state_planes), (size_t)rows * p.hidden)) return rc;
+    if (p.attention_only) {
+      const DflEncoderLayer& y = p.layers[0];
+      if (int rc = gemm(f32 ? at(w.state_planes) : state, y.qkv_w, y.qkv_b, nullptr, rows, 3 * width, p.hidden, DFL_ACT_NONE, qkv, true)) return rc;
+      return attention(y, qkv, p.outs[0], 0);
+    }
     for (int l = 0; l < p.n_layers; ++l) {
       const DflEncoderLayer& y = p.layers[l];
       const bool last = l == p.n_layers - 1, convolve = l == 0 && p.conv_w;
       void* next = !packed && p.outs[l] ? p.outs[l] : at(w.state[l & 1]);
-      if (int rc = gemm(state, y.qkv_w, y.qkv_b, nullptr, rows, 3 * width, p.hidden, DFL_ACT_NONE, qkv)) return rc;
+      if (int rc = gemm(f32 ? at(w.state_planes) : state, y.qkv_w, y.qkv_b, nullptr, rows, 3 * width, p.hidden, DFL_ACT_NONE, qkv, true)) return rc;
       if (int rc = attention(y, qkv, at(w.context), l)) return rc;
       if (int rc = gemm(at(w.context), y.attn_out_w, y.attn_out_b, at(w.dense), rows, p.hidden, width, DFL_ACT_NONE)) return rc;
-      if (int rc = norm(at(w.dense), state, y.attn_norm_w, y.attn_norm_b, at(w.mixed), rows, y.attn_norm_eps)) return rc;
-      if (int rc = gemm(at(w.mixed), y.ffn_in_w, y.ffn_in_b, at(w.inner), rows, p.ffn, p.hidden, DFL_ACT_GELU)) return rc;
-      if (int rc = gemm(at(w.inner), y.ffn_out_w, y.ffn_out_b, at(w.dense), rows, p.hidden, p.ffn, DFL_ACT_NONE)) return rc;
+      if (int rc = norm(at(w.dense), state, y.attn_norm_w, y.attn_norm_b, at(w.mixed), rows, y.attn_norm_eps, nullptr, nullptr,
+                        f32 ? at(w.mixed_planes) : nullptr)) return rc;
+      void* inner = f32 ? at(w.inner_planes) : at(w.inner);
+      if (int rc = gemm(f32 ? at(w.mixed_planes) : at(w.mixed), y.ffn_in_w, y.ffn_in_b, inner, rows, p.ffn, p.hidden, DFL_ACT_GELU, nullptr, true)) return rc;
+      if (int rc = gemm(inner, y.ffn_out_w, y.ffn_out_b, at(w.dense), rows, p.hidden, p.ffn, DFL_ACT_NONE)) return rc;
       // a packed state is also written out at its unpacked rows where the convolution or the caller reads it
       if (int rc = norm(at(w.dense), at(w.mixed), y.ffn_norm_w, y.ffn_norm_b, next, rows, y.ffn_norm_eps, nullptr,
-                        packed && (last || convolve) ? unpacked : nullptr)) return rc;
+                        packed && (last || convolve) ? unpacked : nullptr, f32 && !last ? at(w.state_planes) : nullptr)) return rc;
       if (convolve) {
         if (int rc = convolution(packed ? unpacked : next, packed ? unpacked : next)) return rc;
         if (packed && !last) {

@@ -64,23 +64,29 @@ int encode_tensor_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uin
   return DFL_OK;
 }
 
-int encode_tensor_map_pieces(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t batch,
-                             uint64_t row_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_rows,
-                             uint32_t box_batch, uint32_t box_pieces) {
+int encode_tensor_map_4d(CUtensorMap* map, const void* base, const uint64_t (&dims)[4], const uint64_t (&strides)[3],
+                         const uint32_t (&box)[4]) {
   EncodeTiledFn encode = resolve_encode_tiled();
   if (!encode) return fail(DFL_ERR_DRIVER, "cuTensorMapEncodeTiled entry point not available");
-  if ((row_stride_bytes & 15) || (batch_stride_bytes & 15))
+  if ((strides[0] & 15) || (strides[1] & 15) || (strides[2] & 15))
     return fail(DFL_ERR_ALIGNMENT, "tensor-map strides must be multiples of 16 bytes");
-  if (box_pieces > 1 && inner % 64) return fail(DFL_ERR_BAD_ARG, "rows of whole 128-byte pieces expected");
-  const cuuint64_t dims[4] = {box_pieces > 1 ? 64 : inner, rows, batch, box_pieces > 1 ? inner / 64 : 1};
-  const cuuint64_t strides[3] = {row_stride_bytes, batch_stride_bytes, box_pieces > 1 ? 128 : row_stride_bytes};
-  const cuuint32_t box[4] = {64, box_rows, box_batch, box_pieces};
-  const cuuint32_t elem_strides[4] = {1, 1, 1, 1};
-  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, const_cast<void*>(base), dims, strides, box, elem_strides,
+  const cuuint64_t d[4] = {dims[0], dims[1], dims[2], dims[3]}, st[3] = {strides[0], strides[1], strides[2]};
+  const cuuint32_t bx[4] = {box[0], box[1], box[2], box[3]}, elem_strides[4] = {1, 1, 1, 1};
+  CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT16, 4, const_cast<void*>(base), d, st, bx, elem_strides,
                       CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                       CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(DFL_ERR_DRIVER, "cuTensorMapEncodeTiled failed with CUresult %d", (int)r);
   return DFL_OK;
+}
+
+int encode_tensor_map_pieces(CUtensorMap* map, const void* base, uint64_t inner, uint64_t rows, uint64_t batch,
+                             uint64_t row_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_rows,
+                             uint32_t box_batch, uint32_t box_pieces) {
+  if (box_pieces > 1 && inner % 64) return fail(DFL_ERR_BAD_ARG, "rows of whole 128-byte pieces expected");
+  const uint64_t dims[4] = {box_pieces > 1 ? 64 : inner, rows, batch, box_pieces > 1 ? inner / 64 : 1};
+  const uint64_t strides[3] = {row_stride_bytes, batch_stride_bytes, box_pieces > 1 ? 128 : row_stride_bytes};
+  const uint32_t box[4] = {64, box_rows, box_batch, box_pieces};
+  return encode_tensor_map_4d(map, base, dims, strides, box);
 }
 
 // Library-owned status word for kernels whose caller passes none.

@@ -472,6 +472,10 @@ int encode_tensor_map_3d(CUtensorMap* map, const void* base, uint64_t inner, uin
                          uint64_t row_stride_bytes, uint64_t batch_stride_bytes, uint32_t box_inner,
                          uint32_t box_rows, int swizzle_bytes);
 
+// 4-D map over 2-byte elements with the 128-byte swizzle; strides in bytes, of dimensions 1..3.
+int encode_tensor_map_4d(CUtensorMap* map, const void* base, const uint64_t (&dims)[4], const uint64_t (&strides)[3],
+                         const uint32_t (&box)[4]);
+
 // 4-D map of K-major operands for k-blocks of 64 elements, 128-byte swizzle.  box_pieces = 1: {inner, rows, batch, 1},
 // a load at x = 64 * k-block brings one block (zeros beyond `inner`).  box_pieces > 1: {64, rows, batch, inner / 64}, a
 // load at piece k-block brings `box_pieces` consecutive blocks, one 128-byte-swizzle tile behind the other; `inner` must

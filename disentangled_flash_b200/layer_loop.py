@@ -1,7 +1,9 @@
 """The prepared layer loop of one bucket as a single native call (``dfl_encoder_fwd``).
 
-Built by ``DebertaV2InferenceEncoder.prepare_for_inference`` for a bucket whose layers all have the Hugging Face shape
-in a 16-bit type; the encoder's Python loop serves everything else.  Holds the pointers of every parameter the loop reads
+Built by ``DebertaV2InferenceEncoder.prepare_for_inference`` for a bucket whose layers all have the Hugging Face shape;
+the encoder's Python loop serves everything else.  In FP32 the weight matrices are held as bf16 planes
+(``dfl_split_planes``) for the tensor-core GEMMs, made once per encoder; a weight modified in place after that sends the
+calls to the Python loop until the next preparation.  A convolution branch stays the caller's module in FP32.  Holds the pointers of every parameter the loop reads
 and compares them with the modules' current ones before each call, so a parameter that was exchanged or moved after the
 preparation is never read at its old place.
 """
@@ -9,23 +11,30 @@ preparation is never read at its old place.
 from __future__ import annotations
 
 import ctypes
-import math
 from typing import Any
 
 import torch
 from torch import nn
 
 from . import _cabi
+from .attention import fill_attention_fields
 
+_ATTENTION_FIELDS = (("qkv_w", "attention.self", "_cached_qkv_weight"), ("qkv_b", "attention.self", "_cached_qkv_bias"))
 _LAYER_FIELDS = (
-    ("qkv_w", "attention.self", "_cached_qkv_weight"), ("qkv_b", "attention.self", "_cached_qkv_bias"),
     ("attn_out_w", "attention.output.dense", "weight"), ("attn_out_b", "attention.output.dense", "bias"),
     ("attn_norm_w", "attention.output.LayerNorm", "weight"), ("attn_norm_b", "attention.output.LayerNorm", "bias"),
     ("ffn_in_w", "intermediate.dense", "weight"), ("ffn_in_b", "intermediate.dense", "bias"),
     ("ffn_out_w", "output.dense", "weight"), ("ffn_out_b", "output.dense", "bias"),
     ("ffn_norm_w", "output.LayerNorm", "weight"), ("ffn_norm_b", "output.LayerNorm", "bias"),
 )
+_PLANE_FIELDS = ("attn_out_w", "ffn_in_w", "ffn_out_w")   # weight matrices given as planes in FP32
 _data_ptr = torch.Tensor.data_ptr
+
+
+def version_of(tensor: torch.Tensor) -> int:
+    """How often ``tensor`` has been modified in place (inference tensors do not count)."""
+
+    return -1 if tensor.is_inference() else tensor._version
 
 
 def _module_at(root: nn.Module, path: str) -> nn.Module:
@@ -46,24 +55,28 @@ class LayerLoop:
         first = encoder.layer[0].attention.self
         weight = first.query_proj.weight
         dtype, device = weight.dtype, weight.device
-        if device.type != "cuda" or dtype not in (torch.float16, torch.bfloat16):
+        f32 = dtype == torch.float32
+        if device.type != "cuda" or dtype not in (torch.float16, torch.bfloat16, torch.float32):
             return None
-        if not (all(a and b for a, b in encoder._fused_output_blocks) and all(encoder._fused_intermediates)):
+        if not (all(a and b for a, b in encoder._fused_output_blocks) and (f32 or all(encoder._fused_intermediates))):
             return None
-        if encoder.conv is not None and not conv_covered:
+        if encoder.conv is not None and not (conv_covered or f32):
             return None
         self = LayerLoop()
-        self.plans, self.length, self.device, self.dtype = plans, length, device, dtype
+        self.plans, self.length, self.device, self.dtype, self.f32 = plans, length, device, dtype, f32
         self.attention = [layer.attention.self for layer in encoder.layer]
         hidden, ffn = weight.shape[1], encoder.layer[0].intermediate.dense.weight.shape[0]
         width = first.all_head_size
         if hidden % 8 or ffn % 8 or first.attention_head_size not in (32, 64, 128):
+            return None
+        if f32 and not _cabi.f32_planes_supported(first.attention_head_size, length):
             return None
         n = len(encoder.layer)
         self.layers = (_cabi.DflEncoderLayer * n)()
         # (owner dict, key) of every tensor the loop reads, and where it was
         self._owners: list[dict] = []
         self._keys: list[str] = []
+        self._planes: list[torch.Tensor] = []
 
         def read(module: nn.Module, key: str) -> torch.Tensor | None:
             for owner in (module._parameters, module._buffers):
@@ -76,27 +89,32 @@ class LayerLoop:
                     return tensor
             return None
 
-        shapes = {"qkv_w": (3 * width, hidden), "attn_out_w": (hidden, width), "ffn_in_w": (ffn, hidden),
+        shapes = {"attn_out_w": (hidden, width), "ffn_in_w": (ffn, hidden),
                   "ffn_out_w": (hidden, ffn), "attn_norm_w": (hidden,), "ffn_norm_w": (hidden,)}
         try:
             for index, layer in enumerate(encoder.layer):
                 entry, plan = self.layers[index], plans[index]
+                for _, path, key in _ATTENTION_FIELDS:
+                    read(_module_at(layer, path), key)
+                module = layer.attention.self
+                if module._cached_qkv_weight.shape != (3 * width, hidden) or (f32 and module._cached_qkv_planes is None):
+                    return None
+                fill_attention_fields(entry, module, plan)
                 for field, path, key in _LAYER_FIELDS:
-                    tensor = read(_module_at(layer, path), key)
+                    owner = _module_at(layer, path)
+                    tensor = read(owner, key)
                     if field in shapes and (tensor is None or tuple(tensor.shape) != shapes[field]):
                         return None
+                    if f32 and field in _PLANE_FIELDS:
+                        tensor = encoder._weight_planes_of(tensor)
+                        self._planes.append(tensor)
                     setattr(entry, field, None if tensor is None else tensor.data_ptr())
                 entry.attn_norm_eps = float(layer.attention.output.LayerNorm.eps)
                 entry.ffn_norm_eps = float(layer.output.LayerNorm.eps)
-                module = layer.attention.self
-                has_c2p, has_p2c = module.has_c2p, module.has_p2c
-                if has_c2p != first.has_c2p or has_p2c != first.has_p2c or module.pos_att_type != first.pos_att_type:
+                if (module.has_c2p, module.has_p2c, module.pos_att_type) != (first.has_c2p, first.has_p2c, first.pos_att_type):
                     return None
-                for field, wanted in (("rel_key", has_c2p), ("rel_query", has_p2c), ("pos_key", has_c2p), ("pos_query", has_p2c)):
-                    tensor = getattr(plan, field) if wanted else None
-                    setattr(entry, field, None if tensor is None else tensor.data_ptr())
             p = _cabi.DflEncoderParams()
-            if encoder.conv is not None:
+            if encoder.conv is not None and not f32:
                 norm = encoder.conv.LayerNorm
                 bias = read(encoder.conv.conv, "bias")
                 gamma, beta = read(norm, "weight"), read(norm, "bias")
@@ -108,18 +126,21 @@ class LayerLoop:
                 p.conv_norm_eps = float(norm.eps)
         except _NotCovered:
             return None
-        self._pointers = self._current_pointers()
+        self._pointers = self._current_state()
         lut = plans[0].delta_to_local
         p.layers, p.n_layers = self.layers, n
         p.seq_len, p.hidden, p.heads, p.head_dim, p.ffn = length, hidden, first.num_attention_heads, first.attention_head_size, ffn
         p.lut, p.n_active = lut.data_ptr(), plans[0].active_slots.numel()
-        terms = 1 + int("c2p" in first.pos_att_type) + int("p2c" in first.pos_att_type)
-        p.scale, p.dtype = 1.0 / math.sqrt(first.attention_head_size * terms), _cabi.dtype_code(dtype)
+        p.scale, p.dtype = first._score_scale(), _cabi.dtype_code(dtype)
         self.params, self.n_layers, self.hidden = p, n, hidden
         return self
 
-    def _current_pointers(self) -> list[int]:
-        return list(map(_data_ptr, map(dict.__getitem__, self._owners, self._keys)))
+    def _current_state(self) -> list[int]:
+        """Address of every tensor the loop reads; in FP32, where copies of the weights are read, their versions too."""
+
+        tensors = list(map(dict.__getitem__, self._owners, self._keys))
+        state = list(map(_data_ptr, tensors))
+        return state + list(map(version_of, tensors)) if self.f32 else state
 
     def covers(self, encoder: nn.Module, plans: Any, hidden: torch.Tensor, mask: torch.Tensor) -> bool:
         """Whether this call can take the native loop (the state it was built from still holds)."""
@@ -133,14 +154,14 @@ class LayerLoop:
         for fused in encoder._fused_output_blocks:
             if not (fused[0] and fused[1]):
                 return False
-        if not all(encoder._fused_intermediates):
+        if not self.f32 and not all(encoder._fused_intermediates):
             return False
         for module in self.attention:
             if module.training or module._algo != _cabi.ALGO_AUTO:
                 return False
         try:
-            return self._current_pointers() == self._pointers
-        except (KeyError, TypeError):   # a parameter was deleted or set to None
+            return self._current_state() == self._pointers
+        except (KeyError, TypeError, AttributeError):   # a parameter was deleted or set to None
             return False
 
     def _call(self, hidden: torch.Tensor, mask: torch.Tensor, outs: Any, status: torch.Tensor | None) -> _cabi.DflEncoderParams:
@@ -156,17 +177,35 @@ class LayerLoop:
         return p
 
     def run(self, hidden: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None,
-            trace: list[torch.Tensor] | None) -> torch.Tensor:
-        outs = (ctypes.c_void_p * self.n_layers)()
+            trace: list[torch.Tensor] | None, conv: Any = None) -> torch.Tensor:
+        """``conv``: a convolution branch that is not part of the native loop, called after layer 0."""
+
+        if conv is not None:
+            first: list[torch.Tensor] = []
+            state = conv(hidden, self._run(hidden, mask, status, first, 0, 1), mask)
+            if trace is not None:
+                trace.append(state)
+            return self._run(state, mask, status, trace, 1, self.n_layers) if self.n_layers > 1 else state
+        return self._run(hidden, mask, status, trace, 0, self.n_layers)
+
+    def _run(self, hidden: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None,
+             trace: list[torch.Tensor] | None, begin: int, end: int) -> torch.Tensor:
+        n = end - begin
+        outs = (ctypes.c_void_p * n)()
         out = torch.empty(hidden.shape, dtype=self.dtype, device=self.device)
-        outs[self.n_layers - 1] = out.data_ptr()
+        outs[n - 1] = out.data_ptr()
         if trace is not None:
-            for layer in range(self.n_layers - 1):
+            for layer in range(n - 1):
                 state = torch.empty(hidden.shape, dtype=self.dtype, device=self.device)
                 outs[layer] = state.data_ptr()
                 trace.append(state)
             trace.append(out)
-        _cabi.encoder_fwd(self._call(hidden, mask, outs, status), self.device)
+        p = self._call(hidden, mask, outs, status)
+        if n != self.n_layers:
+            p.n_layers = n
+            p.layers = ctypes.cast(ctypes.addressof(self.layers) + begin * ctypes.sizeof(_cabi.DflEncoderLayer),
+                                   ctypes.POINTER(_cabi.DflEncoderLayer))
+        _cabi.encoder_fwd(p, self.device)
         return out
 
     def run_packed(self, hidden: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None, out: torch.Tensor,

@@ -120,6 +120,9 @@ typedef struct DflLinearParams {
   int32_t out_seqs;
 } DflLinearParams;
 DFL_API int dfl_qkv_proj(const DflLinearParams* p, void* stream);
+/* F32 with x and w given as bf16 planes [3][M][K] / [3][N][K] (dfl_split_planes): the same on the tensor cores, at least as
+ * accurate as the fp32 multiply-add chain of dfl_qkv_proj; K a multiple of 8. */
+DFL_API int dfl_qkv_proj_planes(const DflLinearParams* p, void* stream);
 
 /*
  * Prune projected position tables to the active slots:
@@ -391,10 +394,18 @@ DFL_API int dfl_embed_layernorm(const DflEmbedLayerNormParams* p, void* stream);
  * LayerNorm), and after layer 0 the optional convolution branch.  Every step is one of the functions above; the call
  * exists because a forward of a small batch is bound by what the host spends per launch, and because a kernel that is
  * known to follow one of this library's may load its weights before that one has finished.
- * F16/BF16, hidden == heads * head_dim not required, hidden and ffn multiples of 8, hidden as dfl_add_layernorm takes it.
+ * hidden == heads * head_dim is not required; hidden and ffn are multiples of 8, hidden as dfl_add_layernorm takes it.
  * Attention: rel_key / rel_query where given (dfl_attention_rel_fwd), else pos_key / pos_query (dfl_pos_scores +
  * dfl_attention_fwd, `lut` required).
+ *
+ * F32: the four weight matrices and pos_key / pos_query are given as bf16 planes [3][...] whose sum is the fp32 tensor
+ * (dfl_split_planes, once per weight); the GEMMs run on the tensor cores with six plane products per product and
+ * fp32 sums, at least as accurate as a fp32 multiply-add chain (finite operands; an infinite operand gives NaN).  Biases
+ * and norm parameters stay fp32.  No convolution branch and no packed rows in F32.
  */
+/* planes[3][n] (bf16) with planes[0] + planes[1] + planes[2] == x exactly; n a multiple of 4 */
+DFL_API int dfl_f32_planes_supported(int head_dim, int seq_len);   /* whether the F32 form covers the attention's sizes */
+DFL_API int dfl_split_planes(const void* x, void* planes, int64_t n, void* stream);
 typedef struct DflEncoderLayer {
   const void *qkv_w, *qkv_b;              /* [3*heads*head_dim, hidden], [3*heads*head_dim] or NULL */
   const void *attn_out_w, *attn_out_b;    /* [hidden, heads*head_dim], [hidden] or NULL */
@@ -427,6 +438,8 @@ typedef struct DflEncoderParams {
    * event 2l+1 after the attention of layer l. */
   void* const* attention_events;
   int32_t launches;                /* out: kernels this call has launched */
+  int32_t attention_only;          /* non-zero: layer 0 up to its attention; outs[0] is the context
+                                      [batch, seq_len, heads*head_dim] and only the qkv and table entries are read */
   /* Packed form (packed_rows > 0, rel_* form only, seq_len a multiple of 32): between the attention kernels the layers
    * run on the valid positions, packed in groups of 32 rows.  outs[n_layers-1] receives the unpacked result; positions
    * no group covers are left as they are there.  No other entry of outs may be given. */
