@@ -8,27 +8,30 @@
 // with x running over one contiguous window of 255 table rows.  Both are produced by tcgen05.mma from 128-row
 // table blocks (L2 resident), rounded to the input type exactly like the separate score GEMMs round their output,
 // and parked in shared memory, where the softmax threads pick them up along diagonals.
-//   C2P depends on the query rows only: D[r, m] = q_r . rel_key[x_lo + m] with TMEM lanes = query rows.  Per query
-//       row a shared-memory ring of two 128-column blocks is kept (the window of a key tile is two blocks; the next
-//       key tile needs one new block, written in place of the block that left the window).
+//   C2P depends on the query rows only: D[r, m] = q_r . rel_key[x_lo + m] with TMEM lanes = query rows.  The window of a
+//       key tile is two 128-column blocks; the next key tile needs one new block.  Converter warps round a block's rows and
+//       store each shifted by its row, so that key x of the tile ends up in column x: a softmax thread adds its 64 scores
+//       from eight 16-byte loads.
 //   P2C is new for every key tile: D[n, m] = k_n . rel_query[x_lo + m] with TMEM lanes = keys n, computed in two
-//       halves of 128 table rows through one 128-column accumulator.  Converter warps round each key's row and
-//       store the 136-column span the 128 queries of the tile can reach; a softmax thread then reads, for key n,
-//       element (n & 7) + 128 - r of row n: the 32 lanes of a warp read 32 consecutive elements.
+//       halves of 128 table rows through one 128-column accumulator.  Here the diagonal runs across the lanes' columns and
+//       the softmax threads need it transposed: converter warps round each key's row and store it, shifted by its key, as
+//       row n of a K-major B operand, and S gets it by one more MMA, S += I . tile^T with an identity matrix as A.  The
+//       tensor pipe is idle three quarters of the time otherwise; it transposes and adds exactly (one product by 1.0 and
+//       zeros, fp32 accumulation).
 //
 // Persistent: one CTA per SM walks (batch, head, 128-query tile) items in 128-key tiles; every role keeps running
-// counters so that the barrier phases carry over from item to item and the loader / MMA issuer run ahead.
+// counters so that the barrier phases carry over from item to item and the loader / MMA issuers run ahead.
 //   warps 0-7   softmax: two threads per query row (warps w and w+4 own the same TMEM lanes; each takes 64 of the
-//               128 keys of a tile, 32 of the 64 packed P columns and half of the output columns).  Two passes over
-//               the keys in rolled loops of 32: scores + relative terms + mask + maximum, written back to the S
-//               columns; then exp2, rounding, row sum and the P store.
-//   warps 8-11  converters for the C2P block and P2C accumulators (TMEM -> 16-bit -> shared memory)
-//   warp 12     issuer of every MMA (C2P block, S, P2C halves, PV) and TMEM owner
-//   warp 13     per-item mask analysis (kept-key bits, skipped key tiles), one item ahead, and TMA producer
-// The first MMAs of an item (first C2P block, S and P2C of its first key tile) are issued while the softmax threads
-// still work on the last key tile of the previous item; the second C2P block of an item goes through the P and O
-// columns, which are idle between the read-out of one item and the first PV of the next.
-//   warps 14-15 idle (they complete the fourth warpgroup, whose registers go to the softmax warps)
+//               128 keys of a tile, 32 of the 64 packed P columns and half of the output columns).  One pass: the 64
+//               scores stay in registers from the S load to the P store.
+//   warps 8-11  converters of the P2C halves (TMEM -> 16-bit -> shared memory), warps 12-15 of the C2P blocks
+//   warp 16     issuer of the score MMAs (C2P block, P2C halves, S with the P2C tile added) and TMEM owner
+//   warp 17     per-item mask analysis (kept-key bits, skipped key tiles), one item ahead, and TMA producer
+//   warp 18     issuer of the PV MMAs; warp 19 is idle (it completes the fifth warpgroup)
+// What bounds it: instruction issue and fetch.  With everything unrolled (156 KB of code) a third of the issue slots were
+// lost to instruction fetch; the waits, the loader and the MMA loops are therefore rolled (88 KB), which was worth 17 %.
+// 32 x 12 heads x 512 x d 64, fp16, both terms: 185 -> 173 us, C2P only 145 -> 117 us against two passes over the keys with
+// the diagonals read by the softmax threads.
 #include <type_traits>
 
 #include "attention_tc_common.cuh"
@@ -44,36 +47,43 @@ using attn::Pack2;
 constexpr int BM = 128;              // query rows per item (= TMEM lanes)
 constexpr int BK = 128;              // keys per tile
 constexpr int kSoftmaxWarps = 8;
-constexpr int kMmaWarp = 12;
-constexpr int kTmaWarp = 13;
-constexpr int kThreads = 512;
-constexpr int kSoftmaxRegs = 152;    // 256 x 152 + 128 x 120 + 128 x 88 = 65536 registers
-constexpr int kConvRegs = 120;
-constexpr int kMiscRegs = 88;
-// The kernel is launched with 65536 / kThreads = 128 registers per thread.  `setmaxnreg.inc` waits until the pool
-// holds what it asks for, so the three budgets must not ask for more than the SM has (a wait that nothing could
+constexpr int kC2pWarp = 12;         // warps 8-11 convert the P2C halves, 12-15 the C2P blocks
+constexpr int kMmaWarp = 16;
+constexpr int kTmaWarp = 17;
+constexpr int kPvWarp = 18;
+constexpr int kThreads = 640;
+constexpr int kSoftmaxRegs = 128;    // 256 x 128 + 256 x 80 + 128 x 64 = 61440 registers
+constexpr int kConvRegs = 80;
+constexpr int kMiscRegs = 64;
+// The kernel is launched with 65536 / kThreads registers per thread, rounded down to the allocation unit of 8: 96.
+// `setmaxnreg.inc` waits until the pool holds what it asks for, so the three budgets must not ask for more than the SM has (a wait that nothing could
 // bound); `setmaxnreg.dec` with a value above the launch allocation is an illegal instruction.
-constexpr int kLaunchRegs = 65536 / kThreads;
-static_assert(8 * 32 * kSoftmaxRegs + 4 * 32 * kConvRegs + 4 * 32 * kMiscRegs <= kThreads * kLaunchRegs,
+constexpr int kLaunchRegs = 65536 / kThreads / 8 * 8;
+static_assert(8 * 32 * kSoftmaxRegs + 8 * 32 * kConvRegs + 4 * 32 * kMiscRegs <= kThreads * kLaunchRegs,
               "register budgets of the three warpgroup kinds exceed what the launch allocates");
 static_assert(kSoftmaxRegs >= kLaunchRegs && kConvRegs <= kLaunchRegs && kMiscRegs <= kLaunchRegs &&
                   kSoftmaxRegs % 8 == 0 && kConvRegs % 8 == 0 && kMiscRegs % 8 == 0,
               "setmaxnreg.inc raises and setmaxnreg.dec lowers the launch allocation, in multiples of 8");
-constexpr int kConsumerWarps = 13;   // softmax, converters, MMA issuer: every warp that reads an item slot
+constexpr int kConsumerWarps = 18;   // softmax, converters, both MMA issuers: every warp that reads an item slot
 
 constexpr int kItemSlots = 3;        // the loader analyses one item ahead of the one whose tiles it loads
 constexpr int kMaxSeqLen = 2048;
 constexpr int kMaskWords = kMaxSeqLen / 32;   // kept-key bits per item
 
-// C2P ring: per query row two 128-column blocks and the first 16 columns once more (a 16-key run never wraps).
-// 580 bytes = 145 words per row: the diagonal 16-bit reads of a warp and its 32-bit stores are conflict free.
-constexpr int RING_COLS = 256;
-constexpr int RING_MIRROR = 16;
-constexpr int RING_PITCH = 580;
-// P2C staging: per key 17 chunks of 8 columns (the chunk-aligned span of table rows its 128 queries reach).
-// 272 bytes = 68 words per row: eight consecutive rows cover all 32 banks with their 16-byte stores.
-constexpr int STG_CHUNKS = 17;
-constexpr int STG_PITCH = STG_CHUNKS * 16;
+// C2P rows: per query row two tiles of 128 16-bit scores, tile T of the CTA's running count in half T & 1, key x of the tile
+// at column x: the softmax thread of the row reads its 64 keys as eight 16-byte words.  35 16-byte units per row: eight
+// consecutive rows hit different bank groups with those reads, and the converters' 4-byte stores conflict at most 2-way.
+constexpr int ROW_PITCH = 560;
+// P2C tile: the B operand of the MMA that adds it to S, K-major without swizzle: 8-row core matrices of 128 bytes, rows =
+// keys, K = query rows.  Chunks of eight query rows are STG_CHUNK bytes apart (32 bytes more than 16 core matrices, so
+// that the 4-byte stores of 32 neighbouring keys, each shifted by its key, fall into 32 different banks).
+constexpr int STG_CHUNK = 16 * 128 + 32;
+constexpr int STG_BYTES = 16 * STG_CHUNK;
+// Identity operand of that MMA: 240 rows x 16 columns, row 112 + k holds a one in column k and the others are zero; k-step
+// kk of the 128 x 128 identity is the 128-row window that starts at row 112 - 16 kk.
+constexpr int EYE_ROWS = 240;
+constexpr int EYE_CHUNK = EYE_ROWS * 16;   // bytes between the two 8-column chunks
+constexpr int EYE_BYTES = 2 * EYE_CHUNK;
 
 // TMEM columns (all 512; one CTA per SM)
 constexpr int COL_S = 0;      // 128  S = Q K^T of the current tile (fp32)
@@ -95,16 +105,16 @@ struct RLayout {
   static constexpr int offV = offK + 2 * kTile;
   static constexpr int offRK = offV + kVStages * kTile;
   static constexpr int offRQ = offRK + kRkStages * kTile;   // 2 stages
-  static constexpr int offRing = offRQ + 2 * kTile;
-  static constexpr int offStg = offRing + BM * RING_PITCH;
-  static constexpr int offBar = offStg + BK * STG_PITCH;
+  static constexpr int offRows = offRQ + 2 * kTile;
+  static constexpr int offStg = offRows + BM * ROW_PITCH;
+  static constexpr int offEye = offStg + STG_BYTES;
+  static constexpr int offBar = offEye + EYE_BYTES;
   static constexpr int kBarBytes = 512;
-  // exchange area: row maxima [2 parities][2 halves][BM], row sums [2 halves][BM], then the mean-of-V scratch
-  // ([256 / D groups][D] partial sums, [D] column mean)
+  // exchange area: [2 parities][2 halves][BM] row maxima (row sums at the end of an item, partial sums of the mean-of-V
+  // path), then the [D] column mean of V
   static constexpr int offXmax = offBar + kBarBytes;
-  static constexpr int offXsum = offXmax + 2 * 2 * BM * 4;
-  static constexpr int offMeanV = offXsum + 2 * BM * 4;
-  static constexpr int offItem = offMeanV + 1024 + 256;
+  static constexpr int offMeanV = offXmax + 2 * 2 * BM * 4;
+  static constexpr int offItem = offMeanV + 256;
   static constexpr int kItemBytes = 288;
   static constexpr int total = offItem + kItemSlots * kItemBytes + 1024;   // + alignment slack
   static_assert(offStg % 16 == 0 && offBar % 16 == 0 && offItem % 16 == 0, "alignment");
@@ -126,16 +136,14 @@ struct RBarriers {
   uint64_t rk_full[2], rk_empty[2], rq_full[2], rq_empty[2];
   uint64_t s_full, s_free;          // S accumulator: MMA -> softmax, softmax (8 warps) -> MMA
   uint64_t xc_full, xc_free;        // C2P block accumulator: MMA -> converters (4 warps) -> MMA
-  uint64_t b1_full;                 // second C2P block of an item, in the P and O columns
   uint64_t xp_full, xp_free;        // P2C half accumulator: MMA -> converters (4 warps) -> MMA
-  uint64_t pt_ready, pt_release;    // P2C staging tile: converters -> softmax -> converters
+  uint64_t pt_ready, pt_release;    // P2C tile in shared memory: converters -> MMA (its reads complete) -> converters
   uint64_t p_full, o_ready, o_free; // P stored (8 warps); PV complete; output accumulator read out (8 warps)
-  uint64_t c2p_ready, ring_release; // C2P ring blocks of a tile: converters -> softmax -> converters
+  uint64_t c2p_ready, ring_release; // C2P rows of a tile: converters -> softmax -> converters
   uint64_t pair2[4];                // the two warps of a lane quarter: row maximum (row sum) posted
   uint64_t item_full[kItemSlots], item_empty[kItemSlots];
   uint64_t xbar;                    // the eight softmax warps (mean-of-V path)
   uint32_t tmem_base;
-  int abort_flag;
 };
 static_assert(sizeof(RBarriers) <= 512, "barrier block too large");
 
@@ -148,43 +156,20 @@ __device__ __forceinline__ void setmaxnreg_dec() {
   asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(N));
 }
 
-// tcgen05.mma with shared-memory descriptors passed as 32-bit halves (hi is shared by both operands) and the
-// accumulate flag as a compile-time constant: the issuing thread spends no instructions on building descriptors.
-template <int ACC>
-__device__ __forceinline__ void umma_ss_lohi(uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo, uint32_t hi, uint32_t idesc) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 da, db;\n\tsetp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 da, {%1, %3};\n\tmov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], da, db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_lo), "r"(b_lo), "r"(hi), "r"(idesc), "n"(ACC)
-      : "memory");
-}
-__device__ __forceinline__ void umma_ts_lohi(uint32_t d_tmem, uint32_t a_tmem, uint32_t b_lo, uint32_t hi, uint32_t idesc,
-                                             uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t.reg .b64 db;\n\tsetp.ne.b32 p, %5, 0;\n\t"
-      "mov.b64 db, {%2, %3};\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], db, %4, p;\n\t}"
-      ::"r"(d_tmem), "r"(a_tmem), "r"(b_lo), "r"(hi), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
-// 16-bit shared-memory load, zero-extended into a 32-bit register (32-bit destinations keep every value in its
-// own register; the address arithmetic of unrolled callers folds into the instruction's immediate offset).
-__device__ __forceinline__ uint32_t lds_u16_r32(uint32_t saddr) {
-  uint32_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
+__device__ __forceinline__ uint4 lds_v4(uint32_t saddr) {
+  uint4 v;
+  asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(saddr) : "memory");
   return v;
 }
-__device__ __forceinline__ uint32_t lds_u32(uint32_t saddr) {
-  uint32_t v;
-  asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(saddr) : "memory");
-  return v;
-}
-// low 32 bits of {hi, lo} >> amount (amount 0 or 16: one element of a pair of packed 16-bit values)
-__device__ __forceinline__ uint32_t funnel_r(uint32_t lo, uint32_t hi, uint32_t amount) {
+// {hi, lo} >> amount, low 32 bits; amount 0 or 16 (wrap), 16 or 32 (clamp)
+__device__ __forceinline__ uint32_t funnel_wrap(uint32_t lo, uint32_t hi, uint32_t amount) {
   uint32_t v;
   asm("shf.r.wrap.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(lo), "r"(hi), "r"(amount));
+  return v;
+}
+__device__ __forceinline__ uint32_t funnel_clamp(uint32_t lo, uint32_t hi, uint32_t amount) {
+  uint32_t v;
+  asm("shf.r.clamp.b32 %0, %1, %2, %3;" : "=r"(v) : "r"(lo), "r"(hi), "r"(amount));
   return v;
 }
 __device__ __forceinline__ float max3(float a, float b, float c) {
@@ -195,8 +180,17 @@ __device__ __forceinline__ float max3(float a, float b, float c) {
 __device__ __forceinline__ void sts_u32(uint32_t saddr, uint32_t v) {
   asm volatile("st.shared.u32 [%0], %1;" ::"r"(saddr), "r"(v) : "memory");
 }
-__device__ __forceinline__ void sts_v4(uint32_t saddr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
-  asm volatile("st.shared.v4.u32 [%0], {%1, %2, %3, %4};" ::"r"(saddr), "r"(a), "r"(b), "r"(c), "r"(d) : "memory");
+__device__ __forceinline__ void sts_u32_if(uint32_t saddr, uint32_t v, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.shared.u32 [%0], %1;\n\t}" ::"r"(saddr), "r"(v), "r"((int)on) : "memory");
+}
+// Two scores rounded to T and packed.  FP16 saturates: a score beyond 65504 would be an infinity, and the MMA that adds
+// the P2C tile to S multiplies the other rows' entries of that key by zero.
+template <typename T>
+__device__ __forceinline__ uint32_t pack_scores(float lo, float hi) {
+  uint32_t v;
+  if constexpr (__is_same(T, __half)) asm("cvt.rn.satfinite.f16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  else asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(v) : "f"(hi), "f"(lo));
+  return v;
 }
 
 // 32 consecutive fp32 TMEM columns of this thread's lane into arr[off .. off+31] (a register array indexed by
@@ -216,20 +210,6 @@ __device__ __forceinline__ void sts_v4(uint32_t saddr, uint32_t a, uint32_t b, u
       : "r"(taddr)                                                                                                  \
       : "memory")
 
-#define DFL_TMEM_ST32_F(taddr, arr, off)                                                                            \
-  asm volatile(                                                                                                     \
-      "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "                                                               \
-      "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, "                                    \
-      "%17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31, %32};"                            \
-      ::"r"(taddr), "f"(arr[off + 0]), "f"(arr[off + 1]), "f"(arr[off + 2]), "f"(arr[off + 3]), "f"(arr[off + 4]),   \
-        "f"(arr[off + 5]), "f"(arr[off + 6]), "f"(arr[off + 7]), "f"(arr[off + 8]), "f"(arr[off + 9]),               \
-        "f"(arr[off + 10]), "f"(arr[off + 11]), "f"(arr[off + 12]), "f"(arr[off + 13]), "f"(arr[off + 14]),          \
-        "f"(arr[off + 15]), "f"(arr[off + 16]), "f"(arr[off + 17]), "f"(arr[off + 18]), "f"(arr[off + 19]),          \
-        "f"(arr[off + 20]), "f"(arr[off + 21]), "f"(arr[off + 22]), "f"(arr[off + 23]), "f"(arr[off + 24]),          \
-        "f"(arr[off + 25]), "f"(arr[off + 26]), "f"(arr[off + 27]), "f"(arr[off + 28]), "f"(arr[off + 29]),          \
-        "f"(arr[off + 30]), "f"(arr[off + 31])                                                                       \
-      : "memory")
-
 // s0 += lo half of w, s1 += hi half of w (w = two packed values of type T), in fp32.
 template <typename T>
 __device__ __forceinline__ void add_pair(float& s0, float& s1, uint32_t w);
@@ -246,25 +226,29 @@ __device__ __forceinline__ void add_pair<__nv_bfloat16>(float& s0, float& s1, ui
       : "r"(w));
 }
 
-// Kept-key bits of batch row b: word w (keys [32w, 32w+32)) built from its 32 mask elements.
-__device__ __forceinline__ uint32_t kept_bits_word(const DflAttnRelParams& p, int b, int w) {
-  const int L = p.seq_len;
-  uint32_t kb = 0;
-  const int jw = 32 * w;
-  const long long base = (long long)b * L + jw;
-  if (jw + 32 <= L && p.mask_elem_size == 1 && ((reinterpret_cast<uintptr_t>(p.mask) + base) & 15) == 0) {
-    const uint4* m16 = reinterpret_cast<const uint4*>(reinterpret_cast<const unsigned char*>(p.mask) + base);
-    const uint4 lo = m16[0], hi = m16[1];
-    const uint32_t wds[8] = {lo.x, lo.y, lo.z, lo.w, hi.x, hi.y, hi.z, hi.w};
+// Kept-key bits of batch row b, one word of 32 keys per lane: lane l gets words l (lo) and l + 32 (hi).  Warp-collective:
+// the mask is read 32 elements at a time, four words in flight.
+__device__ __forceinline__ void kept_bits(const DflAttnRelParams& p, int b, int lane, uint32_t& lo, uint32_t& hi) {
+  const int L = p.seq_len, n_words = (L + 31) / 32;
+  const long long base = (long long)b * L;
+  lo = hi = 0;
+#pragma unroll 1
+  for (int w0 = 0; w0 < n_words; w0 += 4) {
+    bool keep[4];
 #pragma unroll
-    for (int x = 0; x < 32; ++x)
-      if ((wds[x >> 2] >> ((x & 3) * 8)) & 0xffu) kb |= 1u << x;
-  } else if (jw < L) {
-#pragma unroll 8
-    for (int x = 0; x < 32; ++x)
-      if (jw + x < L && mask_keep(p.mask, p.mask_elem_size, base + x)) kb |= 1u << x;
+    for (int x = 0; x < 4; ++x) {
+      const int j = 32 * (w0 + x) + lane;
+      keep[x] = j < L && mask_keep(p.mask, p.mask_elem_size, base + j);
+    }
+#pragma unroll
+    for (int x = 0; x < 4; ++x) {
+      const uint32_t bits = __ballot_sync(0xffffffffu, keep[x]);
+      if (lane == ((w0 + x) & 31)) {
+        if (w0 + x < 32) lo = bits;
+        else hi = bits;
+      }
+    }
   }
-  return kb;
 }
 
 // Key tiles before the first and after the last kept key contribute nothing to a kept query row (their
@@ -308,11 +292,10 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   extern __shared__ unsigned char smem_dyn[];
   unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
   RBarriers* bars = reinterpret_cast<RBarriers*>(smem + LO::offBar);
-  volatile int* abort_flag = &bars->abort_flag;
   ItemSlot* slots = reinterpret_cast<ItemSlot*>(smem + LO::offItem);
 
   const int L = p.seq_len, H = p.heads;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, threadIdx.x >> 5, 0), lane = threadIdx.x & 31;
   const bool has_c2p = p.rel_key != nullptr, has_p2c = p.rel_query != nullptr;
   int fail_code = 0;   // code of the bounded wait of this thread that expired first, if any
 
@@ -334,7 +317,6 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       ptx::mbar_init(&bars->item_full[s], 1);
       ptx::mbar_init(&bars->item_empty[s], kConsumerWarps);
     }
-    ptx::mbar_init(&bars->b1_full, 1);
     ptx::mbar_init(&bars->s_full, 1);
     ptx::mbar_init(&bars->s_free, kSoftmaxWarps);   // one elected lane per softmax warp
     ptx::mbar_init(&bars->xc_full, 1);
@@ -342,7 +324,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     ptx::mbar_init(&bars->xp_full, 1);
     ptx::mbar_init(&bars->xp_free, 4);              // converter warps
     ptx::mbar_init(&bars->pt_ready, 4);
-    ptx::mbar_init(&bars->pt_release, kSoftmaxWarps);
+    ptx::mbar_init(&bars->pt_release, 1);
     ptx::mbar_init(&bars->p_full, kSoftmaxWarps);
     ptx::mbar_init(&bars->o_ready, 1);
     ptx::mbar_init(&bars->o_free, kSoftmaxWarps);
@@ -350,9 +332,18 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     ptx::mbar_init(&bars->ring_release, kSoftmaxWarps);
     for (int s = 0; s < 4; ++s) ptx::mbar_init(&bars->pair2[s], 2);
     ptx::mbar_init(&bars->xbar, kSoftmaxWarps);
-    bars->abort_flag = 0;
     ptx::fence_mbar_init();
   }
+  // identity operand: zeros with ones on rows 112 .. 127
+  for (int e = threadIdx.x; e < EYE_BYTES / 16; e += kThreads) {
+    const int chunk = e / EYE_ROWS, col = e - chunk * EYE_ROWS - (EYE_ROWS - BM) - 8 * chunk;   // column of the one, if in [0, 8)
+    const uint32_t one = __is_same(T, __half) ? 0x3C00u : 0x3F80u;
+    uint32_t w[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) w[j] = col == 2 * j ? one : (col == 2 * j + 1 ? one << 16 : 0u);
+    *reinterpret_cast<uint4*>(smem + LO::offEye + e * 16) = make_uint4(w[0], w[1], w[2], w[3]);
+  }
+  ptx::fence_proxy_async_smem();
   if (warp == kTmaWarp && lane == 0) {
     ptx::prefetch_tensormap(&tmap_q);
     ptx::prefetch_tensormap(&tmap_k);
@@ -375,7 +366,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   // A bounded wait whose verdict is the same in every lane of the warp (the tcgen05.ld/st/wait instructions that
   // follow are warp-collective and must not be reached by part of a warp).
   auto wwait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
-    return __all_sync(0xffffffffu, ptx::mbar_wait_inline(bar, parity, abort_flag, fail_code, code));
+    return ptx::mbar_wait_warp(bar, parity, fail_code, code);
   };
 
   // The set-up above overlaps the tail of the previous kernel of the stream; Q, K, V, the mask and the status word
@@ -384,9 +375,8 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
   // Every role walks the same item sequence (item number k of this CTA is item blockIdx.x + k * gridDim.x; it uses
   // item slot k % 3 in phase (k / 3) & 1) and keeps its own running counters.  Register budgets are set per
-  // warpgroup (warps 0-3, 4-7: softmax; 8-11: converters; 12-15: the rest), at the head of the branch the whole
-  // warpgroup takes.  The loops over a tile's keys are rolled on purpose: the kernel is bound by instruction fetch
-  // as soon as the code of a tile no longer fits the instruction caches.
+  // warpgroup (warps 0-7: softmax; 8-15: converters; 16-19: the rest), at the head of the branch the whole warpgroup
+  // takes.
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
     // ----------------------------------------------------------------- softmax
@@ -399,16 +389,12 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const uint32_t t_s = tmem_base + lane_base + COL_S + hf * 64;
     const uint32_t t_p = tmem_base + lane_base + COL_P + hf * 32;
     const uint32_t t_o = tmem_base + lane_base + COL_O + hf * OW;
-    const uint32_t ring_row = ptx::smem_u32(smem + LO::offRing) + (uint32_t)(r * RING_PITCH);
-    const uint32_t odd16 = (uint32_t)(r & 1) * 16u;   // a row's window starts on an odd column iff r is odd
-    // P2C of (row r, key n) is element (n & 7) + 128 - r of staging row n
-    const uint32_t stg_base = ptx::smem_u32(smem + LO::offStg) + (uint32_t)(hf * 64 * STG_PITCH + 2 * (128 - r));
-    float* xmax = reinterpret_cast<float*>(smem + LO::offXmax);
-    float* xsum = reinterpret_cast<float*>(smem + LO::offXsum);
+    const uint32_t c2p_row = ptx::smem_u32(smem + LO::offRows) + (uint32_t)(r * ROW_PITCH + hf * 128);   // this thread's 64 keys
+    float* xchg = reinterpret_cast<float*>(smem + LO::offXmax);
     uint64_t* pair2 = &bars->pair2[q4];
     // Two running counts give every barrier phase of this role: c_t = key tiles started (all items), c_i = items with
-    // kept rows finished.  Per tile one phase each of s_full, c2p_ready, pt_ready and o_ready, per tile and per item
-    // one of pair2; an item of padded rows only uses xbar exactly twice (phases 0 and 1).
+    // kept rows finished.  Per tile one phase each of s_full, c2p_ready and o_ready, per tile and per item one of pair2;
+    // an item of padded rows only uses xbar exactly four times.
     uint32_t c_t = 0, c_i = 0;
     bool ok = true;
 
@@ -433,14 +419,14 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         // the column mean of V.  No score, no softmax: one pass over V by the 256 softmax threads.
         // 16-byte loads, every thread sums 8 columns over a stride of rows; the row groups of a warp are folded with
         // shuffles and the eight warps through shared memory (the row-exchange words are idle during such an item).
-        float* part = xmax;                                                  // [8 warps][D] partial sums
-        T* mean = reinterpret_cast<T*>(smem + LO::offMeanV + 1024);          // [D]
+        float* part = xchg;                                          // [8 warps][D] partial sums
+        T* mean = reinterpret_cast<T*>(smem + LO::offMeanV);         // [D]
         constexpr int kChunks = D / 8;             // 16-byte chunks per row of V
         constexpr int kRowStep = 256 / kChunks;    // rows covered by the 256 threads at once
         const int tid = threadIdx.x, chunk = tid % kChunks, rgrp = tid / kChunks;
         const uint4* V4 = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + (long long)bh * L * D);
         float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 4
+#pragma unroll 2
         for (int row = rgrp; row < L; row += kRowStep) {
           const uint4 raw = __ldg(V4 + (long long)row * kChunks + chunk);
           const T* e = reinterpret_cast<const T*>(&raw);
@@ -452,13 +438,18 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
           for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
         }
+        // every warp has read its partner's row sums of the item before
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->xbar);
+        ok = wwait(&bars->xbar, 0u, 34);
+        if (!ok) break;
         if (lane < kChunks) {
 #pragma unroll
           for (int j = 0; j < 8; ++j) part[warp * D + lane * 8 + j] = acc[j];
         }
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->xbar);
-        ok = wwait(&bars->xbar, 0u, 34);
+        ok = wwait(&bars->xbar, 1u, 36);
         if (!ok) break;
         if (tid < D) {
           float total = 0.0f;
@@ -468,7 +459,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->xbar);
-        ok = wwait(&bars->xbar, 1u, 35);
+        ok = wwait(&bars->xbar, 0u, 35);
         if (!ok) break;
         const int rows = out_rows - i0 < BM ? out_rows - i0 : BM;
         constexpr int kVec = D / 8;  // 16-byte chunks per output row
@@ -478,6 +469,10 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           const int rr = e / kVec, v = e - rr * kVec;
           *reinterpret_cast<uint4*>(out + (long long)rr * H * D + v * 8) = mine;
         }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->xbar);   // the exchange words are free again
+        ok = wwait(&bars->xbar, 1u, 37);
+        if (!ok) break;
       } else {
         const int i = i0 + r;
         const bool row_ok = i < L;
@@ -488,89 +483,73 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           const int t = t_begin + u;
           const uint32_t kb0 = sl->kbits[4 * t + 2 * hf], kb1 = sl->kbits[4 * t + 2 * hf + 1];
           const int n_in = L - t * BK - hf * 64;   // in-range keys among this thread's 64 (may be <= 0 or >= 64)
-          // ring column of (row r, key x of the tile): (128 * (u & 1) + 128 - r + x) mod 256
-          const uint32_t cb = (128u * (uint32_t)(u & 1) + 128u - (uint32_t)r + 64u * (uint32_t)hf) & 255u;
-
           const uint32_t tile_phase = c_t & 1u;
           ++c_t;
           ok = wwait(&bars->s_full, tile_phase, 41);
-          if (ok && has_c2p) ok = wwait(&bars->c2p_ready, tile_phase, 42);
-          if (ok && has_p2c) ok = wwait(&bars->pt_ready, tile_phase, 44);
           if (!ok) break;
           ptx::tc_fence_after();
 
-          // ---- pass 1 over the thread's 64 keys in two chunks of 32: S from TMEM (the next chunk in flight), the two
-          // relative terms from shared memory, mask, running maximum; the biased scores go back to the S columns.
-          float cur[32], nxt[32];
-          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
-          DFL_TMEM_LD32_F(t_s, nxt, 0);
-#pragma unroll 1
-          for (int q = 0; q < 2; ++q) {
+          // Scores of the thread's 64 keys: Q.K plus the P2C term from tensor memory (the MMA issuer has added the
+          // term), the C2P term from the thread's row in shared memory.  They stay in registers until P is stored.
+          float s[64];
+          DFL_TMEM_LD32_F(t_s, s, 0);
+          DFL_TMEM_LD32_F(t_s + 32, s, 32);
+          if (has_c2p) {
+            ok = wwait(&bars->c2p_ready, tile_phase, 42);
+            if (!ok) break;
+            const uint32_t caddr = c2p_row + (tile_phase ? 256u : 0u);
+            uint4 w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = lds_v4(caddr + 16u * j);
             ptx::tmem_wait_ld();
 #pragma unroll
-            for (int x = 0; x < 32; ++x) cur[x] = nxt[x];
-            if (q == 0) DFL_TMEM_LD32_F(t_s + 32, nxt, 0);
-            if (has_p2c) {
-              const uint32_t paddr = stg_base + (uint32_t)(q * 32 * STG_PITCH);
+            for (int half = 0; half < 2; ++half) {
 #pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                // per 16 keys: 16 loads issued before the 16 adds that use them (a warp issues in order)
-                uint32_t pv[16];
-#pragma unroll
-                for (int x = 0; x < 16; ++x)
-                  pv[x] = lds_u16_r32(paddr + (uint32_t)((16 * j + x) * STG_PITCH + 2 * (x & 7)));
-#pragma unroll
-                for (int x = 0; x < 16; ++x) cur[16 * j + x] = Pack2<T>::add(cur[16 * j + x], (uint16_t)pv[x]);
+              for (int j = 0; j < 4; ++j) {
+                const int x = 32 * half + 8 * j;
+                add_pair<T>(s[x], s[x + 1], w[j].x);
+                add_pair<T>(s[x + 2], s[x + 3], w[j].y);
+                add_pair<T>(s[x + 4], s[x + 5], w[j].z);
+                add_pair<T>(s[x + 6], s[x + 7], w[j].w);
               }
-              // the staging tile is read: the converters may fill it for the next tile while the C2P terms of this
-              // chunk, the mask and pass 2 are still to come
-              if (q == 1) {
+              if (half == 0) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) w[j] = lds_v4(caddr + 64u + 16u * j);
+                ptx::tc_fence_before();
                 __syncwarp();
-                if (lane == 0) ptx::mbar_arrive(&bars->pt_release);
+                if (lane == 0) {   // S and the C2P row are in registers: both may be overwritten for the next tiles
+                  ptx::mbar_arrive(&bars->s_free);
+                  ptx::mbar_arrive(&bars->ring_release);
+                }
               }
             }
-            if (has_c2p) {
-#pragma unroll
-              for (int j = 0; j < 2; ++j) {
-                // 16 keys are read as nine aligned 32-bit words and shifted by one element where the run starts on
-                // an odd column; the run stays below column 272 (the first 16 columns are mirrored behind the ring)
-                const uint32_t w0 = (cb + 32u * (uint32_t)q + 16u * j) & 255u;
-                const uint32_t caddr = ring_row + 2u * (w0 & ~1u);
-                uint32_t cw[9];
-#pragma unroll
-                for (int x = 0; x < 9; ++x) cw[x] = lds_u32(caddr + 4u * x);
-#pragma unroll
-                for (int x = 0; x < 8; ++x)
-                  add_pair<T>(cur[16 * j + 2 * x], cur[16 * j + 2 * x + 1], funnel_r(cw[x], cw[x + 1], odd16));
-              }
-            }
-            // mask: keys >= L and padded keys -> -inf; a padded query row -> 0 on every in-range key
-            const uint32_t kbq = q ? kb1 : kb0;
-            if (!q_keep) {
-              const int n_q = n_in - 32 * q;
-#pragma unroll
-              for (int x = 0; x < 32; ++x) cur[x] = x < n_q ? 0.0f : -INFINITY;
-            } else if (kbq != 0xffffffffu) {
-#pragma unroll
-              for (int x = 0; x < 32; ++x)
-                if (!((kbq >> x) & 1u)) cur[x] = -INFINITY;
-            }
-#pragma unroll
-            for (int x = 0; x < 32; x += 2) mx[(x >> 1) & 3] = max3(mx[(x >> 1) & 3], cur[x], cur[x + 1]);
-            DFL_TMEM_ST32_F(t_s + 32 * q, cur, 0);
+          } else {
+            ptx::tmem_wait_ld();
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&bars->s_free);
           }
-          // the ring blocks and the staging tile of this tile are read
-          __syncwarp();
-          if (lane == 0 && has_c2p) ptx::mbar_arrive(&bars->ring_release);
+          // mask: keys >= L and padded keys -> -inf; a padded query row -> 0 on every in-range key
+          if (!q_keep) {
+#pragma unroll
+            for (int x = 0; x < 64; ++x) s[x] = x < n_in ? 0.0f : -INFINITY;
+          } else if ((kb0 & kb1) != 0xffffffffu) {
+#pragma unroll
+            for (int x = 0; x < 32; ++x) {
+              if (!((kb0 >> x) & 1u)) s[x] = -INFINITY;
+              if (!((kb1 >> x) & 1u)) s[32 + x] = -INFINITY;
+            }
+          }
+          float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
+#pragma unroll
+          for (int x = 0; x < 64; x += 2) mx[(x >> 1) & 3] = max3(mx[(x >> 1) & 3], s[x], s[x + 1]);
           const float my_max = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));
           // the row maximum of the tile needs the other half of the keys: exchange through shared memory
           const uint32_t pair_phase = (c_t + c_i + 1u) & 1u;   // c_t - 1 tiles and c_i items before this exchange
-          float* xm = xmax + pair_phase * (2 * BM);
+          float* xm = xchg + pair_phase * (2 * BM);
           xm[hf * BM + r] = my_max;
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(pair2);
-          ptx::tmem_wait_st();
-          DFL_TMEM_LD32_F(t_s, nxt, 0);   // first chunk of pass 2, in flight during the exchange
           ok = wwait(pair2, pair_phase, 45);
           if (!ok) break;
           const float tile_max = fmaxf(my_max, xm[(1 - hf) * BM + r]);
@@ -604,32 +583,21 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
           const float neg_m = -(m_run == -INFINITY ? 0.0f : m_run) * cscale;
 
-          // ---- pass 2: P = exp2(biased score * scale - reference), rounded, to the P columns; row sum.
+          // P = exp2(score * scale - reference), rounded, to the P columns; row sum.
           // The row sum is taken over P as rounded for the tensor core, so that the weights P/l the output is
           // built from sum to one exactly.  (The reference sums the unrounded values, kernel.py:316-333; with the
           // lazy reference maximum the largest P of a row is not the exactly representable 1.0, and an unrounded
           // sum would leave the rounding error of the dominant key uncompensated.)
           float sum[4] = {0.0f, 0.0f, 0.0f, 0.0f};
-#pragma unroll 1
+#pragma unroll
           for (int q = 0; q < 2; ++q) {
-            ptx::tmem_wait_ld();
-#pragma unroll
-            for (int x = 0; x < 32; ++x) cur[x] = nxt[x];
-            if (q == 0) {
-              DFL_TMEM_LD32_F(t_s + 32, nxt, 0);
-            } else {
-              // the whole S half is in registers: the accumulator is free for the next tile's S
-              ptx::tc_fence_before();
-              __syncwarp();
-              if (lane == 0) ptx::mbar_arrive(&bars->s_free);
-            }
-#pragma unroll
-            for (int x = 0; x < 32; ++x) cur[x] = fmaf(cur[x], cscale, neg_m);
-#pragma unroll
-            for (int x = 0; x < 32; ++x) cur[x] = ptx::ex2_approx(cur[x]);
             uint32_t packed[16];
 #pragma unroll
-            for (int x = 0; x < 32; x += 2) packed[x / 2] = Pack2<T>::pack(cur[x], cur[x + 1]);
+            for (int x = 0; x < 32; ++x) s[32 * q + x] = fmaf(s[32 * q + x], cscale, neg_m);
+#pragma unroll
+            for (int x = 0; x < 32; ++x) s[32 * q + x] = ptx::ex2_approx(s[32 * q + x]);
+#pragma unroll
+            for (int x = 0; x < 32; x += 2) packed[x / 2] = Pack2<T>::pack(s[32 * q + x], s[32 * q + x + 1]);
 #pragma unroll
             for (int x = 0; x < 16; ++x) add_pair<T>(sum[(2 * x) & 3], sum[(2 * x + 1) & 3], packed[x]);
             // the P buffer is the A operand of the previous tile's PV until that MMA completes
@@ -653,13 +621,15 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         ok = wwait(&bars->o_ready, (c_t & 1u) ^ 1u, 48);   // the item's last PV: c_t - 1 completed before it
         if (!ok) break;
         ptx::tc_fence_after();
-        xsum[hf * BM + r] = l_run;
+        const uint32_t sum_phase = (c_t + c_i) & 1u;
+        float* xs = xchg + sum_phase * (2 * BM);
+        xs[hf * BM + r] = l_run;
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(pair2);
-        ok = wwait(pair2, (c_t + c_i) & 1u, 49);
+        ok = wwait(pair2, sum_phase, 49);
         ++c_i;
         if (!ok) break;
-        const float inv = 1.0f / (l_run + xsum[(1 - hf) * BM + r]);
+        const float inv = 1.0f / (l_run + xs[(1 - hf) * BM + r]);
         uint32_t o[OW];
         attn::tmem_ld_n(t_o, o);
         ptx::tmem_wait_ld();
@@ -686,97 +656,131 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   } else if (warp < kMmaWarp) {
     setmaxnreg_dec<kConvRegs>();
     // -------------------------------------------------------------- converters
-    // Thread (quarter q4, lane) owns TMEM lane 32*q4 + lane of both transit accumulators:
-    //   C2P blocks: query row r of the tile; the block's 128 columns are rounded and stored to ring row r.
-    //   P2C halves: key n of the tile.  Of the 256 table rows of the tile's window, the 128 queries reach rows
-    //     n+1 .. n+128; the chunk-aligned span [8*(n/8), 8*(n/8) + 136) is stored to staging row n.
-    // Jobs are taken in the order the MMA issuer produces them.
+    // Thread (quarter q4, lane) owns TMEM lane 32*q4 + lane of both transit accumulators and moves its row, rounded to T,
+    // to where the consumer reads it without a shift of its own:
+    //   C2P block c (lane = query row r): column m is the score of key x = m + r of tile c - 1 where that is below 128,
+    //     of key x - 128 of tile c otherwise (the block is the upper half of one tile's window and the lower half of the
+    //     next one's).  Consecutive m land at consecutive columns of the row buffer, modulo its two tiles.
+    //   P2C halves (lane = key n): table column w of the tile's 256 is the score of query row 128 + n - w; the row goes to
+    //     row n of the K-major B operand of the MMA that adds the tile to S.
+    // Both destinations are shifted by the lane, and a 4-byte store takes two neighbouring columns: a funnel shift pairs
+    // them from the packed words at hand for odd (C2P) or even (P2C) rows.
     const int q4 = warp & 3;
     const int row = q4 * 32 + lane;
-    const int c_first = row >> 3;   // first chunk of the staging span (chunks are 8 table rows = 16 bytes)
     const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
     const uint32_t t_xp = tmem_base + lane_base + COL_XP;
     const uint32_t t_xc = tmem_base + lane_base + COL_XC;
-    const uint32_t t_b1 = tmem_base + lane_base + COL_P;   // second block of an item: P and O columns
-    const uint32_t stg_row = ptx::smem_u32(smem + LO::offStg) + (uint32_t)(row * STG_PITCH) - (uint32_t)(c_first * 16);
-    const uint32_t ring_row = ptx::smem_u32(smem + LO::offRing) + (uint32_t)(row * RING_PITCH);
-    uint32_t c_xp = 0, c_xc = 0, c_b1 = 0, c_pt = 0;
+    // C2P: word k of a block (columns 2k, 2k+1; for odd rows 2k-1, 2k) goes to column 128 * tile + 2k + row_even
+    const int row_even = row & ~1;
+    const uint32_t row_addr = ptx::smem_u32(smem + LO::offRows) + (uint32_t)(row * ROW_PITCH + 2 * row_even);
+    const uint32_t c_shift = (row & 1) ? 16u : 32u;
+    uint32_t carry = 0;         // last packed word of the previous block of this row
+    // P2C: word k holds query rows 128 + row_even - 2k and + 1
+    const uint32_t p_shift = (row & 1) ? 0u : 16u;
+    uint32_t stg_addr[4];       // where word k = 0, 1, 2, 3 (mod 4) would go
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int qr = 128 + row_even - 2 * j;
+      stg_addr[j] = ptx::smem_u32(smem + LO::offStg) + (uint32_t)((qr >> 3) * STG_CHUNK + (row >> 3) * 128 + (row & 7) * 16 + (qr & 7) * 2);
+    }
+    uint32_t c_xp = 0, c_xc = 0, c_pt = 0;
     uint32_t rel_seen = 0;      // phases of ring_release (one per key tile) waited for so far
     uint32_t tiles_before = 0;  // key tiles of all earlier items
     bool ok = true;
 
-    // One C2P block: TMEM (two pieces of 64 columns) -> 16-bit -> ring block `pos` of this thread's row.  The ring
-    // position must be free: `need` key tiles in total must have been read by all softmax warps.
-    auto convert_block = [&](uint32_t t_src, uint64_t* full, uint32_t full_parity, bool frees_xc, int pos, uint32_t need) -> bool {
-      if (!wwait(full, full_parity, 18)) return false;
+    // One C2P block: upper part of running tile `upper`, lower part of tile upper + 1; the first block of an item has no
+    // upper part.  The two row buffers must be free: `need` key tiles in total must have been read.
+    auto convert_block = [&](bool first, uint32_t upper, uint32_t need) -> bool {
+      if (!wwait(&bars->xc_full, c_xc & 1u, 18)) return false;
+      ++c_xc;
       ptx::tc_fence_after();
+      uint32_t prev = carry;
+      uint32_t v[32];
+      ptx::tmem_ld32(t_xc, v);
+      while (rel_seen < need) {
+        if (!wwait(&bars->ring_release, rel_seen & 1u, 17)) return false;
+        ++rel_seen;
+      }
 #pragma unroll 1
-      for (int piece = 0; piece < 2; ++piece) {
-        uint32_t r0[32], r1[32];
-        ptx::tmem_ld32(t_src + piece * 64, r0);
-        ptx::tmem_ld32(t_src + piece * 64 + 32, r1);
+      for (int j = 0; j < 4; ++j) {   // 32 columns at a time, the next ones in flight while these are stored
         ptx::tmem_wait_ld();
-        if (piece == 1 && frees_xc) {   // the block is in registers: the accumulator is free for the next block's MMA
+        if (j == 3) {   // the block is in registers: the accumulator is free for the next block's MMA
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&bars->xc_free);
         }
-        if (piece == 0) {
-          while (rel_seen < need) {
-            if (!wwait(&bars->ring_release, rel_seen & 1u, 17)) return false;
-            ++rel_seen;
+        uint32_t w[16];
+#pragma unroll
+        for (int k = 0; k < 16; ++k) w[k] = pack_scores<T>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
+        if (j < 3) ptx::tmem_ld32(t_xc + 32 * (j + 1), v);
+        const uint32_t top = w[15];
+#pragma unroll
+        for (int k = 15; k > 0; --k) w[k] = funnel_clamp(w[k - 1], w[k], c_shift);
+        w[0] = funnel_clamp(prev, w[0], c_shift);
+        prev = top;
+        // column 2k + row_even below 128: tile `upper`; from 128 on: the next tile, whose buffer is the other half
+        const uint32_t up = row_addr + (upper & 1u) * 256u + 64u * j, down = row_addr + ((upper & 1u) ? 0u : 256u) - 256u + 64u * j;
+        const int turn = j + q4;   // columns of this warp and chunk: 32 * turn .. 32 * turn + 61
+        if (turn >= 4) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) sts_u32(down + 4 * k, w[k]);
+        } else if (turn == 3) {
+          const int last_up = 127 - 32 * j - row_even;   // 2k <= last_up: tile `upper`
+#pragma unroll
+          for (int k = 0; k < 16; ++k) {
+            const bool below = 2 * k <= last_up;
+            sts_u32_if((below ? up : down) + 4 * k, w[k], !(first && below));
           }
-        }
-        const uint32_t dst = ring_row + (uint32_t)(pos * 256 + piece * 128);
+        } else if (!first) {
 #pragma unroll
-        for (int x = 0; x < 32; x += 2) {
-          const uint32_t w = Pack2<T>::pack(__uint_as_float(r0[x]), __uint_as_float(r0[x + 1]));
-          sts_u32(dst + 2 * x, w);
-          if (x < RING_MIRROR && pos == 0 && piece == 0) sts_u32(dst + RING_COLS * 2 + 2 * x, w);
+          for (int k = 0; k < 16; ++k) sts_u32(up + 4 * k, w[k]);
         }
-#pragma unroll
-        for (int x = 0; x < 32; x += 2)
-          sts_u32(dst + 64 + 2 * x, Pack2<T>::pack(__uint_as_float(r1[x]), __uint_as_float(r1[x + 1])));
       }
+      carry = prev;
       return true;
     };
-    // One half (128 table rows) of a tile's P2C accumulator -> staging.  half 0 also waits for the staging tile.
+    // One half (128 table columns) of a tile's P2C accumulator.  A warp's 32 keys take words 16 * q4 + 1 .. 16 * q4 + 79 of
+    // the tile's 128: 32-column chunks q4 .. 3 of the first half and 0 .. q4 of the second.
+    uint32_t p_prev = 0;
     auto convert_half = [&](int half) -> bool {
       if (!wwait(&bars->xp_full, c_xp & 1u, 19)) return false;
+      ++c_xp;
       ptx::tc_fence_after();
-      // A warp's 32 keys reach chunks 4*q4 .. 4*q4 + 19 of the window's 32: quarters 2 and 3 never store anything of
-      // the first 64 columns of the first half, quarters 0 and 1 nothing of the last 64 of the second half.
-      const int p_begin = (half == 0 && q4 >= 2) ? 1 : 0;
-      const int p_end = (half == 1 && q4 <= 1) ? 1 : 2;
+      const int begin = half == 0 ? q4 : 0, end = half == 0 ? 4 : q4 + 1;
+      uint32_t v[32];
+      ptx::tmem_ld32(t_xp + 32 * begin, v);
+      if (half == 0 && !wwait(&bars->pt_release, (c_pt & 1u) ^ 1u, 20)) return false;   // the previous tile has been read
 #pragma unroll 1
-      for (int piece = p_begin; piece < p_end; ++piece) {
-        uint32_t r0[32], r1[32];
-        ptx::tmem_ld32(t_xp + piece * 64, r0);
-        ptx::tmem_ld32(t_xp + piece * 64 + 32, r1);
+      for (int j = begin; j < end; ++j) {
         ptx::tmem_wait_ld();
-        if (piece == p_end - 1) {   // what this warp needs of the half is in registers: its share of xp_free
+        if (j == end - 1) {   // what this warp needs of the half is in registers: its share of xp_free
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&bars->xp_free);
         }
-        if (half == 0 && piece == p_begin) {
-          // the staging tile must have been read by all softmax warps (previous tile)
-          if (!wwait(&bars->pt_release, (c_pt & 1u) ^ 1u, 20)) return false;
-        }
-        // 8 chunks of 8 table rows; chunk c of the window goes to position c - c_first if that is in [0, 16]
+        uint32_t w[16];
 #pragma unroll
-        for (int c = 0; c < 8; ++c) {
-          const uint32_t (&src)[32] = c < 4 ? r0 : r1;
-          const int x = (c & 3) * 8;
-          const uint32_t w0 = Pack2<T>::pack(__uint_as_float(src[x + 0]), __uint_as_float(src[x + 1]));
-          const uint32_t w1 = Pack2<T>::pack(__uint_as_float(src[x + 2]), __uint_as_float(src[x + 3]));
-          const uint32_t w2 = Pack2<T>::pack(__uint_as_float(src[x + 4]), __uint_as_float(src[x + 5]));
-          const uint32_t w3 = Pack2<T>::pack(__uint_as_float(src[x + 6]), __uint_as_float(src[x + 7]));
-          const int chunk = half * 16 + piece * 8 + c;
-          if (chunk >= c_first && chunk <= c_first + (STG_CHUNKS - 1)) sts_v4(stg_row + (uint32_t)(chunk * 16), w0, w1, w2, w3);
+        for (int k = 0; k < 16; ++k) w[k] = pack_scores<T>(__uint_as_float(v[2 * k + 1]), __uint_as_float(v[2 * k]));
+        if (j + 1 < end) ptx::tmem_ld32(t_xp + 32 * (j + 1), v);
+        const uint32_t top = w[15];
+#pragma unroll
+        for (int k = 15; k > 0; --k) w[k] = funnel_wrap(w[k], w[k - 1], p_shift);
+        w[0] = funnel_wrap(w[0], p_prev, p_shift);
+        p_prev = top;
+        const int chunk = half * 4 + j;                              // words 16 * chunk + k
+        const uint32_t down = (uint32_t)(chunk * 4 * STG_CHUNK);     // 32 columns are four chunks of eight query rows
+        const int turn = chunk - q4;
+        if (turn >= 1 && turn <= 3) {
+#pragma unroll
+          for (int k = 0; k < 16; ++k) sts_u32(stg_addr[k & 3] - down - (uint32_t)((k >> 2) * STG_CHUNK), w[k]);
+        } else {
+          // words 1 + row_even / 2 .. 64 + row_even / 2 are query rows of the tile
+          const int lo = 1 + row_even / 2 - 16 * chunk, hi = 64 + row_even / 2 - 16 * chunk;
+#pragma unroll
+          for (int k = 0; k < 16; ++k)
+            sts_u32_if(stg_addr[k & 3] - down - (uint32_t)((k >> 2) * STG_CHUNK), w[k], k >= lo && k <= hi);
         }
       }
-      ++c_xp;
       return true;
     };
 
@@ -788,39 +792,28 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       const ItemSlot* sl = &slots[slot];
       const int n = sl->t_end - sl->t_begin;
       if (sl->any_kept != 0) {
-        // Jobs of the item in production order: block 0 | P2C of tile 0 | block 1 | per further tile u: first half,
-        // block u + 1, second half.  One flat loop with one copy of each conversion routine: the converter's code
-        // shares the instruction cache with the softmax warps of its scheduler.
-        for (int u = 0; u < n && ok; ++u) {
-#pragma unroll 1
-          for (int jb = 0; jb < 4 && ok; ++jb) {
-            // kind: 0 nothing, 1 C2P block from the XC accumulator, 2 C2P block from the P/O columns, 3 P2C half
-            int kind, arg;
-            if (u == 0) {
-              kind = jb == 0 ? 1 : (jb == 3 ? 2 : 3);
-              arg = jb == 0 ? 0 : (jb == 3 ? 1 : jb - 1);          // ring position / half
-            } else {
-              kind = jb == 0 ? 0 : (jb == 2 ? 1 : 3);
-              arg = jb == 2 ? ((u + 1) & 1) : (jb == 1 ? 0 : 1);   // block u + 1 replaces block u - 1
-            }
-            if (kind == 3) {
-              if (has_p2c) ok = convert_half(arg);
-            } else if (kind != 0 && has_c2p) {
-              const bool from_xc = kind == 1;
-              ok = convert_block(from_xc ? t_xc : t_b1, from_xc ? &bars->xc_full : &bars->b1_full,
-                                 (from_xc ? c_xc : c_b1) & 1u, from_xc, arg, tiles_before + (uint32_t)u);
-              if (from_xc) ++c_xc; else ++c_b1;
+        if (warp >= kC2pWarp) {
+          // block 0, then per key tile u block u + 1
+          for (int u = -1; u < n && ok && has_c2p; ++u) {
+            const uint32_t upper = tiles_before + (uint32_t)u;
+            ok = convert_block(u < 0, upper, upper == 0xffffffffu ? 0u : upper);
+            if (ok && u >= 0) {
+              __syncwarp();
+              if (lane == 0) ptx::mbar_arrive(&bars->c2p_ready);
             }
           }
-          if (!ok) break;
-          __syncwarp();
-          if (lane == 0) {
-            if (has_c2p) ptx::mbar_arrive(&bars->c2p_ready);
-            if (has_p2c) ptx::mbar_arrive(&bars->pt_ready);
+        } else {
+          for (int u = 0; u < n && ok && has_p2c; ++u) {
+            ok = convert_half(0) && convert_half(1);
+            if (!ok) break;
+            ptx::fence_proxy_async_smem();   // the tile is read by the tensor core
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&bars->pt_ready);
+            ++c_pt;
           }
-          ++c_pt;
         }
-        if (has_c2p) tiles_before += (uint32_t)n;
+        if (!ok) break;
+        tiles_before += (uint32_t)n;
       }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
@@ -829,9 +822,10 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     setmaxnreg_dec<kMiscRegs>();
     if (warp == kTmaWarp) {
       // ------------------------------------------------- mask analysis + TMA producer
-      // Running counts of loads; stage = count % stages, phase = (count / stages) & 1.  Loads are issued in the
-      // order the MMA issuer consumes them (a stage that is still in use blocks only loads needed after its release).
-      struct LoadItem {
+      // One stream of loads in the order the MMAs consume them, each waiting for its stage; V runs one key tile behind, so
+      // that what the next scores need never waits for a PV.  Running counts: stage = count % stages, phase =
+      // (count / stages) & 1.
+      struct Item {
         int t_begin, n, i0, bh, h;
         bool any_kept;
       };
@@ -839,14 +833,14 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       bool ok = true;
 
       // Mask analysis of item number k2 (item it2), published through its slot.  Warp-collective.
-      auto analyze = [&](int k2, int it2, LoadItem& f) -> bool {
+      auto analyze = [&](int k2, int it2, Item& f) -> bool {
         const int slot = k2 % kItemSlots;
         const int qt = it2 / n_bh, bh = it2 - qt * n_bh, b = bh / H;
         const int i0 = qt * BM;
         ItemSlot* sl = &slots[slot];
         if (!wwait(&bars->item_empty[slot], ((uint32_t)(k2 / kItemSlots) & 1u) ^ 1u, 30)) return false;
-        const uint32_t kb_lo = kept_bits_word(p, b, lane);
-        const uint32_t kb_hi = L > 1024 ? kept_bits_word(p, b, lane + 32) : 0u;
+        uint32_t kb_lo, kb_hi;
+        kept_bits(p, b, lane, kb_lo, kb_hi);
         const TileRange range = tile_range(kb_lo, kb_hi, i0, L, lane);
         sl->kbits[lane] = kb_lo;
         sl->kbits[lane + 32] = kb_hi;
@@ -859,275 +853,200 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->item_full[slot]);
-        f.t_begin = range.t_begin;
-        f.n = range.t_end - range.t_begin;
-        f.i0 = i0;
-        f.bh = bh;
-        f.h = bh - b * H;
-        f.any_kept = range.any_kept;
+        f = {range.t_begin, range.t_end - range.t_begin, i0, bh, bh - b * H, range.any_kept};
         return true;
       };
-      // table row of column 0 of block 0: pair (row r, key x) of tile u uses column 128 - r + x of blocks u, u+1
-      auto table_row0 = [&](const LoadItem& f) { return f.t_begin * BK - f.i0 - BM + (L - 1); };
-      auto load_rk = [&](const LoadItem& f, int c) -> bool {
-        const uint32_t st = c_rk % LO::kRkStages, ph = (c_rk / LO::kRkStages) & 1u;
-        if (!ptx::mbar_wait_inline(&bars->rk_empty[st], ph ^ 1u, abort_flag, fail_code, 11)) return false;
-        ptx::mbar_arrive_expect_tx(&bars->rk_full[st], (uint32_t)LO::kTile);
-        ptx::tma_load_3d(smem + LO::offRK + st * LO::kTile, &tmap_fk, &bars->rk_full[st], 0, table_row0(f) + c * BK, f.h);
-        ++c_rk;
-        return true;
-      };
-      auto load_rq = [&](const LoadItem& f, int c) -> bool {
-        const uint32_t st = c_rq & 1u, ph = (c_rq >> 1) & 1u;
-        if (!ptx::mbar_wait_inline(&bars->rq_empty[st], ph ^ 1u, abort_flag, fail_code, 12)) return false;
-        ptx::mbar_arrive_expect_tx(&bars->rq_full[st], (uint32_t)LO::kTile);
-        ptx::tma_load_3d(smem + LO::offRQ + st * LO::kTile, &tmap_fq, &bars->rq_full[st], 0, table_row0(f) + c * BK, f.h);
-        ++c_rq;
-        return true;
-      };
-      auto load_k = [&](const LoadItem& f, int u) -> bool {
-        const uint32_t st = c_k & 1u, ph = (c_k >> 1) & 1u;
-        if (!ptx::mbar_wait_inline(&bars->k_empty[st], ph ^ 1u, abort_flag, fail_code, 1)) return false;
-        ptx::mbar_arrive_expect_tx(&bars->k_full[st], (uint32_t)LO::kTile);
-        ptx::tma_load_3d(smem + LO::offK + st * LO::kTile, &tmap_k, &bars->k_full[st], 0, (f.t_begin + u) * BK, f.bh);
-        ++c_k;
-        return true;
-      };
-      auto load_v = [&](const LoadItem& f, int u) -> bool {
-        const uint32_t st = c_v % LO::kVStages, ph = (c_v / LO::kVStages) & 1u;
-        if (!ptx::mbar_wait_inline(&bars->v_empty[st], ph ^ 1u, abort_flag, fail_code, 2)) return false;
-        ptx::mbar_arrive_expect_tx(&bars->v_full[st], (uint32_t)LO::kTile);
-        ptx::tma_load_3d(smem + LO::offV + st * LO::kTile, &tmap_v, &bars->v_full[st], 0, (f.t_begin + u) * BK, f.bh);
-        ++c_v;
-        return true;
-      };
-      // what the first MMAs of an item need: Q, first rel_key block, K of the first tile, first two rel_query blocks
-      auto prologue_loads = [&](const LoadItem& f) -> bool {
-        if (!ptx::mbar_wait_inline(&bars->q_empty, (c_q & 1u) ^ 1u, abort_flag, fail_code, 3)) return false;
-        ptx::mbar_arrive_expect_tx(&bars->q_full, (uint32_t)LO::kTile);
-        ptx::tma_load_3d(smem + LO::offQ, &tmap_q, &bars->q_full, 0, f.i0, f.bh);
-        ++c_q;
-        if (has_c2p && !load_rk(f, 0)) return false;
-        if (!load_k(f, 0)) return false;
-        if (has_p2c && !(load_rq(f, 0) && load_rq(f, 1))) return false;
-        return true;
+      // one 128-row tile into stage count % stages of the buffers at `offset`
+      auto load = [&](const CUtensorMap* map, int offset, uint64_t* full, uint64_t* empty, uint32_t& count, uint32_t stages, int row,
+                      int z, int code) {
+        const uint32_t st = stages == 1 ? 0u : count & 1u, ph = (stages == 1 ? count : count >> 1) & 1u;
+        ++count;
+        ok = ok && wwait(&empty[st], ph ^ 1u, code);
+        if (ok && lane == 0) {
+          ptx::mbar_arrive_expect_tx(&full[st], (uint32_t)LO::kTile);
+          ptx::tma_load_3d(smem + offset + st * LO::kTile, map, &full[st], 0, row, z);
+        }
+        __syncwarp();
       };
 
-      LoadItem cur{}, nxt{};
-      int it = blockIdx.x, k = 0;
-      if (it < n_items) {
-        ok = analyze(0, it, cur);
-        if (ok && cur.any_kept && lane == 0) ok = prologue_loads(cur);
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-      }
-      for (; it < n_items && ok; it += gridDim.x, ++k) {
+      Item cur{}, nxt{};
+      int k = 0, v_row = -1, v_bh = 0;   // the tile whose V is still to be loaded, if v_row >= 0
+      if ((int)blockIdx.x < n_items) ok = analyze(0, blockIdx.x, cur);
+#pragma unroll 1
+      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
         const bool has_next = n_items - it > (int)gridDim.x;
-        // what the item needs right at its start goes out before the next item's mask is analysed
-        if (cur.any_kept && lane == 0) {
-          if (has_c2p) ok = load_rk(cur, 1);
-          if (ok && cur.n > 1) {
-            ok = load_k(cur, 1);
-            if (ok && has_c2p) ok = load_rk(cur, 2);
-            if (ok && has_p2c) ok = load_rq(cur, 2);
+        // table row of column 0 of block 0: pair (row r, key x) of tile u uses column 128 - r + x of blocks u, u + 1
+        const int row0 = cur.t_begin * BK - cur.i0 - BM + (L - 1);
+        const int steps = cur.any_kept ? cur.n : 0;
+        // step -1 brings Q and the first table blocks, step u brings K(u) and the table blocks u + 1
+#pragma unroll 1
+        for (int u = -1; u < steps && ok; ++u) {
+          if (steps > 0) {
+            if (u < 0) load(&tmap_q, LO::offQ, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
+            else load(&tmap_k, LO::offK, bars->k_full, bars->k_empty, c_k, 2, (cur.t_begin + u) * BK, cur.bh, 1);
+            if (has_p2c) load(&tmap_fq, LO::offRQ, bars->rq_full, bars->rq_empty, c_rq, 2, row0 + (u + 1) * BK, cur.h, 12);
+            if (has_c2p) load(&tmap_fk, LO::offRK, bars->rk_full, bars->rk_empty, c_rk, LO::kRkStages, row0 + (u + 1) * BK, cur.h, 11);
           }
-        }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
-        if (ok && has_next) ok = analyze(k + 1, it + (int)gridDim.x, nxt);
-        if (!ok) break;
-        const bool next_kept = has_next && nxt.any_kept;
-        if (lane == 0) {
-          if (cur.any_kept) {
-            for (int u = 0; u < cur.n && ok; ++u) {
-              if (u + 1 < cur.n) {
-                if (u > 0) {
-                  ok = load_k(cur, u + 1);
-                  if (ok && has_c2p) ok = load_rk(cur, u + 2);
-                  if (ok && has_p2c) ok = load_rq(cur, u + 2);
-                }
-              } else if (next_kept) {
-                ok = prologue_loads(nxt);
-              }
-              if (ok) ok = load_v(cur, u);
-            }
-          } else if (next_kept) {
-            ok = prologue_loads(nxt);
+          if (v_row >= 0 && (u >= 0 || steps == 0)) {
+            load(&tmap_v, LO::offV, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
+            v_row = -1;
           }
+          if (u >= 0) {
+            v_row = (cur.t_begin + u) * BK;
+            v_bh = cur.bh;
+          }
+          // The next item is analysed once the loads its predecessor starts with are on their way.  Its slot is that of
+          // the item three before it, which is complete only if its last V has been loaded: the load above, whatever
+          // kind the items in between are.
+          if (ok && has_next && (u == 0 || steps == 0)) ok = analyze(k + 1, it + (int)gridDim.x, nxt);
         }
-        ok = __shfl_sync(0xffffffffu, ok ? 1 : 0, 0) != 0;
         cur = nxt;
       }
+      if (v_row >= 0) load(&tmap_v, LO::offV, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
     } else if (warp == kMmaWarp) {
       // -------------------------------------------------------------- MMA issuer
-      // One thread issues every MMA; descriptors are kept as precomputed 32-bit halves (only the start-address
-      // field moves).  Order per key tile u (steady state): the next tile's first P2C half, new C2P block and second
-      // P2C half while the softmax threads work on tile u, the next tile's S as soon as they have read S(u), then
-      // PV(u) as soon as P(u) is stored.  In the item's last tile the place of the next tile's MMAs is taken by the
-      // first MMAs of the next item.
-      if (lane == 0) {
-        constexpr int is_bf16 = __is_same(T, __nv_bfloat16) ? 1 : 0;
-        constexpr uint32_t idesc_nn = ptx::make_idesc_f16(is_bf16, BM, 128, 0, 0);   // 128 x 128, both K-major
-        constexpr uint32_t idesc_pv = ptx::make_idesc_f16(is_bf16, BM, D, 0, 1);     // 128 x D, V is MN-major
-        constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
-        constexpr uint32_t sbo = 8 * LO::kRowBytes;
-        constexpr int kSteps = LO::kRowBytes / 32;   // K=16 steps over d
-        // shared-memory descriptor = {lo, hi}: lo = start>>4 | (leading offset>>4) << 16, hi = stride offset>>4 |
-        // version 1 << 14 | swizzle << 29; every operand here shares hi
-        constexpr uint32_t desc_hi = ((sbo >> 4) & 0x3FFFu) | (1u << 14) | (mode << 29);
-        constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4;
-        constexpr uint32_t kPvStepUnits = (16u * LO::kRowBytes) >> 4;   // 16 keys further down the V tile
-        auto desc_lo = [](uint32_t addr, uint32_t lbo) { return ((addr >> 4) & 0x3FFFu) | ((lbo >> 4) << 16); };
-        const uint32_t q_lo = desc_lo(ptx::smem_u32(smem + LO::offQ), 16);
-        const uint32_t k_lo = desc_lo(ptx::smem_u32(smem + LO::offK), 16);
-        const uint32_t rk_lo = desc_lo(ptx::smem_u32(smem + LO::offRK), 16);
-        const uint32_t rq_lo = desc_lo(ptx::smem_u32(smem + LO::offRQ), 16);
-        const uint32_t v_lo = ((ptx::smem_u32(smem + LO::offV) >> 4) & 0x3FFFu) | (kTileUnits << 16);
-        uint32_t c_q = 0, c_k = 0, c_v = 0, c_rk = 0;   // loads consumed (stage / phase as in the loader)
-        uint32_t c_s = 0, c_xc = 0, c_xp = 0, c_p = 0;  // S tiles, C2P blocks through XC, P2C halves, PVs issued
-        uint32_t rq_alloc = 0;                          // rel_query blocks handed to items so far
-        uint32_t c_items = 0;                           // items with kept rows started so far
-        bool ok = true;
+      // MMAs that produce scores.  The whole warp walks the items, one elected lane issues (umma_ss_f16_warp); descriptors
+      // are precomputed and only their start-address field moves.  Per key tile: first P2C half, C2P block of the tile
+      // after it, second P2C half, then S as soon as the softmax threads have read the previous tile's S, and the P2C
+      // tile on top of it as soon as the converters have finished it.  This warp never waits for P (the PV MMAs have an
+      // issuer of their own), so the relative terms of the next tiles are produced while the softmax is at work.
+      constexpr int is_bf16 = __is_same(T, __nv_bfloat16) ? 1 : 0;
+      constexpr uint32_t idesc_nn = ptx::make_idesc_f16(is_bf16, BM, 128, 0, 0);   // 128 x 128, both K-major
+      constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
+      constexpr uint32_t sbo = 8 * LO::kRowBytes;
+      constexpr int kSteps = LO::kRowBytes / 32;   // K=16 steps over d
+      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4;
+      const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offQ), 16, sbo, mode);
+      const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, sbo, mode);
+      const uint64_t rk_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRK), 16, sbo, mode);
+      const uint64_t rq_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRQ), 16, sbo, mode);
+      const uint64_t eye_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offEye) + (EYE_ROWS - BM) * 16, EYE_CHUNK, 128, 0);
+      const uint64_t stg_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offStg), STG_CHUNK, 128, 0);
+      uint32_t c_q = 0, c_k = 0, c_rk = 0;            // loads consumed (stage / phase as in the loader)
+      uint32_t c_s = 0, c_xc = 0, c_xp = 0;           // S tiles, C2P blocks, P2C halves issued
+      uint32_t rq_alloc = 0;                          // rel_query blocks handed to items so far
+      bool ok = true;
 
-        // D[128 x 128] = A[128 x d] * B[128 x d]^T, both operands K-major tiles in shared memory
-        auto mma_nn = [&](uint32_t d_tmem, uint32_t a_lo, uint32_t b_lo) {
-#pragma unroll
-          for (int kk = 0; kk < kSteps; ++kk) {
-            if (kk == 0) umma_ss_lohi<0>(d_tmem, a_lo, b_lo, desc_hi, idesc_nn);
-            else umma_ss_lohi<1>(d_tmem, a_lo + 2u * kk, b_lo + 2u * kk, desc_hi, idesc_nn);
-          }
-        };
-        auto wait1 = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
-          return ptx::mbar_wait_inline(bar, parity, abort_flag, fail_code, code);
-        };
-        // new C2P block = Q . rel_key block^T, into the block accumulator, or (second block of an item) into the
-        // P and O columns, which the caller has made sure are idle
-        auto issue_c = [&](bool second_block) -> bool {
-          const uint32_t st = c_rk % LO::kRkStages, ph = (c_rk / LO::kRkStages) & 1u;
-          if (!wait1(&bars->rk_full[st], ph, 13)) return false;
-          if (!second_block && !wait1(&bars->xc_free, (c_xc & 1u) ^ 1u, 14)) return false;
+      // D[128 x 128] = A[128 x d] * B[128 x d]^T, both operands K-major tiles in shared memory
+      auto mma_nn = [&](uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc) {
+#pragma unroll 1
+        for (int kk = 0; kk < kSteps; ++kk)
+          ptx::umma_ss_f16_warp(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc_nn, kk != 0 ? 1u : 0u);
+      };
+      // new C2P block = Q . rel_key block^T
+      auto issue_c = [&]() -> bool {
+        const uint32_t st = c_rk % LO::kRkStages, ph = (c_rk / LO::kRkStages) & 1u;
+        if (!wwait(&bars->rk_full[st], ph, 13)) return false;
+        if (!wwait(&bars->xc_free, (c_xc & 1u) ^ 1u, 14)) return false;
+        ptx::tc_fence_after();
+        mma_nn(tmem_base + COL_XC, q_desc, rk_desc + st * kTileUnits);
+        ptx::umma_commit_warp(&bars->rk_empty[st]);
+        ptx::umma_commit_warp(&bars->xc_full);
+        ++c_rk;
+        ++c_xc;
+        return true;
+      };
+      // S = Q . K^T of the tile whose K is in stage kst, plus I . (P2C tile)^T
+      auto issue_s = [&](uint32_t kst) -> bool {
+        if (!wwait(&bars->s_free, (c_s & 1u) ^ 1u, 6)) return false;
+        ptx::tc_fence_after();
+        mma_nn(tmem_base + COL_S, q_desc, k_desc + kst * kTileUnits);
+        if (has_p2c) {
+          if (!wwait(&bars->pt_ready, c_s & 1u, 9)) return false;
           ptx::tc_fence_after();
-          mma_nn(tmem_base + (second_block ? COL_P : COL_XC), q_lo, rk_lo + st * kTileUnits);
-          ptx::umma_commit(&bars->rk_empty[st]);
-          ptx::umma_commit(second_block ? &bars->b1_full : &bars->xc_full);
-          ++c_rk;
-          if (!second_block) ++c_xc;
-          return true;
-        };
-        // S = Q . K^T of the tile whose K is in stage kst
-        auto issue_s = [&](uint32_t kst) -> bool {
-          if (!wait1(&bars->s_free, (c_s & 1u) ^ 1u, 6)) return false;
-          ptx::tc_fence_after();
-          mma_nn(tmem_base + COL_S, q_lo, k_lo + kst * kTileUnits);
-          ptx::umma_commit(&bars->s_full);
-          ++c_s;
-          return true;
-        };
-        // one half of the P2C accumulator: XP[n, m] = K . rel_query block^T; `first` = first use of the table block
-        // (wait for its load), `last` = last use (release its stage)
-        auto issue_pt = [&](uint32_t kst, uint32_t blk, bool first, bool last) -> bool {
-          const uint32_t st = blk & 1u, ph = (blk >> 1) & 1u;
-          if (first && !wait1(&bars->rq_full[st], ph, 15)) return false;
-          if (!wait1(&bars->xp_free, (c_xp & 1u) ^ 1u, 16)) return false;
-          ptx::tc_fence_after();
-          mma_nn(tmem_base + COL_XP, k_lo + kst * kTileUnits, rq_lo + st * kTileUnits);
-          if (last) ptx::umma_commit(&bars->rq_empty[st]);
-          ptx::umma_commit(&bars->xp_full);
-          ++c_xp;
-          return true;
-        };
-        // The first MMAs of an item with n key tiles: first C2P block, both P2C halves of tile 0, S(0).  rq0 receives
-        // the number of the item's first rel_query block (tile u uses blocks rq0 + u and rq0 + u + 1).
-        auto item_head = [&](int n, uint32_t& rq0) -> bool {
-          if (!wait1(&bars->q_full, c_q & 1u, 4)) return false;
-          ++c_q;
-          if (has_c2p && !issue_c(false)) return false;
+#pragma unroll 1
+          for (int kk = 0; kk < BM / 16; ++kk)
+            ptx::umma_ss_f16_warp(tmem_base + COL_S, eye_desc - (uint64_t)(16 * kk), stg_desc + (uint64_t)(2 * kk * (STG_CHUNK >> 4)),
+                                  idesc_nn, 1u);
+          ptx::umma_commit_warp(&bars->pt_release);
+        }
+        ptx::umma_commit_warp(&bars->s_full);
+        ++c_s;
+        return true;
+      };
+      // one half of the P2C accumulator: XP[n, w] = K . rel_query block^T; `first` = first use of the table block
+      // (wait for its load), `last` = last use (release its stage)
+      auto issue_pt = [&](uint32_t kst, uint32_t blk, bool first, bool last) -> bool {
+        const uint32_t st = blk & 1u, ph = (blk >> 1) & 1u;
+        if (first && !wwait(&bars->rq_full[st], ph, 15)) return false;
+        if (!wwait(&bars->xp_free, (c_xp & 1u) ^ 1u, 16)) return false;
+        ptx::tc_fence_after();
+        mma_nn(tmem_base + COL_XP, k_desc + kst * kTileUnits, rq_desc + st * kTileUnits);
+        if (last) ptx::umma_commit_warp(&bars->rq_empty[st]);
+        ptx::umma_commit_warp(&bars->xp_full);
+        ++c_xp;
+        return true;
+      };
+      int k = 0;
+      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
+        const int slot = k % kItemSlots;
+        ok = wwait(&bars->item_full[slot], (uint32_t)(k / kItemSlots) & 1u, 31);
+        if (!ok) break;
+        const bool any_kept = slots[slot].any_kept != 0;
+        const int n = slots[slot].t_end - slots[slot].t_begin;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
+        if (!any_kept) continue;
+        ok = wwait(&bars->q_full, c_q & 1u, 4);
+        ++c_q;
+        // step -1: C2P block 0; step u: key tile u (C2P blocks u and u + 1, rel_query blocks rq_alloc + u and + 1)
+#pragma unroll 1
+        for (int u = -1; u < n && ok; ++u) {
           const uint32_t kst = c_k & 1u;
-          if (!wait1(&bars->k_full[kst], (c_k >> 1) & 1u, 5)) return false;
-          rq0 = rq_alloc;
-          if (has_p2c) {
-            if (!(issue_pt(kst, rq0, true, true) && issue_pt(kst, rq0 + 1u, true, n == 1))) return false;
-            rq_alloc += (uint32_t)n + 1u;
+          if (u >= 0) ok = wwait(&bars->k_full[kst], (c_k >> 1) & 1u, 5);
+#pragma unroll 1
+          for (int half = 0; half < 2 && ok; ++half) {
+            if (u >= 0 && has_p2c)
+              ok = issue_pt(kst, rq_alloc + (uint32_t)(u + half), half == 1 || u == 0, half == 0 || u + 1 == n);
+            if (ok && half == 0 && has_c2p) ok = issue_c();
           }
-          if (!issue_s(kst)) return false;
-          ptx::umma_commit(&bars->k_empty[kst]);
+          if (u < 0 || !ok) continue;
+          ok = issue_s(kst);
+          if (!ok) break;
+          ptx::umma_commit_warp(&bars->k_empty[kst]);
           ++c_k;
-          return true;
-        };
-        struct ItemInfo {
-          bool any_kept;
-          int n;
-        };
-        auto get_item = [&](int k2, ItemInfo& f) -> bool {
-          const int slot = k2 % kItemSlots;
-          if (!wait1(&bars->item_full[slot], (uint32_t)(k2 / kItemSlots) & 1u, 31)) return false;
-          f.any_kept = slots[slot].any_kept != 0;
-          f.n = slots[slot].t_end - slots[slot].t_begin;
-          return true;
-        };
-
-        ItemInfo cur{false, 0}, nxt{false, 0};
-        uint32_t cur_rq = 0, nxt_rq = 0;
-        int it = blockIdx.x, k = 0;
-        if (it < n_items) {
-          ok = get_item(0, cur);
-          if (ok && cur.any_kept) ok = item_head(cur.n, cur_rq);
         }
-        for (; it < n_items && ok; it += gridDim.x, ++k) {
-          const bool has_next = n_items - it > (int)gridDim.x;
-          // The output accumulator of the previous item with kept rows has been read out (o_free completes one phase per
-          // such item; this thread is never more than one phase behind, so parities cannot alias).
-          if (cur.any_kept) {
-            if (c_items > 0) ok = wait1(&bars->o_free, (c_items - 1u) & 1u, 38);
-            ++c_items;
-          }
+        if (!ok) break;
+        rq_alloc += (uint32_t)n + 1u;
+        ptx::umma_commit_warp(&bars->q_empty);
+      }
+    } else if (warp == kPvWarp) {
+      // ----------------------------------------------------------- O (+)= P . V of every key tile, as soon as P is stored
+      constexpr uint32_t idesc_pv = ptx::make_idesc_f16(__is_same(T, __nv_bfloat16) ? 1 : 0, BM, D, 0, 1);   // V is MN-major
+      constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
+      constexpr uint32_t kPvStepUnits = (16u * LO::kRowBytes) >> 4;   // 16 keys further down the V tile
+      const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offV), LO::kTile, 8 * LO::kRowBytes, mode);
+      uint32_t c_v = 0, c_items = 0;   // tiles, and items with kept rows, so far
+      bool ok = true;
+      int k = 0;
+      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
+        const int slot = k % kItemSlots;
+        ok = wwait(&bars->item_full[slot], (uint32_t)(k / kItemSlots) & 1u, 39);
+        if (!ok) break;
+        const bool any_kept = slots[slot].any_kept != 0;
+        const int n = slots[slot].t_end - slots[slot].t_begin;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
+        if (!any_kept) continue;
+        for (int u = 0; u < n; ++u) {
+          const uint32_t vst = c_v % LO::kVStages, vph = (c_v / LO::kVStages) & 1u;
+          ok = wwait(&bars->v_full[vst], vph, 8);
+          // The output accumulator of the previous item with kept rows has been read out (o_free completes one phase
+          // per such item; this warp is never more than one phase behind, so parities cannot alias).
+          if (ok && u == 0 && c_items > 0) ok = wwait(&bars->o_free, (c_items - 1u) & 1u, 38);
+          if (ok) ok = wwait(&bars->p_full, c_v & 1u, 7);
           if (!ok) break;
-          if (cur.any_kept) {
-            const int n = cur.n;
-            if (has_c2p) ok = issue_c(true);
-            if (ok && n == 1) ptx::umma_commit(&bars->q_empty);
-            for (int u = 0; u < n && ok; ++u) {
-              if (u + 1 < n) {
-                // ---- front of tile u + 1
-                const uint32_t kst = c_k & 1u;
-                ok = wait1(&bars->k_full[kst], (c_k >> 1) & 1u, 5);
-                if (ok && has_p2c) ok = issue_pt(kst, cur_rq + (uint32_t)(u + 1), false, true);
-                if (ok && has_c2p) ok = issue_c(false);
-                if (ok && has_p2c) ok = issue_pt(kst, cur_rq + (uint32_t)(u + 2), true, u + 2 == n);
-                if (ok) ok = issue_s(kst);   // waits until the softmax threads have read the current tile's S
-                if (!ok) break;
-                ptx::umma_commit(&bars->k_empty[kst]);
-                ++c_k;
-                if (u + 2 == n) ptx::umma_commit(&bars->q_empty);   // S(n-1) and the last C2P block are issued
-              } else if (has_next) {
-                // The next item's slot is read only now: the loader publishes it after loads whose stages this
-                // thread's earlier MMAs of the current item release.
-                ok = get_item(k + 1, nxt);
-                if (ok && nxt.any_kept) ok = item_head(nxt.n, nxt_rq);
-                if (!ok) break;
-              }
-              // ---- PV(u): O (+)= P . V
-              const uint32_t vst = c_v % LO::kVStages, vph = (c_v / LO::kVStages) & 1u;
-              ok = wait1(&bars->p_full, c_p & 1u, 7) && wait1(&bars->v_full[vst], vph, 8);
-              if (!ok) break;
-              ptx::tc_fence_after();
-              const uint32_t vt_lo = v_lo + vst * kTileUnits;
-#pragma unroll
-              for (int kk = 0; kk < BK / 16; ++kk)
-                umma_ts_lohi(tmem_base + COL_O, tmem_base + COL_P + kk * 8, vt_lo + kk * kPvStepUnits, desc_hi, idesc_pv,
-                             (u > 0 || kk > 0) ? 1u : 0u);
-              ptx::umma_commit(&bars->v_empty[vst]);
-              ptx::umma_commit(&bars->o_ready);
-              ++c_v;
-              ++c_p;
-            }
-          } else if (has_next) {
-            ok = get_item(k + 1, nxt);
-            if (ok && nxt.any_kept) ok = item_head(nxt.n, nxt_rq);
-          }
-          if (!ok) break;
-          ptx::mbar_arrive(&bars->item_empty[k % kItemSlots]);
-          cur = nxt;
-          cur_rq = nxt_rq;
+          ptx::tc_fence_after();
+          const uint64_t vt_desc = v_desc + vst * (uint32_t)(LO::kTile >> 4);
+#pragma unroll 1
+          for (int kk = 0; kk < BK / 16; ++kk)
+            ptx::umma_ts_f16_warp(tmem_base + COL_O, tmem_base + COL_P + kk * 8, vt_desc + kk * kPvStepUnits, idesc_pv,
+                                  (u > 0 || kk > 0) ? 1u : 0u);
+          ptx::umma_commit_warp(&bars->v_empty[vst]);
+          ptx::umma_commit_warp(&bars->o_ready);
+          ++c_v;
         }
+        ++c_items;
       }
     }
   }

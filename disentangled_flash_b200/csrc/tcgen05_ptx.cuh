@@ -91,32 +91,29 @@ __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, volati
   return mbar_wait_slow(bar, parity, abort_flag, gstatus, code);
 }
 
-// Fully inlined bounded wait, for kernels that change their register budget with setmaxnreg (such kernels
-// cannot contain calls to separately compiled device functions).  It is inlined at every wait of those kernels, and
-// they are sensitive to instruction-cache footprint, so it is kept small: the clock (low 32 bits of the nanosecond
-// timer, enough for a limit of two seconds) and the CTA's abort flag are looked at once per 64 failed polls (each of
-// which may park the thread for a couple of microseconds), and
-// the code of the wait that gave up is left in a register of the caller instead of being written from here.
-__device__ __forceinline__ uint32_t globaltimer_lo() {
-  uint32_t t;
-  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
-  return t;
-}
-__device__ __forceinline__ bool mbar_wait_inline(uint64_t* bar, uint32_t parity, volatile int* abort_flag, int& fail_code,
-                                                 int code, uint32_t limit_ns = (uint32_t)kWaitLimitNs) {
-  if (mbar_try_wait(bar, parity)) return true;
-  const uint32_t t0 = globaltimer_lo();
-  uint32_t spins = 0;
-  while (!mbar_try_wait_hint(bar, parity, 2000u)) {
-    if ((++spins & 63u) != 0) continue;
-    if (*abort_flag) return false;   // another wait of the CTA gave up
-    if (globaltimer_lo() - t0 > limit_ns) {
-      *abort_flag = 1;     // every other wait of the CTA gives up at its next look
-      fail_code = code;    // reported by the caller once, when it leaves its role
+// Fully inlined bounded wait of a whole converged warp, for kernels that change their register budget with setmaxnreg (such
+// kernels cannot contain calls to separately compiled device functions).  It is inlined at every wait of those kernels,
+// which are bound by instruction fetch once their code outgrows the instruction caches, so it is as small as it can be: a
+// counted loop of polls, each of which may park the warp for up to two microseconds (it resumes at once when the phase
+// completes).  kWaitPolls of them last between a few hundredths of a second and two seconds; the code of the wait that
+// gave up is left in a register of the caller, whose role then ends.  The verdict is the same in every lane.
+constexpr uint32_t kWaitPolls = 1u << 20;
+__device__ __forceinline__ bool mbar_wait_warp(uint64_t* bar, uint32_t parity, int& fail_code, int code) {
+  uint32_t polls = kWaitPolls;
+#pragma unroll 1
+  while (!__all_sync(0xffffffffu, mbar_try_wait_hint(bar, parity, 2000u))) {
+    if (--polls == 0) {
+      fail_code = code;
       return false;
     }
   }
   return true;
+}
+
+__device__ __forceinline__ uint32_t globaltimer_lo() {
+  uint32_t t;
+  asm volatile("mov.u32 %0, %%globaltimer_lo;" : "=r"(t));
+  return t;
 }
 
 // generic-proxy writes to shared memory -> visible to the async proxy (TMA / tcgen05)
