@@ -12,8 +12,8 @@
 //       key tile is two 128-column blocks; the next key tile needs one new block.  Converter warps round a block's rows and
 //       store each shifted by its row, so that key x of the tile ends up in column x: a softmax thread adds its 64 scores
 //       from eight 16-byte loads.
-//   P2C is new for every key tile: D[n, m] = k_n . rel_query[x_lo + m] with TMEM lanes = keys n, computed in two
-//       halves of 128 table rows through one 128-column accumulator.  Here the diagonal runs across the lanes' columns and
+//   P2C is new for every key tile: D[n, m] = k_n . rel_query[x_lo + m] with TMEM lanes = keys n, computed in four
+//       parts of 64 table rows through two 64-column accumulators.  Here the diagonal runs across the lanes' columns and
 //       the softmax threads need it transposed: converter warps round each key's row and store it, shifted by its key, as
 //       row n of a K-major B operand, and S gets it by one more MMA, S += I . tile^T with an identity matrix as A.  The
 //       tensor pipe is idle three quarters of the time otherwise; it transposes and adds exactly (one product by 1.0 and
@@ -24,10 +24,10 @@
 //   warps 0-7   softmax: two threads per query row (warps w and w+4 own the same TMEM lanes; each takes 64 of the
 //               128 keys of a tile, 32 of the 64 packed P columns and half of the output columns).  One pass: the 64
 //               scores stay in registers from the S load to the P store.
-//   warps 8-11  converters of the P2C halves (TMEM -> 16-bit -> shared memory), warps 12-15 of the C2P blocks
-//   warp 16     issuer of the score MMAs (C2P block, P2C halves, S with the P2C tile added) and TMEM owner
+//   warps 8-11  converters of the P2C parts (TMEM -> 16-bit -> shared memory), warps 12-15 of the C2P blocks
+//   warp 16     issuer of the C2P block MMAs and of S with the P2C tile added, and TMEM owner
 //   warp 17     per-item mask analysis (kept-key bits, skipped key tiles), one item ahead, and TMA producer
-//   warp 18     issuer of the PV MMAs; warp 19 is idle (it completes the fifth warpgroup)
+//   warp 18     issuer of the PV MMAs, warp 19 of the P2C parts
 // What bounds it: instruction issue and fetch.  With everything unrolled (156 KB of code) a third of the issue slots were
 // lost to instruction fetch; the waits, the loader and the MMA loops are therefore rolled (88 KB), which was worth 17 %.
 // 32 x 12 heads x 512 x d 64, fp16, both terms: 185 -> 173 us, C2P only 145 -> 117 us against two passes over the keys with
@@ -47,10 +47,11 @@ using attn::Pack2;
 constexpr int BM = 128;              // query rows per item (= TMEM lanes)
 constexpr int BK = 128;              // keys per tile
 constexpr int kSoftmaxWarps = 8;
-constexpr int kC2pWarp = 12;         // warps 8-11 convert the P2C halves, 12-15 the C2P blocks
+constexpr int kC2pWarp = 12;         // warps 8-11 convert the P2C parts, 12-15 the C2P blocks
 constexpr int kMmaWarp = 16;
 constexpr int kTmaWarp = 17;
 constexpr int kPvWarp = 18;
+constexpr int kPartWarp = 19;
 constexpr int kThreads = 640;
 constexpr int kSoftmaxRegs = 128;    // 256 x 128 + 256 x 80 + 128 x 64 = 61440 registers
 constexpr int kConvRegs = 80;
@@ -64,7 +65,7 @@ static_assert(8 * 32 * kSoftmaxRegs + 8 * 32 * kConvRegs + 4 * 32 * kMiscRegs <=
 static_assert(kSoftmaxRegs >= kLaunchRegs && kConvRegs <= kLaunchRegs && kMiscRegs <= kLaunchRegs &&
                   kSoftmaxRegs % 8 == 0 && kConvRegs % 8 == 0 && kMiscRegs % 8 == 0,
               "setmaxnreg.inc raises and setmaxnreg.dec lowers the launch allocation, in multiples of 8");
-constexpr int kConsumerWarps = 18;   // softmax, converters, both MMA issuers: every warp that reads an item slot
+constexpr int kConsumerWarps = 19;   // softmax, converters, MMA issuers: every warp that reads an item slot
 
 constexpr int kItemSlots = 3;        // the loader analyses one item ahead of the one whose tiles it loads
 constexpr int kMaxSeqLen = 2048;
@@ -90,7 +91,7 @@ constexpr int COL_S = 0;      // 128  S = Q K^T of the current tile (fp32)
 constexpr int COL_P = 128;    // 64   P of the current tile (16-bit pairs), A operand of the PV MMA
 constexpr int COL_O = 192;    // 64   O accumulator (first D columns used)
 constexpr int COL_XC = 256;   // 128  one new C2P block for the 128 query rows
-constexpr int COL_XP = 384;   // 128  one half (128 table rows) of the P2C accumulator of a key tile
+constexpr int COL_XP = 384;   // 2 x 64  two of the four parts (64 table rows each) of the P2C accumulator of a key tile
 constexpr int kTmemCols = 512;
 
 template <int D>
@@ -136,7 +137,7 @@ struct RBarriers {
   uint64_t rk_full[2], rk_empty[2], rq_full[2], rq_empty[2];
   uint64_t s_full, s_free;          // S accumulator: MMA -> softmax, softmax (8 warps) -> MMA
   uint64_t xc_full, xc_free;        // C2P block accumulator: MMA -> converters (4 warps) -> MMA
-  uint64_t xp_full, xp_free;        // P2C half accumulator: MMA -> converters (4 warps) -> MMA
+  uint64_t xp_full[2], xp_free[2];  // P2C part accumulators: MMA -> converters (4 warps) -> MMA
   uint64_t pt_ready, pt_release;    // P2C tile in shared memory: converters -> MMA (its reads complete) -> converters
   uint64_t p_full, o_ready, o_free; // P stored (8 warps); PV complete; output accumulator read out (8 warps)
   uint64_t c2p_ready, ring_release; // C2P rows of a tile: converters -> softmax -> converters
@@ -305,7 +306,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     ptx::mbar_init(&bars->q_empty, 1);
     for (int s = 0; s < 2; ++s) {
       ptx::mbar_init(&bars->k_full[s], 1);
-      ptx::mbar_init(&bars->k_empty[s], 1);
+      ptx::mbar_init(&bars->k_empty[s], has_p2c ? 2 : 1);   // its issuers: Q K^T, and P2C parts
       ptx::mbar_init(&bars->v_full[s], 1);
       ptx::mbar_init(&bars->v_empty[s], 1);
       ptx::mbar_init(&bars->rk_full[s], 1);
@@ -321,8 +322,10 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     ptx::mbar_init(&bars->s_free, kSoftmaxWarps);   // one elected lane per softmax warp
     ptx::mbar_init(&bars->xc_full, 1);
     ptx::mbar_init(&bars->xc_free, 4);              // converter warps
-    ptx::mbar_init(&bars->xp_full, 1);
-    ptx::mbar_init(&bars->xp_free, 4);              // converter warps
+    for (int s = 0; s < 2; ++s) {
+      ptx::mbar_init(&bars->xp_full[s], 1);
+      ptx::mbar_init(&bars->xp_free[s], 4);         // converter warps
+    }
     ptx::mbar_init(&bars->pt_ready, 4);
     ptx::mbar_init(&bars->pt_release, 1);
     ptx::mbar_init(&bars->p_full, kSoftmaxWarps);
@@ -661,7 +664,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     //   C2P block c (lane = query row r): column m is the score of key x = m + r of tile c - 1 where that is below 128,
     //     of key x - 128 of tile c otherwise (the block is the upper half of one tile's window and the lower half of the
     //     next one's).  Consecutive m land at consecutive columns of the row buffer, modulo its two tiles.
-    //   P2C halves (lane = key n): table column w of the tile's 256 is the score of query row 128 + n - w; the row goes to
+    //   P2C parts (lane = key n): table column w of the tile's 256 is the score of query row 128 + n - w; the row goes to
     //     row n of the K-major B operand of the MMA that adds the tile to S.
     // Both destinations are shifted by the lane, and a 4-byte store takes two neighbouring columns: a funnel shift pairs
     // them from the packed words at hand for odd (C2P) or even (P2C) rows.
@@ -739,43 +742,48 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       carry = prev;
       return true;
     };
-    // One half (128 table columns) of a tile's P2C accumulator.  A warp's 32 keys take words 16 * q4 + 1 .. 16 * q4 + 79 of
-    // the tile's 128: 32-column chunks q4 .. 3 of the first half and 0 .. q4 of the second.
+    // One part (64 table columns) of a tile's P2C accumulator.  A warp's 32 keys take words 16 * q4 + 1 .. 16 * q4 + 79 of
+    // the tile's 128: 32-column chunks q4 .. q4 + 4 of the eight, two chunks per part.
     uint32_t p_prev = 0;
-    auto convert_half = [&](int half) -> bool {
-      if (!wwait(&bars->xp_full, c_xp & 1u, 19)) return false;
+    auto convert_part = [&](int part) -> bool {
+      const int buf = part & 1;
+      if (!wwait(&bars->xp_full[buf], (c_xp >> 1) & 1u, 19)) return false;
       ++c_xp;
       ptx::tc_fence_after();
-      const int begin = half == 0 ? q4 : 0, end = half == 0 ? 4 : q4 + 1;
+      const int begin = max(q4, 2 * part), end = min(q4 + 5, 2 * part + 2);
+      if (begin >= end) {   // nothing for this warp's keys: its share of xp_free
+        if (lane == 0) ptx::mbar_arrive(&bars->xp_free[buf]);
+        return true;
+      }
+      const uint32_t t_part = t_xp + 64 * buf - 64 * part;
       uint32_t v[32];
-      ptx::tmem_ld32(t_xp + 32 * begin, v);
-      if (half == 0 && !wwait(&bars->pt_release, (c_pt & 1u) ^ 1u, 20)) return false;   // the previous tile has been read
+      ptx::tmem_ld32(t_part + 32 * begin, v);
+      if (begin == q4 && !wwait(&bars->pt_release, (c_pt & 1u) ^ 1u, 20)) return false;   // the previous tile has been read
 #pragma unroll 1
       for (int j = begin; j < end; ++j) {
         ptx::tmem_wait_ld();
-        if (j == end - 1) {   // what this warp needs of the half is in registers: its share of xp_free
+        if (j == end - 1) {   // what this warp needs of the part is in registers
           ptx::tc_fence_before();
           __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&bars->xp_free);
+          if (lane == 0) ptx::mbar_arrive(&bars->xp_free[buf]);
         }
         uint32_t w[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) w[k] = pack_scores<T>(__uint_as_float(v[2 * k + 1]), __uint_as_float(v[2 * k]));
-        if (j + 1 < end) ptx::tmem_ld32(t_xp + 32 * (j + 1), v);
+        if (j + 1 < end) ptx::tmem_ld32(t_part + 32 * (j + 1), v);
         const uint32_t top = w[15];
 #pragma unroll
         for (int k = 15; k > 0; --k) w[k] = funnel_wrap(w[k], w[k - 1], p_shift);
         w[0] = funnel_wrap(w[0], p_prev, p_shift);
         p_prev = top;
-        const int chunk = half * 4 + j;                              // words 16 * chunk + k
-        const uint32_t down = (uint32_t)(chunk * 4 * STG_CHUNK);     // 32 columns are four chunks of eight query rows
-        const int turn = chunk - q4;
+        const uint32_t down = (uint32_t)(j * 4 * STG_CHUNK);     // words 16 * j + k; 32 columns are four chunks of eight query rows
+        const int turn = j - q4;
         if (turn >= 1 && turn <= 3) {
 #pragma unroll
           for (int k = 0; k < 16; ++k) sts_u32(stg_addr[k & 3] - down - (uint32_t)((k >> 2) * STG_CHUNK), w[k]);
         } else {
           // words 1 + row_even / 2 .. 64 + row_even / 2 are query rows of the tile
-          const int lo = 1 + row_even / 2 - 16 * chunk, hi = 64 + row_even / 2 - 16 * chunk;
+          const int lo = 1 + row_even / 2 - 16 * j, hi = 64 + row_even / 2 - 16 * j;
 #pragma unroll
           for (int k = 0; k < 16; ++k)
             sts_u32_if(stg_addr[k & 3] - down - (uint32_t)((k >> 2) * STG_CHUNK), w[k], k >= lo && k <= hi);
@@ -804,7 +812,8 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
         } else {
           for (int u = 0; u < n && ok && has_p2c; ++u) {
-            ok = convert_half(0) && convert_half(1);
+#pragma unroll 1
+            for (int part = 0; part < 4 && ok; ++part) ok = convert_part(part);
             if (!ok) break;
             ptx::fence_proxy_async_smem();   // the tile is read by the tensor core
             __syncwarp();
@@ -878,13 +887,14 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         // table row of column 0 of block 0: pair (row r, key x) of tile u uses column 128 - r + x of blocks u, u + 1
         const int row0 = cur.t_begin * BK - cur.i0 - BM + (L - 1);
         const int steps = cur.any_kept ? cur.n : 0;
-        // step -1 brings Q and the first table blocks, step u brings K(u) and the table blocks u + 1
+        // step -1 brings Q and the first table blocks, step u the table blocks u + 1; K runs one step ahead (its P2C parts
+        // are multiplied while the tile before is still with the converters), V one behind
 #pragma unroll 1
         for (int u = -1; u < steps && ok; ++u) {
           if (steps > 0) {
-            if (u < 0) load(&tmap_q, LO::offQ, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
-            else load(&tmap_k, LO::offK, bars->k_full, bars->k_empty, c_k, 2, (cur.t_begin + u) * BK, cur.bh, 1);
             if (has_p2c) load(&tmap_fq, LO::offRQ, bars->rq_full, bars->rq_empty, c_rq, 2, row0 + (u + 1) * BK, cur.h, 12);
+            if (u + 1 < steps) load(&tmap_k, LO::offK, bars->k_full, bars->k_empty, c_k, 2, (cur.t_begin + u + 1) * BK, cur.bh, 1);
+            if (u < 0) load(&tmap_q, LO::offQ, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
             if (has_c2p) load(&tmap_fk, LO::offRK, bars->rk_full, bars->rk_empty, c_rk, LO::kRkStages, row0 + (u + 1) * BK, cur.h, 11);
           }
           if (v_row >= 0 && (u >= 0 || steps == 0)) {
@@ -905,11 +915,11 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       if (v_row >= 0) load(&tmap_v, LO::offV, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
     } else if (warp == kMmaWarp) {
       // -------------------------------------------------------------- MMA issuer
-      // MMAs that produce scores.  The whole warp walks the items, one elected lane issues (umma_ss_f16_warp); descriptors
-      // are precomputed and only their start-address field moves.  Per key tile: first P2C half, C2P block of the tile
-      // after it, second P2C half, then S as soon as the softmax threads have read the previous tile's S, and the P2C
-      // tile on top of it as soon as the converters have finished it.  This warp never waits for P (the PV MMAs have an
-      // issuer of their own), so the relative terms of the next tiles are produced while the softmax is at work.
+      // C2P blocks and S.  In each issuing role the whole warp walks the items and one elected lane issues
+      // (umma_ss_f16_warp); descriptors are precomputed and only their start-address field moves.  Per key tile: C2P block
+      // of the tile after it, Q K^T as soon as the softmax threads have read the previous tile's S, and the P2C tile on
+      // top of it as soon as the converters have finished it.  The P2C parts and the PV MMAs have issuers of their own:
+      // an issue costs its warp about as long as the MMA runs, and neither waits for what this warp waits for.
       constexpr int is_bf16 = __is_same(T, __nv_bfloat16) ? 1 : 0;
       constexpr uint32_t idesc_nn = ptx::make_idesc_f16(is_bf16, BM, 128, 0, 0);   // 128 x 128, both K-major
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
@@ -919,12 +929,10 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offQ), 16, sbo, mode);
       const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, sbo, mode);
       const uint64_t rk_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRK), 16, sbo, mode);
-      const uint64_t rq_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRQ), 16, sbo, mode);
       const uint64_t eye_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offEye) + (EYE_ROWS - BM) * 16, EYE_CHUNK, 128, 0);
       const uint64_t stg_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offStg), STG_CHUNK, 128, 0);
       uint32_t c_q = 0, c_k = 0, c_rk = 0;            // loads consumed (stage / phase as in the loader)
-      uint32_t c_s = 0, c_xc = 0, c_xp = 0;           // S tiles, C2P blocks, P2C halves issued
-      uint32_t rq_alloc = 0;                          // rel_query blocks handed to items so far
+      uint32_t c_s = 0, c_xc = 0;                     // S tiles, C2P blocks issued
       bool ok = true;
 
       // D[128 x 128] = A[128 x d] * B[128 x d]^T, both operands K-major tiles in shared memory
@@ -946,37 +954,6 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         ++c_xc;
         return true;
       };
-      // S = Q . K^T of the tile whose K is in stage kst, plus I . (P2C tile)^T
-      auto issue_s = [&](uint32_t kst) -> bool {
-        if (!wwait(&bars->s_free, (c_s & 1u) ^ 1u, 6)) return false;
-        ptx::tc_fence_after();
-        mma_nn(tmem_base + COL_S, q_desc, k_desc + kst * kTileUnits);
-        if (has_p2c) {
-          if (!wwait(&bars->pt_ready, c_s & 1u, 9)) return false;
-          ptx::tc_fence_after();
-#pragma unroll 1
-          for (int kk = 0; kk < BM / 16; ++kk)
-            ptx::umma_ss_f16_warp(tmem_base + COL_S, eye_desc - (uint64_t)(16 * kk), stg_desc + (uint64_t)(2 * kk * (STG_CHUNK >> 4)),
-                                  idesc_nn, 1u);
-          ptx::umma_commit_warp(&bars->pt_release);
-        }
-        ptx::umma_commit_warp(&bars->s_full);
-        ++c_s;
-        return true;
-      };
-      // one half of the P2C accumulator: XP[n, w] = K . rel_query block^T; `first` = first use of the table block
-      // (wait for its load), `last` = last use (release its stage)
-      auto issue_pt = [&](uint32_t kst, uint32_t blk, bool first, bool last) -> bool {
-        const uint32_t st = blk & 1u, ph = (blk >> 1) & 1u;
-        if (first && !wwait(&bars->rq_full[st], ph, 15)) return false;
-        if (!wwait(&bars->xp_free, (c_xp & 1u) ^ 1u, 16)) return false;
-        ptx::tc_fence_after();
-        mma_nn(tmem_base + COL_XP, k_desc + kst * kTileUnits, rq_desc + st * kTileUnits);
-        if (last) ptx::umma_commit_warp(&bars->rq_empty[st]);
-        ptx::umma_commit_warp(&bars->xp_full);
-        ++c_xp;
-        return true;
-      };
       int k = 0;
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
         const int slot = k % kItemSlots;
@@ -989,26 +966,75 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (!any_kept) continue;
         ok = wwait(&bars->q_full, c_q & 1u, 4);
         ++c_q;
-        // step -1: C2P block 0; step u: key tile u (C2P blocks u and u + 1, rel_query blocks rq_alloc + u and + 1)
+        // step -1: C2P block 0; step u: key tile u (C2P block u + 1)
 #pragma unroll 1
         for (int u = -1; u < n && ok; ++u) {
-          const uint32_t kst = c_k & 1u;
-          if (u >= 0) ok = wwait(&bars->k_full[kst], (c_k >> 1) & 1u, 5);
-#pragma unroll 1
-          for (int half = 0; half < 2 && ok; ++half) {
-            if (u >= 0 && has_p2c)
-              ok = issue_pt(kst, rq_alloc + (uint32_t)(u + half), half == 1 || u == 0, half == 0 || u + 1 == n);
-            if (ok && half == 0 && has_c2p) ok = issue_c();
-          }
+          if (has_c2p) ok = issue_c();
           if (u < 0 || !ok) continue;
-          ok = issue_s(kst);
+          const uint32_t kst = c_k & 1u;
+          ok = wwait(&bars->k_full[kst], (c_k >> 1) & 1u, 5) && wwait(&bars->s_free, (c_s & 1u) ^ 1u, 6);
           if (!ok) break;
+          ptx::tc_fence_after();
+          mma_nn(tmem_base + COL_S, q_desc, k_desc + kst * kTileUnits);
           ptx::umma_commit_warp(&bars->k_empty[kst]);
+          if (u + 1 == n) ptx::umma_commit_warp(&bars->q_empty);
+          if (has_p2c) {
+            ok = wwait(&bars->pt_ready, c_s & 1u, 9);
+            if (!ok) break;
+            ptx::tc_fence_after();
+#pragma unroll 1
+            for (int kk = 0; kk < BM / 16; ++kk)
+              ptx::umma_ss_f16_warp(tmem_base + COL_S, eye_desc - (uint64_t)(16 * kk), stg_desc + (uint64_t)(2 * kk * (STG_CHUNK >> 4)),
+                                    idesc_nn, 1u);
+            ptx::umma_commit_warp(&bars->pt_release);
+          }
+          ptx::umma_commit_warp(&bars->s_full);
           ++c_k;
+          ++c_s;
         }
+      }
+    } else if (warp == kPartWarp) {
+      // ------------------------------- P2C parts, as far ahead as their two accumulators allow
+      // XP[n, w] = K . rel_query^T over 64 table rows; parts 0 and 1 of a tile take them from its first table block, 2 and
+      // 3 from the second one, which is the first one of the next tile.
+      constexpr uint32_t idesc_part = ptx::make_idesc_f16(__is_same(T, __nv_bfloat16) ? 1 : 0, BM, 64, 0, 0);
+      constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
+      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4;
+      const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, 8 * LO::kRowBytes, mode);
+      const uint64_t rq_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRQ), 16, 8 * LO::kRowBytes, mode);
+      uint32_t c_k = 0, c_rq = 0, c_xp = 0;   // key tiles consumed, table blocks released, parts issued
+      bool ok = true;
+      int k = 0;
+      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
+        const int slot = k % kItemSlots;
+        ok = wwait(&bars->item_full[slot], (uint32_t)(k / kItemSlots) & 1u, 40);
         if (!ok) break;
-        rq_alloc += (uint32_t)n + 1u;
-        ptx::umma_commit_warp(&bars->q_empty);
+        const int n = slots[slot].any_kept != 0 && has_p2c ? slots[slot].t_end - slots[slot].t_begin : 0;
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
+#pragma unroll 1
+        for (uint32_t x = 0; x < 4u * (uint32_t)n && ok; ++x) {   // part x & 3 of key tile x >> 2
+          const uint32_t part = x & 3u, kst = c_k & 1u, buf = c_xp & 1u;
+          if (part == 0) ok = wwait(&bars->k_full[kst], (c_k >> 1) & 1u, 43);
+          if (ok && (x == 0 || part == 2)) ok = wwait(&bars->rq_full[c_rq & 1u], (c_rq >> 1) & 1u, 15);   // first use of a block
+          ok = ok && wwait(&bars->xp_free[buf], ((c_xp >> 1) & 1u) ^ 1u, 16);
+          if (!ok) break;
+          ptx::tc_fence_after();
+          const uint64_t a_desc = k_desc + kst * kTileUnits, b_desc = rq_desc + (c_rq & 1u) * kTileUnits + buf * (kTileUnits / 2);
+#pragma unroll 1
+          for (int kk = 0; kk < LO::kRowBytes / 32; ++kk)
+            ptx::umma_ss_f16_warp(tmem_base + COL_XP + 64 * buf, a_desc + 2u * kk, b_desc + 2u * kk, idesc_part, kk != 0 ? 1u : 0u);
+          ptx::umma_commit_warp(&bars->xp_full[buf]);
+          ++c_xp;
+          if (part == 1 || x + 1 == 4u * (uint32_t)n) {   // last use of the block
+            ptx::umma_commit_warp(&bars->rq_empty[c_rq & 1u]);
+            ++c_rq;
+          }
+          if (part == 3) {
+            ptx::umma_commit_warp(&bars->k_empty[kst]);
+            ++c_k;
+          }
+        }
       }
     } else if (warp == kPvWarp) {
       // ----------------------------------------------------------- O (+)= P . V of every key tile, as soon as P is stored
