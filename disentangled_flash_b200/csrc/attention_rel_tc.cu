@@ -116,7 +116,7 @@ struct RLayout {
   static constexpr int offXmax = offBar + kBarBytes;
   static constexpr int offMeanV = offXmax + 2 * 2 * BM * 4;
   static constexpr int offItem = offMeanV + 256;
-  static constexpr int kItemBytes = 288;
+  static constexpr int kItemBytes = 304;
   static constexpr int total = offItem + kItemSlots * kItemBytes + 1024;   // + alignment slack
   static_assert(offStg % 16 == 0 && offBar % 16 == 0 && offItem % 16 == 0, "alignment");
   static_assert(total <= 232448, "shared memory budget");
@@ -126,10 +126,12 @@ struct RLayout {
 struct ItemSlot {
   int t_begin, t_end;   // key tiles [t_begin, t_end) are processed
   int any_kept;         // 0: every query row of the tile is padding -> mean-of-V path, no pipeline work
-  int bh, i0;           // batch*heads + head, first query row
+  int bh, h, i0;        // batch*heads + head, head, first query row
+  int out_rows;         // rows of the sequence the output holds, from out_row0 on: [B,L,H*d], or packed rows (see
+  long long out_row0;   // DflAttnRelParams.out_row_base)
   uint32_t kbits[kMaskWords];   // kept-key bits of the batch row, word w = keys [32w, 32w+32)
 };
-static_assert(sizeof(ItemSlot) <= 288, "item slot too large");
+static_assert(sizeof(ItemSlot) <= 304, "item slot too large");
 
 struct RBarriers {
   uint64_t q_full, q_empty;
@@ -409,12 +411,10 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       const ItemSlot* sl = &slots[slot];
       const int t_begin = sl->t_begin, n = sl->t_end - sl->t_begin;
       const bool any_kept = sl->any_kept != 0;
-      const int bh = sl->bh, b = bh / H, h = bh - b * H;
+      const int bh = sl->bh, h = sl->h;
       const int i0 = sl->i0;
-
-      // where the item's rows go: [B,L,H*d], or packed rows of the sequence (see DflAttnRelParams.out_row_base)
-      const long long out_row0 = p.out_row_base ? (long long)p.out_row_base[b] : (long long)b * L;
-      const int out_rows = p.out_row_base ? p.out_row_count[b] : L;
+      const long long out_row0 = sl->out_row0;
+      const int out_rows = sl->out_rows;
       if (!any_kept && out_rows <= i0) {
         // a tile of padded positions that the packed output does not hold: nothing to compute, nothing to store
       } else if (!any_kept) {
@@ -620,10 +620,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         if (!ok) break;
 
-        // ---- the item's last PV, then normalise and store this thread's half of the output columns
-        ok = wwait(&bars->o_ready, (c_t & 1u) ^ 1u, 48);   // the item's last PV: c_t - 1 completed before it
-        if (!ok) break;
-        ptx::tc_fence_after();
+        // ---- row sums, the item's last PV, then normalise and store this thread's half of the output columns
         const uint32_t sum_phase = (c_t + c_i) & 1u;
         float* xs = xchg + sum_phase * (2 * BM);
         xs[hf * BM + r] = l_run;
@@ -633,25 +630,43 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         ++c_i;
         if (!ok) break;
         const float inv = 1.0f / (l_run + xs[(1 - hf) * BM + r]);
+        ok = wwait(&bars->o_ready, (c_t & 1u) ^ 1u, 48);   // the item's last PV: c_t - 1 completed before it
+        if (!ok) break;
+        ptx::tc_fence_after();
         uint32_t o[OW];
         attn::tmem_ld_n(t_o, o);
         ptx::tmem_wait_ld();
-        // the accumulator is in registers: the next item's second C2P block and first PV may overwrite it
+        // the accumulator is in registers: the next item's first PV may overwrite it
         ptx::tc_fence_before();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->o_free);
-        if (row_ok && i < out_rows) {
-          T* out = reinterpret_cast<T*>(p.out) + (out_row0 + i) * ((long long)H * D) + (long long)h * D + hf * OW;
+        // Lanes of one row each would touch 32 cache lines per store (1900 cycles an item).  The OW / 8 lanes of a group
+        // transpose their 16-byte chunks instead: lane c of the group ends up with chunk c of every row of the group, and a
+        // store covers whole 2 * OW byte segments.
+        constexpr int kGroup = OW / 8;
+        uint32_t w[kGroup][4];
 #pragma unroll
-          for (int v = 0; v < OW / 8; ++v) {
-            uint4 pk;
-            pk.x = Pack2<T>::pack(__uint_as_float(o[v * 8 + 0]) * inv, __uint_as_float(o[v * 8 + 1]) * inv);
-            pk.y = Pack2<T>::pack(__uint_as_float(o[v * 8 + 2]) * inv, __uint_as_float(o[v * 8 + 3]) * inv);
-            pk.z = Pack2<T>::pack(__uint_as_float(o[v * 8 + 4]) * inv, __uint_as_float(o[v * 8 + 5]) * inv);
-            pk.w = Pack2<T>::pack(__uint_as_float(o[v * 8 + 6]) * inv, __uint_as_float(o[v * 8 + 7]) * inv);
-            *reinterpret_cast<uint4*>(out + v * 8) = pk;
+        for (int x = 0; x < OW / 2; ++x)
+          w[x / 4][x % 4] = Pack2<T>::pack(__uint_as_float(o[2 * x]) * inv, __uint_as_float(o[2 * x + 1]) * inv);
+#pragma unroll
+        for (int bit = 1; bit < kGroup; bit <<= 1) {
+          const bool upper = (lane & bit) != 0;
+#pragma unroll
+          for (int c = 0; c < kGroup; ++c) {
+            if (c & bit) continue;
+#pragma unroll
+            for (int x = 0; x < 4; ++x) {   // the lower lane keeps chunk c and takes the partner's, the upper one chunk c + bit
+              const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? w[c][x] : w[c | bit][x], bit);
+              if (upper) w[c][x] = got;
+              else w[c | bit][x] = got;
+            }
           }
         }
+        const int row0 = i0 + (r & ~(kGroup - 1)), rows = min(L, out_rows) - row0;
+        T* out = reinterpret_cast<T*>(p.out) + (out_row0 + row0) * ((long long)H * D) + (long long)h * D + hf * OW + (lane & (kGroup - 1)) * 8;
+#pragma unroll
+        for (int c = 0; c < kGroup; ++c)
+          if (c < rows) *reinterpret_cast<uint4*>(out + (long long)c * H * D) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
       }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
@@ -858,6 +873,9 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           sl->t_end = range.t_end;
           sl->any_kept = range.any_kept ? 1 : 0;
           sl->bh = bh;
+          sl->h = bh - b * H;
+          sl->out_row0 = p.out_row_base ? (long long)p.out_row_base[b] : (long long)b * L;
+          sl->out_rows = p.out_row_base ? p.out_row_count[b] : L;
           sl->i0 = i0;
         }
         __syncwarp();
