@@ -35,7 +35,7 @@ Workspace plan_workspace(const DflEncoderParams& p) {
     return here;
   };
   const bool f32 = p.dtype == DFL_F32, layers = !p.attention_only;
-  w.qkv = take(p.packed_rows > 0 ? 0 : 3 * padded(positions * width * (f32 ? kPlaneBytes : es)));
+  w.qkv = take(p.packed_rows > 0 && p.row_groups ? 0 : 3 * padded(positions * width * (f32 ? kPlaneBytes : es)));
   if (layers) {
     w.context = take(rows * width * (f32 ? kPlaneBytes : es));
     w.dense = take(rows * p.hidden * es);
@@ -94,9 +94,11 @@ int validate(const DflEncoderParams& p) {
   if ((long long)p.batch * p.heads > 65535) return fail(DFL_ERR_TOO_LARGE, "batch*heads > 65535");
   if (p.packed_rows > 0) {
     if (two_call(p)) return fail(DFL_ERR_UNSUPPORTED, "packed rows need the rel_key / rel_query form");
-    if (p.packed_rows % 32 || p.seq_len % 32) return fail(DFL_ERR_BAD_ARG, "packed rows come in groups of 32");
-    if (!p.pack_rows || !p.row_groups || !p.row_base || !p.row_count || !p.qkv[0] || !p.qkv[1] || !p.qkv[2])
-      return fail(DFL_ERR_BAD_ARG, "null packed-row table or buffer");
+    if (!p.pack_rows || !p.row_base || !p.row_count) return fail(DFL_ERR_BAD_ARG, "null packed-row table");
+    if (p.row_groups) {
+      if (p.packed_rows % 32 || p.seq_len % 32) return fail(DFL_ERR_BAD_ARG, "row groups are 32 rows of one sequence");
+      if (!p.qkv[0] || !p.qkv[1] || !p.qkv[2]) return fail(DFL_ERR_BAD_ARG, "null qkv buffer");
+    }
   }
   return DFL_OK;
 }
@@ -122,7 +124,7 @@ struct Loop {
     if (heads_out) {
       for (int i = 0; i < 3; ++i) g.out[i] = heads_out[i];
       g.head_split = 1; g.heads = p.heads; g.head_dim = p.head_dim; g.rows_per_seq = p.seq_len;
-      if (p.packed_rows > 0) {
+      if (p.packed_rows > 0 && p.row_groups) {
         g.row_groups = p.row_groups;
         g.out_seqs = p.batch;
       }
@@ -232,9 +234,13 @@ struct Loop {
   int run() {
     const bool packed = p.packed_rows > 0;
     const int rows = packed ? p.packed_rows : p.batch * p.seq_len, width = p.heads * p.head_dim;
+    // Q, K, V of packed rows: projected from the packed rows where groups of 32 of them have a place in the head-major
+    // buffers, from the unpacked state (which every layer then writes as well) otherwise
+    const bool grouped = packed && p.row_groups;
+    const int qkv_rows = grouped ? rows : p.batch * p.seq_len;
     void* qkv[3];
     for (int i = 0; i < 3; ++i)
-      qkv[i] = packed ? p.qkv[i] : at(w.qkv + (size_t)i * padded((size_t)rows * width * (p.dtype == DFL_F32 ? kPlaneBytes : dtype_size(p.dtype))));
+      qkv[i] = grouped ? p.qkv[i] : at(w.qkv + (size_t)i * padded((size_t)qkv_rows * width * (p.dtype == DFL_F32 ? kPlaneBytes : dtype_size(p.dtype))));
     const void* state = p.x;
     const bool f32 = p.dtype == DFL_F32;
     void* unpacked = p.outs[p.n_layers - 1];
@@ -254,7 +260,8 @@ struct Loop {
       const DflEncoderLayer& y = p.layers[l];
       const bool last = l == p.n_layers - 1, convolve = l == 0 && p.conv_w;
       void* next = !packed && p.outs[l] ? p.outs[l] : at(w.state[l & 1]);
-      if (int rc = gemm(f32 ? at(w.state_planes) : state, y.qkv_w, y.qkv_b, nullptr, rows, 3 * width, p.hidden, DFL_ACT_NONE, qkv, true)) return rc;
+      const void* input = f32 ? at(w.state_planes) : (packed && !grouped ? (l == 0 ? p.x : unpacked) : state);
+      if (int rc = gemm(input, y.qkv_w, y.qkv_b, nullptr, qkv_rows, 3 * width, p.hidden, DFL_ACT_NONE, qkv, true)) return rc;
       if (int rc = attention(y, qkv, at(w.context), l)) return rc;
       if (int rc = gemm(at(w.context), y.attn_out_w, y.attn_out_b, at(w.dense), rows, p.hidden, width, DFL_ACT_NONE)) return rc;
       if (int rc = norm(at(w.dense), state, y.attn_norm_w, y.attn_norm_b, at(w.mixed), rows, y.attn_norm_eps, nullptr, nullptr,
@@ -262,9 +269,10 @@ struct Loop {
       void* inner = f32 ? at(w.inner_planes) : at(w.inner);
       if (int rc = gemm(f32 ? at(w.mixed_planes) : at(w.mixed), y.ffn_in_w, y.ffn_in_b, inner, rows, p.ffn, p.hidden, DFL_ACT_GELU, nullptr, true)) return rc;
       if (int rc = gemm(inner, y.ffn_out_w, y.ffn_out_b, at(w.dense), rows, p.hidden, p.ffn, DFL_ACT_NONE)) return rc;
-      // a packed state is also written out at its unpacked rows where the convolution or the caller reads it
+      // a packed state is also written out at its unpacked rows where the convolution, the next projection or the caller
+      // reads it
       if (int rc = norm(at(w.dense), at(w.mixed), y.ffn_norm_w, y.ffn_norm_b, next, rows, y.ffn_norm_eps, nullptr,
-                        packed && (last || convolve) ? unpacked : nullptr, f32 && !last ? at(w.state_planes) : nullptr)) return rc;
+                        packed && (last || convolve || !grouped) ? unpacked : nullptr, f32 && !last ? at(w.state_planes) : nullptr)) return rc;
       if (convolve) {
         if (int rc = convolution(packed ? unpacked : next, packed ? unpacked : next)) return rc;
         if (packed && !last) {

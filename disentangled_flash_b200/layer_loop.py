@@ -210,17 +210,20 @@ class LayerLoop:
 
     def run_packed(self, hidden: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None, out: torch.Tensor,
                    tables: tuple[torch.Tensor, torch.Tensor, torch.Tensor, torch.Tensor],
-                   qkv: tuple[torch.Tensor, ...]) -> None:
-        """``tables`` = (pack_rows, row_groups, row_base, row_count); the result goes to the covered rows of ``out``."""
+                   qkv: tuple[torch.Tensor, ...] | None) -> None:
+        """``tables`` = (pack_rows, row_groups, row_base, row_count); the result goes to the covered rows of ``out``.
+        ``qkv``: the head-major buffers of the grouped projection, None where the bucket has no row groups."""
 
         outs = (ctypes.c_void_p * self.n_layers)()
         outs[self.n_layers - 1] = out.data_ptr()
         p = self._call(hidden, mask, outs, status)
         pack_rows, row_groups, row_base, row_count = tables
-        p.packed_rows, p.pack_rows, p.row_groups = pack_rows.numel(), pack_rows.data_ptr(), row_groups.data_ptr()
+        p.packed_rows, p.pack_rows = pack_rows.numel(), pack_rows.data_ptr()
         p.row_base, p.row_count = row_base.data_ptr(), row_count.data_ptr()
-        for i in range(3):
-            p.qkv[i] = qkv[i].data_ptr()
+        if qkv is not None:
+            p.row_groups = row_groups.data_ptr()
+            for i in range(3):
+                p.qkv[i] = qkv[i].data_ptr()
         _cabi.encoder_fwd(p, self.device)
 
 

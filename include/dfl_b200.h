@@ -440,12 +440,14 @@ typedef struct DflEncoderParams {
   int32_t launches;                /* out: kernels this call has launched */
   int32_t attention_only;          /* non-zero: layer 0 up to its attention; outs[0] is the context
                                       [batch, seq_len, heads*head_dim] and only the qkv and table entries are read */
-  /* Packed form (packed_rows > 0, rel_* form only, seq_len a multiple of 32): between the attention kernels the layers
-   * run on the valid positions, packed in groups of 32 rows.  outs[n_layers-1] receives the unpacked result; positions
-   * no group covers are left as they are there.  No other entry of outs may be given. */
-  int32_t packed_rows;             /* T, a multiple of 32 */
+  /* Packed form (packed_rows > 0, rel_* form only): between the attention kernels the layers run on the valid positions,
+   * packed.  outs[n_layers-1] receives the unpacked result; positions no packed row holds are left as they are there
+   * (finite; with row_groups NULL they are read as the state of padded positions).  No other entry of outs may be given.
+   * With seq_len a multiple of 32 and every sequence packed in groups of 32 rows, row_groups and qkv let the QKV projection
+   * read the packed rows too; with row_groups NULL it reads the unpacked state and qkv is not used. */
+  int32_t packed_rows;             /* T */
   const int32_t* pack_rows;        /* device [T]: row of [batch*seq_len] each packed row holds */
-  const int32_t* row_groups;       /* device [T/32]: first of them per group */
+  const int32_t* row_groups;       /* device [T/32]: first of them per group, or NULL */
   const int32_t* row_base;         /* device [batch]: first packed row of a sequence */
   const int32_t* row_count;        /* device [batch]: packed rows of a sequence */
   void* qkv[3];                    /* [batch, heads, seq_len, head_dim] each, finite contents, kept from call to call */
