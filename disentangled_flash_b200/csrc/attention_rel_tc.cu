@@ -72,9 +72,9 @@ constexpr int kMaxSeqLen = 2048;
 constexpr int kMaskWords = kMaxSeqLen / 32;   // kept-key bits per item
 
 // C2P rows: per query row two tiles of 128 16-bit scores, tile T of the CTA's running count in half T & 1, key x of the tile
-// at column x: the softmax thread of the row reads its 64 keys as eight 16-byte words.  35 16-byte units per row: eight
-// consecutive rows hit different bank groups with those reads, and the converters' 4-byte stores conflict at most 2-way.
-constexpr int ROW_PITCH = 560;
+// at column x: the softmax thread of the row reads its 64 keys as eight 16-byte words.  33 16-byte units per row: eight
+// consecutive rows hit different bank groups with those reads, and the converters' 4-byte stores conflict 2-way.
+constexpr int ROW_PITCH = 528;
 // P2C tile: the B operand of the MMA that adds it to S, K-major without swizzle: 8-row core matrices of 128 bytes, rows =
 // keys, K = query rows.  Chunks of eight query rows are STG_CHUNK bytes apart (32 bytes more than 16 core matrices, so
 // that the 4-byte stores of 32 neighbouring keys, each shifted by its key, fall into 32 different banks).
@@ -89,24 +89,35 @@ constexpr int EYE_BYTES = 2 * EYE_CHUNK;
 // TMEM columns (all 512; one CTA per SM)
 constexpr int COL_S = 0;      // 128  S = Q K^T of the current tile (fp32)
 constexpr int COL_P = 128;    // 64   P of the current tile (16-bit pairs), A operand of the PV MMA
-constexpr int COL_O = 192;    // 64   O accumulator (first D columns used)
-constexpr int COL_XC = 256;   // 128  one new C2P block for the 128 query rows
+constexpr int COL_O = 192;    // D    O accumulator
+                              // XC: one new C2P block for the 128 query rows, 128 columns from 256 on; half a block at a
+                              // time, 64 columns from 320 on, with d = 128
 constexpr int COL_XP = 384;   // 2 x 64  two of the four parts (64 table rows each) of the P2C accumulator of a key tile
 constexpr int kTmemCols = 512;
 
 template <int D>
 struct RLayout {
-  static_assert(D == 32 || D == 64, "head dims 32 and 64");
-  static constexpr int kRowBytes = D * 2;
-  static constexpr int kTile = 128 * kRowBytes;        // Q tile, K tile, V tile, one 128-row table block
-  static constexpr int kVStages = D == 64 ? 1 : 2;     // d = 64 fills shared memory: V and rel_key blocks are
-  static constexpr int kRkStages = D == 64 ? 1 : 2;    // reloaded within the tile time after their single use
+  static_assert(D == 32 || D == 64 || D == 128, "head dims 32, 64 and 128");
+  // An operand tile is kSub sub-tiles of at most 64 columns, one swizzled 64- or 128-byte row per tile row.  The table blocks
+  // and V come in kPieces pieces: at d = 128 in 64-row halves, the only way one stage of each fits beside Q and K.
+  static constexpr int kSub = D > 64 ? 2 : 1;
+  static constexpr int kPieces = D > 64 ? 2 : 1;
+  static constexpr int kPieceRows = 128 / kPieces;
+  static constexpr int kRowBytes = D * 2 / kSub;
+  static constexpr int kTile = 128 * D * 2;            // Q tile, K tile
+  static constexpr int kPiece = kPieceRows * D * 2;    // piece of V or of a 128-row table block
+  static constexpr int kSteps = D / 16;                // K=16 steps over d
+  static constexpr int kKStages = D > 64 ? 1 : 2, kRqStages = D > 64 ? 1 : 2;
+  static constexpr int kVStages = D == 32 ? 2 : 1;     // d = 64 fills shared memory: V and rel_key blocks are
+  static constexpr int kRkStages = D == 32 ? 2 : 1;    // reloaded within the tile time after their single use
+  static constexpr int kXcCols = 128 / kPieces;        // C2P accumulator
+  static constexpr int kColXc = D > 64 ? 320 : 256;
   static constexpr int offQ = 0;
-  static constexpr int offK = offQ + kTile;                 // 2 stages
-  static constexpr int offV = offK + 2 * kTile;
-  static constexpr int offRK = offV + kVStages * kTile;
-  static constexpr int offRQ = offRK + kRkStages * kTile;   // 2 stages
-  static constexpr int offRows = offRQ + 2 * kTile;
+  static constexpr int offK = offQ + kTile;
+  static constexpr int offV = offK + kKStages * kTile;
+  static constexpr int offRK = offV + kVStages * kPiece;
+  static constexpr int offRQ = offRK + kRkStages * kPiece;
+  static constexpr int offRows = offRQ + kRqStages * kPiece;
   static constexpr int offStg = offRows + BM * ROW_PITCH;
   static constexpr int offEye = offStg + STG_BYTES;
   static constexpr int offBar = offEye + EYE_BYTES;
@@ -114,7 +125,7 @@ struct RLayout {
   // exchange area: [2 parities][2 halves][BM] row maxima (row sums at the end of an item, partial sums of the mean-of-V
   // path), then the [D] column mean of V
   static constexpr int offXmax = offBar + kBarBytes;
-  static constexpr int offMeanV = offXmax + 2 * 2 * BM * 4;
+  static constexpr int offMeanV = offXmax + (D > 64 ? 8 * D * 4 : 2 * 2 * BM * 4);
   static constexpr int offItem = offMeanV + 256;
   static constexpr int kItemBytes = 304;
   static constexpr int total = offItem + kItemSlots * kItemBytes + 1024;   // + alignment slack
@@ -283,6 +294,19 @@ __device__ __forceinline__ TileRange tile_range(uint32_t kb_lo, uint32_t kb_hi, 
     r.t_end = (last >> 2) + 1;
   }
   return r;
+}
+
+// D[128 x N] = A[128 x d] * B[N x d]^T, both operands K-major tiles in shared memory; a_sub, b_sub: descriptor units from
+// one 64-column sub-tile to the next.  One converged warp.
+template <int D>
+__device__ __forceinline__ void mma_over_d(uint32_t d_tmem, uint64_t a_desc, uint32_t a_sub, uint64_t b_desc, uint32_t b_sub,
+                                           uint32_t idesc) {
+#pragma unroll 1
+  for (int kk = 0; kk < D / 16; ++kk) {
+    ptx::umma_ss_f16_warp(d_tmem, a_desc, b_desc, idesc, kk != 0 ? 1u : 0u);
+    a_desc += D > 64 && kk == 3 ? a_sub - 6u : 2u;
+    b_desc += D > 64 && kk == 3 ? b_sub - 6u : 2u;
+  }
 }
 
 template <typename T, int D>
@@ -633,40 +657,45 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         ok = wwait(&bars->o_ready, (c_t & 1u) ^ 1u, 48);   // the item's last PV: c_t - 1 completed before it
         if (!ok) break;
         ptx::tc_fence_after();
-        uint32_t o[OW];
-        attn::tmem_ld_n(t_o, o);
-        ptx::tmem_wait_ld();
-        // the accumulator is in registers: the next item's first PV may overwrite it
-        ptx::tc_fence_before();
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->o_free);
-        // Lanes of one row each would touch 32 cache lines per store (1900 cycles an item).  The OW / 8 lanes of a group
+        // Lanes of one row each would touch 32 cache lines per store (1900 cycles an item).  The kGroup lanes of a group
         // transpose their 16-byte chunks instead: lane c of the group ends up with chunk c of every row of the group, and a
-        // store covers whole 2 * OW byte segments.
-        constexpr int kGroup = OW / 8;
-        uint32_t w[kGroup][4];
-#pragma unroll
-        for (int x = 0; x < OW / 2; ++x)
-          w[x / 4][x % 4] = Pack2<T>::pack(__uint_as_float(o[2 * x]) * inv, __uint_as_float(o[2 * x + 1]) * inv);
-#pragma unroll
-        for (int bit = 1; bit < kGroup; bit <<= 1) {
-          const bool upper = (lane & bit) != 0;
-#pragma unroll
-          for (int c = 0; c < kGroup; ++c) {
-            if (c & bit) continue;
-#pragma unroll
-            for (int x = 0; x < 4; ++x) {   // the lower lane keeps chunk c and takes the partner's, the upper one chunk c + bit
-              const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? w[c][x] : w[c | bit][x], bit);
-              if (upper) w[c][x] = got;
-              else w[c | bit][x] = got;
-            }
-          }
-        }
+        // store covers whole segments.
+        constexpr int OC = OW < 32 ? OW : 32;   // columns at a time
+        constexpr int kGroup = OC / 8;
         const int row0 = i0 + (r & ~(kGroup - 1)), rows = min(L, out_rows) - row0;
         T* out = reinterpret_cast<T*>(p.out) + (out_row0 + row0) * ((long long)H * D) + (long long)h * D + hf * OW + (lane & (kGroup - 1)) * 8;
 #pragma unroll
-        for (int c = 0; c < kGroup; ++c)
-          if (c < rows) *reinterpret_cast<uint4*>(out + (long long)c * H * D) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+        for (int c0 = 0; c0 < OW; c0 += OC) {
+          uint32_t o[OC];
+          attn::tmem_ld_n(t_o + c0, o);
+          ptx::tmem_wait_ld();
+          if (c0 + OC == OW) {   // the accumulator is in registers: the next item's first PV may overwrite it
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&bars->o_free);
+          }
+          uint32_t w[kGroup][4];
+#pragma unroll
+          for (int x = 0; x < OC / 2; ++x)
+            w[x / 4][x % 4] = Pack2<T>::pack(__uint_as_float(o[2 * x]) * inv, __uint_as_float(o[2 * x + 1]) * inv);
+#pragma unroll
+          for (int bit = 1; bit < kGroup; bit <<= 1) {
+            const bool upper = (lane & bit) != 0;
+#pragma unroll
+            for (int c = 0; c < kGroup; ++c) {
+              if (c & bit) continue;
+#pragma unroll
+              for (int x = 0; x < 4; ++x) {   // the lower lane keeps chunk c and takes the partner's, the upper one chunk c + bit
+                const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? w[c][x] : w[c | bit][x], bit);
+                if (upper) w[c][x] = got;
+                else w[c | bit][x] = got;
+              }
+            }
+          }
+#pragma unroll
+          for (int c = 0; c < kGroup; ++c)
+            if (c < rows) *reinterpret_cast<uint4*>(out + (long long)c * H * D + c0) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+        }
       }
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
@@ -687,7 +716,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     const int row = q4 * 32 + lane;
     const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
     const uint32_t t_xp = tmem_base + lane_base + COL_XP;
-    const uint32_t t_xc = tmem_base + lane_base + COL_XC;
+    const uint32_t t_xc = tmem_base + lane_base + LO::kColXc;
     // C2P: word k of a block (columns 2k, 2k+1; for odd rows 2k-1, 2k) goes to column 128 * tile + 2k + row_even
     const int row_even = row & ~1;
     const uint32_t row_addr = ptx::smem_u32(smem + LO::offRows) + (uint32_t)(row * ROW_PITCH + 2 * row_even);
@@ -709,6 +738,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     // One C2P block: upper part of running tile `upper`, lower part of tile upper + 1; the first block of an item has no
     // upper part.  The two row buffers must be free: `need` key tiles in total must have been read.
     auto convert_block = [&](bool first, uint32_t upper, uint32_t need) -> bool {
+      constexpr int kChunksOfXc = LO::kXcCols / 32;   // the accumulator holds a block, or half of it at a time
       if (!wwait(&bars->xc_full, c_xc & 1u, 18)) return false;
       ++c_xc;
       ptx::tc_fence_after();
@@ -721,8 +751,14 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       }
 #pragma unroll 1
       for (int j = 0; j < 4; ++j) {   // 32 columns at a time, the next ones in flight while these are stored
+        if (LO::kPieces > 1 && j == kChunksOfXc) {
+          if (!wwait(&bars->xc_full, c_xc & 1u, 18)) return false;
+          ++c_xc;
+          ptx::tc_fence_after();
+          ptx::tmem_ld32(t_xc, v);
+        }
         ptx::tmem_wait_ld();
-        if (j == 3) {   // the block is in registers: the accumulator is free for the next block's MMA
+        if (j % kChunksOfXc == kChunksOfXc - 1) {   // in registers: the accumulator is free for the next MMA
           ptx::tc_fence_before();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&bars->xc_free);
@@ -730,7 +766,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         uint32_t w[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) w[k] = pack_scores<T>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-        if (j < 3) ptx::tmem_ld32(t_xc + 32 * (j + 1), v);
+        if (j % kChunksOfXc != kChunksOfXc - 1) ptx::tmem_ld32(t_xc + 32 * (j % kChunksOfXc + 1), v);
         const uint32_t top = w[15];
 #pragma unroll
         for (int k = 15; k > 0; --k) w[k] = funnel_clamp(w[k - 1], w[k], c_shift);
@@ -883,15 +919,17 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         f = {range.t_begin, range.t_end - range.t_begin, i0, bh, bh - b * H, range.any_kept};
         return true;
       };
-      // one 128-row tile into stage count % stages of the buffers at `offset`
-      auto load = [&](const CUtensorMap* map, int offset, uint64_t* full, uint64_t* empty, uint32_t& count, uint32_t stages, int row,
-                      int z, int code) {
+      // one tile or piece of `bytes` bytes into stage count % stages of the buffers at `offset`
+      auto load = [&](const CUtensorMap* map, int offset, int bytes, uint64_t* full, uint64_t* empty, uint32_t& count, uint32_t stages,
+                      int row, int z, int code) {
         const uint32_t st = stages == 1 ? 0u : count & 1u, ph = (stages == 1 ? count : count >> 1) & 1u;
         ++count;
         ok = ok && wwait(&empty[st], ph ^ 1u, code);
         if (ok && lane == 0) {
-          ptx::mbar_arrive_expect_tx(&full[st], (uint32_t)LO::kTile);
-          ptx::tma_load_3d(smem + offset + st * LO::kTile, map, &full[st], 0, row, z);
+          ptx::mbar_arrive_expect_tx(&full[st], (uint32_t)bytes);
+#pragma unroll
+          for (int c = 0; c < LO::kSub; ++c)
+            ptx::tma_load_3d(smem + offset + st * bytes + c * (bytes / LO::kSub), map, &full[st], 64 * c, row, z);
         }
         __syncwarp();
       };
@@ -906,22 +944,43 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         const int row0 = cur.t_begin * BK - cur.i0 - BM + (L - 1);
         const int steps = cur.any_kept ? cur.n : 0;
         // step -1 brings Q and the first table blocks, step u the table blocks u + 1; K runs one step ahead (its P2C parts
-        // are multiplied while the tile before is still with the converters), V one behind
+        // are multiplied while the tile before is still with the converters), V one behind.  With pieces, in the order in
+        // which a single stage of each is consumed: step u brings the four rel_query pieces of tile u around the two of
+        // rel_key block u + 1, then K of tile u + 1; V is loaded by the warp that issues the PV MMAs.
 #pragma unroll 1
         for (int u = -1; u < steps && ok; ++u) {
           if (steps > 0) {
-            if (has_p2c) load(&tmap_fq, LO::offRQ, bars->rq_full, bars->rq_empty, c_rq, 2, row0 + (u + 1) * BK, cur.h, 12);
-            if (u + 1 < steps) load(&tmap_k, LO::offK, bars->k_full, bars->k_empty, c_k, 2, (cur.t_begin + u + 1) * BK, cur.bh, 1);
-            if (u < 0) load(&tmap_q, LO::offQ, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
-            if (has_c2p) load(&tmap_fk, LO::offRK, bars->rk_full, bars->rk_empty, c_rk, LO::kRkStages, row0 + (u + 1) * BK, cur.h, 11);
+            if (LO::kPieces == 1 && has_p2c)
+              load(&tmap_fq, LO::offRQ, LO::kPiece, bars->rq_full, bars->rq_empty, c_rq, LO::kRqStages, row0 + (u + 1) * BK, cur.h, 12);
+            if (LO::kPieces > 1) {
+              if (u < 0) load(&tmap_q, LO::offQ, LO::kTile, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
+#pragma unroll 1
+              for (int x = 0; x < 6; ++x) {   // rel_query, rel_query, rel_key, rel_key, rel_query, rel_query
+                const int row = row0 + (u + (x >= 2 ? 1 : 0)) * BK + (x & 1) * LO::kPieceRows;
+                if ((x >> 1) == 1) {
+                  if (has_c2p) load(&tmap_fk, LO::offRK, LO::kPiece, bars->rk_full, bars->rk_empty, c_rk, LO::kRkStages, row, cur.h, 11);
+                } else if (u >= 0 && has_p2c) {
+                  load(&tmap_fq, LO::offRQ, LO::kPiece, bars->rq_full, bars->rq_empty, c_rq, LO::kRqStages, row, cur.h, 12);
+                }
+              }
+            }
+            if (u + 1 < steps)
+              load(&tmap_k, LO::offK, LO::kTile, bars->k_full, bars->k_empty, c_k, LO::kKStages, (cur.t_begin + u + 1) * BK, cur.bh, 1);
+            if (LO::kPieces == 1) {
+              if (u < 0) load(&tmap_q, LO::offQ, LO::kTile, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
+              if (has_c2p)
+                load(&tmap_fk, LO::offRK, LO::kPiece, bars->rk_full, bars->rk_empty, c_rk, LO::kRkStages, row0 + (u + 1) * BK, cur.h, 11);
+            }
           }
-          if (v_row >= 0 && (u >= 0 || steps == 0)) {
-            load(&tmap_v, LO::offV, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
-            v_row = -1;
-          }
-          if (u >= 0) {
-            v_row = (cur.t_begin + u) * BK;
-            v_bh = cur.bh;
+          if (LO::kPieces == 1) {
+            if (v_row >= 0 && (u >= 0 || steps == 0)) {
+              load(&tmap_v, LO::offV, LO::kPiece, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
+              v_row = -1;
+            }
+            if (u >= 0) {
+              v_row = (cur.t_begin + u) * BK;
+              v_bh = cur.bh;
+            }
           }
           // The next item is analysed once the loads its predecessor starts with are on their way.  Its slot is that of
           // the item three before it, which is complete only if its last V has been loaded: the load above, whatever
@@ -930,7 +989,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         cur = nxt;
       }
-      if (v_row >= 0) load(&tmap_v, LO::offV, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
+      if (v_row >= 0) load(&tmap_v, LO::offV, LO::kPiece, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
     } else if (warp == kMmaWarp) {
       // -------------------------------------------------------------- MMA issuer
       // C2P blocks and S.  In each issuing role the whole warp walks the items and one elected lane issues
@@ -942,8 +1001,8 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       constexpr uint32_t idesc_nn = ptx::make_idesc_f16(is_bf16, BM, 128, 0, 0);   // 128 x 128, both K-major
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
       constexpr uint32_t sbo = 8 * LO::kRowBytes;
-      constexpr int kSteps = LO::kRowBytes / 32;   // K=16 steps over d
-      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4;
+      constexpr uint32_t idesc_c = ptx::make_idesc_f16(is_bf16, BM, LO::kXcCols, 0, 0);
+      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4, kPieceUnits = (uint32_t)LO::kPiece >> 4;
       const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offQ), 16, sbo, mode);
       const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, sbo, mode);
       const uint64_t rk_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRK), 16, sbo, mode);
@@ -953,23 +1012,20 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       uint32_t c_s = 0, c_xc = 0;                     // S tiles, C2P blocks issued
       bool ok = true;
 
-      // D[128 x 128] = A[128 x d] * B[128 x d]^T, both operands K-major tiles in shared memory
-      auto mma_nn = [&](uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc) {
-#pragma unroll 1
-        for (int kk = 0; kk < kSteps; ++kk)
-          ptx::umma_ss_f16_warp(d_tmem, a_desc + 2u * kk, b_desc + 2u * kk, idesc_nn, kk != 0 ? 1u : 0u);
-      };
-      // new C2P block = Q . rel_key block^T
+      // new C2P block = Q . rel_key block^T, piece by piece
       auto issue_c = [&]() -> bool {
-        const uint32_t st = c_rk % LO::kRkStages, ph = (c_rk / LO::kRkStages) & 1u;
-        if (!wwait(&bars->rk_full[st], ph, 13)) return false;
-        if (!wwait(&bars->xc_free, (c_xc & 1u) ^ 1u, 14)) return false;
-        ptx::tc_fence_after();
-        mma_nn(tmem_base + COL_XC, q_desc, rk_desc + st * kTileUnits);
-        ptx::umma_commit_warp(&bars->rk_empty[st]);
-        ptx::umma_commit_warp(&bars->xc_full);
-        ++c_rk;
-        ++c_xc;
+#pragma unroll 1
+        for (int piece = 0; piece < LO::kPieces; ++piece) {
+          const uint32_t st = c_rk % LO::kRkStages, ph = (c_rk / LO::kRkStages) & 1u;
+          if (!wwait(&bars->rk_full[st], ph, 13)) return false;
+          if (!wwait(&bars->xc_free, (c_xc & 1u) ^ 1u, 14)) return false;
+          ptx::tc_fence_after();
+          mma_over_d<D>(tmem_base + LO::kColXc, q_desc, kTileUnits / LO::kSub, rk_desc + st * kPieceUnits, kPieceUnits / LO::kSub, idesc_c);
+          ptx::umma_commit_warp(&bars->rk_empty[st]);
+          ptx::umma_commit_warp(&bars->xc_full);
+          ++c_rk;
+          ++c_xc;
+        }
         return true;
       };
       int k = 0;
@@ -989,11 +1045,11 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         for (int u = -1; u < n && ok; ++u) {
           if (has_c2p) ok = issue_c();
           if (u < 0 || !ok) continue;
-          const uint32_t kst = c_k & 1u;
-          ok = wwait(&bars->k_full[kst], (c_k >> 1) & 1u, 5) && wwait(&bars->s_free, (c_s & 1u) ^ 1u, 6);
+          const uint32_t kst = c_k % LO::kKStages;
+          ok = wwait(&bars->k_full[kst], (c_k / LO::kKStages) & 1u, 5) && wwait(&bars->s_free, (c_s & 1u) ^ 1u, 6);
           if (!ok) break;
           ptx::tc_fence_after();
-          mma_nn(tmem_base + COL_S, q_desc, k_desc + kst * kTileUnits);
+          mma_over_d<D>(tmem_base + COL_S, q_desc, kTileUnits / LO::kSub, k_desc + kst * kTileUnits, kTileUnits / LO::kSub, idesc_nn);
           ptx::umma_commit_warp(&bars->k_empty[kst]);
           if (u + 1 == n) ptx::umma_commit_warp(&bars->q_empty);
           if (has_p2c) {
@@ -1017,7 +1073,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       // 3 from the second one, which is the first one of the next tile.
       constexpr uint32_t idesc_part = ptx::make_idesc_f16(__is_same(T, __nv_bfloat16) ? 1 : 0, BM, 64, 0, 0);
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
-      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4;
+      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4, kPieceUnits = (uint32_t)LO::kPiece >> 4;
       const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, 8 * LO::kRowBytes, mode);
       const uint64_t rq_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRQ), 16, 8 * LO::kRowBytes, mode);
       uint32_t c_k = 0, c_rq = 0, c_xp = 0;   // key tiles consumed, table blocks released, parts issued
@@ -1032,20 +1088,19 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
 #pragma unroll 1
         for (uint32_t x = 0; x < 4u * (uint32_t)n && ok; ++x) {   // part x & 3 of key tile x >> 2
-          const uint32_t part = x & 3u, kst = c_k & 1u, buf = c_xp & 1u;
-          if (part == 0) ok = wwait(&bars->k_full[kst], (c_k >> 1) & 1u, 43);
-          if (ok && (x == 0 || part == 2)) ok = wwait(&bars->rq_full[c_rq & 1u], (c_rq >> 1) & 1u, 15);   // first use of a block
+          const uint32_t part = x & 3u, kst = c_k % LO::kKStages, buf = c_xp & 1u, rst = c_rq % LO::kRqStages;
+          if (part == 0) ok = wwait(&bars->k_full[kst], (c_k / LO::kKStages) & 1u, 43);
+          if (ok && (LO::kPieces > 1 || x == 0 || part == 2))   // first use of a block, or a piece for this part only
+            ok = wwait(&bars->rq_full[rst], (c_rq / LO::kRqStages) & 1u, 15);
           ok = ok && wwait(&bars->xp_free[buf], ((c_xp >> 1) & 1u) ^ 1u, 16);
           if (!ok) break;
           ptx::tc_fence_after();
-          const uint64_t a_desc = k_desc + kst * kTileUnits, b_desc = rq_desc + (c_rq & 1u) * kTileUnits + buf * (kTileUnits / 2);
-#pragma unroll 1
-          for (int kk = 0; kk < LO::kRowBytes / 32; ++kk)
-            ptx::umma_ss_f16_warp(tmem_base + COL_XP + 64 * buf, a_desc + 2u * kk, b_desc + 2u * kk, idesc_part, kk != 0 ? 1u : 0u);
+          mma_over_d<D>(tmem_base + COL_XP + 64 * buf, k_desc + kst * kTileUnits, kTileUnits / LO::kSub,
+                        rq_desc + rst * kPieceUnits + (LO::kPieces > 1 ? 0u : buf * (kPieceUnits / 2)), kPieceUnits / LO::kSub, idesc_part);
           ptx::umma_commit_warp(&bars->xp_full[buf]);
           ++c_xp;
-          if (part == 1 || x + 1 == 4u * (uint32_t)n) {   // last use of the block
-            ptx::umma_commit_warp(&bars->rq_empty[c_rq & 1u]);
+          if (LO::kPieces > 1 || part == 1 || x + 1 == 4u * (uint32_t)n) {   // last use of the block or piece
+            ptx::umma_commit_warp(&bars->rq_empty[rst]);
             ++c_rq;
           }
           if (part == 3) {
@@ -1059,8 +1114,8 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       constexpr uint32_t idesc_pv = ptx::make_idesc_f16(__is_same(T, __nv_bfloat16) ? 1 : 0, BM, D, 0, 1);   // V is MN-major
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
       constexpr uint32_t kPvStepUnits = (16u * LO::kRowBytes) >> 4;   // 16 keys further down the V tile
-      const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offV), LO::kTile, 8 * LO::kRowBytes, mode);
-      uint32_t c_v = 0, c_items = 0;   // tiles, and items with kept rows, so far
+      const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offV), LO::kPiece / LO::kSub, 8 * LO::kRowBytes, mode);
+      uint32_t c_v = 0, c_t = 0, c_items = 0;   // pieces of V, key tiles, and items with kept rows, so far
       bool ok = true;
       int k = 0;
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
@@ -1068,27 +1123,44 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         ok = wwait(&bars->item_full[slot], (uint32_t)(k / kItemSlots) & 1u, 39);
         if (!ok) break;
         const bool any_kept = slots[slot].any_kept != 0;
-        const int n = slots[slot].t_end - slots[slot].t_begin;
+        const int t_begin = slots[slot].t_begin, n = slots[slot].t_end - t_begin, bh = slots[slot].bh;
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
         if (!any_kept) continue;
-        for (int u = 0; u < n; ++u) {
-          const uint32_t vst = c_v % LO::kVStages, vph = (c_v / LO::kVStages) & 1u;
-          ok = wwait(&bars->v_full[vst], vph, 8);
-          // The output accumulator of the previous item with kept rows has been read out (o_free completes one phase
-          // per such item; this warp is never more than one phase behind, so parities cannot alias).
-          if (ok && u == 0 && c_items > 0) ok = wwait(&bars->o_free, (c_items - 1u) & 1u, 38);
-          if (ok) ok = wwait(&bars->p_full, c_v & 1u, 7);
-          if (!ok) break;
-          ptx::tc_fence_after();
-          const uint64_t vt_desc = v_desc + vst * (uint32_t)(LO::kTile >> 4);
+        for (int u = 0; u < n && ok; ++u) {
 #pragma unroll 1
-          for (int kk = 0; kk < BK / 16; ++kk)
-            ptx::umma_ts_f16_warp(tmem_base + COL_O, tmem_base + COL_P + kk * 8, vt_desc + kk * kPvStepUnits, idesc_pv,
-                                  (u > 0 || kk > 0) ? 1u : 0u);
-          ptx::umma_commit_warp(&bars->v_empty[vst]);
+          for (int piece = 0; piece < LO::kPieces && ok; ++piece) {
+            const uint32_t vst = c_v % LO::kVStages, vph = (c_v / LO::kVStages) & 1u;
+            if (LO::kPieces > 1) {   // loaded here, as soon as the piece before it has been read
+              ok = wwait(&bars->v_empty[vst], vph ^ 1u, 10);
+              if (ok && lane == 0) {
+                ptx::mbar_arrive_expect_tx(&bars->v_full[vst], (uint32_t)LO::kPiece);
+#pragma unroll
+                for (int c = 0; c < LO::kSub; ++c)
+                  ptx::tma_load_3d(smem + LO::offV + c * (LO::kPiece / LO::kSub), &tmap_v, &bars->v_full[vst], 64 * c,
+                                   (t_begin + u) * BK + piece * LO::kPieceRows, bh);
+              }
+              __syncwarp();
+            }
+            if (ok) ok = wwait(&bars->v_full[vst], vph, 8);
+            // The output accumulator of the previous item with kept rows has been read out (o_free completes one phase
+            // per such item; this warp is never more than one phase behind, so parities cannot alias).
+            if (ok && u == 0 && piece == 0 && c_items > 0) ok = wwait(&bars->o_free, (c_items - 1u) & 1u, 38);
+            if (ok && piece == 0) ok = wwait(&bars->p_full, c_t & 1u, 7);
+            if (!ok) break;
+            ptx::tc_fence_after();
+            const uint64_t vt_desc = v_desc + vst * (uint32_t)(LO::kPiece >> 4);
+            const uint32_t p_cols = tmem_base + COL_P + piece * (LO::kPieceRows / 2);
+#pragma unroll 1
+            for (int kk = 0; kk < LO::kPieceRows / 16; ++kk)
+              ptx::umma_ts_f16_warp(tmem_base + COL_O, p_cols + kk * 8, vt_desc + kk * kPvStepUnits, idesc_pv,
+                                    (u > 0 || piece > 0 || kk > 0) ? 1u : 0u);
+            ptx::umma_commit_warp(&bars->v_empty[vst]);
+            ++c_v;
+          }
+          if (!ok) break;
           ptx::umma_commit_warp(&bars->o_ready);
-          ++c_v;
+          ++c_t;
         }
         ++c_items;
       }
@@ -1122,14 +1194,15 @@ int launch_rel_typed(const DflAttnRelParams& p, cudaStream_t stream) {
   const int L = p.seq_len, BH = p.batch * p.heads, R = 2 * L - 1;
   const uint64_t row = (uint64_t)D * sizeof(T), seq = (uint64_t)L * row, table = (uint64_t)R * row;
   CUtensorMap tq, tk, tv, tfk, tfq;
-  int rc = encode_tensor_map_3d(&tq, p.q, D, L, BH, row, seq, D, BM, LO::kRowBytes);
-  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tk, p.k, D, L, BH, row, seq, D, BK, LO::kRowBytes);
-  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tv, p.v, D, L, BH, row, seq, D, BK, LO::kRowBytes);
+  constexpr int kCols = D / LO::kSub;
+  int rc = encode_tensor_map_3d(&tq, p.q, D, L, BH, row, seq, kCols, BM, LO::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tk, p.k, D, L, BH, row, seq, kCols, BK, LO::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tv, p.v, D, L, BH, row, seq, kCols, LO::kPieceRows, LO::kRowBytes);
   // a disabled term reuses the other table's map; it is never dereferenced
   const void* fk = p.rel_key ? p.rel_key : p.rel_query;
   const void* fq = p.rel_query ? p.rel_query : p.rel_key;
-  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfk, fk, D, R, p.heads, row, table, D, BK, LO::kRowBytes);
-  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfq, fq, D, R, p.heads, row, table, D, BK, LO::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfk, fk, D, R, p.heads, row, table, kCols, LO::kPieceRows, LO::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfq, fq, D, R, p.heads, row, table, kCols, LO::kPieceRows, LO::kRowBytes);
   if (rc != DFL_OK) return rc;
 
   auto kernel = attention_rel_kernel<T, D>;
@@ -1155,16 +1228,23 @@ int launch_rel_typed(const DflAttnRelParams& p, cudaStream_t stream) {
 }  // namespace
 
 bool attention_rel_supported(const DflAttnRelParams& p) {
-  return p.dtype != DFL_F32 && (p.head_dim == 32 || p.head_dim == 64) && (p.rel_key || p.rel_query) &&
-         p.seq_len >= 1 && p.seq_len <= kMaxSeqLen;
+  // d = 128 beyond 96 positions: plans of shorter buckets have no relative tables at this head dim, which is part of the
+  // interface.  Above the line one launch beats three at every size: 130 positions 38.8 -> 19.4 us (1 x 8 heads), 512
+  // positions 212 -> 100 us (16 x 8 heads).
+  return p.dtype != DFL_F32 && (p.head_dim == 32 || p.head_dim == 64 || (p.head_dim == 128 && p.seq_len > 96)) &&
+         (p.rel_key || p.rel_query) && p.seq_len >= 1 && p.seq_len <= kMaxSeqLen;
+}
+
+template <typename T>
+int launch_rel(const DflAttnRelParams& p, cudaStream_t stream) {
+  return p.head_dim == 128  ? launch_rel_typed<T, 128>(p, stream)
+         : p.head_dim == 64 ? launch_rel_typed<T, 64>(p, stream)
+                            : launch_rel_typed<T, 32>(p, stream);
 }
 
 int launch_attention_rel(const DflAttnRelParams& p, cudaStream_t stream) {
   if (!attention_rel_supported(p)) return fail(DFL_ERR_UNSUPPORTED, "configuration not covered by the relative-table kernel");
-  if (p.dtype == DFL_F16)
-    return p.head_dim == 64 ? launch_rel_typed<__half, 64>(p, stream) : launch_rel_typed<__half, 32>(p, stream);
-  return p.head_dim == 64 ? launch_rel_typed<__nv_bfloat16, 64>(p, stream)
-                          : launch_rel_typed<__nv_bfloat16, 32>(p, stream);
+  return p.dtype == DFL_F16 ? launch_rel<__half>(p, stream) : launch_rel<__nv_bfloat16>(p, stream);
 }
 
 int launch_expand_rel_tables(const void* pos, const int32_t* lut, void* rel, int heads, int n_active, int seq_len,
