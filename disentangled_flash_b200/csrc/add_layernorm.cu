@@ -20,6 +20,23 @@ namespace {
 
 constexpr int kWarpsPerBlock = 8;
 
+// Two instantiations.  With many rows the kernel is bound by the bytes it keeps in flight, so by the warps an SM holds:
+// the register budget is cut to what the row itself needs, and every row has a warp of its own (the block scheduler
+// evens out what a grid-stride loop leaves unbalanced).  16384 x 768 fp16 17.4 -> 13.9 us, 4096 x 1536 14.5 -> 9.9 us,
+// against one wave of grid-stride blocks at 99 to 124 registers.  With few rows it is bound by its chain of latencies
+// (loads, two reductions, loads, stores): gamma and beta are fetched together with the row.  A forward of 1 x 32 tokens at
+// hidden 768 530 -> 491 us (25 launches), of 8 x 64 at hidden 1536 1850 -> 1780 us (49 launches).
+constexpr int min_blocks(int floats_per_lane, bool few) {
+  return few                     ? 1
+         : floats_per_lane <= 16 ? 5
+         : floats_per_lane <= 24 ? 4
+         : floats_per_lane <= 32 ? 3
+         : floats_per_lane <= 64 ? 2
+                                 : 1;
+}
+// Few: the rows that fit the SMs at the registers of that form, two blocks of eight warps up to 24 values a lane, one beyond.
+constexpr int few_blocks_per_sm(int floats_per_lane) { return floats_per_lane <= 24 ? 2 : 1; }
+
 template <typename T>
 struct Vec16 {
   static constexpr int kElems = 16 / sizeof(T);
@@ -109,13 +126,14 @@ __device__ __forceinline__ long long load_index(const void* idx, int elem, long 
 }
 
 // Vector j of lane l covers columns (j*32 + l) * E .. +E: a warp reads 512 contiguous bytes per vector index.
-template <typename T, int VEC>
-__global__ void __launch_bounds__(kWarpsPerBlock * 32)
+template <typename T, int VEC, bool FEW>
+__global__ void __launch_bounds__(kWarpsPerBlock * 32, min_blocks(VEC * Vec16<T>::kElems, FEW))
 add_layernorm_kernel(const uint4* x, const uint4* residual, const uint4* __restrict__ gamma,
                      const uint4* __restrict__ beta, uint4* out, long long rows, int hidden, float eps,
                      const void* __restrict__ row_mask, int mask_elem, uint4* out2,
                      const int32_t* __restrict__ out2_rows, const RowSource src, uint2* planes) {
   constexpr int E = Vec16<T>::kElems;
+  constexpr bool kEarly = FEW && VEC <= 12;   // four raw rows in registers
   const int lane = threadIdx.x & 31;
   const int vecs_per_row = hidden / E;
   const float inv_n = 1.0f / (float)hidden;
@@ -151,6 +169,15 @@ add_layernorm_kernel(const uint4* x, const uint4* residual, const uint4* __restr
       for (int j = 0; j < VEC; ++j) {
         const int c = j * 32 + lane;
         rres[j] = c < vecs_per_row ? ld_stream(rr + c) : make_uint4(0, 0, 0, 0);
+      }
+    }
+    uint4 rg[kEarly ? VEC : 1], rb[kEarly ? VEC : 1];
+    if constexpr (kEarly) {
+#pragma unroll
+      for (int j = 0; j < VEC; ++j) {
+        const int c = j * 32 + lane;
+        rg[j] = c < vecs_per_row ? ld_stream(gamma + c) : make_uint4(0, 0, 0, 0);
+        rb[j] = c < vecs_per_row && beta ? ld_stream(beta + c) : make_uint4(0, 0, 0, 0);
       }
     }
     float v[VEC * E];
@@ -192,8 +219,8 @@ add_layernorm_kernel(const uint4* x, const uint4* residual, const uint4* __restr
       const int c = j * 32 + lane;
       if (c < vecs_per_row) {
         float g[E], b[E], y[E];
-        unpack<T>(__ldg(gamma + c), g);
-        if (beta) unpack<T>(__ldg(beta + c), b);
+        unpack<T>(kEarly ? rg[kEarly ? j : 0] : __ldg(gamma + c), g);
+        if (beta) unpack<T>(kEarly ? rb[kEarly ? j : 0] : __ldg(beta + c), b);
 #pragma unroll
         for (int e = 0; e < E; ++e) y[e] = fmaf((v[j * E + e] - mean) * rstd, g[e], beta ? b[e] * keep : 0.f);
         const uint4 packed = pack<T>(y);
@@ -217,11 +244,12 @@ void launch_one(const void* x, const void* residual, const void* gamma, const vo
                 int hidden, float eps, const void* row_mask, int mask_elem, void* out2, const int32_t* out2_rows,
                 const RowSource& src, void* planes, int sm_count, cudaStream_t stream) {
   const long long wanted = (rows + kWarpsPerBlock - 1) / kWarpsPerBlock;
-  const long long cap = (long long)sm_count * 8;   // 8 CTAs of 8 warps per SM: one wave, grid-stride beyond it
-  const int blocks = (int)(wanted < cap ? wanted : cap);
-  launch_after_predecessor(add_layernorm_kernel<T, VEC>, dim3(blocks), dim3(kWarpsPerBlock * 32), 0, stream,
-                           (const uint4*)x, (const uint4*)residual, (const uint4*)gamma, (const uint4*)beta, (uint4*)out,
-                           rows, hidden, eps, row_mask, mask_elem, (uint4*)out2, out2_rows, src, (uint2*)planes);
+  const bool few = wanted <= (long long)sm_count * few_blocks_per_sm(VEC * Vec16<T>::kElems);
+  const int blocks = (int)(wanted < 0x7fffffffLL ? wanted : 0x7fffffffLL);
+  launch_after_predecessor(few ? add_layernorm_kernel<T, VEC, true> : add_layernorm_kernel<T, VEC, false>, dim3(blocks),
+                           dim3(kWarpsPerBlock * 32), 0, stream, (const uint4*)x, (const uint4*)residual, (const uint4*)gamma,
+                           (const uint4*)beta, (uint4*)out, rows, hidden, eps, row_mask, mask_elem, (uint4*)out2, out2_rows, src,
+                           (uint2*)planes);
 }
 
 template <typename T>
@@ -283,7 +311,7 @@ int launch_rows(const void* x, const void* residual, const void* gamma, const vo
                 const int32_t* out2_rows, const RowSource& src, void* planes, cudaStream_t stream) {
   static KernelDeviceConfig config;   // only the SM count of the current device is needed (no shared memory)
   int sm_count = 0;
-  if (int rc = configure_kernel(config, add_layernorm_kernel<float, 1>, 0, &sm_count, "add_layernorm_kernel")) return rc;
+  if (int rc = configure_kernel(config, add_layernorm_kernel<float, 1, true>, 0, &sm_count, "add_layernorm_kernel")) return rc;
   switch (dtype) {
     case DFL_F16: return launch_typed<__half>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, planes, sm_count, stream);
     case DFL_BF16: return launch_typed<__nv_bfloat16>(x, residual, gamma, beta, out, rows, hidden, eps, row_mask, mask_elem, out2, out2_rows, src, planes, sm_count, stream);
