@@ -1242,8 +1242,9 @@ int launch_rel(const DflAttnRelParams& p, cudaStream_t stream) {
                             : launch_rel_typed<T, 32>(p, stream);
 }
 
-int launch_attention_rel(const DflAttnRelParams& p, cudaStream_t stream) {
+int launch_attention_rel(const DflAttnRelParams& p, cudaStream_t stream, bool tables_early) {
   if (!attention_rel_supported(p)) return fail(DFL_ERR_UNSUPPORTED, "configuration not covered by the relative-table kernel");
+  if (attention_rel_small_covers(p)) return launch_attention_rel_small(p, tables_early, stream);
   return p.dtype == DFL_F16 ? launch_rel<__half>(p, stream) : launch_rel<__nv_bfloat16>(p, stream);
 }
 

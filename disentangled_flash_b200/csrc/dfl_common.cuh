@@ -221,7 +221,10 @@ bool attention_f32_planes_supported(int head_dim, int seq_len);
 int launch_attention_f32_planes(const DflAttnParams& p, int out_planes, cudaStream_t stream);
 int launch_attention_tc(const DflAttnParams& p, cudaStream_t stream);
 bool attention_rel_supported(const DflAttnRelParams& p);
-int launch_attention_rel(const DflAttnRelParams& p, cudaStream_t stream);
+// tables_early: rel_key / rel_query were complete before the kernel ahead of this one in the stream started
+int launch_attention_rel(const DflAttnRelParams& p, cudaStream_t stream, bool tables_early = false);
+bool attention_rel_small_covers(const DflAttnRelParams& p);
+int launch_attention_rel_small(const DflAttnRelParams& p, bool tables_early, cudaStream_t stream);
 int add_layernorm_max_hidden(size_t elem_size);
 int launch_add_layernorm(const void* x, const void* residual, const void* gamma, const void* beta, void* out,
                          long long rows, int hidden, float eps, int dtype, const void* row_mask, int mask_elem,

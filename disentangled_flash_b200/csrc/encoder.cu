@@ -179,7 +179,7 @@ struct Loop {
         a.out_row_count = p.row_count;
       }
       ++p.launches;
-      rc = dfl_attention_rel_fwd(&a, stream);
+      rc = launch_attention_rel(a, stream, true);   // the projection ran between the tables and this launch
     } else {
       DflAttnParams a{};
       const int ld = (p.n_active + 7) / 8 * 8;

@@ -1,0 +1,40 @@
+"""The short-sequence form of the relative-table attention: row and key remainders of its three sizes, masks and single
+terms, the packed output, and the batch size at which 65 .. 128 positions go to the other kernel."""
+
+import pytest
+import torch
+
+from helpers import assert_close, make_core_case, oracle_core
+from test_gpu_rel_attention import DTYPES, dev, expand, run_rel
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("dtype_name", sorted(DTYPES))
+@pytest.mark.parametrize("d", (32, 64))
+@pytest.mark.parametrize("batch,heads,length,mask,mode", (
+    (1, 1, 1, "none", "both"), (3, 2, 15, "right", "c2p"), (2, 3, 16, "left", "p2c"), (3, 5, 17, "heavy", "both"),
+    (2, 2, 31, "all", "both"), (40, 12, 33, "right", "both"), (3, 2, 48, "left", "c2p"), (2, 2, 63, "heavy", "p2c"),
+    (3, 3, 81, "left", "both"), (2, 2, 113, "all", "p2c"), (12, 12, 127, "right", "both"), (16, 12, 127, "right", "both")))
+def test_short_sequences(dtype_name, d, batch, heads, length, mask, mode):
+    dtype = DTYPES[dtype_name]
+    case = make_core_case(batch, heads, length, d, dtype, seed=length, mask=mask, mode=mode)
+    got = run_rel(case)
+    assert_close(got, oracle_core(case), dtype, f"L={length} d={d} mask={mask} mode={mode}")
+    assert torch.equal(got, run_rel(case)), "two identical launches differ"
+
+
+@pytest.mark.parametrize("length", (24, 64, 90))
+def test_short_packed_output(length):
+    from disentangled_flash_b200 import _cabi as c
+
+    case = make_core_case(3, 2, length, 64, torch.float16, seed=7, mask="right")
+    full = run_rel(case)
+    counts = [min(length, -(-int(n) // 32) * 32) for n in case["mask"].sum(dim=1)]
+    bases = [0, counts[0], counts[0] + counts[1]]
+    rel_key, rel_query = expand(case)
+    tables = tuple(torch.tensor(x, dtype=torch.int32, device=dev) for x in (bases, counts))
+    packed = c.attention_rel_fwd(case["q"].to(dev), case["k"].to(dev), case["v"].to(dev), rel_key, rel_query,
+                                 case["mask"].to(dev), case["scale"], packed_rows=(*tables, sum(counts)))
+    for b in range(3):
+        assert torch.equal(packed[bases[b]:bases[b] + counts[b]], full[b, :counts[b]]), b
