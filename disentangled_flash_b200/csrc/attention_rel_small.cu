@@ -268,10 +268,13 @@ int launch_small(const DflAttnRelParams& p, bool tables_early, cudaStream_t stre
   return check_launch("attention_rel_small_kernel");
 }
 
+// Sizes of 2, 4, 6 and 8 warps: a row's windows are as wide as the size.  80 positions in six warps instead of eight
+// 8.1 -> 7.4 us (4 x 12 heads), a forward of 8 x 96 tokens 553 -> 537 us.
 template <typename T, int D>
 int launch_rows(const DflAttnRelParams& p, bool tables_early, cudaStream_t stream) {
   return p.seq_len <= 32   ? launch_small<T, D, 2>(p, tables_early, stream)
          : p.seq_len <= 64 ? launch_small<T, D, 4>(p, tables_early, stream)
+         : p.seq_len <= 96 ? launch_small<T, D, 6>(p, tables_early, stream)
                            : launch_small<T, D, 8>(p, tables_early, stream);
 }
 
