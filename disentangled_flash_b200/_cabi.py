@@ -368,6 +368,9 @@ def linear_heads(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | Non
     m, k = x2.shape
     if weight.shape != (n_out * heads * head_dim, k):
         raise ValueError(f"weight shape {tuple(weight.shape)} does not match [{n_out * heads * head_dim}, {k}]")
+    for name, t in (("weight", weight), ("bias", bias)):
+        if t is not None and (t.dtype != x.dtype or t.device != x.device):
+            raise TypeError(f"{name} must be of the dtype and on the device of x ({x.dtype}, {x.device})")
     p = DflLinearParams()
     if row_groups is not None:
         if outs is None or len(outs) != n_out:

@@ -146,31 +146,47 @@ class _LayerCall:
     ``attention_only``): less host time per call, and in FP32 the tensor-core GEMMs over bf16 planes."""
 
     def __init__(self, module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> None:
-        self.plan, self.qkv_weight = plan, module._cached_qkv_weight
         weight = module._cached_qkv_weight
+        # what the addresses below were taken from; held, so that they stay valid as long as this object
+        self.plan, self.tensors, self.terms = plan, self._tensors(module), (module.has_c2p, module.has_p2c)
         self.layers = (_cabi.DflEncoderLayer * 1)()
         fill_attention_fields(self.layers[0], module, plan)
         p = self.params = _cabi.DflEncoderParams()
         p.layers, p.n_layers, p.attention_only = self.layers, 1, 1
         p.seq_len, p.hidden, p.heads = plan.sequence_length, weight.shape[1], module.num_attention_heads
-        p.head_dim, p.dtype, p.scale = module.attention_head_size, _cabi.dtype_code(weight.dtype), module._score_scale()
+        p.head_dim, p.dtype = module.attention_head_size, _cabi.dtype_code(weight.dtype)
         p.lut, p.n_active = plan.delta_to_local.data_ptr(), plan.active_slots.numel()
         self.width = module.all_head_size
 
     @staticmethod
-    def covers(module: "DisentangledFlashAttention", length: int) -> bool:
+    def _tensors(module: "DisentangledFlashAttention") -> tuple[torch.Tensor | None, ...]:
+        return module._cached_qkv_weight, module._cached_qkv_bias, module._cached_qkv_planes
+
+    @staticmethod
+    def covers(module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> bool:
         if module._algo != _cabi.ALGO_AUTO or module._cached_qkv_weight.shape[1] % 8:
             return False
-        f32 = module._cached_qkv_weight.dtype == torch.float32
-        return not f32 or (module._cached_qkv_planes is not None and _cabi.f32_planes_supported(module.attention_head_size, length))
+        if module._cached_qkv_weight.dtype != torch.float32:
+            return True
+        if module._cached_qkv_planes is None or not _cabi.f32_planes_supported(module.attention_head_size, plan.sequence_length):
+            return False
+        # a plan without planes (of a module prepared otherwise, or built field by field) has its terms in fp32 only
+        return not ((module.has_c2p and plan.pos_key_planes is None) or (module.has_p2c and plan.pos_query_planes is None))
 
-    def __call__(self, hidden_states: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None) -> torch.Tensor:
+    def serves(self, module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> bool:
+        """Whether this object was made from the module's and the plan's present tensors and terms."""
+
+        return (self.plan is plan and self.terms == (module.has_c2p, module.has_p2c)
+                and all(a is b for a, b in zip(self.tensors, self._tensors(module))))
+
+    def __call__(self, module: "DisentangledFlashAttention", hidden_states: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         p = _cabi.DflEncoderParams()
         ctypes.pointer(p)[0] = self.params   # a copy: several threads may run one module
         out = torch.empty(*hidden_states.shape[:2], self.width, dtype=hidden_states.dtype, device=hidden_states.device)
         p.x, p.mask, p.mask_elem_size, p.batch = hidden_states.data_ptr(), mask.data_ptr(), mask.element_size(), hidden_states.shape[0]
         p.outs = (ctypes.c_void_p * 1)(out.data_ptr())
-        p.status = None if status is None else status.data_ptr()
+        status = module._status_word
+        p.scale, p.status = module._score_scale(), None if status is None else status.data_ptr()
         _cabi.encoder_fwd(p, hidden_states.device)
         return out
 
@@ -251,7 +267,7 @@ class DisentangledFlashAttention(nn.Module):
         # shares one word between its layers (set_status_word) and reads it in check_device_status()
         self.register_buffer("_status_word", None, persistent=False)
         self._position_projection_cache: dict[tuple[int, str], B200PreparedPositionPlan] = {}
-        self._layer_calls: dict[int, _LayerCall] = {}   # per sequence length
+        self._layer_calls: dict[int, _LayerCall | None] = {}   # per sequence length
         self._algo = _cabi.ALGO_AUTO
         self.register_load_state_dict_post_hook(_invalidate_attention_cache_after_load)
 
@@ -440,6 +456,36 @@ class DisentangledFlashAttention(nn.Module):
         if torch.is_grad_enabled():
             raise RuntimeError("DisentangledFlashAttention requires torch.no_grad() or torch.inference_mode()")
 
+    def _require_inputs_of_this_module(self, hidden_states: torch.Tensor, attention_mask: torch.Tensor) -> None:
+        """Refuse what the kernels, which see addresses only, would read past its end or on another device."""
+
+        weight = self._cached_qkv_weight
+        batch_size, sequence_length = hidden_states.shape[:2]
+        if hidden_states.shape[-1] != weight.shape[1] or hidden_states.numel() != batch_size * sequence_length * weight.shape[1]:
+            raise ValueError(f"hidden_states shape {tuple(hidden_states.shape)} does not match [B, L, {weight.shape[1]}]")
+        if hidden_states.device != weight.device:
+            raise RuntimeError(f"hidden_states is on {hidden_states.device}, the module on {weight.device}")
+        if attention_mask.device != hidden_states.device:
+            raise RuntimeError(f"attention_mask must be on the device of hidden_states ({hidden_states.device}), "
+                               f"got {attention_mask.device}")
+
+    def _require_plan_of_this_module(self, plan: B200PreparedPositionPlan, device: torch.device) -> None:
+        """Refuse a plan whose tables have another geometry, type or device than this module's."""
+
+        dtype, heads, head_dim = self._cached_qkv_weight.dtype, self.num_attention_heads, self.attention_head_size
+        distances, slots = 2 * plan.sequence_length - 1, plan.active_slots.numel()
+        wanted = [("delta_to_local", plan.delta_to_local, (distances,), torch.int32)]
+        for enabled, names in ((self.has_c2p, ("pos_key", "rel_key")), (self.has_p2c, ("pos_query", "rel_query"))):
+            if enabled:
+                wanted.append((names[0], getattr(plan, names[0]), (heads, slots, head_dim), dtype))
+                wanted.append((names[1], getattr(plan, names[1]), (heads, distances, head_dim), dtype))
+                wanted.append((names[0] + "_planes", getattr(plan, names[0] + "_planes"), (3, heads, slots, head_dim), torch.bfloat16))
+        for name, table, shape, wanted_dtype in wanted:
+            if table is not None and (table.shape != shape or table.dtype != wanted_dtype or table.device != device
+                                      or not table.is_contiguous()):
+                raise ValueError(f"the plan's {name} is {tuple(table.shape)} of {table.dtype} on {table.device}: this module takes "
+                                 f"{shape} of {wanted_dtype} on {device}")
+
     def _project_qkv(self, hidden_states: torch.Tensor):
         """Fused QKV projection; returns ``q, k, v`` head-major ``[B, H, L, d]``.
 
@@ -471,6 +517,7 @@ class DisentangledFlashAttention(nn.Module):
             raise RuntimeError("fused QKV projection is not prepared; call prepare_for_inference() first")
         if hidden_states.dtype != self._cached_qkv_weight.dtype:
             raise TypeError("hidden_states dtype does not match the module's parameters")
+        self._require_inputs_of_this_module(hidden_states, attention_mask)
         base_mask = _require_2d_padding_mask(attention_mask, batch_size, sequence_length)
         if self.has_c2p and plan.pos_key is None:
             raise ValueError("prepared plan has no content-to-position keys")
@@ -478,11 +525,12 @@ class DisentangledFlashAttention(nn.Module):
             raise ValueError("prepared plan has no position-to-content queries")
 
         if not torch.compiler.is_compiling():
+            self._require_plan_of_this_module(plan, hidden_states.device)
             call = self._layer_calls.get(sequence_length)
-            if call is None or call.plan is not plan or call.qkv_weight is not self._cached_qkv_weight:
-                call = self._layer_calls[sequence_length] = _LayerCall(self, plan) if _LayerCall.covers(self, sequence_length) else None
+            if call is None or not call.serves(self, plan):
+                call = self._layer_calls[sequence_length] = _LayerCall(self, plan) if _LayerCall.covers(self, plan) else None
             if call is not None and self._algo == _cabi.ALGO_AUTO:
-                return call(hidden_states.contiguous(), base_mask, self._status_word), None
+                return call(self, hidden_states.contiguous(), base_mask), None
         uses_lut = self.has_c2p or self.has_p2c
         output = (_attention_forward_op if torch.compiler.is_compiling() else _attention_forward)(
             hidden_states.contiguous(),
@@ -527,6 +575,9 @@ class DisentangledFlashAttention(nn.Module):
         rel_query = plan.rel_query if self.has_p2c else None
         if rel_key is None and rel_query is None:
             raise NotImplementedError("packed rows need the single-launch attention path (expanded position tables)")
+        if attention_mask.device != hidden_states.device:
+            raise RuntimeError(f"attention_mask must be on the device of hidden_states ({hidden_states.device}), "
+                               f"got {attention_mask.device}")
         base_mask = _require_2d_padding_mask(attention_mask, batch_size, sequence_length)
         row_groups, buffers = packed_input if packed_input is not None else (None, None)
         query, key, value = _cabi.linear_heads(
