@@ -183,6 +183,9 @@ class LayerLoop:
         if conv is not None:
             first: list[torch.Tensor] = []
             state = conv(hidden, self._run(hidden, mask, status, first, 0, 1), mask)
+            if state.shape != hidden.shape or state.dtype != self.dtype or state.device != self.device:
+                raise ValueError(f"the convolution branch returned {tuple(state.shape)} of {state.dtype} on {state.device}, "
+                                 f"the layers take {tuple(hidden.shape)} of {self.dtype} on {self.device}")
             if trace is not None:
                 trace.append(state)
             return self._run(state, mask, status, trace, 1, self.n_layers) if self.n_layers > 1 else state
