@@ -11,6 +11,7 @@ preparation is never read at its old place.
 from __future__ import annotations
 
 import ctypes
+from collections.abc import Callable
 from typing import Any
 
 import torch
@@ -177,12 +178,12 @@ class LayerLoop:
         return p
 
     def run(self, hidden: torch.Tensor, mask: torch.Tensor, status: torch.Tensor | None,
-            trace: list[torch.Tensor] | None, conv: Any = None) -> torch.Tensor:
-        """``conv``: a convolution branch that is not part of the native loop, called after layer 0."""
+            trace: list[torch.Tensor] | None, conv: Callable[[torch.Tensor], torch.Tensor] | None = None) -> torch.Tensor:
+        """``conv``: a convolution branch that is not part of the native loop, called with the state after layer 0."""
 
         if conv is not None:
             first: list[torch.Tensor] = []
-            state = conv(hidden, self._run(hidden, mask, status, first, 0, 1), mask)
+            state = conv(self._run(hidden, mask, status, first, 0, 1))
             if state.shape != hidden.shape or state.dtype != self.dtype or state.device != self.device:
                 raise ValueError(f"the convolution branch returned {tuple(state.shape)} of {state.dtype} on {state.device}, "
                                  f"the layers take {tuple(hidden.shape)} of {self.dtype} on {self.device}")
