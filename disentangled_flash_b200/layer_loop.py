@@ -3,15 +3,19 @@
 Built by ``DebertaV2InferenceEncoder.prepare_for_inference`` for a bucket whose layers all have the Hugging Face shape;
 the encoder's Python loop serves everything else.  In FP32 the weight matrices are held as bf16 planes
 (``dfl_split_planes``) for the tensor-core GEMMs, made once per encoder; a weight modified in place after that sends the
-calls to the Python loop until the next preparation.  A convolution branch stays the caller's module in FP32.  Holds the pointers of every parameter the loop reads
-and compares them with the modules' current ones before each call, so a parameter that was exchanged or moved after the
-preparation is never read at its old place.
+calls to the Python loop until the next preparation.  A convolution branch stays the caller's module in FP32.
+
+The native call reads the modules' parameters by address.  Before each call the state the addresses were taken from is
+compared with the present one: the modules, where and in which form their parameters lie, and the settings that went into
+the call.  Whatever was exchanged, moved or changed after the preparation, the call then takes the Python loop, which
+reads the modules as they are.
 """
 
 from __future__ import annotations
 
 import ctypes
 from collections.abc import Callable
+from operator import itemgetter
 from typing import Any
 
 import torch
@@ -29,7 +33,8 @@ _LAYER_FIELDS = (
     ("ffn_norm_w", "output.LayerNorm", "weight"), ("ffn_norm_b", "output.LayerNorm", "bias"),
 )
 _PLANE_FIELDS = ("attn_out_w", "ffn_in_w", "ffn_out_w")   # weight matrices given as planes in FP32
-_data_ptr = torch.Tensor.data_ptr
+_data_ptr, _dtype = torch.Tensor.data_ptr, torch.Tensor.dtype.__get__
+_shape, _stride = torch.Tensor.shape.__get__, torch.Tensor.stride
 
 
 def version_of(tensor: torch.Tensor) -> int:
@@ -38,18 +43,21 @@ def version_of(tensor: torch.Tensor) -> int:
     return -1 if tensor.is_inference() else tensor._version
 
 
-def _module_at(root: nn.Module, path: str) -> nn.Module:
-    for name in path.split("."):
-        root = getattr(root, name)
-    return root
-
-
 class LayerLoop:
     """One bucket of one encoder.  ``build`` returns None where the loop does not cover the encoder."""
 
     def __init__(self) -> None:
         self.plans: Any = None
         self.length = 0
+        # The state a call is compared with (see covers()).  A dict of sub-modules or of instance attributes belongs to its
+        # module, so an exchanged module shows up in the dict of its parent.
+        self._children: list[dict] = []   # module._modules of every module on the way to a parameter
+        self._owners: list[dict] = []     # (dict, key) of every tensor the loop reads
+        self._keys: list[str] = []
+        self._matrices: list[int] = []    # which of them have more than one dimension
+        self._settings: list[dict] = []   # (instance attributes, name): eps, training, the activation, ...
+        self._names: list[str] = []
+        self._hooks: list[dict] = []      # forward hooks of modules the native call stands in for
 
     @staticmethod
     def build(encoder: nn.Module, length: int, plans: Any, conv_covered: bool) -> "LayerLoop | None":
@@ -57,7 +65,7 @@ class LayerLoop:
         weight = first.query_proj.weight
         dtype, device = weight.dtype, weight.device
         f32 = dtype == torch.float32
-        if device.type != "cuda" or dtype not in (torch.float16, torch.bfloat16, torch.float32):
+        if dtype not in (torch.float16, torch.bfloat16, torch.float32):
             return None
         if not (all(a and b for a, b in encoder._fused_output_blocks) and (f32 or all(encoder._fused_intermediates))):
             return None
@@ -65,7 +73,7 @@ class LayerLoop:
             return None
         self = LayerLoop()
         self.plans, self.length, self.device, self.dtype, self.f32 = plans, length, device, dtype, f32
-        self.attention = [layer.attention.self for layer in encoder.layer]
+        self.layer, self.conv = encoder.layer, encoder.conv
         hidden, ffn = weight.shape[1], encoder.layer[0].intermediate.dense.weight.shape[0]
         width = first.all_head_size
         if hidden % 8 or ffn % 8 or first.attention_head_size not in (32, 64, 128):
@@ -74,9 +82,6 @@ class LayerLoop:
             return None
         n = len(encoder.layer)
         self.layers = (_cabi.DflEncoderLayer * n)()
-        # (owner dict, key) of every tensor the loop reads, and where it was
-        self._owners: list[dict] = []
-        self._keys: list[str] = []
         self._planes: list[torch.Tensor] = []
 
         def read(module: nn.Module, key: str) -> torch.Tensor | None:
@@ -87,23 +92,34 @@ class LayerLoop:
                         raise _NotCovered
                     self._owners.append(owner)
                     self._keys.append(key)
+                    if tensor.dim() > 1:
+                        self._matrices.append(len(self._keys) - 1)
                     return tensor
+            self._settings += [module._parameters, module._buffers]   # none, and none may appear
+            self._names += [key, key]
             return None
 
         shapes = {"attn_out_w": (hidden, width), "ffn_in_w": (ffn, hidden),
                   "ffn_out_w": (hidden, ffn), "attn_norm_w": (hidden,), "ffn_norm_w": (hidden,)}
         try:
+            self._walk(encoder.layer)
             for index, layer in enumerate(encoder.layer):
                 entry, plan = self.layers[index], plans[index]
+                self._walk(layer, layer.attention, layer.attention.output, layer.intermediate, layer.output)
                 for _, path, key in _ATTENTION_FIELDS:
-                    read(_module_at(layer, path), key)
+                    read(layer.get_submodule(path), key)
                 module = layer.attention.self
                 if module._cached_qkv_weight.shape != (3 * width, hidden) or (f32 and module._cached_qkv_planes is None):
                     return None
+                if module.training or module._algo != _cabi.ALGO_AUTO:
+                    return None
+                self._watch(module, "training", "_algo", "relative_attention", "pos_att_type")
                 fill_attention_fields(entry, module, plan)
+                if f32:
+                    self._owners.append(module._buffers)
+                    self._keys.append("_cached_qkv_planes")
                 for field, path, key in _LAYER_FIELDS:
-                    owner = _module_at(layer, path)
-                    tensor = read(owner, key)
+                    tensor = read(layer.get_submodule(path), key)
                     if field in shapes and (tensor is None or tuple(tensor.shape) != shapes[field]):
                         return None
                     if f32 and field in _PLANE_FIELDS:
@@ -112,10 +128,22 @@ class LayerLoop:
                     setattr(entry, field, None if tensor is None else tensor.data_ptr())
                 entry.attn_norm_eps = float(layer.attention.output.LayerNorm.eps)
                 entry.ffn_norm_eps = float(layer.output.LayerNorm.eps)
+                self._watch(layer.attention.output.LayerNorm, "eps")
+                self._watch(layer.output.LayerNorm, "eps")
+                activation = layer.intermediate.intermediate_act_fn
+                self._watch(layer.intermediate, "intermediate_act_fn")
+                if isinstance(activation, nn.Module):
+                    self._watch(activation, "approximate", "act")
+                if f32:   # the Python loop calls this block as the module it is
+                    self._stand_in_for(layer.intermediate)
+                    self._stand_in_for(layer.intermediate.dense, nn.Linear)
+                    if isinstance(activation, nn.Module):
+                        self._stand_in_for(activation)
                 if (module.has_c2p, module.has_p2c, module.pos_att_type) != (first.has_c2p, first.has_p2c, first.pos_att_type):
                     return None
             p = _cabi.DflEncoderParams()
             if encoder.conv is not None and not f32:
+                self._walk(encoder.conv)
                 norm = encoder.conv.LayerNorm
                 bias = read(encoder.conv.conv, "bias")
                 gamma, beta = read(norm, "weight"), read(norm, "bias")
@@ -125,9 +153,23 @@ class LayerLoop:
                 p.conv_norm_w, p.conv_norm_b = gamma.data_ptr(), None if beta is None else beta.data_ptr()
                 p.conv_taps, p.conv_activation = self._conv_weight.shape[0], encoder._conv_activation_code
                 p.conv_norm_eps = float(norm.eps)
+                self._watch(norm, "eps")
+                if not encoder._conv_fused[length]:   # the Python loop calls this branch as the module it is
+                    self._watch(encoder.conv, "conv_act")
+                    self._stand_in_for(encoder.conv)
+                    self._stand_in_for(encoder.conv.conv, nn.Conv1d)
+                    self._stand_in_for(norm, nn.LayerNorm)
+                    dropout = encoder.conv._modules.get("dropout")
+                    if dropout is not None:
+                        if dropout.training:
+                            return None
+                        self._stand_in_for(dropout)
+                        self._watch(dropout, "training")
         except _NotCovered:
             return None
-        self._pointers = self._current_state()
+        self._pick = itemgetter(*self._matrices)
+        state = self._current_state()
+        self._state = (*state[:4], list(map(dict.copy, self._children)), *state[5:])
         lut = plans[0].delta_to_local
         p.layers, p.n_layers = self.layers, n
         p.seq_len, p.hidden, p.heads, p.head_dim, p.ffn = length, hidden, first.num_attention_heads, first.attention_head_size, ffn
@@ -136,12 +178,31 @@ class LayerLoop:
         self.params, self.n_layers, self.hidden = p, n, hidden
         return self
 
-    def _current_state(self) -> list[int]:
-        """Address of every tensor the loop reads; in FP32, where copies of the weights are read, their versions too."""
+    def _walk(self, *modules: nn.Module) -> None:
+        self._children += [module._modules for module in modules]
+
+    def _watch(self, module: nn.Module, *names: str) -> None:
+        self._settings += [module.__dict__] * len(names)
+        self._names += names
+
+    def _stand_in_for(self, module: nn.Module, kind: type[nn.Module] | None = None) -> None:
+        """The native call does what ``module`` does: not if it (a ``kind``) has a forward of its own, or hooks."""
+
+        if kind is not None and type(module).forward is not kind.forward:
+            raise _NotCovered
+        self._watch(module, "forward")
+        self._hooks += [module._forward_hooks, module._forward_pre_hooks]
+
+    def _current_state(self) -> tuple:
+        """What the addresses in the native call depend on, some 30 us for 12 layers: per tensor the address and the type,
+        of a matrix also its form (``.data = other`` changes them under the same name); in FP32, where copies of the
+        weights are read, the versions too."""
 
         tensors = list(map(dict.__getitem__, self._owners, self._keys))
-        state = list(map(_data_ptr, tensors))
-        return state + list(map(version_of, tensors)) if self.f32 else state
+        matrices = self._pick(tensors)
+        return (list(map(_data_ptr, tensors)), list(map(_dtype, tensors)), list(map(_shape, matrices)), list(map(_stride, matrices)),
+                self._children, list(map(dict.get, self._settings, self._names)),
+                list(map(version_of, tensors)) if self.f32 else None)
 
     def covers(self, encoder: nn.Module, plans: Any, hidden: torch.Tensor, mask: torch.Tensor) -> bool:
         """Whether this call can take the native loop (the state it was built from still holds)."""
@@ -152,17 +213,16 @@ class LayerLoop:
             return False
         if mask.shape != hidden.shape[:2] or mask.device != self.device or torch.is_grad_enabled():
             return False
+        if encoder.layer is not self.layer or encoder.conv is not self.conv or any(self._hooks):
+            return False
         for fused in encoder._fused_output_blocks:
             if not (fused[0] and fused[1]):
                 return False
         if not self.f32 and not all(encoder._fused_intermediates):
             return False
-        for module in self.attention:
-            if module.training or module._algo != _cabi.ALGO_AUTO:
-                return False
         try:
-            return self._current_state() == self._pointers
-        except (KeyError, TypeError, AttributeError):   # a parameter was deleted or set to None
+            return self._current_state() == self._state
+        except (KeyError, TypeError, AttributeError, RuntimeError):   # a parameter was deleted, or set to or from None
             return False
 
     def _call(self, hidden: torch.Tensor, mask: torch.Tensor, outs: Any, status: torch.Tensor | None) -> _cabi.DflEncoderParams:
