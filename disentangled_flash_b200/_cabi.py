@@ -55,6 +55,7 @@ EXPORTED_SYMBOLS = (
     "dfl_attention_rel_fwd",
     "dfl_qkv_proj_planes",
     "dfl_split_planes",
+    "dfl_refresh_planes",
     "dfl_f32_planes_supported",
     "dfl_encoder_workspace_bytes",
     "dfl_encoder_fwd",
@@ -156,7 +157,8 @@ class DflEncoderParams(Structure):
         ("scale", c_float), ("attention_events", POINTER(c_void_p)), ("launches", c_int32), ("attention_only", c_int32),
         ("packed_rows", c_int32),
         ("pack_rows", c_void_p), ("row_groups", c_void_p), ("row_base", c_void_p), ("row_count", c_void_p),
-        ("qkv", c_void_p * 3),
+        ("qkv", c_void_p * 3), ("conv_w_module", c_int32),
+        ("plane_sources", c_void_p), ("n_plane_sources", c_int32), ("n_plane_pieces", ctypes.c_int64),
     ]
 
 
@@ -229,6 +231,8 @@ def load_library() -> ctypes.CDLL:
     lib.dfl_f32_planes_supported.argtypes = [c_int, c_int]
     lib.dfl_split_planes.restype = c_int
     lib.dfl_split_planes.argtypes = [c_void_p, c_void_p, ctypes.c_int64, c_void_p]
+    lib.dfl_refresh_planes.restype = c_int
+    lib.dfl_refresh_planes.argtypes = [c_void_p, c_int32, ctypes.c_int64, c_void_p]
     lib.dfl_encoder_workspace_bytes.restype = ctypes.c_size_t
     lib.dfl_encoder_workspace_bytes.argtypes = [POINTER(DflEncoderParams)]
     lib.dfl_encoder_fwd.restype = c_int
@@ -759,6 +763,36 @@ def split_planes(x: torch.Tensor) -> torch.Tensor:
     with _on_device(x.device):
         _check(lib.dfl_split_planes(x.data_ptr(), planes.data_ptr(), x.numel(), _stream(x.device)), "dfl_split_planes")
     return planes
+
+
+class FollowingPlanes:
+    """The bf16 planes of FP32 matrices, kept equal to them by ``refresh`` (``dfl_refresh_planes``; also the first launch of
+    an ``encoder_fwd`` given them).  Holds no reference to the matrices: the caller compares their addresses."""
+
+    PIECE = 1024   # DFL_PLANE_PIECE
+
+    def __init__(self, matrices: list[torch.Tensor]) -> None:
+        self.addresses = [m.data_ptr() for m in matrices]
+        device = matrices[0].device
+        pieces = [-(-m.numel() // self.PIECE) for m in matrices]
+        for m in matrices:
+            if m.dtype != torch.float32 or m.device != device or not m.is_contiguous() or m.numel() % 4 or m.data_ptr() % 16:
+                raise ValueError("planes follow contiguous, 16-byte aligned FP32 matrices of one device")
+        self.planes = [torch.empty(3, *m.shape, dtype=torch.bfloat16, device=device) for m in matrices]
+        self.n_sources, self.n_pieces = len(matrices), sum(pieces)
+        self.digests = torch.zeros(self.n_pieces, 2, dtype=torch.int64, device=device)
+        rows, first = [], 0
+        for m, planes, count in zip(matrices, self.planes, pieces):
+            rows.append([m.data_ptr(), planes.data_ptr(), self.digests.data_ptr() + 16 * first, m.numel(), first])
+            first += count
+        self.sources = torch.tensor(rows, dtype=torch.int64).to(device)
+        self.refresh()
+
+    def refresh(self) -> None:
+        device = self.sources.device
+        with _on_device(device):
+            _check(load_library().dfl_refresh_planes(self.sources.data_ptr(), self.n_sources, self.n_pieces, _stream(device)),
+                   "dfl_refresh_planes")
 
 
 def linear_heads_planes(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tensor | None, *, heads: int, head_dim: int,

@@ -288,7 +288,39 @@ __global__ void __launch_bounds__(256) copy_rows_kernel(const uint4* __restrict_
       dst[r * vecs_per_row + c] = from >= 0 ? src[from * vecs_per_row + c] : make_uint4(0, 0, 0, 0);
   }
 }
+
+// dst[t][o][i] = src[o][i][t], 2-byte elements, eight i per thread, a block's part of src through shared memory.  It runs
+// beside the kernel ahead of it: the work comes first and the wait last, so that whatever waits for this kernel has waited
+// for that one too.
+__global__ void __launch_bounds__(256) conv_weight_kernel(const uint4* __restrict__ src, uint4* __restrict__ dst, long long n, int taps) {
+  extern __shared__ uint4 part[];   // [256 * taps]
+  const long long first = blockIdx.x * 256ll;   // of the n groups of eight i
+  const int groups = (int)(n - first < 256 ? n - first : 256);
+#pragma unroll 3
+  for (int x = threadIdx.x; x < groups * taps; x += 256) part[x] = src[first * taps + x];
+  __syncthreads();
+  if ((int)threadIdx.x < groups) {
+    const uint16_t* mine = reinterpret_cast<const uint16_t*>(part) + threadIdx.x * 8 * taps;
+    for (int t = 0; t < taps; ++t) {
+      uint32_t v[8];
+#pragma unroll
+      for (int j = 0; j < 8; ++j) v[j] = mine[j * taps + t];
+      dst[t * n + first + threadIdx.x] = make_uint4(v[0] | v[1] << 16, v[2] | v[3] << 16, v[4] | v[5] << 16, v[6] | v[7] << 16);
+    }
+  }
+  wait_for_predecessor();
+  release_successor();
+}
 }  // namespace
+
+int launch_conv_weight(const void* w, void* out, int c_out, int c_in, int taps, cudaStream_t stream) {
+  if (taps > 12) return fail(DFL_ERR_UNSUPPORTED, "%d taps: at most 12", taps);   // 48 KB of shared memory
+  const long long n = (long long)c_out * (c_in / 8);
+  cudaError_t e = launch_after_predecessor(conv_weight_kernel, dim3((unsigned)((n + 255) / 256)), dim3(256), (size_t)256 * 16 * taps,
+                                           stream, (const uint4*)w, (uint4*)out, n, taps);
+  if (e != cudaSuccess) return fail(DFL_ERR_LAUNCH, "conv_weight_kernel: %s", cudaGetErrorString(e));
+  return check_launch("conv_weight_kernel");
+}
 
 int launch_copy_rows(const void* src, void* dst, const int32_t* rows, long long n_rows, int row_bytes,
                      cudaStream_t stream) {

@@ -267,6 +267,12 @@ int dfl_split_planes(const void* x, void* planes, int64_t n, void* stream) {
   return launch_split_planes(x, planes, n, (cudaStream_t)stream);
 }
 
+int dfl_refresh_planes(const DflPlaneSource* sources_dev, int32_t n_sources, int64_t n_pieces, void* stream) {
+  if (!sources_dev) return fail(DFL_ERR_BAD_ARG, "null pointer");
+  if (n_sources < 1 || n_pieces < 1) return fail(DFL_ERR_BAD_ARG, "non-positive size");
+  return launch_refresh_planes(sources_dev, n_sources, n_pieces, (cudaStream_t)stream);
+}
+
 int dfl_copy_rows(const void* src, void* dst, const int32_t* rows_dev, int64_t n_rows, int32_t row_bytes, void* stream) {
   if (n_rows < 0 || row_bytes < 16 || (row_bytes % 16)) return fail(DFL_ERR_BAD_ARG, "rows of a positive multiple of 16 bytes");
   if (n_rows == 0) return DFL_OK;

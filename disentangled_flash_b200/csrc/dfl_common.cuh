@@ -214,6 +214,10 @@ int launch_gemm_tc(const GemmDesc& g, cudaStream_t stream);
 // FP32 on the tensor cores: g.x is [3][batch][M][K] and g.w [3][w_mod][N][K] bf16 planes (launch_split_planes).
 int launch_gemm_f32_planes(const GemmDesc& g, cudaStream_t stream);
 int launch_split_planes(const void* x, void* planes, long long n, cudaStream_t stream);   // n a multiple of 4
+int launch_refresh_planes(const DflPlaneSource* sources, int n_sources, long long n_pieces, cudaStream_t stream);
+// nn.Conv1d weight [out, in, taps] of 2-byte elements -> [taps, out, in] (in a multiple of 8).  Starts before the kernel ahead of it has finished: that
+// one must not write w, nor it or the kernel before it read `out`.
+int launch_conv_weight(const void* w, void* out, int c_out, int c_in, int taps, cudaStream_t stream);
 
 int launch_attention_simt(const DflAttnParams& p, cudaStream_t stream);
 // FP32 over bf16 planes: p.q, p.k, p.v are [3][B,H,L,d], the scores fp32, the output fp32 or planes [3][B,L,H*d].

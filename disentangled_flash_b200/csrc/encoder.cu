@@ -17,6 +17,7 @@ struct Workspace {
   // F32: bf16 planes of the layer's input, of its first output block, and of the FFN's inside (Q, K, V and the context
   // are planes there too)
   size_t state_planes, mixed_planes, inner_planes;
+  size_t conv_w;   // conv_w_module: the convolution's weight by taps
 };
 
 constexpr size_t kPlaneBytes = 6;   // three bf16 planes per element
@@ -51,6 +52,7 @@ Workspace plan_workspace(const DflEncoderParams& p) {
       w.inner_planes = take(rows * (size_t)p.ffn * kPlaneBytes);
     }
   }
+  if (p.conv_w && p.conv_w_module) w.conv_w = take((size_t)p.conv_taps * p.hidden * p.hidden * es);
   if (two_call(p)) {
     const size_t ld = ((size_t)p.n_active + 7) / 8 * 8;
     for (int i = 0; i < 2; ++i) w.scores[i] = take(positions * p.heads * ld * es);
@@ -89,8 +91,11 @@ int validate(const DflEncoderParams& p) {
     return fail(DFL_ERR_BAD_ARG, "attention_only takes one layer of padded rows");
   if (p.dtype == DFL_F32 && (p.conv_w || p.packed_rows > 0 || !two_call(p)))
     return fail(DFL_ERR_UNSUPPORTED, "F32 has no convolution branch, no packed rows and no rel_key / rel_query form");
+  if (p.plane_sources && (p.dtype != DFL_F32 || p.n_plane_sources < 1 || p.n_plane_pieces < 1))
+    return fail(DFL_ERR_BAD_ARG, "plane sources are an F32 form, with their counts");
   if (p.dtype == DFL_F32 && !attention_f32_planes_supported(p.head_dim, p.seq_len))
     return fail(DFL_ERR_UNSUPPORTED, "head_dim %d at seq_len %d in F32", p.head_dim, p.seq_len);
+  if (p.conv_w && p.conv_w_module && p.conv_taps < 1) return fail(DFL_ERR_BAD_ARG, "conv_taps %d", p.conv_taps);
   if ((long long)p.batch * p.heads > 65535) return fail(DFL_ERR_TOO_LARGE, "batch*heads > 65535");
   if (p.packed_rows > 0) {
     if (two_call(p)) return fail(DFL_ERR_UNSUPPORTED, "packed rows need the rel_key / rel_query form");
@@ -219,7 +224,7 @@ struct Loop {
   // keep * LayerNorm(state + act(keep * conv1d(x))) -> out
   int convolution(const void* state, void* out) {
     GemmDesc g{};
-    g.x = p.x; g.w = p.conv_w; g.bias = p.conv_b; g.out[0] = at(w.inner);
+    g.x = p.x; g.w = p.conv_w_module ? at(w.conv_w) : p.conv_w; g.bias = p.conv_b; g.out[0] = at(w.inner);
     g.M = p.seq_len; g.N = p.hidden; g.K = p.hidden;
     g.batch = p.batch; g.stride_x = g.stride_c = (long long)p.seq_len * p.hidden; g.w_mod = 1; g.ldc = p.hidden;
     g.heads = 1; g.head_dim = p.hidden; g.rows_per_seq = p.seq_len;
@@ -241,6 +246,10 @@ struct Loop {
     void* qkv[3];
     for (int i = 0; i < 3; ++i)
       qkv[i] = grouped ? p.qkv[i] : at(w.qkv + (size_t)i * padded((size_t)qkv_rows * width * (p.dtype == DFL_F32 ? kPlaneBytes : dtype_size(p.dtype))));
+    if (p.plane_sources) {
+      ++p.launches;
+      if (int rc = launch_refresh_planes(p.plane_sources, p.n_plane_sources, p.n_plane_pieces, stream)) return rc;
+    }
     const void* state = p.x;
     const bool f32 = p.dtype == DFL_F32;
     void* unpacked = p.outs[p.n_layers - 1];
@@ -262,6 +271,10 @@ struct Loop {
       void* next = !packed && p.outs[l] ? p.outs[l] : at(w.state[l & 1]);
       const void* input = f32 ? at(w.state_planes) : (packed && !grouped ? (l == 0 ? p.x : unpacked) : state);
       if (int rc = gemm(input, y.qkv_w, y.qkv_b, nullptr, qkv_rows, 3 * width, p.hidden, DFL_ACT_NONE, qkv, true)) return rc;
+      if (convolve && p.conv_w_module) {   // after the projection: the previous forward has finished by then
+        ++p.launches;
+        if (int rc = launch_conv_weight(p.conv_w, at(w.conv_w), p.hidden, p.hidden, p.conv_taps, stream)) return rc;
+      }
       if (int rc = attention(y, qkv, at(w.context), l)) return rc;
       if (int rc = gemm(at(w.context), y.attn_out_w, y.attn_out_b, at(w.dense), rows, p.hidden, width, DFL_ACT_NONE)) return rc;
       if (int rc = norm(at(w.dense), state, y.attn_norm_w, y.attn_norm_b, at(w.mixed), rows, y.attn_norm_eps, nullptr, nullptr,

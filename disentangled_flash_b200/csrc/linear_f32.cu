@@ -48,6 +48,66 @@ __global__ void __launch_bounds__(256) split_planes_kernel(const float4* __restr
   }
 }
 
+// Keeps planes equal to the matrices they were made from: compares a digest of every 4 KB piece (1024 elements) with the one
+// stored when its planes were written, and splits the piece again where they differ.  A warp per piece; HBM bound, 4 bytes
+// per element (a split reads 4 and writes 6): 46 us for 12 layers of hidden 768 (63.7 M elements), 297 us for 24 of 1536
+// (510 M, 6.9 TB/s); 138 and 864 us where everything has changed.  Splitting every matrix anew at each layer of each forward
+// cost 190 and 630 us.
+// The digest is two 64-bit sums over the element's bits x_i and fixed keys k_i: sum (x_2i + k_2i)(x_2i+1 + k_2i+1), the NH
+// hash of Black, Halevi, Krawczyk, Krovetz and Rogaway (UMAC, CRYPTO 1999), and sum x_i (k_i | 1).  One changed element always
+// shows (an odd factor is invertible mod 2^64); several leave both sums as they were with a chance of about 2^-64.
+constexpr int kPieceVecs = DFL_PLANE_PIECE / 4 / 32;   // float4 per lane
+__global__ void __launch_bounds__(256, 3) refresh_planes_kernel(const DflPlaneSource* __restrict__ sources, int n_sources, long long n_pieces) {
+  wait_for_predecessor();
+  release_successor();
+  const int lane = threadIdx.x & 31;
+  const uint32_t seed = (uint32_t)(lane + 1) * 0x9E3779B1u;
+  int at = 0;
+  for (long long piece = blockIdx.x * 8ll + (threadIdx.x >> 5); piece < n_pieces; piece += gridDim.x * 8ll) {
+    while (at + 1 < n_sources && piece >= sources[at + 1].first_piece) ++at;
+    const DflPlaneSource src = sources[at];
+    const long long n4 = src.n / 4, local = piece - src.first_piece, first = local * (DFL_PLANE_PIECE / 4) + lane;
+    float4 v[kPieceVecs];
+    ulonglong2* digest = reinterpret_cast<ulonglong2*>(src.digests) + local;
+    const ulonglong2 then = *digest;
+#pragma unroll
+    for (int j = 0; j < kPieceVecs; ++j)
+      v[j] = first + 32 * j < n4 ? __ldcs(reinterpret_cast<const float4*>(src.w) + first + 32 * j) : make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    unsigned long long nh = 0, linear = 0;
+#pragma unroll
+    for (int j = 0; j < kPieceVecs; ++j) {
+      const uint32_t x[4] = {__float_as_uint(v[j].x), __float_as_uint(v[j].y), __float_as_uint(v[j].z), __float_as_uint(v[j].w)};
+      uint32_t k[4];
+#pragma unroll
+      for (int c = 0; c < 4; ++c) {
+        k[c] = seed * (2u * (uint32_t)(4 * j + c) * 0x45D9F3Bu + 0x2C1B3C6Du);
+        k[c] ^= k[c] >> 15;
+        linear += (unsigned long long)x[c] * (k[c] | 1u);
+      }
+      nh += (unsigned long long)(x[0] + k[0]) * (x[1] + k[1]) + (unsigned long long)(x[2] + k[2]) * (x[3] + k[3]);
+    }
+#pragma unroll
+    for (int o = 16; o > 0; o >>= 1) {
+      nh += __shfl_xor_sync(0xffffffffu, nh, o);
+      linear += __shfl_xor_sync(0xffffffffu, linear, o);
+    }
+    if (then.x == nh && then.y == linear) continue;   // warp-uniform
+    uint2* planes = reinterpret_cast<uint2*>(src.planes);
+#pragma unroll
+    for (int j = 0; j < kPieceVecs; ++j) {
+      if (first + 32 * j >= n4) break;
+      const float f[4] = {v[j].x, v[j].y, v[j].z, v[j].w};
+      uint2 out[kPlanes];
+      split3x4(f, out);
+#pragma unroll
+      for (int q = 0; q < kPlanes; ++q) planes[q * n4 + first + 32 * j] = out[q];
+    }
+    __threadfence();   // another stream that sees the digest sees the planes
+    __syncwarp();
+    if (lane == 0) *digest = make_ulonglong2(nh, linear);
+  }
+}
+
 // 32 finished columns [n, n+32) of the warp's 32 rows: bias, activation, then through the staging buffer so that eight
 // lanes store one row segment; row-major or head-major, in fp32 or as bf16 planes.
 __device__ __forceinline__ void emit32(const GemmDesc& g, const float (&acc)[32], const float* bias, float* stage, int row0,
@@ -440,6 +500,14 @@ int launch_split_planes(const void* x, void* planes, long long n, cudaStream_t s
   cudaError_t e = launch_after_predecessor(split_planes_kernel, dim3(blocks), dim3(256), 0, stream, (const float4*)x, (uint2*)planes, n4);
   if (e != cudaSuccess) return fail(DFL_ERR_LAUNCH, "split_planes_kernel: %s", cudaGetErrorString(e));
   return check_launch("split_planes_kernel");
+}
+
+int launch_refresh_planes(const DflPlaneSource* sources, int n_sources, long long n_pieces, cudaStream_t stream) {
+  const long long wanted = (n_pieces + 7) / 8, cap = 148 * 6;
+  cudaError_t e = launch_after_predecessor(refresh_planes_kernel, dim3((unsigned)(wanted < cap ? wanted : cap)), dim3(256), 0, stream,
+                                           sources, n_sources, n_pieces);
+  if (e != cudaSuccess) return fail(DFL_ERR_LAUNCH, "refresh_planes_kernel: %s", cudaGetErrorString(e));
+  return check_launch("refresh_planes_kernel");
 }
 
 int launch_gemm_f32_planes(const GemmDesc& g, cudaStream_t stream) {

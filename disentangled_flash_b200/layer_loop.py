@@ -1,9 +1,7 @@
 """The prepared layer loop of one bucket as a single native call (``dfl_encoder_fwd``).
 
 Built by ``DebertaV2InferenceEncoder.prepare_for_inference`` for a bucket whose layers all have the Hugging Face shape;
-the encoder's Python loop serves everything else.  In FP32 the weight matrices are held as bf16 planes
-(``dfl_split_planes``) for the tensor-core GEMMs, made once per encoder; a weight modified in place after that sends the
-calls to the Python loop until the next preparation.  A convolution branch stays the caller's module in FP32.
+the encoder's Python loop serves everything else.  A convolution branch stays the caller's module in FP32.
 
 The native call reads the modules' parameters by address.  Before each call the state the addresses were taken from is
 compared with the present one: the modules, where and in which form their parameters lie, and the settings that went into
@@ -32,15 +30,15 @@ _LAYER_FIELDS = (
     ("ffn_out_w", "output.dense", "weight"), ("ffn_out_b", "output.dense", "bias"),
     ("ffn_norm_w", "output.LayerNorm", "weight"), ("ffn_norm_b", "output.LayerNorm", "bias"),
 )
-_PLANE_FIELDS = ("attn_out_w", "ffn_in_w", "ffn_out_w")   # weight matrices given as planes in FP32
+_PLANE_FIELDS = ("attn_out_w", "ffn_in_w", "ffn_out_w")   # weight matrices given as planes in FP32, which follow them
 _data_ptr, _dtype = torch.Tensor.data_ptr, torch.Tensor.dtype.__get__
 _shape, _stride = torch.Tensor.shape.__get__, torch.Tensor.stride
 
 
-def version_of(tensor: torch.Tensor) -> int:
-    """How often ``tensor`` has been modified in place (inference tensors do not count)."""
-
-    return -1 if tensor.is_inference() else tensor._version
+def _module_at(root: nn.Module, path: str) -> nn.Module:
+    for name in path.split("."):
+        root = getattr(root, name)
+    return root
 
 
 class LayerLoop:
@@ -82,7 +80,6 @@ class LayerLoop:
             return None
         n = len(encoder.layer)
         self.layers = (_cabi.DflEncoderLayer * n)()
-        self._planes: list[torch.Tensor] = []
 
         def read(module: nn.Module, key: str) -> torch.Tensor | None:
             for owner in (module._parameters, module._buffers):
@@ -99,6 +96,7 @@ class LayerLoop:
             self._names += [key, key]
             return None
 
+        weights: list[torch.Tensor] = []
         shapes = {"attn_out_w": (hidden, width), "ffn_in_w": (ffn, hidden),
                   "ffn_out_w": (hidden, ffn), "attn_norm_w": (hidden,), "ffn_norm_w": (hidden,)}
         try:
@@ -107,7 +105,7 @@ class LayerLoop:
                 entry, plan = self.layers[index], plans[index]
                 self._walk(layer, layer.attention, layer.attention.output, layer.intermediate, layer.output)
                 for _, path, key in _ATTENTION_FIELDS:
-                    read(layer.get_submodule(path), key)
+                    read(_module_at(layer, path), key)
                 module = layer.attention.self
                 if module._cached_qkv_weight.shape != (3 * width, hidden) or (f32 and module._cached_qkv_planes is None):
                     return None
@@ -119,13 +117,13 @@ class LayerLoop:
                     self._owners.append(module._buffers)
                     self._keys.append("_cached_qkv_planes")
                 for field, path, key in _LAYER_FIELDS:
-                    tensor = read(layer.get_submodule(path), key)
+                    tensor = read(_module_at(layer, path), key)
                     if field in shapes and (tensor is None or tuple(tensor.shape) != shapes[field]):
                         return None
                     if f32 and field in _PLANE_FIELDS:
-                        tensor = encoder._weight_planes_of(tensor)
-                        self._planes.append(tensor)
-                    setattr(entry, field, None if tensor is None else tensor.data_ptr())
+                        weights.append(tensor.detach())
+                    else:
+                        setattr(entry, field, None if tensor is None else tensor.data_ptr())
                 entry.attn_norm_eps = float(layer.attention.output.LayerNorm.eps)
                 entry.ffn_norm_eps = float(layer.output.LayerNorm.eps)
                 self._watch(layer.attention.output.LayerNorm, "eps")
@@ -142,14 +140,23 @@ class LayerLoop:
                 if (module.has_c2p, module.has_p2c, module.pos_att_type) != (first.has_c2p, first.has_p2c, first.pos_att_type):
                     return None
             p = _cabi.DflEncoderParams()
+            if f32:
+                self._weights = encoder._planes_following(weights)
+                for index, planes in enumerate(self._weights.planes):
+                    setattr(self.layers[index // 3], _PLANE_FIELDS[index % 3], planes.data_ptr())
+                p.plane_sources, p.n_plane_sources = self._weights.sources.data_ptr(), self._weights.n_sources
+                p.n_plane_pieces = self._weights.n_pieces
             if encoder.conv is not None and not f32:
                 self._walk(encoder.conv)
                 norm = encoder.conv.LayerNorm
                 bias = read(encoder.conv.conv, "bias")
                 gamma, beta = read(norm, "weight"), read(norm, "bias")
-                read(encoder.conv.conv, "weight")
+                weight = read(encoder.conv.conv, "weight")
                 self._conv_weight = encoder._conv_weight   # [taps, out, in], permuted at prepare time
-                p.conv_w, p.conv_b = self._conv_weight.data_ptr(), None if bias is None else bias.data_ptr()
+                # a bucket for which the Python loop calls the module, which reads its weight at the call, does so too
+                p.conv_w_module = not encoder._conv_fused[length]
+                p.conv_w = (weight if p.conv_w_module else self._conv_weight).data_ptr()
+                p.conv_b = None if bias is None else bias.data_ptr()
                 p.conv_norm_w, p.conv_norm_b = gamma.data_ptr(), None if beta is None else beta.data_ptr()
                 p.conv_taps, p.conv_activation = self._conv_weight.shape[0], encoder._conv_activation_code
                 p.conv_norm_eps = float(norm.eps)
@@ -195,14 +202,12 @@ class LayerLoop:
 
     def _current_state(self) -> tuple:
         """What the addresses in the native call depend on, some 30 us for 12 layers: per tensor the address and the type,
-        of a matrix also its form (``.data = other`` changes them under the same name); in FP32, where copies of the
-        weights are read, the versions too."""
+        of a matrix also its form (``.data = other`` changes them under the same name)."""
 
         tensors = list(map(dict.__getitem__, self._owners, self._keys))
         matrices = self._pick(tensors)
         return (list(map(_data_ptr, tensors)), list(map(_dtype, tensors)), list(map(_shape, matrices)), list(map(_stride, matrices)),
-                self._children, list(map(dict.get, self._settings, self._names)),
-                list(map(version_of, tensors)) if self.f32 else None)
+                self._children, list(map(dict.get, self._settings, self._names)))
 
     def covers(self, encoder: nn.Module, plans: Any, hidden: torch.Tensor, mask: torch.Tensor) -> bool:
         """Whether this call can take the native loop (the state it was built from still holds)."""
@@ -267,6 +272,8 @@ class LayerLoop:
         p = self._call(hidden, mask, outs, status)
         if n != self.n_layers:
             p.n_layers = n
+            if begin > 0:
+                p.plane_sources = None   # done by the call for the first layers
             p.layers = ctypes.cast(ctypes.addressof(self.layers) + begin * ctypes.sizeof(_cabi.DflEncoderLayer),
                                    ctypes.POINTER(_cabi.DflEncoderLayer))
         _cabi.encoder_fwd(p, self.device)

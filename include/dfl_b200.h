@@ -399,13 +399,28 @@ DFL_API int dfl_embed_layernorm(const DflEmbedLayerNormParams* p, void* stream);
  * dfl_attention_fwd, `lut` required).
  *
  * F32: the four weight matrices and pos_key / pos_query are given as bf16 planes [3][...] whose sum is the fp32 tensor
- * (dfl_split_planes, once per weight); the GEMMs run on the tensor cores with six plane products per product and
+ * (dfl_split_planes, once per weight); with plane_sources the call brings planes up to date with their weights first.
+ * The GEMMs run on the tensor cores with six plane products per product and
  * fp32 sums, at least as accurate as a fp32 multiply-add chain (finite operands; an infinite operand gives NaN).  Biases
  * and norm parameters stay fp32.  No convolution branch and no packed rows in F32.
  */
 /* planes[3][n] (bf16) with planes[0] + planes[1] + planes[2] == x exactly; n a multiple of 4 */
 DFL_API int dfl_f32_planes_supported(int head_dim, int seq_len);   /* whether the F32 form covers the attention's sizes */
 DFL_API int dfl_split_planes(const void* x, void* planes, int64_t n, void* stream);
+/*
+ * Planes that follow their fp32 matrices: one launch compares a digest of every DFL_PLANE_PIECE elements with the one kept
+ * from when their planes were written, and rewrites planes and digest where it differs (however the matrix was changed, in
+ * captured graphs too).  `sources` is a device array ordered by first_piece; zeroed digests make the planes from nothing.
+ */
+#define DFL_PLANE_PIECE 1024
+typedef struct DflPlaneSource {
+  const void* w;         /* fp32 [n] */
+  void*       planes;    /* bf16 [3][n] */
+  void*       digests;   /* 16 bytes per piece, 16-byte aligned */
+  int64_t     n;         /* a multiple of 4 */
+  int64_t     first_piece;   /* pieces of the sources before this one; each has ceil(n / DFL_PLANE_PIECE) */
+} DflPlaneSource;
+DFL_API int dfl_refresh_planes(const DflPlaneSource* sources_dev, int32_t n_sources, int64_t n_pieces, void* stream);
 typedef struct DflEncoderLayer {
   const void *qkv_w, *qkv_b;              /* [3*heads*head_dim, hidden], [3*heads*head_dim] or NULL */
   const void *attn_out_w, *attn_out_b;    /* [hidden, heads*head_dim], [hidden] or NULL */
@@ -451,6 +466,12 @@ typedef struct DflEncoderParams {
   const int32_t* row_base;         /* device [batch]: first packed row of a sequence */
   const int32_t* row_count;        /* device [batch]: packed rows of a sequence */
   void* qkv[3];                    /* [batch, heads, seq_len, head_dim] each, finite contents, kept from call to call */
+  int32_t conv_w_module;           /* non-zero: conv_w is the nn.Conv1d weight [hidden, hidden, taps] itself; every call lays
+                                      it out by taps in the workspace, so that a changed weight is used */
+  /* F32, optional: dfl_refresh_planes() as the first launch of the call */
+  const struct DflPlaneSource* plane_sources;
+  int32_t n_plane_sources;
+  int64_t n_plane_pieces;
 } DflEncoderParams;
 DFL_API size_t dfl_encoder_workspace_bytes(const DflEncoderParams* p);
 DFL_API int dfl_encoder_fwd(DflEncoderParams* p, void* stream);

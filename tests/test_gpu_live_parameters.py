@@ -54,3 +54,61 @@ def test_exchanged_modules_are_used(dtype):
     torch.manual_seed(1)
     encoder.layer[1].output.dense = nn.Linear(512, 256).to(dev, dtype)
     assert_follows(encoder, hidden, mask, before, dtype)
+
+
+def _by_data(w):
+    w.data.copy_(torch.randn(w.shape, generator=torch.Generator().manual_seed(9)) * 0.05)
+
+
+def _in_place(w):
+    with torch.no_grad():
+        w.mul_(-1.0)
+
+
+@pytest.mark.parametrize("change", (_in_place, _by_data))
+@pytest.mark.parametrize("which", ("attention.output", "intermediate", "output"))
+@pytest.mark.parametrize("inference", (False, True))   # inference tensors count no changes
+def test_fp32_weights_changed_in_place_are_used(which, change, inference):
+    encoder, hidden, mask = prepared(torch.float32, 40, conv=3, inference=inference)
+    before, _ = both(encoder, hidden, mask)
+    with torch.inference_mode(inference):
+        for layer in encoder.layer:
+            change(layer.get_submodule(which).dense.weight)
+    assert_follows(encoder, hidden, mask, before, torch.float32)
+
+
+@pytest.mark.parametrize("dtype", (torch.float16, torch.bfloat16))
+@pytest.mark.parametrize("length", (17, 64, 255))
+def test_short_convolution_weights_changed_in_place_are_used(dtype, length):
+    encoder, hidden, mask = prepared(dtype, length, conv=3)
+    before, _ = both(encoder, hidden, mask)
+    _by_data(encoder.conv.conv.weight)
+    encoder.conv.conv.weight.data.mul_(4)
+    assert_follows(encoder, hidden, mask, before, dtype)
+
+
+@pytest.mark.parametrize("dtype,conv", ((torch.float32, 0), (torch.float16, 3)))
+def test_a_captured_graph_reads_the_weights_as_they_are(dtype, conv):
+    encoder, hidden, mask = prepared(dtype, 32, conv=conv)
+    bucket = df.capture_deberta_buckets(encoder, 2)[32]
+    before = bucket(hidden, mask).float().cpu()
+    _in_place(encoder.conv.conv.weight if conv else encoder.layer[0].output.dense.weight)
+    got = bucket(hidden, mask).float().cpu()
+    with torch.inference_mode():
+        want = encoder(hidden, mask).last_hidden_state.float().cpu()
+    assert torch.equal(got, want) and (got - before).norm() / want.norm() > 0.05
+
+
+def test_fp32_layers_of_every_width_use_their_own_weights():
+    """Matrices of a few hundred to a few million elements, their planes one after the other in one workspace."""
+
+    for hidden_size, heads, ffn, length in ((256, 4, 264, 3), (512, 8, 2048, 130), (1536, 24, 6144, 64)):
+        cfg = df.DebertaAttentionConfig(hidden_size=hidden_size, num_attention_heads=heads, attention_head_size=64,
+                                        num_hidden_layers=3, intermediate_size=ffn, max_position_embeddings=512,
+                                        position_buckets=64, norm_rel_ebd="layer_norm", conv_kernel_size=0)
+        backbone = hf_modules.Backbone(cfg, vocab_size=8).eval()
+        hf_modules.initialize_parameters(backbone, 5, std=0.03)
+        df.optimize_deberta(backbone.to(dev), sequence_lengths=[length])
+        hidden = torch.randn(2, length, hidden_size, generator=torch.Generator().manual_seed(2)).to(dev)
+        got, want = both(backbone.encoder, hidden, torch.ones(2, length, dtype=torch.bool, device=dev))
+        assert (got - want).norm() / want.norm() < 5e-6

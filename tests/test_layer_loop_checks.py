@@ -49,7 +49,7 @@ LENGTH = 32
 def covered(monkeypatch):
     """``build(dtype, conv)`` -> the encoder, and whether its native loop covers a call now."""
 
-    monkeypatch.setattr(_cabi, "split_planes", lambda x: torch.zeros(3, *x.shape, dtype=torch.bfloat16))
+    monkeypatch.setattr(_cabi.FollowingPlanes, "refresh", lambda self: None)
 
     def build(dtype=torch.float16, conv=0, bias=True, activation=None):
         cfg = df.DebertaAttentionConfig(hidden_size=256, num_attention_heads=4, attention_head_size=64, num_hidden_layers=3,
