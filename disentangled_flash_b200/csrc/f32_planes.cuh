@@ -7,16 +7,16 @@ namespace dfl {
 
 constexpr int kPlanes = 3;
 
+// An infinity is 1 (of its sign), 0 and itself.  A product takes plane 2 of one operand with plane 0 of the other only, so
+// that an infinity meets each element it is multiplied with exactly once, by its sign and size; in plane 0 it would also meet
+// the other operand's planes 1 and 2, which are zeros or of the other sign, and give NaN.
 __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16& b, __nv_bfloat16& c) {
-  a = __float2bfloat16_rn(x);
-  float af = __bfloat162float(a);
-  if (isinf(af)) {   // rounding a finite value up to infinity: truncate instead
-    a = __ushort_as_bfloat16((unsigned short)(__float_as_uint(x) >> 16));
-    af = __bfloat162float(a);
-  }
-  const float r1 = isinf(af) ? 0.0f : x - af;   // exact
+  const bool infinite = isinf(x);
+  a = __float2bfloat16_rn(infinite ? copysignf(1.0f, x) : x);
+  if (isinf(__bfloat162float(a))) a = __ushort_as_bfloat16((unsigned short)(__float_as_uint(x) >> 16));   // rounded up: truncate
+  const float r1 = infinite ? 0.0f : x - __bfloat162float(a);   // exact
   b = __float2bfloat16_rn(r1);
-  c = __float2bfloat16_rn(r1 - __bfloat162float(b));
+  c = __float2bfloat16_rn(infinite ? x : r1 - __bfloat162float(b));
 }
 
 // Four elements of one row as packed plane words.

@@ -10,7 +10,8 @@
 // last, and the epilogue warps add the finished block to sums in registers, rounded to nearest, while the MMA warp fills
 // the other accumulator.  Against an fp64 product the result is at least as accurate as the sequential fp32 chain of the
 // CUDA-core kernel this replaces on the prepared paths (tests/test_gpu_f32_tensor.py).
-// Infinities: inf - inf inside the split sums gives NaN where IEEE arithmetic would give an infinity.
+// Infinities and NaN come out as a fp32 multiply-add chain gives them (f32_planes.cuh), except beside operands below 2^-134,
+// whose leading plane is zero.
 //
 // What bounds it: six bf16 MMAs per product, a sixth of the bf16 tensor rate; a k-block brings 96 KB for 24 MMAs of a
 // 256 x 256 pair tile (3.1 k cycles), far below what an SM can take from L2.

@@ -401,11 +401,12 @@ DFL_API int dfl_embed_layernorm(const DflEmbedLayerNormParams* p, void* stream);
  * F32: the four weight matrices and pos_key / pos_query are given as bf16 planes [3][...] whose sum is the fp32 tensor
  * (dfl_split_planes, once per weight); with plane_sources the call brings planes up to date with their weights first.
  * The GEMMs run on the tensor cores with six plane products per product and
- * fp32 sums, at least as accurate as a fp32 multiply-add chain (finite operands; an infinite operand gives NaN).  Biases
+ * fp32 sums, at least as accurate as a fp32 multiply-add chain, infinities and NaN included.  Biases
  * and norm parameters stay fp32.  No convolution branch and no packed rows in F32.
  */
-/* planes[3][n] (bf16) with planes[0] + planes[1] + planes[2] == x exactly; n a multiple of 4 */
 DFL_API int dfl_f32_planes_supported(int head_dim, int seq_len);   /* whether the F32 form covers the attention's sizes */
+/* planes[3][n] (bf16) with planes[0] + planes[1] + planes[2] == x exactly (an infinity: 1 of its sign, 0, itself); n a
+ * multiple of 4 */
 DFL_API int dfl_split_planes(const void* x, void* planes, int64_t n, void* stream);
 /*
  * Planes that follow their fp32 matrices: one launch compares a digest of every DFL_PLANE_PIECE elements with the one kept
