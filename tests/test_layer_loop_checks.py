@@ -51,7 +51,7 @@ def covered(monkeypatch):
 
     monkeypatch.setattr(_cabi.FollowingPlanes, "refresh", lambda self: None)
 
-    def build(dtype=torch.float16, conv=0, bias=True, activation=None):
+    def build(dtype=torch.float16, conv=0, bias=True, activation=None, misaligned=None):
         cfg = df.DebertaAttentionConfig(hidden_size=256, num_attention_heads=4, attention_head_size=64, num_hidden_layers=3,
                                         intermediate_size=512, max_position_embeddings=64, position_buckets=32,
                                         conv_kernel_size=conv)
@@ -62,6 +62,9 @@ def covered(monkeypatch):
             if activation is not None:
                 layer.intermediate.intermediate_act_fn = activation()
         encoder = df.DebertaV2InferenceEncoder(source, cfg).to(dtype).eval()
+        if misaligned is not None:
+            weight = encoder.get_submodule(misaligned).weight
+            weight.data = torch.zeros(weight.numel() + 1, dtype=dtype)[1:].view_as(weight)
         f32, plans = dtype == torch.float32, []
         for layer in encoder.layer:
             module = layer.attention.self
@@ -75,6 +78,8 @@ def covered(monkeypatch):
             encoder._conv_weight = encoder.conv.conv.weight.detach().permute(2, 0, 1).contiguous()
         plans = tuple(plans)
         loop = LayerLoop.build(encoder, LENGTH, plans, bool(conv))
+        if loop is None:
+            return encoder, None
         hidden, mask = torch.zeros(2, LENGTH, 256, dtype=dtype), torch.ones(2, LENGTH, dtype=torch.bool)
 
         def covers():
@@ -162,3 +167,9 @@ def test_hooks_and_forwards_of_their_own_run_where_the_fp32_loop_would_skip_them
         assert covers()
         touch(encoder.layer[2].intermediate)
         assert not covers()
+
+
+@pytest.mark.parametrize("dtype", (torch.float16, torch.float32))
+@pytest.mark.parametrize("where", ("layer.0.attention.output.dense", "layer.2.output.dense"))
+def test_misaligned_weights_are_left_to_the_python_loop(covered, where, dtype):
+    assert covered(dtype, misaligned=where)[1] is None
