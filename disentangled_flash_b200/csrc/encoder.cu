@@ -96,7 +96,8 @@ int validate(const DflEncoderParams& p) {
   if (p.dtype == DFL_F32 && !attention_f32_planes_supported(p.head_dim, p.seq_len))
     return fail(DFL_ERR_UNSUPPORTED, "head_dim %d at seq_len %d in F32", p.head_dim, p.seq_len);
   if (p.conv_w && p.conv_w_module && p.conv_taps < 1) return fail(DFL_ERR_BAD_ARG, "conv_taps %d", p.conv_taps);
-  if ((long long)p.batch * p.heads > 65535) return fail(DFL_ERR_TOO_LARGE, "batch*heads > 65535");
+  // the two-call attention kernels have batch*heads as a grid's second dimension; the rel form has no such limit
+  if (two_call(p) && (long long)p.batch * p.heads > 65535) return fail(DFL_ERR_TOO_LARGE, "batch*heads > 65535");
   if (p.packed_rows > 0) {
     if (two_call(p)) return fail(DFL_ERR_UNSUPPORTED, "packed rows need the rel_key / rel_query form");
     if (!p.pack_rows || !p.row_base || !p.row_count) return fail(DFL_ERR_BAD_ARG, "null packed-row table");
