@@ -788,6 +788,9 @@ class FollowingPlanes:
         self.sources = torch.tensor(rows, dtype=torch.int64).to(device)
         self.refresh()
 
+    def __reduce__(self):
+        return type(None), ()   # addresses of other tensors: a copy of the owner makes its own
+
     def refresh(self) -> None:
         device = self.sources.device
         with _on_device(device):

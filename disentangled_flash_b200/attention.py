@@ -141,6 +141,22 @@ def _require_2d_padding_mask(attention_mask: torch.Tensor, batch_size: int, sequ
     return attention_mask.contiguous()
 
 
+class NativeCalls(dict):
+    """Native calls by sequence length.  They hold addresses, so a copied or pickled module has an empty one, marked as
+    ``copied``, and makes its calls anew."""
+
+    copied = False
+
+    def __reduce__(self):
+        return _copied_calls, ()
+
+
+def _copied_calls() -> NativeCalls:
+    calls = NativeCalls()
+    calls.copied = True
+    return calls
+
+
 class _LayerCall:
     """The QKV projection and the attention of one layer and length as one native call (``dfl_encoder_fwd`` with
     ``attention_only``): less host time per call, and in FP32 the tensor-core GEMMs over bf16 planes."""
@@ -267,7 +283,7 @@ class DisentangledFlashAttention(nn.Module):
         # shares one word between its layers (set_status_word) and reads it in check_device_status()
         self.register_buffer("_status_word", None, persistent=False)
         self._position_projection_cache: dict[tuple[int, str], B200PreparedPositionPlan] = {}
-        self._layer_calls: dict[int, _LayerCall | None] = {}   # per sequence length
+        self._layer_calls: dict[int, _LayerCall | None] = NativeCalls()   # per sequence length
         self._algo = _cabi.ALGO_AUTO
         self.register_load_state_dict_post_hook(_invalidate_attention_cache_after_load)
 

@@ -1,6 +1,8 @@
 """A prepared encoder reads the blocks around the attention as they are at the call: modules exchanged and parameters changed
 after the preparation give what the encoder's Python loop, which calls them live, gives."""
 
+import copy
+
 import pytest
 import torch
 from torch import nn
@@ -112,3 +114,16 @@ def test_fp32_layers_of_every_width_use_their_own_weights():
         hidden = torch.randn(2, length, hidden_size, generator=torch.Generator().manual_seed(2)).to(dev)
         got, want = both(backbone.encoder, hidden, torch.ones(2, length, dtype=torch.bool, device=dev))
         assert (got - want).norm() / want.norm() < 5e-6
+
+
+@pytest.mark.parametrize("dtype", (torch.float32, torch.float16))
+def test_a_copy_of_a_prepared_encoder_has_weights_of_its_own(dtype):
+    encoder, hidden, mask = prepared(dtype, 40)
+    before, _ = both(encoder, hidden, mask)
+    twin = copy.deepcopy(encoder)
+    _in_place(twin.layer[1].output.dense.weight)
+    with torch.inference_mode():
+        twin(hidden, mask)   # the first call makes the copy's native loop
+    assert 40 in twin._layer_loops
+    assert_follows(twin, hidden, mask, before, dtype)
+    assert torch.equal(both(encoder, hidden, mask)[0], before)

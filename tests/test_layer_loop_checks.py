@@ -1,13 +1,16 @@
 """When the native layer loop may serve a call, and what it checks on the way: everything that needs no GPU.  The loops are
 built over CPU modules whose prepared buffers are made by hand, and the native call is replaced by a recorder."""
 
+import copy
+import io
+
 import pytest
 import torch
 from torch import nn
 
 import hf_modules
 import disentangled_flash_b200 as df
-from disentangled_flash_b200 import _cabi
+from disentangled_flash_b200 import _cabi, attention
 from disentangled_flash_b200.layer_loop import LayerLoop
 
 
@@ -81,6 +84,11 @@ def covered(monkeypatch):
         if loop is None:
             return encoder, None
         hidden, mask = torch.zeros(2, LENGTH, 256, dtype=dtype), torch.ones(2, LENGTH, dtype=torch.bool)
+
+        encoder._layer_loops[LENGTH] = loop
+        encoder._buckets.by_length[LENGTH] = plans
+        encoder._buckets.select(LENGTH)
+        encoder._conv_covered = {LENGTH: bool(conv)}
 
         def covers():
             with torch.no_grad():
@@ -173,3 +181,29 @@ def test_hooks_and_forwards_of_their_own_run_where_the_fp32_loop_would_skip_them
 @pytest.mark.parametrize("where", ("layer.0.attention.output.dense", "layer.2.output.dense"))
 def test_misaligned_weights_are_left_to_the_python_loop(covered, where, dtype):
     assert covered(dtype, misaligned=where)[1] is None
+
+
+def _saved_and_loaded(model):
+    file = io.BytesIO()
+    torch.save(model, file)
+    file.seek(0)
+    return torch.load(file, weights_only=False)
+
+
+@pytest.mark.parametrize("dtype,conv", ((torch.float16, 0), (torch.bfloat16, 3), (torch.float32, 0)))
+@pytest.mark.parametrize("duplicate", (copy.deepcopy, _saved_and_loaded))
+def test_a_copy_of_a_prepared_encoder_makes_native_calls_of_its_own(covered, monkeypatch, dtype, conv, duplicate):
+    encoder, covers = covered(dtype, conv=conv)
+    with torch.no_grad():
+        module = encoder.layer[0].attention.self
+        module._layer_calls[LENGTH] = attention._LayerCall(module, encoder._active_plans[0])
+        twin = duplicate(encoder)
+        monkeypatch.setattr(torch.Tensor, "is_cuda", property(lambda t: True))
+        loop = twin._layer_loop(torch.zeros(2, LENGTH, 256, dtype=dtype), torch.ones(2, LENGTH, dtype=torch.bool), twin._active_plans)
+    assert covers() and not twin.layer[0].attention.self._layer_calls
+    assert loop.layers[1].ffn_norm_w == twin.layer[1].output.LayerNorm.weight.data_ptr() != encoder.layer[1].output.LayerNorm.weight.data_ptr()
+    if dtype == torch.float32:
+        assert twin._weight_planes.addresses == [w for layer in twin.layer for w in (
+            layer.attention.output.dense.weight.data_ptr(), layer.intermediate.dense.weight.data_ptr(), layer.output.dense.weight.data_ptr())]
+    else:
+        assert loop.layers[2].ffn_out_w == twin.layer[2].output.dense.weight.data_ptr()
