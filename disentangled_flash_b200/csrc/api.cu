@@ -44,8 +44,8 @@ int dfl_check_status(int32_t* status_dev, void* stream) {
   if (e != cudaSuccess) return fail(DFL_ERR_LAUNCH, "clearing the status word: %s", cudaGetErrorString(e));
   if (code == 98)   // dfl_embed_layernorm: the one code that is not a wait
     return fail(DFL_ERR_BAD_ARG, "an embedding index was outside its table (that row was read as zeros)");
-  return fail(DFL_ERR_DEVICE_TIMEOUT, "a bounded device-side wait expired (wait code %d); outputs since the last check are invalid",
-              (int)code);
+  return fail(DFL_ERR_DEVICE_TIMEOUT, "a bounded device-side wait expired (wait code %d, %s); outputs since the last check are invalid",
+              (int)code, kernel_of_wait(code));
 }
 
 int dfl_selftest_bounded_wait(int32_t* status_dev, uint32_t limit_us, void* stream) {

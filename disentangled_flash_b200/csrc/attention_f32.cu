@@ -25,6 +25,7 @@ namespace {
 
 constexpr int BM = 128, kSoftmaxWarps = 8, kTmaWarp = 8, kMmaWarp = 9, kThreads = 320;
 constexpr int kMaxSmem = 232448;
+constexpr int kWaits = kWaitsAttentionF32;
 constexpr int COL_S = 0, COL_P = 128, COL_O = 320;   // S: BN fp32; P: three planes of BN / 2; O: D fp32
 constexpr int kTmemCols = 512;
 
@@ -127,10 +128,10 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       ptx::mbar_arrive_expect_tx(&bars->q_full, (uint32_t)T::kQ);
       load(T::offQ, T::kQSub, &tmap_q, &bars->q_full, i0);
       for (int t = 0; t < n_kt; ++t) {
-        if (!ptx::mbar_wait(&bars->k_empty, ((uint32_t)t & 1u) ^ 1u, abort_flag, status_word, 51)) break;
+        if (!ptx::mbar_wait(&bars->k_empty, ((uint32_t)t & 1u) ^ 1u, abort_flag, status_word, kWaits + 51)) break;
         ptx::mbar_arrive_expect_tx(&bars->k_full, (uint32_t)T::kKV);
         load(T::offK, T::kKSub, &tmap_k, &bars->k_full, t * BN);
-        if (!ptx::mbar_wait(&bars->v_empty, ((uint32_t)t & 1u) ^ 1u, abort_flag, status_word, 52)) break;
+        if (!ptx::mbar_wait(&bars->v_empty, ((uint32_t)t & 1u) ^ 1u, abort_flag, status_word, kWaits + 52)) break;
         ptx::mbar_arrive_expect_tx(&bars->v_full, (uint32_t)T::kKV);
         load(T::offV, T::kKSub, &tmap_v, &bars->v_full, t * BN);
       }
@@ -147,7 +148,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, abort_flag, status_word, code)) != 0;
     };
     auto issue_s = [&](int t) -> bool {
-      if (!wait(&bars->k_full, (uint32_t)t & 1u, 53)) return false;
+      if (!wait(&bars->k_full, (uint32_t)t & 1u, kWaits + 53)) return false;
       ptx::tc_fence_after();
 #pragma unroll
       for (int q = 0; q < 6; ++q)
@@ -162,9 +163,9 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       ptx::umma_commit_warp(&bars->s_full);
       return true;
     };
-    bool ok = wait(&bars->q_full, 0, 54) && issue_s(0);
+    bool ok = wait(&bars->q_full, 0, kWaits + 54) && issue_s(0);
     for (int t = 0; t < n_kt && ok; ++t) {
-      ok = wait(&bars->p_full, (uint32_t)t & 1u, 55) && wait(&bars->v_full, (uint32_t)t & 1u, 56);
+      ok = wait(&bars->p_full, (uint32_t)t & 1u, kWaits + 55) && wait(&bars->v_full, (uint32_t)t & 1u, kWaits + 56);
       if (!ok) break;
       ptx::tc_fence_after();
 #pragma unroll 1
@@ -211,7 +212,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       }
     };
     for (int t = 0; t < n_kt && ok; ++t) {
-      ok = wait(&bars->s_full, (uint32_t)t & 1u, 57);
+      ok = wait(&bars->s_full, (uint32_t)t & 1u, kWaits + 57);
       if (!ok) break;
       ptx::tc_fence_after();
       const int j0 = t * BN + hf * HK;
@@ -258,7 +259,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       xmax[(t & 1) * 2 * BM + hf * BM + r] = mx;
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->pair[quarter]);
-      ok = wait(&bars->pair[quarter], (uint32_t)t & 1u, 58);
+      ok = wait(&bars->pair[quarter], (uint32_t)t & 1u, kWaits + 58);
       if (!ok) break;
       const float m_new = fmaxf(m_run, fmaxf(mx, xmax[(t & 1) * 2 * BM + (1 - hf) * BM + r]));
       const float m_use = m_new == -INFINITY ? 0.0f : m_new;
@@ -272,7 +273,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       }
       l_run = l_run * corr + sum;
       if (t > 0) {   // the previous tile's PV: added before its scale is left behind, and P may be overwritten
-        ok = wait(&bars->o_full, (uint32_t)(t - 1) & 1u, 59);
+        ok = wait(&bars->o_full, (uint32_t)(t - 1) & 1u, kWaits + 59);
         if (!ok) break;
         ptx::tc_fence_after();
         add_output(corr);
@@ -293,7 +294,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->p_full);
     }
-    if (ok) ok = wait(&bars->o_full, (uint32_t)(n_kt - 1) & 1u, 60);
+    if (ok) ok = wait(&bars->o_full, (uint32_t)(n_kt - 1) & 1u, kWaits + 60);
     if (ok) {
       ptx::tc_fence_after();
       add_output(1.0f);
@@ -301,7 +302,7 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       xsum[hf * BM + r] = l_run;
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->pair[quarter]);
-      ok = wait(&bars->pair[quarter], (uint32_t)n_kt & 1u, 61);
+      ok = wait(&bars->pair[quarter], (uint32_t)n_kt & 1u, kWaits + 61);
       if (ok && row_ok) {
         const float inv = 1.0f / (l_run + xsum[(1 - hf) * BM + r]);
         const long long at = ((long long)b * L + i) * ((long long)H * D) + (long long)h * D + hf * OW;

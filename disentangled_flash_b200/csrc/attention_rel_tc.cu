@@ -1167,7 +1167,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
   }
 
-  if (fail_code != 0 && status_word != nullptr) atomicCAS(status_word, 0, fail_code);
+  if (fail_code != 0 && status_word != nullptr) atomicCAS(status_word, 0, kWaitsAttentionRel + fail_code);
   ptx::tc_fence_before();
   __syncthreads();
   if (warp == kMmaWarp) ptx::tmem_dealloc(tmem_base, kTmemCols);

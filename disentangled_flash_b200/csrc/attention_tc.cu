@@ -123,7 +123,7 @@ __device__ __forceinline__ void softmax_role(const RoleCtx& c, const DflAttnPara
   for (int kt = 0; kt < c.n_kt && ok; ++kt) {
     const int sb = kt & 1, j0 = kt * BN;
     const uint32_t use = (uint32_t)(kt >> 1) & 1u;
-    ok = ptx::mbar_wait(&bars->s_full[sb], use, abort_flag, c.status_word, 7);
+    ok = ptx::mbar_wait(&bars->s_full[sb], use, abort_flag, c.status_word, attn::kWaits + 7);
     if (!ok) break;
     ptx::tc_fence_after();
     float s[BN];
@@ -133,7 +133,7 @@ __device__ __forceinline__ void softmax_role(const RoleCtx& c, const DflAttnPara
 
     if (has_pos) {
       const int bs = kt % NB;
-      ok = ptx::mbar_wait(&bars->bias_full[bs], (uint32_t)(kt / NB) & 1u, abort_flag, c.status_word, 8);
+      ok = ptx::mbar_wait(&bars->bias_full[bs], (uint32_t)(kt / NB) & 1u, abort_flag, c.status_word, attn::kWaits + 8);
       if (!ok) break;
       const unsigned char* stage = c.smem + LO::offBias + bs * LO::kBias;
       // lut_i[-jj] is the byte offset (2*slot) of pair (i, j0+jj)
@@ -255,7 +255,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       for (int kt = 0; kt < n_kt; ++kt) {
         const int s = kt % KV_STAGES;
         const uint32_t ph = (uint32_t)(kt / KV_STAGES) & 1u;
-        if (!ptx::mbar_wait(&bars->kv_empty[s], ph ^ 1u, abort_flag, status_word, 1)) break;
+        if (!ptx::mbar_wait(&bars->kv_empty[s], ph ^ 1u, abort_flag, status_word, attn::kWaits + 1)) break;
         ptx::mbar_arrive_expect_tx(&bars->kv_full[s], (uint32_t)LO::kKV);
         unsigned char* kv = smem + LO::offKV + s * LO::kKV;
         for (int c = 0; c < LO::kSub; ++c) {
@@ -274,12 +274,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       constexpr uint32_t sbo = 8 * LO::kRowBytes;
       constexpr int kPerSub = LO::kRowBytes / 32;  // K=16 MMA steps per 64-column (or 32-column) sub-tile
       const uint32_t q_addr = ptx::smem_u32(smem + LO::offQ);
-      bool ok = ptx::mbar_wait(&bars->q_full, 0, abort_flag, status_word, 2);
+      bool ok = ptx::mbar_wait(&bars->q_full, 0, abort_flag, status_word, attn::kWaits + 2);
 
       auto issue_qk = [&](int kt) -> bool {
         const int s = kt % KV_STAGES, sb = kt & 1;
-        if (!ptx::mbar_wait(&bars->kv_full[s], (uint32_t)(kt / KV_STAGES) & 1u, abort_flag, status_word, 3)) return false;
-        if (!ptx::mbar_wait(&bars->s_free[sb], ((uint32_t)(kt >> 1) & 1u) ^ 1u, abort_flag, status_word, 4)) return false;
+        if (!ptx::mbar_wait(&bars->kv_full[s], (uint32_t)(kt / KV_STAGES) & 1u, abort_flag, status_word, attn::kWaits + 3)) return false;
+        if (!ptx::mbar_wait(&bars->s_free[sb], ((uint32_t)(kt >> 1) & 1u) ^ 1u, abort_flag, status_word, attn::kWaits + 4)) return false;
         ptx::tc_fence_after();
         const uint32_t k_addr = ptx::smem_u32(smem + LO::offKV + s * LO::kKV);
 #pragma unroll
@@ -299,7 +299,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
         if (kt + 1 < n_kt) ok = issue_qk(kt + 1);  // next S tile overlaps this tile's softmax
         if (!ok) break;
         const int s = kt % KV_STAGES, sb = kt & 1;
-        ok = ptx::mbar_wait(&bars->p_full[sb], (uint32_t)(kt >> 1) & 1u, abort_flag, status_word, 5);
+        ok = ptx::mbar_wait(&bars->p_full[sb], (uint32_t)(kt >> 1) & 1u, abort_flag, status_word, attn::kWaits + 5);
         if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t v_addr = ptx::smem_u32(smem + LO::offKV + s * LO::kKV + LO::kSub * LO::kKSub);
@@ -324,7 +324,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_con
       const size_t row_bytes = (size_t)p.ld_slots * es;
       for (int kt = 0; kt < n_kt; ++kt) {
         const int sb = kt % NB, j0 = kt * BN;
-        if (!ptx::mbar_wait(&bars->bias_empty[sb], ((uint32_t)(kt / NB) & 1u) ^ 1u, abort_flag, status_word, 6)) break;
+        if (!ptx::mbar_wait(&bars->bias_empty[sb], ((uint32_t)(kt / NB) & 1u) ^ 1u, abort_flag, status_word, attn::kWaits + 6)) break;
         unsigned char* stage = smem + LO::offBias + sb * LO::kBias;
         if (warp == 6) {
           // row r of the tile needs slots lut[i-j] for j in [j0, j0+BN): a window of <= BN slots

@@ -12,6 +12,7 @@ namespace attn {
 
 constexpr int BM = 128;  // query rows per CTA (= TMEM lanes)
 constexpr int BN = 64;   // keys per tile
+constexpr int kWaits = kWaitsAttention;
 
 template <typename T>
 struct Pack2;
@@ -104,7 +105,7 @@ __device__ __forceinline__ bool softmax_tile_tail(float (&s)[BN], RowState& st, 
 
   // O accumulated so far (tiles < kt) must be complete before it is rescaled or P(kt) is consumed
   if (kt > 0) {
-    if (!ptx::mbar_wait(o_ready, (uint32_t)(kt - 1) & 1u, abort_flag, status_word, 9)) return false;
+    if (!ptx::mbar_wait(o_ready, (uint32_t)(kt - 1) & 1u, abort_flag, status_word, kWaits + 9)) return false;
     ptx::tc_fence_after();
     if (__any_sync(0xffffffffu, corr != 1.0f)) {
 #pragma unroll
@@ -144,7 +145,7 @@ template <typename T, int D>
 __device__ __forceinline__ void softmax_store_row(const RowState& st, bool ok, bool row_ok, int n_kt, uint32_t t_o,
                                                   T* out_row, uint64_t* o_ready, volatile int* abort_flag,
                                                   int* status_word) {
-  if (ok) ok = ptx::mbar_wait(o_ready, (uint32_t)(n_kt - 1) & 1u, abort_flag, status_word, 10);
+  if (ok) ok = ptx::mbar_wait(o_ready, (uint32_t)(n_kt - 1) & 1u, abort_flag, status_word, kWaits + 10);
   ptx::tc_fence_after();
   const float inv = 1.0f / st.l_run;
 #pragma unroll

@@ -35,6 +35,25 @@ inline int check_launch(const char* what) {
   return DFL_OK;
 }
 
+// What a kernel writes to the status word when one of its waits expires: the number of the wait plus its kernel's hundred, so
+// that the code says which kernel of a forward it was.  98 (dfl_embed_layernorm: an index) and 99 (the self test) are no waits
+// of these.
+enum WaitCodes {
+  kWaitsAttention = 100, kWaitsGemmPair = 200, kWaitsGemmTile = 300, kWaitsAttentionRel = 400, kWaitsGemmF32 = 500,
+  kWaitsAttentionF32 = 600
+};
+inline const char* kernel_of_wait(int code) {
+  switch (code / 100 * 100) {
+    case kWaitsAttention: return "attention_tc_kernel";
+    case kWaitsGemmPair: return "gemm_tc_pair_kernel";
+    case kWaitsGemmTile: return "gemm_tile_kernel";
+    case kWaitsAttentionRel: return "attention_rel_kernel";
+    case kWaitsGemmF32: return "gemm_f32_kernel";
+    case kWaitsAttentionF32: return "attention_f32_kernel";
+  }
+  return code == 99 ? "the self test" : "unknown";
+}
+
 // Launchers keep their one-time configuration (shared-memory opt-in, SM count, symbol addresses) per device.
 constexpr int kMaxDevices = 64;
 

@@ -29,6 +29,7 @@ namespace {
 constexpr int kRows = 128, BK = 64;
 constexpr int kPlaneA = kRows * BK * 2;
 constexpr int kTmaWarp = 8, kMmaWarp = 9, kThreads = 320, kMaxStages = 4, kMaxSmem = 232448;
+constexpr int kWaits = kWaitsGemmF32;
 
 struct F32Args {
   int split, stages, num_kb, tiles_m, tiles_n;
@@ -258,7 +259,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     int s = 0;
     uint32_t ph = 0;
     for (int i = ahead; i < n_kb; ++i) {
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], ph, abort_flag, g.status, 41))) break;
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], ph, abort_flag, g.status, kWaits + 41))) break;
       load_w(kb_begin + i, s);
       load_x(kb_begin + i, s);
       if (++s == a.stages) {
@@ -276,8 +277,8 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       uint32_t ph = 0;
       for (int i = 0; i < n_kb; ++i) {
         const int acc = i & 1;
-        bool ok = ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, 42);
-        ok = ok && ptx::mbar_wait(&acc_empty[acc], ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, g.status, 44);
+        bool ok = ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 42);
+        ok = ok && ptx::mbar_wait(&acc_empty[acc], ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, g.status, kWaits + 44);
         if (!__all_sync(0xffffffffu, ok)) break;
         ptx::tc_fence_after();
         const uint64_t ad = adesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4)), bd = bdesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
@@ -324,7 +325,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
     const uint32_t acc_empty_leader = PAIR ? ptx::map_to_cta(ptx::smem_u32(acc_empty), leader) : ptx::smem_u32(acc_empty);
     for (int kb = 0; kb < n_kb; ++kb) {
       const int acc = kb & 1;
-      ready = ready && ptx::mbar_wait(&acc_full[acc], (uint32_t)(kb >> 1) & 1u, abort_flag, g.status, 43);
+      ready = ready && ptx::mbar_wait(&acc_full[acc], (uint32_t)(kb >> 1) & 1u, abort_flag, g.status, kWaits + 43);
       ready = __all_sync(0xffffffffu, ready);
       if (!ready) break;
       ptx::tc_fence_after();
@@ -383,7 +384,7 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         }
       }
       __syncwarp();
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(recv_bar, 0, abort_flag, g.status, 45))) rows_live = 0;
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(recv_bar, 0, abort_flag, g.status, kWaits + 45))) rows_live = 0;
       const unsigned char* recv = ring + a.ring_bytes + (uint32_t)r * pitch;
 #pragma unroll
       for (int i = 0; i < NCH; ++i) {

@@ -100,6 +100,7 @@ constexpr int kTmaWarp = 8, kMmaWarp = 9;
 constexpr int kThreads = 320;
 constexpr int kTmemCols = 512;      // two 256-column accumulators: epilogue of tile i overlaps main loop of tile i+1
 constexpr int kMaxSmem = 232448;
+constexpr int kWaits = kWaitsGemmPair;
 
 // Output staging for the tiled-store epilogue: per epilogue warp one buffer of 32 rows x 64 columns (128-byte
 // rows in the 128-byte swizzle pattern of the output tensor maps).  Two warps share a scheduler, so one converts
@@ -297,7 +298,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         for (int step = 0; step < num_kb; ++step, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1u;
-          ok = ptx::mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, g.status, 11);
+          ok = ptx::mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, g.status, kWaits + 11);
           if (!ok) break;
           if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[s], 2u * load_bytes);
           const uint32_t leader_full = ptx::map_to_cta(ptx::smem_u32(&full_bar[s]), 0);
@@ -330,14 +331,14 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       int lt = 0;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++lt) {
         const int acc = lt & 1;
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&tmem_empty_bar[acc], ((uint32_t)(lt >> 1) & 1u) ^ 1u, abort_flag, g.status, 14));
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&tmem_empty_bar[acc], ((uint32_t)(lt >> 1) & 1u) ^ 1u, abort_flag, g.status, kWaits + 14));
         if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN;
         for (int kb = 0; kb < num_kb; ++kb, ++it) {
           const int s = it % STAGES;
           const uint32_t ph = (it / STAGES) & 1u;
-          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, 12));
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 12));
           if (!ok) break;
           ptx::tc_fence_after();
           const uint64_t adesc = adesc0 + (uint64_t)(s * (kPairStageBytes >> 4));
@@ -361,7 +362,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       int m0, n0, z;
       tile_coords(tile, m0, n0, z);
       const int acc = lt & 1;
-      if (ready) ready = ptx::mbar_wait(&tmem_full_bar[acc], (uint32_t)(lt >> 1) & 1u, abort_flag, g.status, 13);
+      if (ready) ready = ptx::mbar_wait(&tmem_full_bar[acc], (uint32_t)(lt >> 1) & 1u, abort_flag, g.status, kWaits + 13);
       ptx::tc_fence_after();
       drain_accumulator<T, CONV>(g, tmap_out.m, tiled != 0, staging,
                            tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(acc * TN),

@@ -31,6 +31,7 @@ constexpr int kEpilogueWarps = 8, kTmaWarp = 8, kMmaWarp = 9;
 constexpr int kThreads = 320;
 constexpr int kMaxStages = 16;
 constexpr int kMaxSmem = 232448;
+constexpr int kWaits = kWaitsGemmTile;
 
 struct TileArgs {
   int bn, split, stages;
@@ -234,7 +235,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     int s = 0;
     uint32_t ph = 0;   // phase of empty_bar[s] that the next refill waits for
     for (int i = ahead; i < n_kb; ++i) {
-      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], ph, abort_flag, g.status, 21))) break;
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], ph, abort_flag, g.status, kWaits + 21))) break;
       load_w(kb_begin + i, s);
       load_x(kb_begin + i, s);
       if (++s == a.stages) {
@@ -253,7 +254,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
       uint32_t ph = 0;
       bool ok = true;
       for (int kb = kb_begin; kb < kb_end; ++kb) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, 22));
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 22));
         if (!ok) break;
         ptx::tc_fence_after();
         const uint64_t adesc = adesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
@@ -291,7 +292,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     asm volatile("bar.sync 1, 256;" ::: "memory");   // the eight epilogue warps
     if (g.weights_early) wait_for_predecessor();      // the output may still be read by the kernel before this one
     const RowPlace place = place_row(g, out_row + (r < out_rows ? r : 0), out_z);
-    ready = __all_sync(0xffffffffu, ptx::mbar_wait(acc_bar, 0, abort_flag, g.status, 23));
+    ready = __all_sync(0xffffffffu, ptx::mbar_wait(acc_bar, 0, abort_flag, g.status, kWaits + 23));
     ptx::tc_fence_after();
     const bool live = ready && r < out_rows;
     // staging of the output blocks: in the operand ring once that is idle, behind the receive buffer otherwise
@@ -345,7 +346,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
                                 ptx::map_to_cta(ptx::smem_u32(recv_bar), dst_rank));
         }
       }
-      ready = __all_sync(0xffffffffu, ptx::mbar_wait(recv_bar, 0, abort_flag, g.status, 24)) && ready;
+      ready = __all_sync(0xffffffffu, ptx::mbar_wait(recv_bar, 0, abort_flag, g.status, kWaits + 24)) && ready;
       const unsigned char* recv = ring + a.ring_bytes + (uint32_t)r * pitch;
       auto finish = [&](auto width, int c) {
         constexpr int NC = decltype(width)::value;
