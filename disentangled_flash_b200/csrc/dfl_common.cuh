@@ -183,7 +183,7 @@ struct GemmDesc {
   int dtype;
   int* status;          // device status word of the call, or null (the tcgen05 GEMM then uses the library's word)
   int activation;       // DFL_ACT_*: applied after the bias (row-major epilogue only)
-  // 1-D convolution as a GEMM over taps (tensor-core pair kernel only): k-step (tap, kb) multiplies rows
+  // 1-D convolution as a GEMM over taps (the 16-bit tensor-core kernels): k-step (tap, kb) multiplies rows
   // m + tap - taps/2 of X_z (rows outside [0, M) read as zero: 'same' padding) with weight matrix W[tap].
   int taps;             // 0 or 1: plain GEMM
   const void* row_mask; // [batch, M] or null: output rows whose element is zero are set to 0 before the activation

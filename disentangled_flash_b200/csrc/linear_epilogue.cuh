@@ -1,4 +1,5 @@
-// Pieces shared by the tcgen05 GEMM kernels (linear_tc.cu: large persistent tiles, linear_tile.cu: one tile per CTA).
+// Pieces shared by the two files of the 16-bit tcgen05 GEMM (linear_tc.cu: large persistent tiles, linear_tile.cu: one tile
+// per CTA).
 #pragma once
 
 #include "dfl_common.cuh"
@@ -7,11 +8,10 @@
 namespace dfl {
 
 // Epilogue of one accumulator chunk: 32 consecutive columns [n, n+32) of output row m, as fp32 bit patterns in r.
-// Adds the bias, rounds to T and stores 32 (or 16) bytes at a time, head-major or row-major.
-// CONV: padding mask of the row (`keep_row`) and tanh.
-template <typename T, bool CONV = false>
+// Adds the bias, applies GELU where asked for, rounds to T and stores 32 (or 16) bytes at a time, head-major or row-major.
+template <typename T>
 __device__ __forceinline__ void store_chunk(const GemmDesc& g, const uint32_t (&r)[32], int m, int n, int z, int ncols,
-                                            int hd, const T* bias, bool keep_row = true) {
+                                            int hd, const T* bias) {
   T* dst;
   int valid = 32;
   if (g.head_split) {
@@ -40,16 +40,9 @@ __device__ __forceinline__ void store_chunk(const GemmDesc& g, const uint32_t (&
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] += Elem<T>::to_f(bh[j]);
     }
-    if (CONV && !keep_row) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = 0.0f;
-    }
     if (g.activation == DFL_ACT_GELU) {
 #pragma unroll
       for (int j = 0; j < 8; ++j) f[j] = gelu_erf_fast(f[j]);
-    } else if (CONV && g.activation == DFL_ACT_TANH) {
-#pragma unroll
-      for (int j = 0; j < 8; ++j) f[j] = tanh_fast(f[j]);
     }
     uint4 packed;
     T* ph = reinterpret_cast<T*>(&packed);
@@ -72,7 +65,6 @@ struct TilePlan {
   int bn;      // output columns per tile, a multiple of 32 up to 256
   int split;   // CTAs (or CTA pairs) of a cluster that share one tile's inner product
   int pair;    // 1: two CTAs per 256-row tile (cta_group::2)
-  int smem_kb; // shared memory per CTA
 };
 int launch_gemm_tile(const GemmDesc& g, const TilePlan& plan, cudaStream_t stream);
 

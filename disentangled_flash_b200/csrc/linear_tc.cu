@@ -94,7 +94,7 @@ __device__ int g_gemm_status = 0;
 
 namespace {
 
-constexpr int TM = 128, TN = 256;  // 128 x 256 output tile: 87 flop per operand byte staged through shared memory
+constexpr int TM = 128, TN = 256;  // rows per CTA, columns of an accumulator (the widest tile)
 constexpr int kEpilogueWarps = 8;   // warp w drains TMEM lanes 32*(w&3).. of accumulator columns 128*(w>>2)..
 constexpr int kTmaWarp = 8, kMmaWarp = 9;
 constexpr int kThreads = 320;
@@ -210,8 +210,8 @@ __device__ __forceinline__ void drain_accumulator(const GemmDesc& g, const CUten
 
 // ---------------------------------------------------------------------------------------------------------------
 // CTA-pair form (clusters of two, `cta_group::2`): one 256 x 256 output tile per pair.  Each CTA loads its own 128
-// rows of X and 128 of the tile's 256 rows of W per k-step (32 KB for 128 x 256 x 64 of MMA work, against 48 KB in
-// the single-CTA kernel: the operand stream from L2 is what bounds this GEMM), the leader CTA (cluster rank 0)
+// rows of X and 128 of the tile's 256 rows of W per k-step (32 KB for 128 x 256 x 64 of MMA work; a CTA on its own would
+// take 48 KB, and the operand stream from L2 is what bounds this GEMM), the leader CTA (cluster rank 0)
 // issues M=256, N=256 MMAs that read both CTAs' shared memory and write 128 accumulator lanes in each CTA's TMEM,
 // and each CTA's epilogue warps drain their own lanes.  Barriers: the loads of both CTAs report to the leader's
 // `full` barriers; the leader's commits arrive on the `empty` / `tmem_full` barriers of both CTAs; the epilogue
@@ -470,7 +470,7 @@ double mma_cycles(int bn, bool pair) {   // per 16-deep step of a 128- (pair: 25
   return wide > floor_ ? wide : floor_;
 }
 
-GemmChoice choose_gemm(int M, int ncols, int K, int batch, int num_sms, bool may_pair, bool may_split) {
+GemmChoice choose_gemm(int M, int ncols, int K, int batch, int num_sms, bool may_pair) {
   GemmChoice best{};
   double best_cost = 1e30;
   const int kb = (K + 63) / 64;
@@ -486,7 +486,7 @@ GemmChoice choose_gemm(int M, int ncols, int K, int batch, int num_sms, bool may
       const double cost = kPairStart + waves * kb * per_kb(bn, true, 2.0 * (double)(tiles < slots ? tiles : slots)) + kDrain64 * bn / 64.0;
       if (cost < best_cost) {
         best_cost = cost;
-        best = {true, {bn, 1, 1, 0}};
+        best = {true, {bn, 1, 1}};
       }
     }
   }
@@ -497,7 +497,7 @@ GemmChoice choose_gemm(int M, int ncols, int K, int batch, int num_sms, bool may
       for (int i = 0; i < 6; ++i) {
         const int split = splits[i], cluster = split * (pair ? 2 : 1);
         // a part of a split product takes whole 128-element k-blocks, at least two of them
-        if (split > 1 && (!may_split || bn % (16 * split) || kb < 4 * split || cluster > 8)) continue;
+        if (split > 1 && (bn % (16 * split) || kb < 4 * split || cluster > 8)) continue;
         const long long ctas = tiles * cluster;
         // clusters do not pack every SM of the GPU's processing clusters
         const long long slots = cluster <= 2 ? num_sms : (cluster <= 6 ? num_sms * 132 / 148 : num_sms * 112 / 148);
@@ -507,7 +507,7 @@ GemmChoice choose_gemm(int M, int ncols, int K, int batch, int num_sms, bool may
         if (split > 1) cost += kExchange + (split - 1.0) / split * (M < 128 ? M : 128) * bn * 4.0 / kExchangeBytes;
         if (cost < best_cost) {
           best_cost = cost;
-          best = {false, {bn, split, pair, 226}};
+          best = {false, {bn, split, pair}};
         }
       }
     }
@@ -517,17 +517,17 @@ GemmChoice choose_gemm(int M, int ncols, int K, int batch, int num_sms, bool may
 
 // The choice is a function of the sizes alone; a forward asks for the same few over and over, so every host thread
 // keeps the last ones.
-GemmChoice cached_choice(int M, int ncols, int K, int batch, int num_sms, bool may_pair, bool may_split) {
+GemmChoice cached_choice(int M, int ncols, int K, int batch, int num_sms, bool may_pair) {
   struct Entry {
     int key[5];
     GemmChoice choice;
   };
   static thread_local Entry table[64];
-  const int key[5] = {M, ncols, K, batch, num_sms * 4 + (may_pair ? 2 : 0) + (may_split ? 1 : 0)};
+  const int key[5] = {M, ncols, K, batch, num_sms * 2 + (may_pair ? 1 : 0)};
   const uint32_t h = ((uint32_t)M * 2654435761u ^ (uint32_t)ncols * 40503u ^ (uint32_t)K * 97u ^ (uint32_t)batch * 7u) >> 3;
   Entry& e = table[h & 63u];
   if (memcmp(e.key, key, sizeof(key)) != 0) {
-    e.choice = choose_gemm(M, ncols, K, batch, num_sms, may_pair, may_split);
+    e.choice = choose_gemm(M, ncols, K, batch, num_sms, may_pair);
     memcpy(e.key, key, sizeof(key));
   }
   return e.choice;
@@ -553,9 +553,9 @@ int launch_t(const GemmDesc& g, cudaStream_t stream) {
     if (g.K >= 64 && g.M >= 2 * TM) return launch_pair<T, true>(g, TN, stream);
     const int taps = g.taps > 1 ? g.taps : 1;
     const int rows = g.M <= TM ? (g.M * g.batch + TM - 1) / (TM / g.M * g.M) * TM : (g.M + TM - 1) / TM * TM * g.batch;
-    return launch_gemm_tile(g, cached_choice(rows, ncols, g.K * taps, 1, num_sms, false, true).tile, stream);
+    return launch_gemm_tile(g, cached_choice(rows, ncols, g.K * taps, 1, num_sms, false).tile, stream);
   }
-  const GemmChoice c = cached_choice(g.M, ncols, g.K, g.batch, num_sms, true, true);
+  const GemmChoice c = cached_choice(g.M, ncols, g.K, g.batch, num_sms, true);
   return c.persistent ? launch_pair<T, false>(g, c.tile.bn, stream) : launch_gemm_tile(g, c.tile, stream);
 }
 

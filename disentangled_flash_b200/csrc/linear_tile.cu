@@ -424,12 +424,11 @@ int launch_typed(const GemmDesc& g, const TilePlan& plan, cudaStream_t stream) {
   rc = encode_tensor_map_pieces(&tmap_w, g.w, g.K, g.N, w_batches, (uint64_t)g.K * es, w_stride, PAIR ? a.bn / 2 : a.bn, 1, a.pieces);
   if (rc != DFL_OK) return rc;
 
-  // Operand ring: as many k-blocks as the inner product of one CTA has, within the shared memory of one CTA per SM,
-  // or of two when the grid has more CTAs than SMs (the second one's loads then overlap the first one's epilogue).
+  // Operand ring: as many k-blocks as the inner product of one CTA has, within all the shared memory there is (the
+  // registers of 320 threads leave room for one CTA per SM anyway).
   auto kernel = gemm_tile_kernel<T, PAIR, CONV>;
   static KernelDeviceConfig config;   // per template instantiation
-  int num_sms = 0;
-  rc = configure_kernel(config, kernel, kMaxSmem, &num_sms, "gemm_tile_kernel");
+  rc = configure_kernel(config, kernel, kMaxSmem, nullptr, "gemm_tile_kernel");
   if (rc != DFL_OK) return rc;
   const long long tiles = (long long)a.tiles_n * a.tiles_m * z_tiles;
   const int cluster = a.split * (PAIR ? 2 : 1);
@@ -438,7 +437,7 @@ int launch_typed(const GemmDesc& g, const TilePlan& plan, cudaStream_t stream) {
   const int stage = a.pieces * (kTileA + (PAIR ? a.bn / 2 : a.bn) * BK * 2);
   const int staging = kEpilogueWarps * 2048;
   const int recv = a.split > 1 ? (a.split - 1) * kRows * (a.bn / a.split * 4 + 16) : 0;
-  const int budget = plan.smem_kb * 1024 - 3072 - (a.split > 1 ? recv + staging : 0);
+  const int budget = kMaxSmem - 4096 - (a.split > 1 ? recv + staging : 0);
   const int kb_cta = (a.num_kb + a.split - 1) / a.split;
   a.stages = budget / stage;
   if (a.stages > kb_cta) a.stages = kb_cta;

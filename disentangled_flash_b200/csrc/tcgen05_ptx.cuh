@@ -196,14 +196,6 @@ __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t* bar) {
 }
 __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wait_all;" ::: "memory"); }
 
-// Shared-memory 16-bit load by 32-bit shared address.  The "memory" clobber keeps the compiler from moving
-// the load above the barrier wait that makes the data visible; the hardware still overlaps a batch of them.
-__device__ __forceinline__ uint16_t lds_u16(uint32_t saddr) {
-  uint16_t v;
-  asm volatile("ld.shared.u16 %0, [%1];" : "=h"(v) : "r"(saddr) : "memory");
-  return v;
-}
-
 __device__ __forceinline__ float ex2_approx(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -294,23 +286,6 @@ __device__ __forceinline__ void tmem_relinquish_pair() {
 }
 __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols) {
   asm volatile("tcgen05.dealloc.cta_group::2.sync.aligned.b32 %0, %1;" ::"r"(taddr), "r"(ncols) : "memory");
-}
-// D[tmem of both CTAs] (+)= A[smem of both CTAs] * B[smem of both CTAs]; issued by the leader CTA only.
-__device__ __forceinline__ void umma_ss_f16_pair(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
-                                                 uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::2.kind::f16 [%0], %1, %2, %3, p;\n\t}"
-      ::"r"(d_tmem), "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-// Arrive on the barrier at the same shared-memory offset in both CTAs of the pair (cluster ranks `leader` and
-// leader + 1) when all previously issued MMAs of this thread have completed.
-__device__ __forceinline__ void umma_commit_pair(uint64_t* bar, uint32_t leader = 0) {
-  const uint16_t both = (uint16_t)(3u << leader);
-  asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
-               ::"r"(smem_u32(bar)), "h"(both)
-               : "memory");
 }
 
 // The same instructions for a whole converged warp: the operands are computed by every lane, hence warp-uniform, and
