@@ -12,10 +12,10 @@ The hot function is :meth:`forward_prepared`.  On the current CUDA stream it
 issues ``dfl_qkv_proj`` (fused QKV projection, written head-major
 ``[B,H,L,d]``) followed by
 
-* ``dfl_attention_rel_fwd`` where it applies (FP16/BF16, head dim 32/64,
-  length up to 2048): one persistent kernel that computes the C2P/P2C scores
-  on the tensor cores from the plan's relative-distance tables and consumes
-  them in place (QK^T + relative gathers + mask + softmax + PV), or otherwise
+* ``dfl_attention_rel_fwd`` where it applies (FP16/BF16, head dim 32/64, or 128
+  beyond 96 positions, length up to 2048): one kernel that computes the C2P/P2C
+  scores on the tensor cores from the plan's relative-distance tables and
+  consumes them in place (QK^T + relative gathers + mask + softmax + PV), or otherwise
 * ``dfl_pos_scores`` (the two score GEMMs) and ``dfl_attention_fwd`` (the
   fused kernel fed with their output), the reference's operator boundary.
 
@@ -151,6 +151,13 @@ class NativeCalls(dict):
         return _copied_calls, ()
 
 
+# what a prepared call depends on beside the plan: buffers, and attributes that has_c2p, has_p2c and the scale come from
+_QKV_BUFFERS = ("_cached_qkv_weight", "_cached_qkv_bias", "_cached_qkv_planes")
+_CALL_SETTINGS = ("relative_attention", "pos_att_type", "attention_head_size", "num_attention_heads")
+_data_ptr, _dtype = torch.Tensor.data_ptr, torch.Tensor.dtype.__get__
+_stride, _numel = torch.Tensor.stride, torch.Tensor.numel
+
+
 def _copied_calls() -> NativeCalls:
     calls = NativeCalls()
     calls.copied = True
@@ -163,20 +170,26 @@ class _LayerCall:
 
     def __init__(self, module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> None:
         weight = module._cached_qkv_weight
-        # what the addresses below were taken from; held, so that they stay valid as long as this object
-        self.plan, self.tensors, self.terms = plan, self._tensors(module), (module.has_c2p, module.has_p2c)
+        # The tensors whose addresses the call below takes, and how they lie; held, so that the addresses stay valid.
+        self.plan, self.tensors = plan, tuple(map(module._buffers.get, _QKV_BUFFERS))
+        self.settings = tuple(map(module.__dict__.get, _CALL_SETTINGS))
+        tables = attention_tensors(module, plan).values()
+        if plan.rel_key is None and plan.rel_query is None:
+            tables = (*tables, plan.delta_to_local)
+        self.read = [t for t in tables if t is not None]
+        self.layout = self._layout()
         self.layers = (_cabi.DflEncoderLayer * 1)()
         fill_attention_fields(self.layers[0], module, plan)
         p = self.params = _cabi.DflEncoderParams()
         p.layers, p.n_layers, p.attention_only = self.layers, 1, 1
         p.seq_len, p.hidden, p.heads = plan.sequence_length, weight.shape[1], module.num_attention_heads
-        p.head_dim, p.dtype = module.attention_head_size, _cabi.dtype_code(weight.dtype)
+        p.head_dim, p.dtype, p.scale = module.attention_head_size, _cabi.dtype_code(weight.dtype), module._score_scale()
         p.lut, p.n_active = plan.delta_to_local.data_ptr(), plan.active_slots.numel()
         self.width = module.all_head_size
 
-    @staticmethod
-    def _tensors(module: "DisentangledFlashAttention") -> tuple[torch.Tensor | None, ...]:
-        return module._cached_qkv_weight, module._cached_qkv_bias, module._cached_qkv_planes
+    def _layout(self) -> tuple[list, ...]:
+        read = self.read
+        return list(map(_data_ptr, read)), list(map(_dtype, read)), list(map(_stride, read)), list(map(_numel, read))
 
     @staticmethod
     def covers(module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> bool:
@@ -190,10 +203,13 @@ class _LayerCall:
         return not ((module.has_c2p and plan.pos_key_planes is None) or (module.has_p2c and plan.pos_query_planes is None))
 
     def serves(self, module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> bool:
-        """Whether this object was made from the module's and the plan's present tensors and terms."""
+        """Whether this object was made from the module's and the plan's present tensors, as they lie now, and settings."""
 
-        return (self.plan is plan and self.terms == (module.has_c2p, module.has_p2c)
-                and all(a is b for a, b in zip(self.tensors, self._tensors(module))))
+        weight, bias, planes = self.tensors
+        buffers = module._buffers
+        return (plan is self.plan and weight is buffers["_cached_qkv_weight"] and bias is buffers["_cached_qkv_bias"]
+                and planes is buffers["_cached_qkv_planes"] and self.settings == tuple(map(module.__dict__.get, _CALL_SETTINGS))
+                and self.layout == self._layout())
 
     def __call__(self, module: "DisentangledFlashAttention", hidden_states: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         p = _cabi.DflEncoderParams()
@@ -201,23 +217,26 @@ class _LayerCall:
         out = torch.empty(*hidden_states.shape[:2], self.width, dtype=hidden_states.dtype, device=hidden_states.device)
         p.x, p.mask, p.mask_elem_size, p.batch = hidden_states.data_ptr(), mask.data_ptr(), mask.element_size(), hidden_states.shape[0]
         p.outs = (ctypes.c_void_p * 1)(out.data_ptr())
-        status = module._status_word
-        p.scale, p.status = module._score_scale(), None if status is None else status.data_ptr()
+        status = module._buffers["_status_word"]
+        p.status = None if status is None else status.data_ptr()
         _cabi.encoder_fwd(p, hidden_states.device)
         return out
 
 
-def fill_attention_fields(entry: "_cabi.DflEncoderLayer", module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> None:
+def attention_tensors(module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> dict[str, torch.Tensor | None]:
     """The QKV and position-table entries of one layer of ``dfl_encoder_fwd``."""
 
     f32 = module._cached_qkv_weight.dtype == torch.float32
-    tensors = {
+    return {
         "qkv_w": module._cached_qkv_planes if f32 else module._cached_qkv_weight, "qkv_b": module._cached_qkv_bias,
         "rel_key": plan.rel_key if module.has_c2p else None, "rel_query": plan.rel_query if module.has_p2c else None,
         "pos_key": (plan.pos_key_planes if f32 else plan.pos_key) if module.has_c2p else None,
         "pos_query": (plan.pos_query_planes if f32 else plan.pos_query) if module.has_p2c else None,
     }
-    for field, tensor in tensors.items():
+
+
+def fill_attention_fields(entry: "_cabi.DflEncoderLayer", module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> None:
+    for field, tensor in attention_tensors(module, plan).items():
         setattr(entry, field, None if tensor is None else tensor.data_ptr())
 
 
@@ -283,7 +302,7 @@ class DisentangledFlashAttention(nn.Module):
         # shares one word between its layers (set_status_word) and reads it in check_device_status()
         self.register_buffer("_status_word", None, persistent=False)
         self._position_projection_cache: dict[tuple[int, str], B200PreparedPositionPlan] = {}
-        self._layer_calls: dict[int, _LayerCall | None] = NativeCalls()   # per sequence length
+        self._layer_calls: dict[int, _LayerCall] = NativeCalls()   # per sequence length
         self._algo = _cabi.ALGO_AUTO
         self.register_load_state_dict_post_hook(_invalidate_attention_cache_after_load)
 
@@ -472,19 +491,6 @@ class DisentangledFlashAttention(nn.Module):
         if torch.is_grad_enabled():
             raise RuntimeError("DisentangledFlashAttention requires torch.no_grad() or torch.inference_mode()")
 
-    def _require_inputs_of_this_module(self, hidden_states: torch.Tensor, attention_mask: torch.Tensor) -> None:
-        """Refuse what the kernels, which see addresses only, would read past its end or on another device."""
-
-        weight = self._cached_qkv_weight
-        batch_size, sequence_length = hidden_states.shape[:2]
-        if hidden_states.shape[-1] != weight.shape[1] or hidden_states.numel() != batch_size * sequence_length * weight.shape[1]:
-            raise ValueError(f"hidden_states shape {tuple(hidden_states.shape)} does not match [B, L, {weight.shape[1]}]")
-        if hidden_states.device != weight.device:
-            raise RuntimeError(f"hidden_states is on {hidden_states.device}, the module on {weight.device}")
-        if attention_mask.device != hidden_states.device:
-            raise RuntimeError(f"attention_mask must be on the device of hidden_states ({hidden_states.device}), "
-                               f"got {attention_mask.device}")
-
     def _require_plan_of_this_module(self, plan: B200PreparedPositionPlan, device: torch.device) -> None:
         """Refuse a plan whose tables have another geometry, type or device than this module's."""
 
@@ -529,26 +535,36 @@ class DisentangledFlashAttention(nn.Module):
             raise ValueError(
                 f"prepared length {plan.sequence_length} does not match input length {sequence_length}"
             )
-        if self._cached_qkv_weight is None:
+        weight = self._buffers["_cached_qkv_weight"]
+        if weight is None:
             raise RuntimeError("fused QKV projection is not prepared; call prepare_for_inference() first")
-        if hidden_states.dtype != self._cached_qkv_weight.dtype:
+        if hidden_states.dtype != weight.dtype:
             raise TypeError("hidden_states dtype does not match the module's parameters")
-        self._require_inputs_of_this_module(hidden_states, attention_mask)
+        # Refuse what the kernels, which see addresses only, would read past its end or on another device.
+        device, hidden_size = hidden_states.device, weight.shape[1]
+        if hidden_states.shape[-1] != hidden_size or hidden_states.numel() != batch_size * sequence_length * hidden_size:
+            raise ValueError(f"hidden_states shape {tuple(hidden_states.shape)} does not match [B, L, {hidden_size}]")
+        if device != weight.device:
+            raise RuntimeError(f"hidden_states is on {device}, the module on {weight.device}")
+        if attention_mask.device != device:
+            raise RuntimeError(f"attention_mask must be on the device of hidden_states ({device}), got {attention_mask.device}")
         base_mask = _require_2d_padding_mask(attention_mask, batch_size, sequence_length)
+        tracing = torch.compiler.is_compiling()
+        if not tracing and self._algo == _cabi.ALGO_AUTO:
+            call = self._layer_calls.get(sequence_length)
+            if call is not None and call.serves(self, plan):   # made after the checks below
+                return call(self, hidden_states.contiguous(), base_mask), None
         if self.has_c2p and plan.pos_key is None:
             raise ValueError("prepared plan has no content-to-position keys")
         if self.has_p2c and plan.pos_query is None:
             raise ValueError("prepared plan has no position-to-content queries")
-
-        if not torch.compiler.is_compiling():
-            self._require_plan_of_this_module(plan, hidden_states.device)
-            call = self._layer_calls.get(sequence_length)
-            if call is None or not call.serves(self, plan):
-                call = self._layer_calls[sequence_length] = _LayerCall(self, plan) if _LayerCall.covers(self, plan) else None
-            if call is not None and self._algo == _cabi.ALGO_AUTO:
+        if not tracing:
+            self._require_plan_of_this_module(plan, device)
+            if _LayerCall.covers(self, plan):
+                call = self._layer_calls[sequence_length] = _LayerCall(self, plan)
                 return call(self, hidden_states.contiguous(), base_mask), None
         uses_lut = self.has_c2p or self.has_p2c
-        output = (_attention_forward_op if torch.compiler.is_compiling() else _attention_forward)(
+        output = (_attention_forward_op if tracing else _attention_forward)(
             hidden_states.contiguous(),
             base_mask,
             self._cached_qkv_weight,
@@ -572,8 +588,8 @@ class DisentangledFlashAttention(nn.Module):
                             packed_input: tuple[torch.Tensor, tuple[torch.Tensor, ...]] | None = None) -> torch.Tensor:
         """``forward_prepared`` with the context written as packed rows ``[T, H*d]``: sequence ``b`` owns rows
         ``row_base[b] .. + row_count[b]`` (``packed_rows = (row_base, row_count, T)``); positions beyond
-        ``row_count[b]`` are not stored.  Only on the single-launch attention path (FP16/BF16, head dim 32/64, a
-        relative term); no counterpart in the reference, which keeps padded positions in every tensor.
+        ``row_count[b]`` are not stored.  Only on the single-launch attention path (FP16/BF16, a relative term,
+        expanded tables); no counterpart in the reference, which keeps padded positions in every tensor.
 
         With ``packed_input = (row_groups, (q, k, v))`` the hidden states are packed rows ``[T, hid]`` as well
         (``attention_mask`` still gives batch and length): the projection writes group ``g`` of 32 rows to rows
