@@ -6,8 +6,8 @@
 // x = j - i = e - (L-1) uses, so the two relative terms of a (128 query x 128 key) tile are
 //   C2P[i, j] = q_i . rel_key[x]      P2C[i, j] = k_j . rel_query[x]
 // with x running over one contiguous window of 255 table rows.  Both are produced by tcgen05.mma from 128-row
-// table blocks (L2 resident), rounded to the input type exactly like the separate score GEMMs round their output,
-// and parked in shared memory, where the softmax threads pick them up along diagonals.
+// table blocks (L2 resident) and rounded to the input type exactly like the separate score GEMMs round their output;
+// converter warps undo the diagonal on the way through shared memory:
 //   C2P depends on the query rows only: D[r, m] = q_r . rel_key[x_lo + m] with TMEM lanes = query rows.  The window of a
 //       key tile is two 128-column blocks; the next key tile needs one new block.  Converter warps round a block's rows and
 //       store each shifted by its row, so that key x of the tile ends up in column x: a softmax thread adds its 64 scores
@@ -28,10 +28,11 @@
 //   warp 16     issuer of the C2P block MMAs and of S with the P2C tile added, and TMEM owner
 //   warp 17     per-item mask analysis (kept-key bits, skipped key tiles), one item ahead, and TMA producer
 //   warp 18     issuer of the PV MMAs, warp 19 of the P2C parts
-// What bounds it: instruction issue and fetch.  With everything unrolled (156 KB of code) a third of the issue slots were
-// lost to instruction fetch; the waits, the loader and the MMA loops are therefore rolled (88 KB), which was worth 17 %.
-// 32 x 12 heads x 512 x d 64, fp16, both terms: 185 -> 173 us, C2P only 145 -> 117 us against two passes over the keys with
-// the diagonals read by the softmax threads.
+// What bounds it: the chain of the roles within a tile.  S waits for the P2C operand, which the converters fill (4.5 k cycles a
+// tile of 5.7 to 6.0 k) and the identity MMA empties (1 k) before they may refill it; the tensor pipe is 27 % active.
+// The waits, the loader and the MMA loops are rolled: with everything unrolled (156 KB of code) a third of the issue slots
+// were lost to instruction fetch.  32 x 12 heads x 512 x d 64, fp16: both terms 148 us, C2P alone 110, P2C alone 130 (185 us
+// for both when the softmax threads read the diagonals in two passes over the keys).
 #include <type_traits>
 
 #include "attention_tc_common.cuh"
@@ -1228,9 +1229,10 @@ int launch_rel_typed(const DflAttnRelParams& p, cudaStream_t stream) {
 }  // namespace
 
 bool attention_rel_supported(const DflAttnRelParams& p) {
-  // d = 128 beyond 96 positions: plans of shorter buckets have no relative tables at this head dim, which is part of the
-  // interface.  Above the line one launch beats three at every size: 130 positions 38.8 -> 19.4 us (1 x 8 heads), 512
-  // positions 212 -> 100 us (16 x 8 heads).
+  // d = 128 beyond 96 positions: plans of shorter buckets have no relative tables at this head dim, which callers rely on.
+  // The line is that of the interface, not a crossover: one launch beats three from 16 positions on (us, three / one: 16
+  // positions 13.3 / 13.1 for 1 x 8 heads, 51 / 36 for 64 x 8; 96 positions 18.5 / 13.1 and 87 / 36; 512 positions 212 / 97 for
+  // 16 x 8 heads).
   return p.dtype != DFL_F32 && (p.head_dim == 32 || p.head_dim == 64 || (p.head_dim == 128 && p.seq_len > 96)) &&
          (p.rel_key || p.rel_query) && p.seq_len >= 1 && p.seq_len <= kMaxSeqLen;
 }

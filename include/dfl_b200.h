@@ -44,7 +44,7 @@ extern "C" {
 #define DFL_F32   2
 
 /* kernel family selection: AUTO = tcgen05 kernels for F16/BF16, IEEE-fp32
- * CUDA-core kernels for F32.  SIMT forces the CUDA-core kernels for any
+ * CUDA-core kernels for F32 (the F32 forms over bf16 planes are functions of their own).  SIMT forces the CUDA-core kernels for any
  * dtype; it exists so that tests can cross-check the tensor-core kernels at
  * sizes where a CPU oracle is too slow. */
 #define DFL_ALGO_AUTO  0
@@ -241,9 +241,10 @@ DFL_API size_t dfl_static_scratch_bytes(void);
  * dfl_pos_scores + dfl_attention_fwd (the two torch.matmul calls kernel.py:574-585 followed by the Triton
  * kernel kernel.py:137-429): S = QK^T + q_i.rel_key[j-i] + k_j.rel_query[j-i], the two relative terms
  * rounded to the input type as the separate score GEMMs round their output, scale, 2-D padding mask,
- * softmax, PV.  The score tensors [B,H,L,A] never exist in global memory.  A persistent kernel: one CTA
- * per SM walks (batch, head, 128-query-tile) items.  Covered: FP16/BF16, head_dim 32 or 64, at least one
- * relative term, seq_len <= 2048; dfl_attention_rel_supported() tells, other configurations return
+ * softmax, PV.  The score tensors [B,H,L,A] never exist in global memory.  A persistent kernel (one CTA
+ * per SM walks (batch, head, 128-query-tile) items), or one CTA per (batch, head) for short sequences.
+ * Covered: FP16/BF16, head_dim 32 or 64, or 128 beyond 96 positions, at least one relative term,
+ * seq_len <= 2048; dfl_attention_rel_supported() tells, other configurations return
  * DFL_ERR_UNSUPPORTED (use dfl_pos_scores + dfl_attention_fwd for them).
  */
 typedef struct DflAttnRelParams {

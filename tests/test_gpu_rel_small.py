@@ -1,4 +1,4 @@
-"""The short-sequence form of the relative-table attention: row and key remainders of its three sizes, masks and single
+"""The short-sequence form of the relative-table attention: row and key remainders of its four sizes, masks and single
 terms, the packed output, and the batch size at which 65 .. 128 positions go to the other kernel."""
 
 import pytest
