@@ -64,8 +64,8 @@ WORKLOAD = dict(name="deberta-v3-base-encoder", geometry="v3-base", batch=32, se
 MIXED = dict(name="deberta-v3-large-mixed-buckets", geometry="v3-large", buckets={128: 171, 256: 171, 512: 170})
 FALLBACK_PEAKS = dict(hbm_gbs=6650.0, bf16_tflops=1590.0, bf16_tflops_sustained=1400.0)
 # DRAM bytes of one dfl_attention_rel_fwd launch per sequence of the default workload (12 heads, L=512, d=64, FP16,
-# valid lengths U[256,512]): dram__bytes_read.sum + dram__bytes_write.sum of the ncu capture summarised in
-# profiles/attention_rel_kernel_v3base_b32_l512_d64_fp16.md (81.1 MB read + 12.5 MB written at B=32), per sequence.
+# valid lengths U[256,512]): dram__bytes_read.sum + dram__bytes_write.sum of an ncu capture of the launch inside the
+# workload (81.1 MB read + 12.5 MB written at B=32), per sequence.
 ATTN_DRAM_BYTES_PER_SEQUENCE = (81.146624e6 + 12.506368e6) / 32
 
 
@@ -823,7 +823,7 @@ def run_v2_xlarge(args, ctx: GpuContext) -> None:
                        "batch": batch, "buckets": list(lengths), "valid_lengths": "uniform[L/2, L]",
                        "note": "one encoder, four prepared buckets; eager = activate_shape() + forward, cuda-graph = "
                                "capture_deberta_buckets() replay (inputs copied into the graph's buffers inside the "
-                               "timed region); fp32 = strict IEEE kernels, eager only",
+                               "timed region); fp32 = at fp32 accuracy (bf16 planes on the tensor cores), eager only",
                        "headline_row": "bf16 cuda-graph L=512"},
             "rows": rows}))
 
