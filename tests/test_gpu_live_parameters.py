@@ -127,3 +127,16 @@ def test_a_copy_of_a_prepared_encoder_has_weights_of_its_own(dtype):
     assert 40 in twin._layer_loops
     assert_follows(twin, hidden, mask, before, dtype)
     assert torch.equal(both(encoder, hidden, mask)[0], before)
+
+
+@pytest.mark.parametrize("dtype,length", ((torch.float32, 32), (torch.float16, 32), (torch.float16, 256)))
+def test_a_captured_graph_outlives_the_preparation_it_was_captured_from(dtype, length):
+    encoder, hidden, mask = prepared(dtype, length, conv=0 if dtype == torch.float32 else 3)
+    bucket = df.capture_deberta_buckets(encoder, 2)[length]
+    before = bucket(hidden, mask).clone()
+    held = [t.data_ptr() for t in (*bucket.prepared[0][0][1:], *bucket.prepared[1][0]) if t is not None]
+    encoder.prepare_for_inference([length + 1])
+    fresh = {t.data_ptr() for plan in encoder._active_plans for t in plan[1:] if t is not None}
+    assert held and not fresh & set(held)   # nothing new lies where the graph reads
+    junk = [torch.full((n,), float("nan"), device=dev) for n in (1 << 10, 1 << 16, 1 << 18, 1 << 20) for _ in range(8)]
+    assert torch.equal(bucket(hidden, mask), before) and junk
