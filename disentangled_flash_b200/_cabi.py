@@ -306,8 +306,7 @@ class _on_device:
     __slots__ = ("index", "previous")
 
     def __init__(self, device: torch.device | str):
-        device = torch.device(device)
-        self.index = device.index
+        self.index = device.index if isinstance(device, torch.device) else torch.device(device).index
         self.previous = -1
 
     def __enter__(self) -> None:
@@ -815,12 +814,17 @@ def linear_heads_planes(x: torch.Tensor, weight: torch.Tensor, bias: torch.Tenso
     return out
 
 
-def encoder_fwd(p: DflEncoderParams, device: torch.device) -> None:
-    """The whole layer loop (``dfl_encoder_fwd``) on the current stream; every field but the workspace is the caller's."""
+def encoder_fwd(p: DflEncoderParams, device: torch.device, sizes: dict[int, int] | None = None) -> None:
+    """The whole layer loop (``dfl_encoder_fwd``) on the current stream; every field but the workspace is the caller's.
+    ``sizes``: workspace bytes by batch, kept by a caller whose other sizes do not change."""
 
     lib = load_library()
     ref = ctypes.byref(p)
-    size = lib.dfl_encoder_workspace_bytes(ref)
+    size = None if sizes is None else sizes.get(p.batch)
+    if size is None:
+        size = lib.dfl_encoder_workspace_bytes(ref)
+        if sizes is not None and len(sizes) < 64:
+            sizes[p.batch] = size
     with _on_device(device):
         workspace = torch.empty(size, dtype=torch.uint8, device=device)
         p.workspace, p.workspace_bytes = workspace.data_ptr(), size

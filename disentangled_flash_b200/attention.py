@@ -154,8 +154,7 @@ class NativeCalls(dict):
 # what a prepared call depends on beside the plan: buffers, and attributes that has_c2p, has_p2c and the scale come from
 _QKV_BUFFERS = ("_cached_qkv_weight", "_cached_qkv_bias", "_cached_qkv_planes")
 _CALL_SETTINGS = ("relative_attention", "pos_att_type", "attention_head_size", "num_attention_heads")
-_data_ptr, _dtype = torch.Tensor.data_ptr, torch.Tensor.dtype.__get__
-_stride, _numel = torch.Tensor.stride, torch.Tensor.numel
+_data_ptr = torch.Tensor.data_ptr
 
 
 def _copied_calls() -> NativeCalls:
@@ -170,14 +169,14 @@ class _LayerCall:
 
     def __init__(self, module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> None:
         weight = module._cached_qkv_weight
-        # The tensors whose addresses the call below takes, and how they lie; held, so that the addresses stay valid.
+        # The tensors whose addresses the call below takes; held, so that the addresses stay valid.
         self.plan, self.tensors = plan, tuple(map(module._buffers.get, _QKV_BUFFERS))
         self.settings = tuple(map(module.__dict__.get, _CALL_SETTINGS))
         tables = attention_tensors(module, plan).values()
         if plan.rel_key is None and plan.rel_query is None:
             tables = (*tables, plan.delta_to_local)
         self.read = [t for t in tables if t is not None]
-        self.layout = self._layout()
+        self.addresses = list(map(_data_ptr, self.read))
         self.layers = (_cabi.DflEncoderLayer * 1)()
         fill_attention_fields(self.layers[0], module, plan)
         p = self.params = _cabi.DflEncoderParams()
@@ -186,10 +185,7 @@ class _LayerCall:
         p.head_dim, p.dtype, p.scale = module.attention_head_size, _cabi.dtype_code(weight.dtype), module._score_scale()
         p.lut, p.n_active = plan.delta_to_local.data_ptr(), plan.active_slots.numel()
         self.width = module.all_head_size
-
-    def _layout(self) -> tuple[list, ...]:
-        read = self.read
-        return list(map(_data_ptr, read)), list(map(_dtype, read)), list(map(_stride, read)), list(map(_numel, read))
+        self.workspace_sizes: dict[int, int] = {}
 
     @staticmethod
     def covers(module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> bool:
@@ -203,23 +199,24 @@ class _LayerCall:
         return not ((module.has_c2p and plan.pos_key_planes is None) or (module.has_p2c and plan.pos_query_planes is None))
 
     def serves(self, module: "DisentangledFlashAttention", plan: B200PreparedPositionPlan) -> bool:
-        """Whether this object was made from the module's and the plan's present tensors, as they lie now, and settings."""
+        """Whether this object was made from the module's and the plan's present tensors, where they are now, and settings."""
 
         weight, bias, planes = self.tensors
         buffers = module._buffers
         return (plan is self.plan and weight is buffers["_cached_qkv_weight"] and bias is buffers["_cached_qkv_bias"]
                 and planes is buffers["_cached_qkv_planes"] and self.settings == tuple(map(module.__dict__.get, _CALL_SETTINGS))
-                and self.layout == self._layout())
+                and self.addresses == list(map(_data_ptr, self.read)))
 
     def __call__(self, module: "DisentangledFlashAttention", hidden_states: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         p = _cabi.DflEncoderParams()
         ctypes.pointer(p)[0] = self.params   # a copy: several threads may run one module
-        out = torch.empty(*hidden_states.shape[:2], self.width, dtype=hidden_states.dtype, device=hidden_states.device)
-        p.x, p.mask, p.mask_elem_size, p.batch = hidden_states.data_ptr(), mask.data_ptr(), mask.element_size(), hidden_states.shape[0]
+        device, (batch, length) = hidden_states.device, mask.shape
+        out = torch.empty((batch, length, self.width), dtype=hidden_states.dtype, device=device)
+        p.x, p.mask, p.mask_elem_size, p.batch = hidden_states.data_ptr(), mask.data_ptr(), mask.element_size(), batch
         p.outs = (ctypes.c_void_p * 1)(out.data_ptr())
         status = module._buffers["_status_word"]
         p.status = None if status is None else status.data_ptr()
-        _cabi.encoder_fwd(p, hidden_states.device)
+        _cabi.encoder_fwd(p, device, self.workspace_sizes)
         return out
 
 

@@ -32,7 +32,7 @@ def prepared(monkeypatch):
                                            rel, None if f32 else rel.clone(), planes, planes)
         calls = []
         monkeypatch.setattr(module, "_validate_device_dtype", lambda tensor: None)
-        monkeypatch.setattr(_cabi, "encoder_fwd", lambda p, device: calls.append(("native", p.scale)))
+        monkeypatch.setattr(_cabi, "encoder_fwd", lambda p, *_: calls.append(("native", p.scale)))
         monkeypatch.setattr(attention, "_attention_forward", lambda *a: calls.append(("general", a)) or torch.empty(0))
         return module, plan, calls
 
