@@ -24,15 +24,21 @@
 //   warps 0-7   softmax: two threads per query row (warps w and w+4 own the same TMEM lanes; each takes 64 of the
 //               128 keys of a tile, 32 of the 64 packed P columns and half of the output columns).  One pass: the 64
 //               scores stay in registers from the S load to the P store.
-//   warps 8-11  converters of the P2C parts (TMEM -> 16-bit -> shared memory), warps 12-15 of the C2P blocks
-//   warp 16     issuer of the C2P block MMAs and of S with the P2C tile added, and TMEM owner
-//   warp 17     per-item mask analysis (kept-key bits, skipped key tiles), one item ahead, and TMA producer
-//   warp 18     issuer of the PV MMAs, warp 19 of the P2C parts
-// What bounds it: the chain of the roles within a tile.  S waits for the P2C operand, which the converters fill (4.5 k cycles a
-// tile of 5.7 to 6.0 k) and the identity MMA empties (1 k) before they may refill it; the tensor pipe is 27 % active.
-// The waits, the loader and the MMA loops are rolled: with everything unrolled (156 KB of code) a third of the issue slots
-// were lost to instruction fetch.  32 x 12 heads x 512 x d 64, fp16: both terms 148 us, C2P alone 110, P2C alone 130 (185 us
-// for both when the softmax threads read the diagonals in two passes over the keys).
+//   warps 8-15  converters of the P2C parts (TMEM -> 16-bit -> shared memory), warps 16-23 of the C2P blocks; two warps
+//               per TMEM lane quarter and role, one for each accumulator of the role's pair
+//   warp 24     issuer of S with the P2C tile added, and TMEM owner
+//   warp 25     per-item mask analysis (kept-key bits, skipped key tiles), one item ahead, and TMA producer of Q, K, rel_query
+//   warp 26     issuer of the PV and C2P block MMAs and of the loads of V and rel_key, warp 27 of the P2C parts
+// What bounds it: a 128 x 128 tile takes 5.4 k cycles, of which a softmax thread works 3.5 k and waits 1.2 k for S; S waits
+// for the P2C operand, which the converters fill in 2.5 k once the identity MMA has released it.  No unit is busy: each role is
+// a chain of dependent instructions that its warps cannot overlap with themselves, so what helps is more warps a role and
+// loads far enough ahead.  us, launch after launch, both terms, no padding, before (one converter warp per quarter and role,
+// one loader in MMA order, C2P behind S in one issuer) and now:
+//   32 x 12 heads x 512 x d 64 fp16 155 -> 135     64 x 16 x 256 x 64 bf16 109 -> 95     7 x 12 x 333 x 64 bf16 29.1 -> 26.2
+//   16 x 24 x 256 x d 32 fp16 46.9 -> 38.6         16 x 8 x 512 x d 128 bf16 104 -> 78
+// The converters' register budget matters more than their number: at 48 registers with the next columns in flight while the
+// last are stored they spill, and the kernel took 238 us.  The waits, the loader and the MMA loops are rolled: with everything
+// unrolled (156 KB of code) a third of the issue slots were lost to instruction fetch.
 #include <type_traits>
 
 #include "attention_tc_common.cuh"
@@ -48,25 +54,25 @@ using attn::Pack2;
 constexpr int BM = 128;              // query rows per item (= TMEM lanes)
 constexpr int BK = 128;              // keys per tile
 constexpr int kSoftmaxWarps = 8;
-constexpr int kC2pWarp = 12;         // warps 8-11 convert the P2C parts, 12-15 the C2P blocks
-constexpr int kMmaWarp = 16;
-constexpr int kTmaWarp = 17;
-constexpr int kPvWarp = 18;
-constexpr int kPartWarp = 19;
-constexpr int kThreads = 640;
-constexpr int kSoftmaxRegs = 128;    // 256 x 128 + 256 x 80 + 128 x 64 = 61440 registers
-constexpr int kConvRegs = 80;
-constexpr int kMiscRegs = 64;
-// The kernel is launched with 65536 / kThreads registers per thread, rounded down to the allocation unit of 8: 96.
+constexpr int kC2pWarp = 16;         // warps 8-15 convert the P2C parts, 16-23 the C2P blocks
+constexpr int kMmaWarp = 24;
+constexpr int kTmaWarp = 25;
+constexpr int kPvWarp = 26;
+constexpr int kPartWarp = 27;
+constexpr int kThreads = 896;
+constexpr int kSoftmaxRegs = 128;    // 256 x 128 + 512 x 48 + 128 x 56 = 64512 registers
+constexpr int kConvRegs = 48;
+constexpr int kMiscRegs = 56;
+// The kernel is launched with 65536 / kThreads registers per thread, rounded down to the allocation unit of 8: 72.
 // `setmaxnreg.inc` waits until the pool holds what it asks for, so the three budgets must not ask for more than the SM has (a wait that nothing could
 // bound); `setmaxnreg.dec` with a value above the launch allocation is an illegal instruction.
 constexpr int kLaunchRegs = 65536 / kThreads / 8 * 8;
-static_assert(8 * 32 * kSoftmaxRegs + 8 * 32 * kConvRegs + 4 * 32 * kMiscRegs <= kThreads * kLaunchRegs,
+static_assert(8 * 32 * kSoftmaxRegs + 16 * 32 * kConvRegs + 4 * 32 * kMiscRegs <= kThreads * kLaunchRegs,
               "register budgets of the three warpgroup kinds exceed what the launch allocates");
 static_assert(kSoftmaxRegs >= kLaunchRegs && kConvRegs <= kLaunchRegs && kMiscRegs <= kLaunchRegs &&
                   kSoftmaxRegs % 8 == 0 && kConvRegs % 8 == 0 && kMiscRegs % 8 == 0,
               "setmaxnreg.inc raises and setmaxnreg.dec lowers the launch allocation, in multiples of 8");
-constexpr int kConsumerWarps = 19;   // softmax, converters, MMA issuers: every warp that reads an item slot
+constexpr int kConsumerWarps = 27;   // softmax, converters, MMA issuers: every warp that reads an item slot
 
 constexpr int kItemSlots = 3;        // the loader analyses one item ahead of the one whose tiles it loads
 constexpr int kMaxSeqLen = 2048;
@@ -81,46 +87,53 @@ constexpr int ROW_PITCH = 528;
 // that the 4-byte stores of 32 neighbouring keys, each shifted by its key, fall into 32 different banks).
 constexpr int STG_CHUNK = 16 * 128 + 32;
 constexpr int STG_BYTES = 16 * STG_CHUNK;
-// Identity operand of that MMA: 240 rows x 16 columns, row 112 + k holds a one in column k and the others are zero; k-step
-// kk of the 128 x 128 identity is the 128-row window that starts at row 112 - 16 kk.
-constexpr int EYE_ROWS = 240;
-constexpr int EYE_CHUNK = EYE_ROWS * 16;   // bytes between the two 8-column chunks
-constexpr int EYE_BYTES = 2 * EYE_CHUNK;
+// Identity operand of that MMA, a strip of 16-byte rows: row 120 + c holds a one in column c.  The two chunks of eight columns
+// of a K = 16 step are windows of 128 rows of this strip, EYE_LBO apart: k-step kk of the 128 x 128 identity takes the window
+// from row 112 - 16 kk for the upper eight of its columns and the one eight rows further down for the lower eight (the
+// P2C operand gives its chunks in that order too: they lie in descending order of the query rows).
+constexpr int EYE_ROWS = 248;
+constexpr int EYE_LBO = 128;
+constexpr int EYE_BYTES = EYE_ROWS * 16;
 
 // TMEM columns (all 512; one CTA per SM)
 constexpr int COL_S = 0;      // 128  S = Q K^T of the current tile (fp32)
 constexpr int COL_P = 128;    // 64   P of the current tile (16-bit pairs), A operand of the PV MMA
 constexpr int COL_O = 192;    // D    O accumulator
-                              // XC: one new C2P block for the 128 query rows, 128 columns from 256 on; half a block at a
-                              // time, 64 columns from 320 on, with d = 128
+                              // XC: 2 x 64   halves of a new C2P block for the 128 query rows, from 256 on; with d = 128
+                              // both in turn in the 64 columns from 320 on
 constexpr int COL_XP = 384;   // 2 x 64  two of the four parts (64 table rows each) of the P2C accumulator of a key tile
 constexpr int kTmemCols = 512;
 
 template <int D>
 struct RLayout {
   static_assert(D == 32 || D == 64 || D == 128, "head dims 32, 64 and 128");
-  // An operand tile is kSub sub-tiles of at most 64 columns, one swizzled 64- or 128-byte row per tile row.  The table blocks
-  // and V come in kPieces pieces: at d = 128 in 64-row halves, the only way one stage of each fits beside Q and K.
+  // An operand tile is kSub sub-tiles of at most 64 columns, one swizzled 64- or 128-byte row per tile row.  The tables come
+  // in pieces of 64 rows, V at d = 128 too.
   static constexpr int kSub = D > 64 ? 2 : 1;
-  static constexpr int kPieces = D > 64 ? 2 : 1;
-  static constexpr int kPieceRows = 128 / kPieces;
   static constexpr int kRowBytes = D * 2 / kSub;
   static constexpr int kTile = 128 * D * 2;            // Q tile, K tile
-  static constexpr int kPiece = kPieceRows * D * 2;    // piece of V or of a 128-row table block
-  static constexpr int kSteps = D / 16;                // K=16 steps over d
-  static constexpr int kKStages = D > 64 ? 1 : 2, kRqStages = D > 64 ? 1 : 2;
-  static constexpr int kVStages = D == 32 ? 2 : 1;     // d = 64 fills shared memory: V and rel_key blocks are
-  static constexpr int kRkStages = D == 32 ? 2 : 1;    // reloaded within the tile time after their single use
-  static constexpr int kXcCols = 128 / kPieces;        // C2P accumulator
+  static constexpr int kTab = 64 * D * 2;              // piece of a table
+  static constexpr int kVPieces = D > 64 ? 2 : 1;
+  static constexpr int kVRows = 128 / kVPieces;
+  static constexpr int kVPiece = kVRows * D * 2;
+  static constexpr int kKStages = D > 64 ? 1 : 2;
+  static constexpr int kVStages = D == 32 ? 2 : 1;
+  // d = 64 and 128 fill shared memory.
+  static constexpr int kRkStages = D == 32 ? 4 : (D == 64 ? 3 : 1);
+  static constexpr int kRqStages = D == 32 ? 4 : (D == 64 ? 4 : 1);
+  // P2C operand tiles.  d 64 has room for a second one only if rel_key has one stage and rel_query two: 132 us against 135 at
+  // 32 x 12 heads x 512, but 104 against 95 at 64 x 16 x 256, where items are short and begin with four loads of rel_key.
+  static constexpr int kStgs = D == 32 ? 2 : 1;
+  static constexpr int kXcCols = 64, kXcs = D > 64 ? 1 : 2;   // C2P accumulators
   static constexpr int kColXc = D > 64 ? 320 : 256;
   static constexpr int offQ = 0;
   static constexpr int offK = offQ + kTile;
   static constexpr int offV = offK + kKStages * kTile;
-  static constexpr int offRK = offV + kVStages * kPiece;
-  static constexpr int offRQ = offRK + kRkStages * kPiece;
-  static constexpr int offRows = offRQ + kRqStages * kPiece;
+  static constexpr int offRK = offV + kVStages * kVPiece;
+  static constexpr int offRQ = offRK + kRkStages * kTab;
+  static constexpr int offRows = offRQ + kRqStages * kTab;
   static constexpr int offStg = offRows + BM * ROW_PITCH;
-  static constexpr int offEye = offStg + STG_BYTES;
+  static constexpr int offEye = offStg + kStgs * STG_BYTES;
   static constexpr int offBar = offEye + EYE_BYTES;
   static constexpr int kBarBytes = 512;
   // exchange area: [2 parities][2 halves][BM] row maxima (row sums at the end of an item, partial sums of the mean-of-V
@@ -129,7 +142,7 @@ struct RLayout {
   static constexpr int offMeanV = offXmax + (D > 64 ? 8 * D * 4 : 2 * 2 * BM * 4);
   static constexpr int offItem = offMeanV + 256;
   static constexpr int kItemBytes = 304;
-  static constexpr int total = offItem + kItemSlots * kItemBytes + 1024;   // + alignment slack
+  static constexpr int total = offItem + kItemSlots * kItemBytes;
   static_assert(offStg % 16 == 0 && offBar % 16 == 0 && offItem % 16 == 0, "alignment");
   static_assert(total <= 232448, "shared memory budget");
 };
@@ -148,11 +161,11 @@ static_assert(sizeof(ItemSlot) <= 304, "item slot too large");
 struct RBarriers {
   uint64_t q_full, q_empty;
   uint64_t k_full[2], k_empty[2], v_full[2], v_empty[2];
-  uint64_t rk_full[2], rk_empty[2], rq_full[2], rq_empty[2];
+  uint64_t rk_full[4], rk_empty[4], rq_full[4], rq_empty[4];
   uint64_t s_full, s_free;          // S accumulator: MMA -> softmax, softmax (8 warps) -> MMA
-  uint64_t xc_full, xc_free;        // C2P block accumulator: MMA -> converters (4 warps) -> MMA
+  uint64_t xc_full[2], xc_free[2];  // halves of a C2P block: MMA -> converters (4 warps each) -> MMA
   uint64_t xp_full[2], xp_free[2];  // P2C part accumulators: MMA -> converters (4 warps) -> MMA
-  uint64_t pt_ready, pt_release;    // P2C tile in shared memory: converters -> MMA (its reads complete) -> converters
+  uint64_t pt_ready[2], pt_release[2];   // P2C tiles in shared memory: converters -> MMA (its reads complete) -> converters
   uint64_t p_full, o_ready, o_free; // P stored (8 warps); PV complete; output accumulator read out (8 warps)
   uint64_t c2p_ready, ring_release; // C2P rows of a tile: converters -> softmax -> converters
   uint64_t pair2[4];                // the two warps of a lane quarter: row maximum (row sum) posted
@@ -198,6 +211,9 @@ __device__ __forceinline__ void sts_u32(uint32_t saddr, uint32_t v) {
 __device__ __forceinline__ void sts_u32_if(uint32_t saddr, uint32_t v, bool on) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.shared.u32 [%0], %1;\n\t}" ::"r"(saddr), "r"(v), "r"((int)on) : "memory");
 }
+__device__ __forceinline__ void sts_u16_if(uint32_t saddr, uint32_t v, bool on) {
+  asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.shared.u16 [%0], %1;\n\t}" ::"r"(saddr), "h"((unsigned short)v), "r"((int)on) : "memory");
+}
 // Two scores rounded to T and packed.  FP16 saturates: a score beyond 65504 would be an infinity, and the MMA that adds
 // the P2C tile to S multiplies the other rows' entries of that key by zero.
 template <typename T>
@@ -242,21 +258,21 @@ __device__ __forceinline__ void add_pair<__nv_bfloat16>(float& s0, float& s1, ui
 }
 
 // Kept-key bits of batch row b, one word of 32 keys per lane: lane l gets words l (lo) and l + 32 (hi).  Warp-collective:
-// the mask is read 32 elements at a time, four words in flight.
+// the mask is read 32 elements at a time, sixteen words in flight.
 __device__ __forceinline__ void kept_bits(const DflAttnRelParams& p, int b, int lane, uint32_t& lo, uint32_t& hi) {
   const int L = p.seq_len, n_words = (L + 31) / 32;
   const long long base = (long long)b * L;
   lo = hi = 0;
 #pragma unroll 1
-  for (int w0 = 0; w0 < n_words; w0 += 4) {
-    bool keep[4];
+  for (int w0 = 0; w0 < n_words; w0 += 16) {
+    bool keep[16];
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
+    for (int x = 0; x < 16; ++x) {
       const int j = 32 * (w0 + x) + lane;
       keep[x] = j < L && mask_keep(p.mask, p.mask_elem_size, base + j);
     }
 #pragma unroll
-    for (int x = 0; x < 4; ++x) {
+    for (int x = 0; x < 16; ++x) {
       const uint32_t bits = __ballot_sync(0xffffffffu, keep[x]);
       if (lane == ((w0 + x) & 31)) {
         if (w0 + x < 32) lo = bits;
@@ -302,7 +318,7 @@ __device__ __forceinline__ TileRange tile_range(uint32_t kb_lo, uint32_t kb_hi, 
 template <int D>
 __device__ __forceinline__ void mma_over_d(uint32_t d_tmem, uint64_t a_desc, uint32_t a_sub, uint64_t b_desc, uint32_t b_sub,
                                            uint32_t idesc) {
-#pragma unroll 1
+#pragma unroll
   for (int kk = 0; kk < D / 16; ++kk) {
     ptx::umma_ss_f16_warp(d_tmem, a_desc, b_desc, idesc, kk != 0 ? 1u : 0u);
     a_desc += D > 64 && kk == 3 ? a_sub - 6u : 2u;
@@ -317,8 +333,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
                      const __grid_constant__ CUtensorMap tmap_fq, const DflAttnRelParams p, int* status_word,
                      int n_items) {
   using LO = RLayout<D>;
-  extern __shared__ unsigned char smem_dyn[];
-  unsigned char* smem = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_dyn) + 1023) & ~uintptr_t(1023));
+  extern __shared__ __align__(1024) unsigned char smem[];   // the swizzled tiles need the alignment
   RBarriers* bars = reinterpret_cast<RBarriers*>(smem + LO::offBar);
   ItemSlot* slots = reinterpret_cast<ItemSlot*>(smem + LO::offItem);
 
@@ -330,12 +345,14 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   // ------------------------------------------------------------------ setup (once per CTA)
   if (threadIdx.x == 0) {
     ptx::mbar_init(&bars->q_full, 1);
-    ptx::mbar_init(&bars->q_empty, 1);
+    ptx::mbar_init(&bars->q_empty, has_c2p ? 2 : 1);          // its issuers: Q K^T, and C2P blocks
     for (int s = 0; s < 2; ++s) {
       ptx::mbar_init(&bars->k_full[s], 1);
       ptx::mbar_init(&bars->k_empty[s], has_p2c ? 2 : 1);   // its issuers: Q K^T, and P2C parts
       ptx::mbar_init(&bars->v_full[s], 1);
       ptx::mbar_init(&bars->v_empty[s], 1);
+    }
+    for (int s = 0; s < 4; ++s) {
       ptx::mbar_init(&bars->rk_full[s], 1);
       ptx::mbar_init(&bars->rk_empty[s], 1);
       ptx::mbar_init(&bars->rq_full[s], 1);
@@ -347,26 +364,26 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
     ptx::mbar_init(&bars->s_full, 1);
     ptx::mbar_init(&bars->s_free, kSoftmaxWarps);   // one elected lane per softmax warp
-    ptx::mbar_init(&bars->xc_full, 1);
-    ptx::mbar_init(&bars->xc_free, 4);              // converter warps
     for (int s = 0; s < 2; ++s) {
+      ptx::mbar_init(&bars->xc_full[s], 1);
+      ptx::mbar_init(&bars->xc_free[s], 4);         // converter warps
       ptx::mbar_init(&bars->xp_full[s], 1);
       ptx::mbar_init(&bars->xp_free[s], 4);         // converter warps
+      ptx::mbar_init(&bars->pt_ready[s], 8);
+      ptx::mbar_init(&bars->pt_release[s], 1);
     }
-    ptx::mbar_init(&bars->pt_ready, 4);
-    ptx::mbar_init(&bars->pt_release, 1);
     ptx::mbar_init(&bars->p_full, kSoftmaxWarps);
     ptx::mbar_init(&bars->o_ready, 1);
     ptx::mbar_init(&bars->o_free, kSoftmaxWarps);
-    ptx::mbar_init(&bars->c2p_ready, 4);
+    ptx::mbar_init(&bars->c2p_ready, 8);
     ptx::mbar_init(&bars->ring_release, kSoftmaxWarps);
     for (int s = 0; s < 4; ++s) ptx::mbar_init(&bars->pair2[s], 2);
     ptx::mbar_init(&bars->xbar, kSoftmaxWarps);
     ptx::fence_mbar_init();
   }
-  // identity operand: zeros with ones on rows 112 .. 127
-  for (int e = threadIdx.x; e < EYE_BYTES / 16; e += kThreads) {
-    const int chunk = e / EYE_ROWS, col = e - chunk * EYE_ROWS - (EYE_ROWS - BM) - 8 * chunk;   // column of the one, if in [0, 8)
+  // identity operand: zeros with ones on rows 120 .. 127
+  for (int e = threadIdx.x; e < EYE_ROWS; e += kThreads) {
+    const int col = e - 120;   // column of the one, if in [0, 8)
     const uint32_t one = __is_same(T, __half) ? 0x3C00u : 0x3F80u;
     uint32_t w[4];
 #pragma unroll
@@ -392,7 +409,6 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
   __syncthreads();
   ptx::tc_fence_after();
   const uint32_t tmem_base = bars->tmem_base;
-
   // A bounded wait whose verdict is the same in every lane of the warp (the tcgen05.ld/st/wait instructions that
   // follow are warp-collective and must not be reached by part of a warp).
   auto wwait = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
@@ -711,134 +727,131 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     //     next one's).  Consecutive m land at consecutive columns of the row buffer, modulo its two tiles.
     //   P2C parts (lane = key n): table column w of the tile's 256 is the score of query row 128 + n - w; the row goes to
     //     row n of the K-major B operand of the MMA that adds the tile to S.
-    // Both destinations are shifted by the lane, and a 4-byte store takes two neighbouring columns: a funnel shift pairs
-    // them from the packed words at hand for odd (C2P) or even (P2C) rows.
-    const int q4 = warp & 3;
+    // Both destinations are shifted by the lane, and a 4-byte store takes two neighbouring columns: for odd (C2P) or even
+    // (P2C) rows a funnel shift pairs them from the packed words at hand, and the first and the last of 32 columns are
+    // stored by themselves.  No column needs its neighbours in another warp's hands, so each role has two warps per
+    // quarter, one for the first and one for the second accumulator of its pair: 32 columns are a chain of some 60
+    // instructions, 600 to 1100 cycles, that a warp cannot overlap with itself.
+    const int q4 = warp & 3, group = (warp >> 2) & 1;
     const int row = q4 * 32 + lane;
+    const bool odd = (row & 1) != 0;
     const uint32_t lane_base = (uint32_t)(q4 * 32) << 16;
-    const uint32_t t_xp = tmem_base + lane_base + COL_XP;
-    const uint32_t t_xc = tmem_base + lane_base + LO::kColXc;
-    // C2P: word k of a block (columns 2k, 2k+1; for odd rows 2k-1, 2k) goes to column 128 * tile + 2k + row_even
     const int row_even = row & ~1;
-    const uint32_t row_addr = ptx::smem_u32(smem + LO::offRows) + (uint32_t)(row * ROW_PITCH + 2 * row_even);
-    const uint32_t c_shift = (row & 1) ? 16u : 32u;
-    uint32_t carry = 0;         // last packed word of the previous block of this row
-    // P2C: word k holds query rows 128 + row_even - 2k and + 1
-    const uint32_t p_shift = (row & 1) ? 0u : 16u;
-    uint32_t stg_addr[4];       // where word k = 0, 1, 2, 3 (mod 4) would go
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int qr = 128 + row_even - 2 * j;
-      stg_addr[j] = ptx::smem_u32(smem + LO::offStg) + (uint32_t)((qr >> 3) * STG_CHUNK + (row >> 3) * 128 + (row & 7) * 16 + (qr & 7) * 2);
-    }
-    uint32_t c_xp = 0, c_xc = 0, c_pt = 0;
     uint32_t rel_seen = 0;      // phases of ring_release (one per key tile) waited for so far
     uint32_t tiles_before = 0;  // key tiles of all earlier items
+    uint32_t c_x = 0, c_pt = 0; // accumulators of this group converted, P2C tiles completed
     bool ok = true;
 
-    // One C2P block: upper part of running tile `upper`, lower part of tile upper + 1; the first block of an item has no
-    // upper part.  The two row buffers must be free: `need` key tiles in total must have been read.
+    // Half `group` of a C2P block: upper part of running tile `upper`, lower part of tile upper + 1; the first block of an item
+    // has no upper part.  The two row buffers must be free: `need` key tiles in total must have been read.
     auto convert_block = [&](bool first, uint32_t upper, uint32_t need) -> bool {
-      constexpr int kChunksOfXc = LO::kXcCols / 32;   // the accumulator holds a block, or half of it at a time
-      if (!wwait(&bars->xc_full, c_xc & 1u, 18)) return false;
-      ++c_xc;
+      // word k of a block (columns 2k, 2k+1; for odd rows 2k-1, 2k) goes to column 128 * tile + 2k + row_even
+      const uint32_t row_addr = ptx::smem_u32(smem + LO::offRows) + (uint32_t)(row * ROW_PITCH + 2 * row_even);
+      const uint32_t shift = odd ? 16u : 32u;
+      const uint32_t t_xc = tmem_base + lane_base + LO::kColXc + (LO::kXcs > 1 ? 64 * group : 0);
+      if (!wwait(&bars->xc_full[group], c_x & 1u, 18)) return false;
+      ++c_x;
       ptx::tc_fence_after();
-      uint32_t prev = carry;
-      uint32_t v[32];
-      ptx::tmem_ld32(t_xc, v);
       while (rel_seen < need) {
         if (!wwait(&bars->ring_release, rel_seen & 1u, 17)) return false;
         ++rel_seen;
       }
 #pragma unroll 1
-      for (int j = 0; j < 4; ++j) {   // 32 columns at a time, the next ones in flight while these are stored
-        if (LO::kPieces > 1 && j == kChunksOfXc) {
-          if (!wwait(&bars->xc_full, c_xc & 1u, 18)) return false;
-          ++c_xc;
-          ptx::tc_fence_after();
-          ptx::tmem_ld32(t_xc, v);
-        }
+      for (int j = 2 * group; j < 2 * group + 2; ++j) {   // 32 columns at a time
+        uint32_t v[32];
+        ptx::tmem_ld32(t_xc + 32 * (j & 1), v);
         ptx::tmem_wait_ld();
-        if (j % kChunksOfXc == kChunksOfXc - 1) {   // in registers: the accumulator is free for the next MMA
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&bars->xc_free);
-        }
         uint32_t w[16];
 #pragma unroll
         for (int k = 0; k < 16; ++k) w[k] = pack_scores<T>(__uint_as_float(v[2 * k]), __uint_as_float(v[2 * k + 1]));
-        if (j % kChunksOfXc != kChunksOfXc - 1) ptx::tmem_ld32(t_xc + 32 * (j % kChunksOfXc + 1), v);
-        const uint32_t top = w[15];
+        if (j & 1) {   // in registers: the accumulator is free for the next MMA
+          ptx::tc_fence_before();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->xc_free[group]);
+        }
+        const uint32_t head = w[0], tail = w[15];
 #pragma unroll
-        for (int k = 15; k > 0; --k) w[k] = funnel_clamp(w[k - 1], w[k], c_shift);
-        w[0] = funnel_clamp(prev, w[0], c_shift);
-        prev = top;
+        for (int k = 15; k > 0; --k) w[k] = funnel_clamp(w[k - 1], w[k], shift);
         // column 2k + row_even below 128: tile `upper`; from 128 on: the next tile, whose buffer is the other half
         const uint32_t up = row_addr + (upper & 1u) * 256u + 64u * j, down = row_addr + ((upper & 1u) ? 0u : 256u) - 256u + 64u * j;
-        const int turn = j + q4;   // columns of this warp and chunk: 32 * turn .. 32 * turn + 61
-        if (turn >= 4) {
-#pragma unroll
-          for (int k = 0; k < 16; ++k) sts_u32(down + 4 * k, w[k]);
-        } else if (turn == 3) {
+        const int turn = j + q4;   // columns of this warp and chunk: 32 * turn .. 32 * turn + 62
+        if (turn >= 4 || !first) {
+          const uint32_t to = turn >= 4 ? down : up;
+          sts_u32_if(to, head, !odd);
+          sts_u16_if(to + 2, head, odd);
+        }
+        if (turn >= 3 || !first) sts_u16_if((turn >= 3 ? down : up) + 64, tail >> 16, odd);
+        if (turn == 3) {
           const int last_up = 127 - 32 * j - row_even;   // 2k <= last_up: tile `upper`
 #pragma unroll
-          for (int k = 0; k < 16; ++k) {
+          for (int k = 1; k < 16; ++k) {
             const bool below = 2 * k <= last_up;
             sts_u32_if((below ? up : down) + 4 * k, w[k], !(first && below));
           }
-        } else if (!first) {
+        } else if (turn >= 4 || !first) {
+          const uint32_t to = turn >= 4 ? down : up;
 #pragma unroll
-          for (int k = 0; k < 16; ++k) sts_u32(up + 4 * k, w[k]);
+          for (int k = 1; k < 16; ++k) sts_u32(to + 4 * k, w[k]);
         }
       }
-      carry = prev;
       return true;
     };
-    // One part (64 table columns) of a tile's P2C accumulator.  A warp's 32 keys take words 16 * q4 + 1 .. 16 * q4 + 79 of
-    // the tile's 128: 32-column chunks q4 .. q4 + 4 of the eight, two chunks per part.
-    uint32_t p_prev = 0;
-    auto convert_part = [&](int part) -> bool {
-      const int buf = part & 1;
-      if (!wwait(&bars->xp_full[buf], (c_xp >> 1) & 1u, 19)) return false;
-      ++c_xp;
-      ptx::tc_fence_after();
-      const int begin = max(q4, 2 * part), end = min(q4 + 5, 2 * part + 2);
-      if (begin >= end) {   // nothing for this warp's keys: its share of xp_free
-        if (lane == 0) ptx::mbar_arrive(&bars->xp_free[buf]);
-        return true;
-      }
-      const uint32_t t_part = t_xp + 64 * buf - 64 * part;
-      uint32_t v[32];
-      ptx::tmem_ld32(t_part + 32 * begin, v);
-      if (begin == q4 && !wwait(&bars->pt_release, (c_pt & 1u) ^ 1u, 20)) return false;   // the previous tile has been read
+    // Parts `group` and `group` + 2 (64 table columns each) of a tile's P2C accumulator.  A quarter's 32 keys take words
+    // 16 * q4 + 1 .. 16 * q4 + 79 of the tile's 128: 32-column chunks q4 .. q4 + 4 of the eight, two chunks per part.
+    auto convert_parts = [&]() -> bool {
+      const uint32_t t_xp = tmem_base + lane_base + COL_XP + 64 * group;
+      const uint32_t stg = c_pt % LO::kStgs;
+      const uint32_t shift = odd ? 0u : 16u;
+      bool waited = false;
 #pragma unroll 1
-      for (int j = begin; j < end; ++j) {
-        ptx::tmem_wait_ld();
-        if (j == end - 1) {   // what this warp needs of the part is in registers
-          ptx::tc_fence_before();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&bars->xp_free[buf]);
+      for (int part = group; part < 4; part += 2) {
+        if (!wwait(&bars->xp_full[group], c_x & 1u, 19)) return false;
+        ++c_x;
+        ptx::tc_fence_after();
+        const int begin = max(q4, 2 * part), end = min(q4 + 5, 2 * part + 2);
+        if (begin >= end) {   // nothing for this warp's keys: its share of xp_free
+          if (lane == 0) ptx::mbar_arrive(&bars->xp_free[group]);
+          continue;
         }
-        uint32_t w[16];
+        if (!waited && !wwait(&bars->pt_release[stg], (c_pt / LO::kStgs & 1u) ^ 1u, 20)) return false;   // that tile has been read
+        waited = true;
+#pragma unroll 1
+        for (int j = begin; j < end; ++j) {
+          uint32_t v[32];
+          ptx::tmem_ld32(t_xp + 32 * (j & 1), v);
+          ptx::tmem_wait_ld();
+          uint32_t w[16];
 #pragma unroll
-        for (int k = 0; k < 16; ++k) w[k] = pack_scores<T>(__uint_as_float(v[2 * k + 1]), __uint_as_float(v[2 * k]));
-        if (j + 1 < end) ptx::tmem_ld32(t_part + 32 * (j + 1), v);
-        const uint32_t top = w[15];
+          for (int k = 0; k < 16; ++k) w[k] = pack_scores<T>(__uint_as_float(v[2 * k + 1]), __uint_as_float(v[2 * k]));
+          if (j == end - 1) {   // what this warp needs of the part is in registers
+            ptx::tc_fence_before();
+            __syncwarp();
+            if (lane == 0) ptx::mbar_arrive(&bars->xp_free[group]);
+          }
+          const uint32_t head = w[0], tail = w[15];
 #pragma unroll
-        for (int k = 15; k > 0; --k) w[k] = funnel_wrap(w[k], w[k - 1], p_shift);
-        w[0] = funnel_wrap(w[0], p_prev, p_shift);
-        p_prev = top;
-        const uint32_t down = (uint32_t)(j * 4 * STG_CHUNK);     // words 16 * j + k; 32 columns are four chunks of eight query rows
-        const int turn = j - q4;
-        if (turn >= 1 && turn <= 3) {
+          for (int k = 15; k > 0; --k) w[k] = funnel_wrap(w[k], w[k - 1], shift);
+          // word k holds query rows 128 + row_even - 2 (16 j + k) and + 1; 16 query rows down are two chunks of eight
+          const int qr = 128 + row_even - 32 * j;
+          const uint32_t base = ptx::smem_u32(smem + LO::offStg) + stg * (uint32_t)STG_BYTES + (uint32_t)((row >> 3) * 128 + (row & 7) * 16);
+          uint32_t at[4];   // where words 0, 1, 2, 3 (mod 4) go
 #pragma unroll
-          for (int k = 0; k < 16; ++k) sts_u32(stg_addr[k & 3] - down - (uint32_t)((k >> 2) * STG_CHUNK), w[k]);
-        } else {
-          // words 1 + row_even / 2 .. 64 + row_even / 2 are query rows of the tile
-          const int lo = 1 + row_even / 2 - 16 * j, hi = 64 + row_even / 2 - 16 * j;
+          for (int x = 0; x < 4; ++x) at[x] = base + (uint32_t)((15 - ((qr - 2 * x) >> 3)) * STG_CHUNK + ((qr - 2 * x) & 7) * 2);
+          const int turn = j - q4;
+          if (turn > 0) {
+            sts_u32_if(at[0], head, odd);
+            sts_u16_if(at[0], head >> 16, !odd);
+          }
+          if (turn < 4) sts_u16_if(at[0] + 4 * STG_CHUNK + 2, tail, !odd);
+          if (turn >= 1 && turn <= 3) {
 #pragma unroll
-          for (int k = 0; k < 16; ++k)
-            sts_u32_if(stg_addr[k & 3] - down - (uint32_t)((k >> 2) * STG_CHUNK), w[k], k >= lo && k <= hi);
+            for (int k = 1; k < 16; ++k) sts_u32(at[k & 3] + (uint32_t)((k >> 2) * STG_CHUNK), w[k]);
+          } else {
+            // words 1 + row_even / 2 .. 64 + row_even / 2 are query rows of the tile
+            const int lo = 1 + row_even / 2 - 16 * j, hi = 64 + row_even / 2 - 16 * j;
+#pragma unroll
+            for (int k = 1; k < 16; ++k) sts_u32_if(at[k & 3] + (uint32_t)((k >> 2) * STG_CHUNK), w[k], k >= lo && k <= hi);
+          }
         }
       }
       return true;
@@ -864,12 +877,11 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
         } else {
           for (int u = 0; u < n && ok && has_p2c; ++u) {
-#pragma unroll 1
-            for (int part = 0; part < 4 && ok; ++part) ok = convert_part(part);
+            ok = convert_parts();
             if (!ok) break;
             ptx::fence_proxy_async_smem();   // the tile is read by the tensor core
             __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&bars->pt_ready);
+            if (lane == 0) ptx::mbar_arrive(&bars->pt_ready[c_pt % LO::kStgs]);
             ++c_pt;
           }
         }
@@ -881,18 +893,30 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     }
   } else {
     setmaxnreg_dec<kMiscRegs>();
+    // Q, K, rel_query and the mask analysis have a warp of their own, rel_key and V are loaded by the issuer of their MMAs.  (One
+    // warp for all of them was what the tensor core waited for: 157 us with a lane per stream at 32 x 12 heads x 512 x 64, where
+    // this takes 135.)  `count` loads so far: stage = count % stages, phase = (count / stages) & 1.
+    auto issue_load = [&](const CUtensorMap* map, int offset, int bytes, uint64_t* full, uint32_t stage, int row, int z) {
+      const uint32_t bar = ptx::smem_u32(&full[stage]), to = ptx::smem_u32(smem) + offset + stage * bytes;
+      ptx::mbar_arrive_expect_tx_warp(bar, (uint32_t)bytes);
+#pragma unroll
+      for (int c = 0; c < LO::kSub; ++c) ptx::tma_load_3d_warp(to + c * (bytes / LO::kSub), map, bar, 64 * c, row, z);
+    };
+    auto load = [&](const CUtensorMap* map, int offset, int bytes, uint64_t* full, uint64_t* empty, uint32_t& count, uint32_t stages,
+                    int row, int z, int code) -> bool {
+      const uint32_t st = count % stages, ph = (count / stages) & 1u;
+      ++count;
+      if (!wwait(&empty[st], ph ^ 1u, code)) return false;
+      issue_load(map, offset, bytes, full, st, row, z);
+      return true;
+    };
     if (warp == kTmaWarp) {
-      // ------------------------------------------------- mask analysis + TMA producer
-      // One stream of loads in the order the MMAs consume them, each waiting for its stage; V runs one key tile behind, so
-      // that what the next scores need never waits for a PV.  Running counts: stage = count % stages, phase =
-      // (count / stages) & 1.
+      // ------------------------------------------------- mask analysis, Q and K
+      uint32_t c_q = 0, c_k = 0, c_rq = 0;
+      bool ok = true;
       struct Item {
         int t_begin, n, i0, bh, h;
-        bool any_kept;
       };
-      uint32_t c_q = 0, c_k = 0, c_v = 0, c_rk = 0, c_rq = 0;
-      bool ok = true;
-
       // Mask analysis of item number k2 (item it2), published through its slot.  Warp-collective.
       auto analyze = [&](int k2, int it2, Item& f) -> bool {
         const int slot = k2 % kItemSlots;
@@ -917,118 +941,48 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive(&bars->item_full[slot]);
-        f = {range.t_begin, range.t_end - range.t_begin, i0, bh, bh - b * H, range.any_kept};
+        f = {range.t_begin, range.any_kept ? range.t_end - range.t_begin : 0, i0, bh, bh - b * H};
         return true;
       };
-      // one tile or piece of `bytes` bytes into stage count % stages of the buffers at `offset`
-      auto load = [&](const CUtensorMap* map, int offset, int bytes, uint64_t* full, uint64_t* empty, uint32_t& count, uint32_t stages,
-                      int row, int z, int code) {
-        const uint32_t st = stages == 1 ? 0u : count & 1u, ph = (stages == 1 ? count : count >> 1) & 1u;
-        ++count;
-        ok = ok && wwait(&empty[st], ph ^ 1u, code);
-        if (ok && lane == 0) {
-          ptx::mbar_arrive_expect_tx(&full[st], (uint32_t)bytes);
-#pragma unroll
-          for (int c = 0; c < LO::kSub; ++c)
-            ptx::tma_load_3d(smem + offset + st * bytes + c * (bytes / LO::kSub), map, &full[st], 64 * c, row, z);
-        }
-        __syncwarp();
-      };
-
       Item cur{}, nxt{};
-      int k = 0, v_row = -1, v_bh = 0;   // the tile whose V is still to be loaded, if v_row >= 0
+      int k = 0;
       if ((int)blockIdx.x < n_items) ok = analyze(0, blockIdx.x, cur);
 #pragma unroll 1
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
-        const bool has_next = n_items - it > (int)gridDim.x;
-        // table row of column 0 of block 0: pair (row r, key x) of tile u uses column 128 - r + x of blocks u, u + 1
+        // K and the rel_query pieces of a tile first: its P2C parts are computed ahead of S, those of the first tile while Q waits
+        // for the item before.  The next item is analysed once Q is on its way; the slot it takes is that of the item before
+        // the one that is being computed.
         const int row0 = cur.t_begin * BK - cur.i0 - BM + (L - 1);
-        const int steps = cur.any_kept ? cur.n : 0;
-        // step -1 brings Q and the first table blocks, step u the table blocks u + 1; K runs one step ahead (its P2C parts
-        // are multiplied while the tile before is still with the converters), V one behind.  With pieces, in the order in
-        // which a single stage of each is consumed: step u brings the four rel_query pieces of tile u around the two of
-        // rel_key block u + 1, then K of tile u + 1; V is loaded by the warp that issues the PV MMAs.
 #pragma unroll 1
-        for (int u = -1; u < steps && ok; ++u) {
-          if (steps > 0) {
-            if (LO::kPieces == 1 && has_p2c)
-              load(&tmap_fq, LO::offRQ, LO::kPiece, bars->rq_full, bars->rq_empty, c_rq, LO::kRqStages, row0 + (u + 1) * BK, cur.h, 12);
-            if (LO::kPieces > 1) {
-              if (u < 0) load(&tmap_q, LO::offQ, LO::kTile, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
+        for (int u = 0; u < cur.n && ok; ++u) {
+          ok = load(&tmap_k, LO::offK, LO::kTile, bars->k_full, bars->k_empty, c_k, LO::kKStages, (cur.t_begin + u) * BK, cur.bh, 1);
 #pragma unroll 1
-              for (int x = 0; x < 6; ++x) {   // rel_query, rel_query, rel_key, rel_key, rel_query, rel_query
-                const int row = row0 + (u + (x >= 2 ? 1 : 0)) * BK + (x & 1) * LO::kPieceRows;
-                if ((x >> 1) == 1) {
-                  if (has_c2p) load(&tmap_fk, LO::offRK, LO::kPiece, bars->rk_full, bars->rk_empty, c_rk, LO::kRkStages, row, cur.h, 11);
-                } else if (u >= 0 && has_p2c) {
-                  load(&tmap_fq, LO::offRQ, LO::kPiece, bars->rq_full, bars->rq_empty, c_rq, LO::kRqStages, row, cur.h, 12);
-                }
-              }
-            }
-            if (u + 1 < steps)
-              load(&tmap_k, LO::offK, LO::kTile, bars->k_full, bars->k_empty, c_k, LO::kKStages, (cur.t_begin + u + 1) * BK, cur.bh, 1);
-            if (LO::kPieces == 1) {
-              if (u < 0) load(&tmap_q, LO::offQ, LO::kTile, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
-              if (has_c2p)
-                load(&tmap_fk, LO::offRK, LO::kPiece, bars->rk_full, bars->rk_empty, c_rk, LO::kRkStages, row0 + (u + 1) * BK, cur.h, 11);
-            }
+          for (int part = 0; part < 4 && has_p2c && ok; ++part)
+            ok = load(&tmap_fq, LO::offRQ, LO::kTab, bars->rq_full, bars->rq_empty, c_rq, LO::kRqStages, row0 + u * BK + part * 64, cur.h, 12);
+          if (u == 0) {
+            ok = ok && load(&tmap_q, LO::offQ, LO::kTile, &bars->q_full, &bars->q_empty, c_q, 1, cur.i0, cur.bh, 3);
+            if (ok && n_items - it > (int)gridDim.x) ok = analyze(k + 1, it + (int)gridDim.x, nxt);
           }
-          if (LO::kPieces == 1) {
-            if (v_row >= 0 && (u >= 0 || steps == 0)) {
-              load(&tmap_v, LO::offV, LO::kPiece, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
-              v_row = -1;
-            }
-            if (u >= 0) {
-              v_row = (cur.t_begin + u) * BK;
-              v_bh = cur.bh;
-            }
-          }
-          // The next item is analysed once the loads its predecessor starts with are on their way.  Its slot is that of
-          // the item three before it, which is complete only if its last V has been loaded: the load above, whatever
-          // kind the items in between are.
-          if (ok && has_next && (u == 0 || steps == 0)) ok = analyze(k + 1, it + (int)gridDim.x, nxt);
         }
+        if (ok && cur.n == 0 && n_items - it > (int)gridDim.x) ok = analyze(k + 1, it + (int)gridDim.x, nxt);
         cur = nxt;
       }
-      if (v_row >= 0) load(&tmap_v, LO::offV, LO::kPiece, bars->v_full, bars->v_empty, c_v, LO::kVStages, v_row, v_bh, 2);
     } else if (warp == kMmaWarp) {
       // -------------------------------------------------------------- MMA issuer
-      // C2P blocks and S.  In each issuing role the whole warp walks the items and one elected lane issues
-      // (umma_ss_f16_warp); descriptors are precomputed and only their start-address field moves.  Per key tile: C2P block
-      // of the tile after it, Q K^T as soon as the softmax threads have read the previous tile's S, and the P2C tile on
-      // top of it as soon as the converters have finished it.  The P2C parts and the PV MMAs have issuers of their own:
-      // an issue costs its warp about as long as the MMA runs, and neither waits for what this warp waits for.
+      // S = Q K^T as soon as the softmax threads have read the previous tile's S, and the P2C tile on top of it as soon as the
+      // converters have finished it.  In each issuing role the whole warp walks the items and one elected lane issues
+      // (umma_ss_f16_warp); descriptors are precomputed and only their start-address field moves.  The other MMAs have
+      // issuers of their own: an issue costs its warp about as long as the MMA runs.
       constexpr int is_bf16 = __is_same(T, __nv_bfloat16) ? 1 : 0;
       constexpr uint32_t idesc_nn = ptx::make_idesc_f16(is_bf16, BM, 128, 0, 0);   // 128 x 128, both K-major
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
-      constexpr uint32_t sbo = 8 * LO::kRowBytes;
-      constexpr uint32_t idesc_c = ptx::make_idesc_f16(is_bf16, BM, LO::kXcCols, 0, 0);
-      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4, kPieceUnits = (uint32_t)LO::kPiece >> 4;
-      const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offQ), 16, sbo, mode);
-      const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, sbo, mode);
-      const uint64_t rk_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRK), 16, sbo, mode);
-      const uint64_t eye_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offEye) + (EYE_ROWS - BM) * 16, EYE_CHUNK, 128, 0);
+      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4;
+      const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offQ), 16, 8 * LO::kRowBytes, mode);
+      const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, 8 * LO::kRowBytes, mode);
+      const uint64_t eye_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offEye) + 112 * 16, EYE_LBO, 128, 0);
       const uint64_t stg_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offStg), STG_CHUNK, 128, 0);
-      uint32_t c_q = 0, c_k = 0, c_rk = 0;            // loads consumed (stage / phase as in the loader)
-      uint32_t c_s = 0, c_xc = 0;                     // S tiles, C2P blocks issued
+      uint32_t c_q = 0, c_k = 0;   // loads consumed; c_k is also the count of S tiles
       bool ok = true;
-
-      // new C2P block = Q . rel_key block^T, piece by piece
-      auto issue_c = [&]() -> bool {
-#pragma unroll 1
-        for (int piece = 0; piece < LO::kPieces; ++piece) {
-          const uint32_t st = c_rk % LO::kRkStages, ph = (c_rk / LO::kRkStages) & 1u;
-          if (!wwait(&bars->rk_full[st], ph, 13)) return false;
-          if (!wwait(&bars->xc_free, (c_xc & 1u) ^ 1u, 14)) return false;
-          ptx::tc_fence_after();
-          mma_over_d<D>(tmem_base + LO::kColXc, q_desc, kTileUnits / LO::kSub, rk_desc + st * kPieceUnits, kPieceUnits / LO::kSub, idesc_c);
-          ptx::umma_commit_warp(&bars->rk_empty[st]);
-          ptx::umma_commit_warp(&bars->xc_full);
-          ++c_rk;
-          ++c_xc;
-        }
-        return true;
-      };
       int k = 0;
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
         const int slot = k % kItemSlots;
@@ -1041,43 +995,39 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (!any_kept) continue;
         ok = wwait(&bars->q_full, c_q & 1u, 4);
         ++c_q;
-        // step -1: C2P block 0; step u: key tile u (C2P block u + 1)
 #pragma unroll 1
-        for (int u = -1; u < n && ok; ++u) {
-          if (has_c2p) ok = issue_c();
-          if (u < 0 || !ok) continue;
-          const uint32_t kst = c_k % LO::kKStages;
-          ok = wwait(&bars->k_full[kst], (c_k / LO::kKStages) & 1u, 5) && wwait(&bars->s_free, (c_s & 1u) ^ 1u, 6);
+        for (int u = 0; u < n && ok; ++u) {
+          const uint32_t kst = c_k % LO::kKStages, stg = c_k % LO::kStgs;
+          ok = wwait(&bars->k_full[kst], (c_k / LO::kKStages) & 1u, 5) && wwait(&bars->s_free, (c_k & 1u) ^ 1u, 6);
           if (!ok) break;
           ptx::tc_fence_after();
           mma_over_d<D>(tmem_base + COL_S, q_desc, kTileUnits / LO::kSub, k_desc + kst * kTileUnits, kTileUnits / LO::kSub, idesc_nn);
           ptx::umma_commit_warp(&bars->k_empty[kst]);
           if (u + 1 == n) ptx::umma_commit_warp(&bars->q_empty);
           if (has_p2c) {
-            ok = wwait(&bars->pt_ready, c_s & 1u, 9);
+            ok = wwait(&bars->pt_ready[stg], (c_k / LO::kStgs) & 1u, 9);
             if (!ok) break;
             ptx::tc_fence_after();
-#pragma unroll 1
+            const uint64_t b_desc = stg_desc + stg * (uint32_t)(STG_BYTES >> 4);
+#pragma unroll
             for (int kk = 0; kk < BM / 16; ++kk)
-              ptx::umma_ss_f16_warp(tmem_base + COL_S, eye_desc - (uint64_t)(16 * kk), stg_desc + (uint64_t)(2 * kk * (STG_CHUNK >> 4)),
+              ptx::umma_ss_f16_warp(tmem_base + COL_S, eye_desc - (uint64_t)(16 * kk), b_desc + (uint64_t)((14 - 2 * kk) * (STG_CHUNK >> 4)),
                                     idesc_nn, 1u);
-            ptx::umma_commit_warp(&bars->pt_release);
+            ptx::umma_commit_warp(&bars->pt_release[stg]);
           }
           ptx::umma_commit_warp(&bars->s_full);
           ++c_k;
-          ++c_s;
         }
       }
     } else if (warp == kPartWarp) {
       // ------------------------------- P2C parts, as far ahead as their two accumulators allow
-      // XP[n, w] = K . rel_query^T over 64 table rows; parts 0 and 1 of a tile take them from its first table block, 2 and
-      // 3 from the second one, which is the first one of the next tile.
+      // XP[n, w] = K . rel_query^T over the 64 table rows of one piece
       constexpr uint32_t idesc_part = ptx::make_idesc_f16(__is_same(T, __nv_bfloat16) ? 1 : 0, BM, 64, 0, 0);
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
-      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4, kPieceUnits = (uint32_t)LO::kPiece >> 4;
+      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4, kTabUnits = (uint32_t)LO::kTab >> 4;
       const uint64_t k_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offK), 16, 8 * LO::kRowBytes, mode);
       const uint64_t rq_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRQ), 16, 8 * LO::kRowBytes, mode);
-      uint32_t c_k = 0, c_rq = 0, c_xp = 0;   // key tiles consumed, table blocks released, parts issued
+      uint32_t c_k = 0, c_xp = 0;   // key tiles consumed, parts issued
       bool ok = true;
       int k = 0;
       for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
@@ -1089,21 +1039,16 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
 #pragma unroll 1
         for (uint32_t x = 0; x < 4u * (uint32_t)n && ok; ++x) {   // part x & 3 of key tile x >> 2
-          const uint32_t part = x & 3u, kst = c_k % LO::kKStages, buf = c_xp & 1u, rst = c_rq % LO::kRqStages;
+          const uint32_t part = x & 3u, kst = c_k % LO::kKStages, buf = c_xp & 1u, rst = c_xp % LO::kRqStages;
           if (part == 0) ok = wwait(&bars->k_full[kst], (c_k / LO::kKStages) & 1u, 43);
-          if (ok && (LO::kPieces > 1 || x == 0 || part == 2))   // first use of a block, or a piece for this part only
-            ok = wwait(&bars->rq_full[rst], (c_rq / LO::kRqStages) & 1u, 15);
-          ok = ok && wwait(&bars->xp_free[buf], ((c_xp >> 1) & 1u) ^ 1u, 16);
+          ok = ok && wwait(&bars->rq_full[rst], (c_xp / LO::kRqStages) & 1u, 15) && wwait(&bars->xp_free[buf], ((c_xp >> 1) & 1u) ^ 1u, 16);
           if (!ok) break;
           ptx::tc_fence_after();
-          mma_over_d<D>(tmem_base + COL_XP + 64 * buf, k_desc + kst * kTileUnits, kTileUnits / LO::kSub,
-                        rq_desc + rst * kPieceUnits + (LO::kPieces > 1 ? 0u : buf * (kPieceUnits / 2)), kPieceUnits / LO::kSub, idesc_part);
+          mma_over_d<D>(tmem_base + COL_XP + 64 * buf, k_desc + kst * kTileUnits, kTileUnits / LO::kSub, rq_desc + rst * kTabUnits,
+                        kTabUnits / LO::kSub, idesc_part);
+          ptx::umma_commit_warp(&bars->rq_empty[rst]);
           ptx::umma_commit_warp(&bars->xp_full[buf]);
           ++c_xp;
-          if (LO::kPieces > 1 || part == 1 || x + 1 == 4u * (uint32_t)n) {   // last use of the block or piece
-            ptx::umma_commit_warp(&bars->rq_empty[rst]);
-            ++c_rq;
-          }
           if (part == 3) {
             ptx::umma_commit_warp(&bars->k_empty[kst]);
             ++c_k;
@@ -1111,59 +1056,116 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
       }
     } else if (warp == kPvWarp) {
-      // ----------------------------------------------------------- O (+)= P . V of every key tile, as soon as P is stored
-      constexpr uint32_t idesc_pv = ptx::make_idesc_f16(__is_same(T, __nv_bfloat16) ? 1 : 0, BM, D, 0, 1);   // V is MN-major
+      // ------------------------- C2P half blocks, and O (+)= P . V of every key tile, with the loads of both
+      // Whichever can go next goes: the C2P blocks run an item and a half ahead of the PV MMAs, on a cursor of their own.
+      constexpr int is_bf16 = __is_same(T, __nv_bfloat16) ? 1 : 0;
+      constexpr uint32_t idesc_c = ptx::make_idesc_f16(is_bf16, BM, LO::kXcCols, 0, 0);
+      constexpr uint32_t idesc_pv = ptx::make_idesc_f16(is_bf16, BM, D, 0, 1);   // V is MN-major
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(LO::kRowBytes);
+      constexpr uint32_t kTileUnits = (uint32_t)LO::kTile >> 4, kTabUnits = (uint32_t)LO::kTab >> 4;
       constexpr uint32_t kPvStepUnits = (16u * LO::kRowBytes) >> 4;   // 16 keys further down the V tile
-      const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offV), LO::kPiece / LO::kSub, 8 * LO::kRowBytes, mode);
-      uint32_t c_v = 0, c_t = 0, c_items = 0;   // pieces of V, key tiles, and items with kept rows, so far
-      bool ok = true;
-      int k = 0;
-      for (int it = blockIdx.x; it < n_items && ok; it += gridDim.x, ++k) {
-        const int slot = k % kItemSlots;
-        ok = wwait(&bars->item_full[slot], (uint32_t)(k / kItemSlots) & 1u, 39);
-        if (!ok) break;
-        const bool any_kept = slots[slot].any_kept != 0;
-        const int t_begin = slots[slot].t_begin, n = slots[slot].t_end - t_begin, bh = slots[slot].bh;
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
-        if (!any_kept) continue;
-        for (int u = 0; u < n && ok; ++u) {
+      const uint64_t q_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offQ), 16, 8 * LO::kRowBytes, mode);
+      const uint64_t rk_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRK), 16, 8 * LO::kRowBytes, mode);
+      const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offV), LO::kVPiece / LO::kSub, 8 * LO::kRowBytes, mode);
+      const int n_mine = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
+      auto complete = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, ptx::mbar_test(bar, parity)); };
+      // C2P: items taken, half blocks of the last one still to be loaded and to be issued, coordinates of the next load; counts
+      int kc = 0, halves = 0, rk_loads = 0, rk_row = 0, rk_h = 0;
+      bool have_q = false;
+      uint32_t c_q = 0, c_rk = 0, c_rk_load = 0;
+      // PV: items taken, pieces of V of the last one still to be loaded and to be multiplied, coordinates; counts
+      int kp = 0, pieces = 0, v_loads = 0, v_row = 0, v_bh = 0;
+      bool first = false;               // no piece of the item has been multiplied
+      uint32_t c_v = 0, c_v_load = 0, c_t = 0, c_items = 0;
+      uint32_t idle = 0;
 #pragma unroll 1
-          for (int piece = 0; piece < LO::kPieces && ok; ++piece) {
-            const uint32_t vst = c_v % LO::kVStages, vph = (c_v / LO::kVStages) & 1u;
-            if (LO::kPieces > 1) {   // loaded here, as soon as the piece before it has been read
-              ok = wwait(&bars->v_empty[vst], vph ^ 1u, 10);
-              if (ok && lane == 0) {
-                ptx::mbar_arrive_expect_tx(&bars->v_full[vst], (uint32_t)LO::kPiece);
-#pragma unroll
-                for (int c = 0; c < LO::kSub; ++c)
-                  ptx::tma_load_3d(smem + LO::offV + c * (LO::kPiece / LO::kSub), &tmap_v, &bars->v_full[vst], 64 * c,
-                                   (t_begin + u) * BK + piece * LO::kPieceRows, bh);
-              }
-              __syncwarp();
-            }
-            if (ok) ok = wwait(&bars->v_full[vst], vph, 8);
-            // The output accumulator of the previous item with kept rows has been read out (o_free completes one phase
-            // per such item; this warp is never more than one phase behind, so parities cannot alias).
-            if (ok && u == 0 && piece == 0 && c_items > 0) ok = wwait(&bars->o_free, (c_items - 1u) & 1u, 38);
-            if (ok && piece == 0) ok = wwait(&bars->p_full, c_t & 1u, 7);
-            if (!ok) break;
-            ptx::tc_fence_after();
-            const uint64_t vt_desc = v_desc + vst * (uint32_t)(LO::kPiece >> 4);
-            const uint32_t p_cols = tmem_base + COL_P + piece * (LO::kPieceRows / 2);
-#pragma unroll 1
-            for (int kk = 0; kk < LO::kPieceRows / 16; ++kk)
-              ptx::umma_ts_f16_warp(tmem_base + COL_O, p_cols + kk * 8, vt_desc + kk * kPvStepUnits, idesc_pv,
-                                    (u > 0 || piece > 0 || kk > 0) ? 1u : 0u);
-            ptx::umma_commit_warp(&bars->v_empty[vst]);
-            ++c_v;
+      while (kp < n_mine || halves + pieces > 0) {
+        ++idle;
+        if (halves == 0 && kc < n_mine && complete(&bars->item_full[kc % kItemSlots], (uint32_t)(kc / kItemSlots) & 1u)) {
+          const ItemSlot* sl = &slots[kc % kItemSlots];   // ours until the PV cursor has taken it too
+          ++kc;
+          if (sl->any_kept != 0 && has_c2p) {
+            halves = rk_loads = 2 * (sl->t_end - sl->t_begin) + 2;
+            // table row of column 0 of block 0: pair (row r, key x) of tile u uses column 128 - r + x of blocks u, u + 1
+            rk_row = sl->t_begin * BK - sl->i0 - BM + (L - 1);
+            rk_h = sl->h;
+            have_q = false;
           }
-          if (!ok) break;
-          ptx::umma_commit_warp(&bars->o_ready);
-          ++c_t;
+          idle = 0;
         }
-        ++c_items;
+        if (rk_loads > 0 && complete(&bars->rk_empty[c_rk_load % LO::kRkStages], ((c_rk_load / LO::kRkStages) & 1u) ^ 1u)) {
+          issue_load(&tmap_fk, LO::offRK, LO::kTab, bars->rk_full, c_rk_load % LO::kRkStages, rk_row, rk_h);
+          ++c_rk_load;
+          --rk_loads;
+          rk_row += 64;
+          idle = 0;
+        }
+        if (halves > 0) {
+          if (!have_q) {
+            have_q = complete(&bars->q_full, c_q & 1u);
+            if (have_q) ++c_q;
+          }
+          // its accumulator has been read: by the group's half before, or, with one accumulator, by the other group's
+          const uint32_t st = c_rk % LO::kRkStages;
+          if (have_q && complete(&bars->rk_full[st], (c_rk / LO::kRkStages) & 1u) &&
+              (LO::kXcs > 1 ? complete(&bars->xc_free[c_rk & 1u], ((c_rk >> 1) & 1u) ^ 1u)
+                            : c_rk == 0u || complete(&bars->xc_free[(c_rk - 1u) & 1u], ((c_rk - 1u) >> 1) & 1u))) {
+            ptx::tc_fence_after();
+            mma_over_d<D>(tmem_base + LO::kColXc + (LO::kXcs > 1 ? 64 * (c_rk & 1u) : 0u), q_desc, kTileUnits / LO::kSub,
+                          rk_desc + st * kTabUnits, kTabUnits / LO::kSub, idesc_c);
+            ptx::umma_commit_warp(&bars->rk_empty[st]);
+            ptx::umma_commit_warp(&bars->xc_full[c_rk & 1u]);
+            ++c_rk;
+            if (--halves == 0) ptx::umma_commit_warp(&bars->q_empty);
+            idle = 0;
+          }
+        }
+        if (pieces == 0 && kp < kc) {
+          const int slot = kp % kItemSlots;
+          ++kp;
+          if (slots[slot].any_kept != 0) {
+            pieces = v_loads = (slots[slot].t_end - slots[slot].t_begin) * LO::kVPieces;
+            v_row = slots[slot].t_begin * BK;
+            v_bh = slots[slot].bh;
+            first = true;
+          }
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
+          idle = 0;
+        }
+        if (v_loads > 0 && complete(&bars->v_empty[c_v_load % LO::kVStages], ((c_v_load / LO::kVStages) & 1u) ^ 1u)) {
+          issue_load(&tmap_v, LO::offV, LO::kVPiece, bars->v_full, c_v_load % LO::kVStages, v_row, v_bh);
+          ++c_v_load;
+          --v_loads;
+          v_row += LO::kVRows;
+          idle = 0;
+        }
+        // A tile's P has been stored; before an item's first, the output accumulator of the previous item with kept rows has been
+        // read out (o_free completes one phase per such item, and this warp is never more than one phase behind).
+        const uint32_t part_of_tile = c_v % LO::kVPieces, vst = c_v % LO::kVStages;
+        if (pieces > 0 && (part_of_tile != 0 || complete(&bars->p_full, c_t & 1u)) && complete(&bars->v_full[vst], (c_v / LO::kVStages) & 1u) &&
+            (!first || c_items == 0 || complete(&bars->o_free, (c_items - 1u) & 1u))) {
+          ptx::tc_fence_after();
+          const uint64_t vt_desc = v_desc + vst * (uint32_t)(LO::kVPiece >> 4);
+          const uint32_t p_cols = tmem_base + COL_P + part_of_tile * (LO::kVRows / 2);
+#pragma unroll
+          for (int kk = 0; kk < LO::kVRows / 16; ++kk)
+            ptx::umma_ts_f16_warp(tmem_base + COL_O, p_cols + kk * 8, vt_desc + kk * kPvStepUnits, idesc_pv, !first || kk > 0 ? 1u : 0u);
+          ptx::umma_commit_warp(&bars->v_empty[vst]);
+          first = false;
+          ++c_v;
+          --pieces;
+          if (part_of_tile == LO::kVPieces - 1) {
+            ptx::umma_commit_warp(&bars->o_ready);
+            ++c_t;
+          }
+          if (pieces == 0) ++c_items;
+          idle = 0;
+        }
+        if (idle > ptx::kWaitPolls * 4u) {
+          fail_code = 7;
+          break;
+        }
       }
     }
   }
@@ -1198,12 +1200,12 @@ int launch_rel_typed(const DflAttnRelParams& p, cudaStream_t stream) {
   constexpr int kCols = D / LO::kSub;
   int rc = encode_tensor_map_3d(&tq, p.q, D, L, BH, row, seq, kCols, BM, LO::kRowBytes);
   if (rc == DFL_OK) rc = encode_tensor_map_3d(&tk, p.k, D, L, BH, row, seq, kCols, BK, LO::kRowBytes);
-  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tv, p.v, D, L, BH, row, seq, kCols, LO::kPieceRows, LO::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tv, p.v, D, L, BH, row, seq, kCols, LO::kVRows, LO::kRowBytes);
   // a disabled term reuses the other table's map; it is never dereferenced
   const void* fk = p.rel_key ? p.rel_key : p.rel_query;
   const void* fq = p.rel_query ? p.rel_query : p.rel_key;
-  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfk, fk, D, R, p.heads, row, table, kCols, LO::kPieceRows, LO::kRowBytes);
-  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfq, fq, D, R, p.heads, row, table, kCols, LO::kPieceRows, LO::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfk, fk, D, R, p.heads, row, table, kCols, 64, LO::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tfq, fq, D, R, p.heads, row, table, kCols, 64, LO::kRowBytes);
   if (rc != DFL_OK) return rc;
 
   auto kernel = attention_rel_kernel<T, D>;
