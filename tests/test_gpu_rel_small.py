@@ -38,3 +38,19 @@ def test_short_packed_output(length):
                                  case["mask"].to(dev), case["scale"], packed_rows=(*tables, sum(counts)))
     for b in range(3):
         assert torch.equal(packed[bases[b]:bases[b] + counts[b]], full[b, :counts[b]]), b
+
+
+# One CTA a head with more heads than SMs, two with fewer: a second CTA without rows (16 of 32 positions) and with one (33),
+# uneven groups (six warps), and the numbers of heads at which 128 positions leave this kernel.
+@pytest.mark.parametrize("dtype_name", sorted(DTYPES))
+@pytest.mark.parametrize("batch,heads,length,d,mask,mode", (
+    (2, 3, 16, 64, "none", "both"), (2, 3, 33, 32, "right", "both"), (2, 3, 49, 64, "left", "c2p"), (3, 2, 97, 64, "heavy", "p2c"),
+    (12, 13, 17, 64, "right", "both"), (12, 13, 33, 64, "heavy", "c2p"), (12, 13, 64, 32, "left", "p2c"), (12, 13, 65, 64, "all", "both"),
+    (12, 13, 96, 64, "right", "both"), (12, 13, 96, 32, "heavy", "both"), (13, 17, 128, 32, "right", "both"),
+    (13, 18, 128, 32, "right", "both"), (12, 12, 128, 64, "heavy", "both")))
+def test_one_and_two_ctas_per_head(dtype_name, batch, heads, length, d, mask, mode):
+    dtype = DTYPES[dtype_name]
+    case = make_core_case(batch, heads, length, d, dtype, seed=100 + length, mask=mask, mode=mode)
+    got = run_rel(case)
+    assert_close(got, oracle_core(case), dtype, f"L={length} d={d} heads={batch * heads} mask={mask} mode={mode}")
+    assert torch.equal(got, run_rel(case)), "two identical launches differ"
