@@ -211,6 +211,11 @@ __device__ __forceinline__ void sts_u32(uint32_t saddr, uint32_t v) {
 __device__ __forceinline__ void sts_u32_if(uint32_t saddr, uint32_t v, bool on) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.shared.u32 [%0], %1;\n\t}" ::"r"(saddr), "r"(v), "r"((int)on) : "memory");
 }
+// ... if bit `bit` of `mask` is set
+__device__ __forceinline__ void sts_u32_bit(uint32_t saddr, uint32_t v, uint32_t mask, int bit) {
+  asm volatile("{\n\t.reg .pred p;\n\t.reg .b32 t;\n\tand.b32 t, %2, %3;\n\tsetp.ne.b32 p, t, 0;\n\t@p st.shared.u32 [%0], %1;\n\t}"
+               ::"r"(saddr), "r"(v), "r"(mask), "r"(1u << bit) : "memory");
+}
 __device__ __forceinline__ void sts_u16_if(uint32_t saddr, uint32_t v, bool on) {
   asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.b32 p, %2, 0;\n\t@p st.shared.u16 [%0], %1;\n\t}" ::"r"(saddr), "h"((unsigned short)v), "r"((int)on) : "memory");
 }
@@ -782,12 +787,10 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         }
         if (turn >= 3 || !first) sts_u16_if((turn >= 3 ? down : up) + 64, tail >> 16, odd);
         if (turn == 3) {
-          const int last_up = 127 - 32 * j - row_even;   // 2k <= last_up: tile `upper`
+          // words below 16 - lane / 2 belong to tile `upper`
+          const uint32_t below = (1u << (16 - (lane >> 1))) - 1u, stored = first ? ~below : ~0u;
 #pragma unroll
-          for (int k = 1; k < 16; ++k) {
-            const bool below = 2 * k <= last_up;
-            sts_u32_if((below ? up : down) + 4 * k, w[k], !(first && below));
-          }
+          for (int k = 1; k < 16; ++k) sts_u32_bit(((below >> k) & 1u ? up : down) + 4 * k, w[k], stored, k);
         } else if (turn >= 4 || !first) {
           const uint32_t to = turn >= 4 ? down : up;
 #pragma unroll
@@ -847,10 +850,11 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 #pragma unroll
             for (int k = 1; k < 16; ++k) sts_u32(at[k & 3] + (uint32_t)((k >> 2) * STG_CHUNK), w[k]);
           } else {
-            // words 1 + row_even / 2 .. 64 + row_even / 2 are query rows of the tile
-            const int lo = 1 + row_even / 2 - 16 * j, hi = 64 + row_even / 2 - 16 * j;
+            // of the tile's words 1 + row_even / 2 .. 64 + row_even / 2 are query rows of the tile: the first of the quarter's
+            // chunks begins below them, the last ends above, at 1 + and at lane / 2
+            const uint32_t rows = turn == 0 ? 0xfffffffeu << (lane >> 1) : (2u << (lane >> 1)) - 1u;
 #pragma unroll
-            for (int k = 1; k < 16; ++k) sts_u32_if(at[k & 3] + (uint32_t)((k >> 2) * STG_CHUNK), w[k], k >= lo && k <= hi);
+            for (int k = 1; k < 16; ++k) sts_u32_bit(at[k & 3] + (uint32_t)((k >> 2) * STG_CHUNK), w[k], rows, k);
           }
         }
       }
