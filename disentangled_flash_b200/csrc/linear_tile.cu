@@ -42,7 +42,8 @@ struct TileArgs {
   int tmem_cols;
   uint32_t ring_bytes;        // operand ring; behind it the receive buffer of a split inner product
   uint32_t recv_bytes;
-  uint32_t x_bytes;           // bytes of one X load (a tile of short sequences holds fewer than 128 rows)
+  uint32_t x_bytes;           // bytes of one X load (a tile of few rows or short sequences holds fewer than 128)
+  uint32_t x_piece;           // bytes from one 64-element piece of it to the next
 };
 
 // Where an output row starts: row-major, or head-major (the three outputs share the offset of sequence and position).
@@ -260,7 +261,7 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
         const uint64_t adesc = adesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
         const uint64_t bdesc = bdesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
         for (int p = 0; p < a.pieces; ++p) {
-          const uint64_t ad = adesc + (uint64_t)(p * (kTileA >> 4)), bd = bdesc + (uint64_t)((uint32_t)p * (uint32_t)(w_rows * BK * 2 >> 4));
+          const uint64_t ad = adesc + (uint64_t)((uint32_t)p * (a.x_piece >> 4)), bd = bdesc + (uint64_t)((uint32_t)p * (uint32_t)(w_rows * BK * 2 >> 4));
 #pragma unroll
           for (int k = 0; k < BK / 16; ++k) {
             const uint32_t acc = kb != kb_begin || p != 0 || k != 0 ? 1u : 0u;
@@ -406,14 +407,20 @@ int launch_typed(const GemmDesc& g, const TilePlan& plan, cudaStream_t stream) {
     z_tiles = 1;
   } else {
     a.tiles_m = (g.M + (PAIR ? 2 : 1) * kRows - 1) / ((PAIR ? 2 : 1) * kRows);
+    // Fewer than 128 rows are loaded as what they are, in groups of eight (a swizzle atom): rows beyond the tensor are zeros that a
+    // load takes longer for than for data.  us per launch with 128 rows and with the rows there are (W from HBM, fp16): 32 x 2304
+    // x 768 4.8 / 4.1, 32 x 3072 x 768 with GELU 7.3 / 5.0, 8 x 4608 x 1536 9.8 / 6.5, 64 x 6144 x 1536 8.3 / 8.2.  The MMA reads 128
+    // rows; what lies in the others' place, within the stage, ends in accumulator rows that nobody reads.
+    if (!CONV && !PAIR && g.M < kRows && g.batch == 1) box_rows = (g.M + 7) / 8 * 8;
   }
   // two 64-element pieces per k-block where the layout allows it: half the barrier round trips per inner product
-  a.pieces = g.K % (2 * BK) == 0 && box_rows * box_seqs == kRows ? 2 : 1;
+  a.pieces = g.K % (2 * BK) == 0 && (!CONV || box_rows * box_seqs == kRows) ? 2 : 1;
   a.kb_per_tap = (g.K + BK * a.pieces - 1) / (BK * a.pieces);
   a.num_kb = taps * a.kb_per_tap;
   a.split = plan.split < a.num_kb ? plan.split : a.num_kb;
   if (a.split > 1 && a.bn % (16 * a.split)) return fail(DFL_ERR_UNSUPPORTED, "gemm_tile: %d columns in %d parts", a.bn, a.split);
-  a.x_bytes = (uint32_t)(box_rows * box_seqs * a.pieces * BK * 2);
+  a.x_piece = (uint32_t)(box_rows * box_seqs * BK * 2);
+  a.x_bytes = (uint32_t)a.pieces * a.x_piece;
 
   CUtensorMap tmap_x, tmap_w;
   const uint64_t x_stride = g.batch > 1 ? (uint64_t)g.stride_x * es : (uint64_t)g.M * g.K * es;
