@@ -38,6 +38,7 @@ struct TileArgs {
   int num_kb, kb_per_tap;     // k-blocks (of 64 * pieces elements) of the whole inner product, and of one tap
   int pieces;                 // 64-element pieces per k-block: 1 or 2
   int tiles_m, tiles_n;
+  int rows;                   // rows per CTA, at most 128
   int seqs_per_tile;          // convolution with short sequences: sequences per tile (else 0)
   int tmem_cols;
   uint32_t ring_bytes;        // operand ring; behind it the receive buffer of a split inner product
@@ -162,9 +163,9 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     const int left = g.batch - x_z;
     out_rows = (left < a.seqs_per_tile ? left : a.seqs_per_tile) * g.M;
   } else {
-    x_row = tm * (PAIR ? 2 * kRows : kRows) + (int)half * kRows;
+    x_row = (tm * (PAIR ? 2 : 1) + (int)half) * a.rows;
     out_row = x_row;
-    out_rows = g.M - x_row < kRows ? g.M - x_row : kRows;
+    out_rows = g.M - x_row < a.rows ? g.M - x_row : a.rows;
   }
   if (out_rows < 0) out_rows = 0;          // the second CTA of a pair may lie wholly below the last row
   const int out_z = CONV && a.seqs_per_tile ? 0 : z;
@@ -407,12 +408,15 @@ int launch_typed(const GemmDesc& g, const TilePlan& plan, cudaStream_t stream) {
     z_tiles = 1;
   } else {
     a.tiles_m = (g.M + (PAIR ? 2 : 1) * kRows - 1) / ((PAIR ? 2 : 1) * kRows);
-    // Fewer than 128 rows are loaded as what they are, in groups of eight (a swizzle atom): rows beyond the tensor are zeros that a
-    // load takes longer for than for data.  us per launch with 128 rows and with the rows there are (W from HBM, fp16): 32 x 2304
-    // x 768 4.8 / 4.1, 32 x 3072 x 768 with GELU 7.3 / 5.0, 8 x 4608 x 1536 9.8 / 6.5, 64 x 6144 x 1536 8.3 / 8.2.  The MMA reads 128
-    // rows; what lies in the others' place, within the stage, ends in accumulator rows that nobody reads.
-    if (!CONV && !PAIR && g.M < kRows && g.batch == 1) box_rows = (g.M + 7) / 8 * 8;
+    // The rows are dealt out evenly, in groups of eight (a swizzle atom), instead of 128 to each tile but the last: rows beyond the
+    // tensor are zeros that a load takes longer for than for data.  us per launch with 128 rows and with the rows there are
+    // (W from HBM, fp16): 32 x 2304 x 768 4.8 / 4.1, 32 x 3072 x 768 with GELU 7.3 / 5.0, 8 x 4608 x 1536 9.8 / 6.5, 64 x 6144 x
+    // 1536 8.3 / 8.2; 130 x 1536 x 6144 11.9 / 11.1, 333 x 768 x 3072 8.4 / 8.0.  The MMA reads 128 rows; what lies in the others'
+    // place, within the stage, ends in accumulator rows that nobody reads.
+    const int ctas_m = a.tiles_m * (PAIR ? 2 : 1);
+    if (!CONV) box_rows = ((g.M + ctas_m - 1) / ctas_m + 7) / 8 * 8;
   }
+  a.rows = CONV ? kRows : box_rows;
   // two 64-element pieces per k-block where the layout allows it: half the barrier round trips per inner product
   a.pieces = g.K % (2 * BK) == 0 && (!CONV || box_rows * box_seqs == kRows) ? 2 : 1;
   a.kb_per_tap = (g.K + BK * a.pieces - 1) / (BK * a.pieces);
