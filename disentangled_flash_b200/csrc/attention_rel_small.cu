@@ -13,7 +13,7 @@
 // instructions of it.  What bounds it is the load latency, then the diagonal gathers, which two CTAs halve.  us per launch, fp16,
 // d 64, both terms, attention_rel_tc.cu / one CTA a head / two: 1 x 12 heads x 32 9.2 / 4.0 / 3.3, 4 x 12 x 64 9.4 / 5.6 / 4.4,
 // 4 x 12 x 96 9.4 / 8.1 / 5.9, 4 x 12 x 128 9.3 / 10.8 / 7.1, 8 x 12 x 128 9.6 / 11.5 / 9.4.  A forward (hidden 768, 12 layers)
-// with one and with two: 4 x 128 tokens as a graph 519 -> 479 us, 8 x 128 625 -> 604.
+// with one and with two: 4 x 128 tokens as a graph 519 -> 495 us, 8 x 128 623 -> 605.
 // Rounding is that of attention_rel_tc.cu: relative terms to T (FP16 saturating), P to T (BF16 up to 64 keys: to two of them), the row sum
 // over the rounded P.
 #include <type_traits>
