@@ -1072,7 +1072,12 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       const uint64_t rk_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offRK), 16, 8 * LO::kRowBytes, mode);
       const uint64_t v_desc = ptx::make_smem_desc(ptx::smem_u32(smem + LO::offV), LO::kVPiece / LO::kSub, 8 * LO::kRowBytes, mode);
       const int n_mine = (int)blockIdx.x < n_items ? (n_items - (int)blockIdx.x + (int)gridDim.x - 1) / (int)gridDim.x : 0;
-      auto complete = [&](uint64_t* bar, uint32_t parity) -> bool { return __all_sync(0xffffffffu, ptx::mbar_test(bar, parity)); };
+      // Bounded by a count of passes in which nothing could go (each up to seven polls, 25 to 250 ns).  One more pass then notes
+      // the barrier of the last step that could not be taken: an instantiation of its own, since what the loop carries for a
+      // report costs it up to 5 % of the kernel (d 64, two key tiles an item).
+      constexpr uint32_t kPasses = ptx::kWaitPolls * 4u;
+      uint32_t left = kPasses;
+      int missing = 0;
       // C2P: items taken, half blocks of the last one still to be loaded and to be issued, coordinates of the next load; counts
       int kc = 0, halves = 0, rk_loads = 0, rk_row = 0, rk_h = 0;
       bool have_q = false;
@@ -1081,11 +1086,14 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       int kp = 0, pieces = 0, v_loads = 0, v_row = 0, v_bh = 0;
       bool first = false;               // no piece of the item has been multiplied
       uint32_t c_v = 0, c_v_load = 0, c_t = 0, c_items = 0;
-      uint32_t idle = 0;
-#pragma unroll 1
-      while (kp < n_mine || halves + pieces > 0) {
-        ++idle;
-        if (halves == 0 && kc < n_mine && complete(&bars->item_full[kc % kItemSlots], (uint32_t)(kc / kItemSlots) & 1u)) {
+      auto pass = [&](auto report) __attribute__((always_inline)) {
+        auto complete = [&](uint64_t* bar, uint32_t parity, int code) -> bool {
+          const bool yes = __all_sync(0xffffffffu, ptx::mbar_test(bar, parity));
+          if (decltype(report)::value && !yes) missing = code;
+          return yes;
+        };
+        --left;
+        if (halves == 0 && kc < n_mine && complete(&bars->item_full[kc % kItemSlots], (uint32_t)(kc / kItemSlots) & 1u, 39)) {
           const ItemSlot* sl = &slots[kc % kItemSlots];   // ours until the PV cursor has taken it too
           ++kc;
           if (sl->any_kept != 0 && has_c2p) {
@@ -1095,25 +1103,25 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             rk_h = sl->h;
             have_q = false;
           }
-          idle = 0;
+          left = kPasses;
         }
-        if (rk_loads > 0 && complete(&bars->rk_empty[c_rk_load % LO::kRkStages], ((c_rk_load / LO::kRkStages) & 1u) ^ 1u)) {
+        if (rk_loads > 0 && complete(&bars->rk_empty[c_rk_load % LO::kRkStages], ((c_rk_load / LO::kRkStages) & 1u) ^ 1u, 2)) {
           issue_load(&tmap_fk, LO::offRK, LO::kTab, bars->rk_full, c_rk_load % LO::kRkStages, rk_row, rk_h);
           ++c_rk_load;
           --rk_loads;
           rk_row += 64;
-          idle = 0;
+          left = kPasses;
         }
         if (halves > 0) {
           if (!have_q) {
-            have_q = complete(&bars->q_full, c_q & 1u);
+            have_q = complete(&bars->q_full, c_q & 1u, 10);
             if (have_q) ++c_q;
           }
           // its accumulator has been read: by the group's half before, or, with one accumulator, by the other group's
           const uint32_t st = c_rk % LO::kRkStages;
-          if (have_q && complete(&bars->rk_full[st], (c_rk / LO::kRkStages) & 1u) &&
-              (LO::kXcs > 1 ? complete(&bars->xc_free[c_rk & 1u], ((c_rk >> 1) & 1u) ^ 1u)
-                            : c_rk == 0u || complete(&bars->xc_free[(c_rk - 1u) & 1u], ((c_rk - 1u) >> 1) & 1u))) {
+          if (have_q && complete(&bars->rk_full[st], (c_rk / LO::kRkStages) & 1u, 13) &&
+              (LO::kXcs > 1 ? complete(&bars->xc_free[c_rk & 1u], ((c_rk >> 1) & 1u) ^ 1u, 14)
+                            : c_rk == 0u || complete(&bars->xc_free[(c_rk - 1u) & 1u], ((c_rk - 1u) >> 1) & 1u, 14))) {
             ptx::tc_fence_after();
             mma_over_d<D>(tmem_base + LO::kColXc + (LO::kXcs > 1 ? 64 * (c_rk & 1u) : 0u), q_desc, kTileUnits / LO::kSub,
                           rk_desc + st * kTabUnits, kTabUnits / LO::kSub, idesc_c);
@@ -1121,7 +1129,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             ptx::umma_commit_warp(&bars->xc_full[c_rk & 1u]);
             ++c_rk;
             if (--halves == 0) ptx::umma_commit_warp(&bars->q_empty);
-            idle = 0;
+            left = kPasses;
           }
         }
         if (pieces == 0 && kp < kc) {
@@ -1135,20 +1143,20 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
           }
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&bars->item_empty[slot]);
-          idle = 0;
+          left = kPasses;
         }
-        if (v_loads > 0 && complete(&bars->v_empty[c_v_load % LO::kVStages], ((c_v_load / LO::kVStages) & 1u) ^ 1u)) {
+        if (v_loads > 0 && complete(&bars->v_empty[c_v_load % LO::kVStages], ((c_v_load / LO::kVStages) & 1u) ^ 1u, 11)) {
           issue_load(&tmap_v, LO::offV, LO::kVPiece, bars->v_full, c_v_load % LO::kVStages, v_row, v_bh);
           ++c_v_load;
           --v_loads;
           v_row += LO::kVRows;
-          idle = 0;
+          left = kPasses;
         }
         // A tile's P has been stored; before an item's first, the output accumulator of the previous item with kept rows has been
         // read out (o_free completes one phase per such item, and this warp is never more than one phase behind).
         const uint32_t part_of_tile = c_v % LO::kVPieces, vst = c_v % LO::kVStages;
-        if (pieces > 0 && (part_of_tile != 0 || complete(&bars->p_full, c_t & 1u)) && complete(&bars->v_full[vst], (c_v / LO::kVStages) & 1u) &&
-            (!first || c_items == 0 || complete(&bars->o_free, (c_items - 1u) & 1u))) {
+        if (pieces > 0 && (part_of_tile != 0 || complete(&bars->p_full, c_t & 1u, 7)) && complete(&bars->v_full[vst], (c_v / LO::kVStages) & 1u, 8) &&
+            (!first || c_items == 0 || complete(&bars->o_free, (c_items - 1u) & 1u, 38))) {
           ptx::tc_fence_after();
           const uint64_t vt_desc = v_desc + vst * (uint32_t)(LO::kVPiece >> 4);
           const uint32_t p_cols = tmem_base + COL_P + part_of_tile * (LO::kVRows / 2);
@@ -1164,12 +1172,14 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
             ++c_t;
           }
           if (pieces == 0) ++c_items;
-          idle = 0;
+          left = kPasses;
         }
-        if (idle > ptx::kWaitPolls * 4u) {
-          fail_code = 7;
-          break;
-        }
+      };
+#pragma unroll 1
+      while ((kp < n_mine || halves + pieces > 0) && left != 0u) pass(std::false_type{});
+      if (left == 0u) {
+        pass(std::true_type{});
+        fail_code = missing != 0 ? missing : 44;   // 44: it has completed since
       }
     }
   }

@@ -2,10 +2,10 @@
 // mbarrier, TMA (cp.async.bulk.tensor), tcgen05 MMA / TMEM alloc / ld / st,
 // and UMMA shared-memory / instruction descriptors.
 //
-// Every wait is bounded: a wait that does not complete within kWaitLimitNs sets
-// an abort flag in shared memory (so that all other waits of the CTA return at
-// once), records a code in a global status word, and returns false.  Kernels
-// then fall through to their teardown (TMEM is always freed).
+// Every wait is bounded.  mbar_wait: a wait that does not complete within kWaitLimitNs sets an abort flag in shared
+// memory (so that all other waits of the CTA return at once), records a code in a global status word, and returns
+// false.  mbar_wait_warp (kernels that cannot call): a count of polls, and a code in a register.  Kernels then fall
+// through to their teardown (TMEM is always freed).
 #pragma once
 
 #include <cuda.h>

@@ -56,9 +56,10 @@ DFL_API const char* dfl_status_string(int status);
 DFL_API const char* dfl_last_error(void);
 
 /*
- * Device status word.  The tcgen05 kernels wait on hardware barriers with a time limit (two seconds); a wait
- * that runs out makes its CTA skip the rest of its work, free its tensor memory and return, after writing a
- * non-zero code (which wait gave up) to the `status` word of the call - a device int32 owned by the caller and
+ * Device status word.  The tcgen05 kernels wait on hardware barriers with a limit: two seconds, or, in the
+ * relative-table attention kernel, a count of polls that lasts between a few hundredths of a second and two seconds.
+ * A wait that runs out makes its CTA skip the rest of its work, free its tensor memory and return, after writing a
+ * non-zero code (which barrier did not complete) to the `status` word of the call - a device int32 owned by the caller and
  * zeroed by it before first use; calls given no status word use a word inside the library.  Nothing on the hot
  * path reads the word.  dfl_check_status() is the read-out: it waits for `stream`, copies the word to the host,
  * and if it is non-zero clears it and returns DFL_ERR_DEVICE_TIMEOUT (dfl_last_error() names the code; the
