@@ -243,7 +243,11 @@ DFL_API size_t dfl_static_scratch_bytes(void);
  * kernel kernel.py:137-429): S = QK^T + q_i.rel_key[j-i] + k_j.rel_query[j-i], the two relative terms
  * rounded to the input type as the separate score GEMMs round their output, scale, 2-D padding mask,
  * softmax, PV.  The score tensors [B,H,L,A] never exist in global memory.  A persistent kernel (one CTA
- * per SM walks (batch, head, 128-query-tile) items), or one CTA per (batch, head) for short sequences.
+ * per SM walks (batch, head, 128-query-tile) items), or one or two CTAs per (batch, head) for short sequences.
+ * Which of them depends on seq_len, head_dim and batch * heads, so the bits of a sequence depend on the size of its
+ * batch: up to 96 positions the two short forms (batch * heads up to the number of SMs, and beyond) differ in the order
+ * of their fp32 row and PV sums alone; from 97 to 128 the persistent kernel, whose reference maximum is another, takes
+ * the larger batches.  The same call twice gives the same bits.
  * Covered: FP16/BF16, head_dim 32 or 64, or 128 beyond 96 positions, at least one relative term,
  * seq_len <= 2048; dfl_attention_rel_supported() tells, other configurations return
  * DFL_ERR_UNSUPPORTED (use dfl_pos_scores + dfl_attention_fwd for them).

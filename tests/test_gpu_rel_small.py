@@ -54,3 +54,24 @@ def test_one_and_two_ctas_per_head(dtype_name, batch, heads, length, d, mask, mo
     got = run_rel(case)
     assert_close(got, oracle_core(case), dtype, f"L={length} d={d} heads={batch * heads} mask={mask} mode={mode}")
     assert torch.equal(got, run_rel(case)), "two identical launches differ"
+
+
+# As many heads as SMs or fewer: two CTAs and two warps a row; one batch row more: one.  Scores, maxima and rounded probabilities are
+# the same bits; row sums and P.V are added in fp32 in another order, 2 L roundings of 2^-24 each, before the output is rounded.
+@pytest.mark.parametrize("dtype_name", sorted(DTYPES))
+@pytest.mark.parametrize("length,d", ((24, 64), (33, 32), (64, 64), (64, 32), (96, 64), (96, 32)))
+def test_one_cta_a_head_is_as_exact_as_two(dtype_name, length, d):
+    dtype = DTYPES[dtype_name]
+    heads = 12
+    few = torch.cuda.get_device_properties(0).multi_processor_count // heads
+    case = make_core_case(few + 1, heads, length, d, dtype, seed=300 + length, mask="heavy")
+    one = run_rel(case)[:few].double().cpu()
+    case.update({name: case[name][:few].contiguous() for name in ("q", "k", "v", "mask")})
+    two = run_rel(case).double().cpu()
+    want = oracle_core(case, compute=torch.float64)
+    step = 2.0 ** -10 if dtype == torch.float16 else 2.0 ** -7   # of the output type
+    bound = step * torch.maximum(one.abs(), two.abs()) + 2 * length * 2.0 ** -24 * case["v"].abs().max().double()
+    assert ((one - two).abs() <= bound).all(), ((one - two).abs() - bound).max().item()
+    # output steps that fall the other way, at random: a few of 10^5 and more elements
+    errors = [(got - want).norm().item() for got in (one, two)]
+    assert max(errors) <= 1.01 * min(errors), errors
