@@ -451,9 +451,10 @@ int launch_pair(const GemmDesc& g, int bn, cudaStream_t stream) {
 // ------------------------------------------------------------------------------------------------ choice of kernel
 // Cost of one GEMM in SM cycles, from the quantities that bound it: the MMA rate of the tile width, the rate at which
 // an SM takes operands from L2, waves over the SMs, the accumulator drain, and the exchange of a split inner product.
-// The constants were fitted to measured launches, weights streaming from HBM.  Against every plan at 172 sizes (32 to 16384
-// rows, N and K of hidden 768, 1024 and 1536) the choice it makes is 1.7 % above the best one on average, within 5 % at 158 of
-// them, and 41 % at worst (32 x 3072 x 1024: 8.4 against 6.0 us).
+// The constants were fitted to measured launches that loaded 128 rows of X for every tile, weights streaming from HBM, and an X
+// load is still charged as 128 rows where a tile has fewer.  Against every plan at 172 sizes (32 to 16384 rows, N and K of hidden
+// 768, 1024 and 1536), tiles loading the rows they have, the choice is 1.1 % above the best one on average (1.3 % at row counts
+// that do not fill their tiles), within 5 % at 162 of them, and 26 % at worst (1024 x 1536 x 6144: 24.6 against 19.5 us).
 constexpr double kSmIngest = 83.0;      // operand bytes per cycle and SM ...
 constexpr double kSharedIngest = 0.46;  // ... and how much slower when every SM pulls
 constexpr double kDrain64 = 1460.0;     // draining 64 accumulator columns of a tile that nothing overlaps
