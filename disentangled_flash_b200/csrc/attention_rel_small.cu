@@ -365,6 +365,8 @@ int device_sm_count() {
 // Two CTAs a head while that does not take more CTAs than the SMs hold two of; with more heads the second CTA would only repeat
 // the loads and the P2C windows.  us per launch, two / one, d 64: 48 items of 64 positions 4.4 / 5.6, 192 6.8 / 6.5, 384
 // 10.5 / 7.6; 144 items of 96 positions 7.1 / 8.6, 192 12.4 / 9.9; 48 items of 128 positions 7.1 / 10.8, 144 9.5 / 11.3.
+// The line is drawn for d 64.  At d 32 and 65 to 96 positions two CTAs are behind at 192 heads (96 positions: 8.4 / 8.1) and 4 to 17 %
+// ahead again from 384 on (12.4 / 14.3, 768 20.8 / 21.6), where one is chosen all the same.
 // Beyond 96 positions one CTA a head is never the choice (see attention_rel_small_covers).
 template <typename T, int D>
 int launch_parts(const DflAttnRelParams& p, bool tables_early, cudaStream_t stream) {
