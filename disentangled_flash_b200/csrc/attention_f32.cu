@@ -224,9 +224,11 @@ attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     };
     for (int t = 0; t < n_kt && ok; ++t) {
       const int j0 = t * BN + hf * HK;
-      // The position scores do not depend on S: the first of the tile's are on their way while it is waited for.  (8 x 12 heads
-      // x 128 x d 64 25.4 -> 24.1 us, 8 x 24 x 256 132 -> 126.  All of a tile's at once do not fit the registers; rows of
-      // C2P copied to shared memory first, 29.4 and 147.)
+      // The position scores do not depend on S: the first of the tile's are on their way while it is waited for.  us per launch
+      // without / with: d 32 8 x 24 heads x 128 35.6 / 35.5, 16 x 24 x 256 178 / 173, 8 x 24 x 512 305 / 295 (its 112 bytes of
+      // spills cost less than it gives); d 64 8 x 12 x 128 23.7 / 22.9, 8 x 24 x 256 113 / 108, 8 x 12 x 512 184 / 172 (96
+      // bytes, 40 without); d 128 8 x 8 x 128 43.5 / 37.8, 16 x 8 x 256 171 / 143, 8 x 8 x 512 254 / 211; one term alone 2 to 17 %
+      // faster.  All of a tile's at once do not fit the registers; rows of C2P copied to shared memory first, 25 -> 29 us.
       float a[16], d[16];
       gather(j0, a, d);
       ok = wait(&bars->s_full, (uint32_t)t & 1u, kWaits + 57);
