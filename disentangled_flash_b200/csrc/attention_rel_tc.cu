@@ -36,6 +36,9 @@
 // one loader in MMA order, C2P behind S in one issuer) and now:
 //   32 x 12 heads x 512 x d 64 fp16 155 -> 135     64 x 16 x 256 x 64 bf16 109 -> 95     7 x 12 x 333 x 64 bf16 29.1 -> 26.2
 //   16 x 24 x 256 x d 32 fp16 46.9 -> 38.6         16 x 8 x 512 x d 128 bf16 104 -> 78
+// The same sizes in that order with lengths uniform in [L/2, L], and without padding C2P alone and P2C alone (kernel times):
+//   140 -> 121, 114 -> 99, 28.6 -> 25.6, 46.8 -> 41.0, 103 -> 77;   114 -> 94, 84 -> 79, 22.4 -> 20.8, 34.6 -> 32.0, 76 -> 56.6;
+//   134 -> 113, 93 -> 79, 25.7 -> 22.5, 40.0 -> 32.3, 85 -> 71
 // The converters' register budget matters more than their number: at 48 registers with the next columns in flight while the
 // last are stored they spill, and the kernel took 238 us.  The waits, the loader and the MMA loops are rolled: with everything
 // unrolled (156 KB of code) a third of the issue slots were lost to instruction fetch.
@@ -426,7 +429,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
 
   // Every role walks the same item sequence (item number k of this CTA is item blockIdx.x + k * gridDim.x; it uses
   // item slot k % 3 in phase (k / 3) & 1) and keeps its own running counters.  Register budgets are set per
-  // warpgroup (warps 0-7: softmax; 8-15: converters; 16-19: the rest), at the head of the branch the whole warpgroup
+  // warpgroup (warps 0-7: softmax; 8-23: converters; 24-27: the rest), at the head of the branch the whole warpgroup
   // takes.
   if (warp < kSoftmaxWarps) {
     setmaxnreg_inc<kSoftmaxRegs>();
