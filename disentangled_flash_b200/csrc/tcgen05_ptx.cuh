@@ -282,8 +282,10 @@ __device__ __forceinline__ void cluster_sync_all() {
 __device__ __forceinline__ void cluster_sync_all_relaxed() {
   asm volatile("barrier.cluster.arrive.relaxed.aligned;\n\tbarrier.cluster.wait.aligned;" ::: "memory");
 }
-__device__ __forceinline__ void mbar_arrive_cluster(uint32_t cluster_addr) {
-  asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
+// Arrival on a barrier of another CTA of the cluster, without ordering this CTA's memory accesses at cluster scope (which would
+// wait for its outstanding stores): for hand-overs of tensor memory, whose accesses the tcgen05 fences around the barrier order.
+__device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
+  asm volatile("mbarrier.arrive.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
 // TMA load into this CTA's shared memory whose completion bytes are reported to a barrier given by its cluster
 // address (the pair leader's barrier).
