@@ -48,23 +48,6 @@ struct Barriers {
 };
 static_assert(sizeof(Barriers) <= 256, "barrier block too large");
 
-// Eight fp32 values into four packed words of each plane.
-__device__ __forceinline__ void split_eight(const float* p, uint32_t (&w)[kPlanes][4]) {
-#pragma unroll
-  for (int j = 0; j < 4; ++j) {
-    const float a = p[2 * j], b = p[2 * j + 1];   // probabilities: finite, no special cases
-    const __nv_bfloat162 h0 = __floats2bfloat162_rn(a, b);
-    const float2 f0 = __bfloat1622float2(h0);
-    const float ra = a - f0.x, rb = b - f0.y;
-    const __nv_bfloat162 h1 = __floats2bfloat162_rn(ra, rb);
-    const float2 f1 = __bfloat1622float2(h1);
-    const __nv_bfloat162 h2 = __floats2bfloat162_rn(ra - f1.x, rb - f1.y);
-    w[0][j] = *reinterpret_cast<const uint32_t*>(&h0);
-    w[1][j] = *reinterpret_cast<const uint32_t*>(&h1);
-    w[2][j] = *reinterpret_cast<const uint32_t*>(&h2);
-  }
-}
-
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
 attention_f32_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k,

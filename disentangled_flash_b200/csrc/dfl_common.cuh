@@ -281,6 +281,11 @@ int launch_attention_simt(const DflAttnParams& p, cudaStream_t stream);
 // FP32 over bf16 planes: p.q, p.k, p.v are [3][B,H,L,d], the scores fp32, the output fp32 or planes [3][B,L,H*d].
 bool attention_f32_planes_supported(int head_dim, int seq_len);
 int launch_attention_f32_planes(const DflAttnParams& p, int out_planes, cudaStream_t stream);
+// The same with the position scores computed in the kernel: p.c2p and p.p2c are unused, pos_key / pos_query [3][H][n_active][d] planes.
+// The tables, lut and mask were complete before the kernel ahead of this one in the stream started.
+bool attention_f32_rel_supported(int head_dim, int seq_len);
+int launch_attention_f32_rel(const DflAttnParams& p, const void* pos_key, const void* pos_query, int n_active, int out_planes,
+                             cudaStream_t stream);
 int launch_attention_tc(const DflAttnParams& p, cudaStream_t stream);
 bool attention_rel_supported(const DflAttnRelParams& p);
 // tables_early: rel_key / rel_query were complete before the kernel ahead of this one in the stream started

@@ -22,6 +22,9 @@ struct Workspace {
 
 constexpr size_t kPlaneBytes = 6;   // three bf16 planes per element
 
+// F32 whose attention kernel computes the position scores itself: nothing of them in the workspace
+bool scores_in_kernel(const DflEncoderParams& p) { return p.dtype == DFL_F32 && attention_f32_rel_supported(p.head_dim, p.seq_len); }
+
 bool two_call(const DflEncoderParams& p) { return !p.layers[0].rel_key && !p.layers[0].rel_query; }
 
 Workspace plan_workspace(const DflEncoderParams& p) {
@@ -53,7 +56,7 @@ Workspace plan_workspace(const DflEncoderParams& p) {
     }
   }
   if (p.conv_w && p.conv_w_module) w.conv_w = take((size_t)p.conv_taps * p.hidden * p.hidden * es);
-  if (two_call(p)) {
+  if (two_call(p) && !scores_in_kernel(p)) {
     const size_t ld = ((size_t)p.n_active + 7) / 8 * 8;
     for (int i = 0; i < 2; ++i) w.scores[i] = take(positions * p.heads * ld * es);
   }
@@ -189,7 +192,9 @@ struct Loop {
     } else {
       DflAttnParams a{};
       const int ld = (p.n_active + 7) / 8 * 8;
-      if ((y.pos_key || y.pos_query) && p.dtype == DFL_F32) {
+      const bool in_kernel = (y.pos_key || y.pos_query) && scores_in_kernel(p);
+      if (in_kernel) {
+      } else if ((y.pos_key || y.pos_query) && p.dtype == DFL_F32) {
         if (y.pos_key) {
           a.c2p = at(w.scores[0]);
           if (int rc2 = scores_f32(qkv[0], y.pos_key, at(w.scores[0]), ld)) return rc2;
@@ -215,7 +220,9 @@ struct Loop {
       a.batch = p.batch; a.heads = p.heads; a.seq_len = p.seq_len; a.head_dim = p.head_dim;
       a.mask_elem_size = p.mask_elem_size; a.scale = p.scale; a.dtype = p.dtype; a.algo = DFL_ALGO_AUTO;
       ++p.launches;
-      rc = p.dtype == DFL_F32 ? launch_attention_f32_planes(a, p.attention_only ? 0 : 1, stream) : dfl_attention_fwd(&a, stream);
+      const int out_planes = p.attention_only ? 0 : 1;
+      rc = in_kernel ? launch_attention_f32_rel(a, y.pos_key, y.pos_query, p.n_active, out_planes, stream)
+                     : (p.dtype == DFL_F32 ? launch_attention_f32_planes(a, out_planes, stream) : dfl_attention_fwd(&a, stream));
     }
     if (rc == DFL_OK && p.attention_events && cudaEventRecord((cudaEvent_t)p.attention_events[2 * layer + 1], stream) != cudaSuccess)
       return fail(DFL_ERR_LAUNCH, "recording a timing event");

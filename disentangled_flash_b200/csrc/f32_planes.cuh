@@ -31,4 +31,21 @@ __device__ __forceinline__ void split3x4(const float (&f)[4], uint2 (&out)[kPlan
   }
 }
 
+// Eight probabilities into four packed words of each plane.
+__device__ __forceinline__ void split_eight(const float* p, uint32_t (&w)[kPlanes][4]) {
+#pragma unroll
+  for (int j = 0; j < 4; ++j) {
+    const float a = p[2 * j], b = p[2 * j + 1];   // probabilities: finite, no special cases
+    const __nv_bfloat162 h0 = __floats2bfloat162_rn(a, b);
+    const float2 f0 = __bfloat1622float2(h0);
+    const float ra = a - f0.x, rb = b - f0.y;
+    const __nv_bfloat162 h1 = __floats2bfloat162_rn(ra, rb);
+    const float2 f1 = __bfloat1622float2(h1);
+    const __nv_bfloat162 h2 = __floats2bfloat162_rn(ra - f1.x, rb - f1.y);
+    w[0][j] = *reinterpret_cast<const uint32_t*>(&h0);
+    w[1][j] = *reinterpret_cast<const uint32_t*>(&h1);
+    w[2][j] = *reinterpret_cast<const uint32_t*>(&h2);
+  }
+}
+
 }  // namespace dfl

@@ -208,6 +208,16 @@ __device__ __forceinline__ void bulk_wait_group() {
 __device__ __forceinline__ void cp_async_16(void* smem_dst, const void* gsrc) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_u32(smem_dst)), "l"(gsrc) : "memory");
 }
+// Zeros instead of the source's bytes where `valid` is false (the address must be a readable one all the same).
+__device__ __forceinline__ void cp_async_16_or_zero(uint32_t smem_dst, const void* gsrc, bool valid) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(smem_dst), "l"(gsrc), "r"(valid ? 16u : 0u));
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+// Wait until at most N of this thread's groups are still in flight.
+template <int N>
+__device__ __forceinline__ void cp_async_wait_group() {
+  asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
 // The mbarrier receives one arrival once all cp.async issued so far by this thread have landed
 // (the arrival is pre-counted in the barrier's init count: ".noinc").
 __device__ __forceinline__ void cp_async_mbar_arrive_noinc(uint64_t* bar) {
