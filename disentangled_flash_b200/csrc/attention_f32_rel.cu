@@ -212,7 +212,9 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
     constexpr uint32_t idesc_rel = ptx::make_idesc_f16(1, BM, kPiece, 0, 0), idesc_qk = ptx::make_idesc_f16(1, BM, BN, 0, 0);
     constexpr uint32_t idesc_pv = ptx::make_idesc_f16(1, BM, D, 0, 1);
     constexpr int kSteps = D / 16, kVSteps = kPiece / 16;
-    constexpr int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};   // plane products, smallest first
+    // plane products, smallest first: (2,0) (1,1) (0,2) (1,0) (0,1) (0,0), two bits each; rolled, see the softmax
+    auto pa = [](int q) { return (0x46u >> (2 * q)) & 3u; };
+    auto pb = [](int q) { return (0x124u >> (2 * q)) & 3u; };
     const uint64_t kd = ptx::make_smem_desc(ptx::smem_u32(smem + T::offK), 16, sbo, mode);
     const uint64_t rd = ptx::make_smem_desc(ptx::smem_u32(smem + T::offRing), 16, sbo, mode);
     const uint64_t vd = ptx::make_smem_desc(ptx::smem_u32(smem + T::offRing), T::kPiecePlane, sbo, mode);
@@ -232,19 +234,19 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
           const uint32_t d_tmem = tmem_base + COL_ACC + a * kPiece;
           const uint64_t bd = rd + (uint64_t)((s * T::kStage) >> 4);
           if (term == 0) {
-#pragma unroll
+#pragma unroll 1
             for (int q = 0; q < 6; ++q)
 #pragma unroll
               for (int k = 0; k < kSteps; ++k)
-                ptx::umma_ts_f16_warp(d_tmem, tmem_base + COL_Q + (uint32_t)(pa[q] * (D / 2) + k * 8),
-                                      bd + (uint64_t)((pb[q] * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
+                ptx::umma_ts_f16_warp(d_tmem, tmem_base + COL_Q + (uint32_t)(pa(q) * (D / 2) + k * 8),
+                                      bd + (uint64_t)((pb(q) * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
           } else {
-#pragma unroll
+#pragma unroll 1
             for (int q = 0; q < 6; ++q)
 #pragma unroll
               for (int k = 0; k < kSteps; ++k)
-                ptx::umma_ss_f16_warp(d_tmem, kd + (uint64_t)((pa[q] * T::kKPlane + k * 32) >> 4),
-                                      bd + (uint64_t)((pb[q] * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
+                ptx::umma_ss_f16_warp(d_tmem, kd + (uint64_t)((pa(q) * T::kKPlane + k * 32) >> 4),
+                                      bd + (uint64_t)((pb(q) * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
           }
           ptx::umma_commit_warp(&bars->empty[s]);
           ptx::umma_commit_warp(&bars->acc_full[a]);
@@ -255,12 +257,12 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
            (t == 0 || wait(&bars->o_full, (uint32_t)(t - 1) & 1u, kCode + 79));
       if (!ok) break;
       ptx::tc_fence_after();
-#pragma unroll
+#pragma unroll 1
       for (int q = 0; q < 6; ++q)
 #pragma unroll
         for (int k = 0; k < kSteps; ++k)
-          ptx::umma_ts_f16_warp(tmem_base + COL_SP, tmem_base + COL_Q + (uint32_t)(pa[q] * (D / 2) + k * 8),
-                                kd + (uint64_t)((pb[q] * T::kKPlane + k * 32) >> 4), idesc_qk, q != 0 || k != 0 ? 1u : 0u);
+          ptx::umma_ts_f16_warp(tmem_base + COL_SP, tmem_base + COL_Q + (uint32_t)(pa(q) * (D / 2) + k * 8),
+                                kd + (uint64_t)((pb(q) * T::kKPlane + k * 32) >> 4), idesc_qk, q != 0 || k != 0 ? 1u : 0u);
       ptx::umma_commit_warp(&bars->k_empty);
       ptx::umma_commit_warp(&bars->s_full);
       const int n_v = value_pieces(t);
@@ -272,8 +274,8 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
       for (int q = 0; q < 6; ++q)
 #pragma unroll 1
         for (int v = 0; v < n_v; ++v) {
-          const uint32_t a = tmem_base + COL_SP + (uint32_t)(pa[q] * (BN / 2) + v * (kPiece / 2));
-          const uint64_t bq = vd + (uint64_t)((((pc + v) % kStages) * T::kStage + pb[q] * T::kPiecePlane) >> 4);
+          const uint32_t a = tmem_base + COL_SP + (uint32_t)(pa(q) * (BN / 2) + v * (kPiece / 2));
+          const uint64_t bq = vd + (uint64_t)((((pc + v) % kStages) * T::kStage + pb(q) * T::kPiecePlane) >> 4);
 #pragma unroll
           for (int k = 0; k < kVSteps; ++k)
             ptx::umma_ts_f16_warp(tmem_base + COL_O, a + (uint32_t)(k * 8), bq + (uint64_t)((k * 16 * T::kRowBytes) >> 4), idesc_pv,
@@ -354,7 +356,7 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
     };
     for (int t = 0; t < n_kt && ok; ++t) {
       const int p0 = first_piece(), p1 = last_piece(t);
-      if (t > 0 && (has_c2p || has_p2c)) ok = sync_compute(kCode + 83);   // every warp has read the previous tile's scores
+      if (t > 0) ok = sync_compute(kCode + 83);   // every warp has read the previous tile's scores
       if (has_c2p) {
 #pragma unroll 1
         for (int pi = p0; pi <= p1 && ok; ++pi) {
@@ -394,46 +396,38 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
           }
         }
       }
-      if (ok && (has_c2p || has_p2c)) ok = sync_compute(kCode + 85);
+      if (ok) ok = sync_compute(kCode + 85);
       ok = ok && wait(&bars->s_full, (uint32_t)t & 1u, kCode + 86);
       if (!ok) break;
       ptx::tc_fence_after();
+      // Two passes over the row, 16 keys at a time in rolled loops: scores, scaled and masked, back to the row in shared memory
+      // and their maximum; then probabilities.  (All 64 in registers and everything unrolled: a CTA's first tile spent 23 k cycles
+      // here, mostly on fetching instructions, later ones 9.4 k.)
       const int j0 = t * BN + hf * HK;
-      float s[HK];
-#pragma unroll
-      for (int c0 = 0; c0 < HK; c0 += 32) {
-        float v[32];
-        ptx::tmem_ld32_f(t_s + c0, v);
+      float4* row = reinterpret_cast<float4*>(rel + r * kPitch + hf * HK);
+      float mx = -INFINITY;
+#pragma unroll 1
+      for (int c0 = 0; c0 < HK; c0 += 16) {
+        float v[16];
+        ptx::tmem_ld16_f(t_s + c0, v);
+        const int left = L - (j0 + c0);
+        uint32_t bits = keep_s[(j0 + c0) >> 5] >> (c0 & 16);
+        if (!q_keep) bits = left >= 16 ? 0xffffu : (left > 0 ? (1u << left) - 1u : 0u);   // attends to all L keys alike
         ptx::tmem_wait_ld();
 #pragma unroll
-        for (int c = 0; c < 32; ++c) s[c0 + c] = v[c];
-      }
-      if (has_c2p || has_p2c) {
-        const float4* row = reinterpret_cast<const float4*>(rel + r * kPitch + hf * HK);
+        for (int c = 0; c < 4; ++c) {
+          const float4 x = row[c0 / 4 + c];
+          const float add[4] = {x.x, x.y, x.z, x.w};
 #pragma unroll
-        for (int c = 0; c < HK / 4; ++c) {
-          const float4 x = row[c];
-          s[4 * c] += x.x;
-          s[4 * c + 1] += x.y;
-          s[4 * c + 2] += x.z;
-          s[4 * c + 3] += x.w;
+          for (int k = 0; k < 4; ++k) {
+            const float scaled = q_keep ? (v[4 * c + k] + add[k]) * scale_log2 : 0.0f;
+            v[4 * c + k] = (bits >> (4 * c + k)) & 1u ? scaled : -INFINITY;
+            mx = fmaxf(mx, v[4 * c + k]);
+          }
+          row[c0 / 4 + c] = make_float4(v[4 * c], v[4 * c + 1], v[4 * c + 2], v[4 * c + 3]);
         }
       }
-      float mx = -INFINITY;
-#pragma unroll
-      for (int w = 0; w < HK / 32; ++w) {
-        const uint32_t bits = keep_s[(j0 >> 5) + w];
-#pragma unroll
-        for (int c = 0; c < 32; ++c) {
-          const int j = j0 + 32 * w + c;
-          float v = s[32 * w + c] * scale_log2;
-          if (!q_keep) v = j < L ? 0.0f : -INFINITY;
-          else if (!((bits >> c) & 1u)) v = -INFINITY;
-          s[32 * w + c] = v;
-          mx = fmaxf(mx, v);
-        }
-      }
-      // row maximum over both halves of the tile; both have S in registers, so that P may take its place
+      // row maximum over both halves of the tile; both have read S, so that P may take its place
       xmax[(t & 1) * 2 * BM + hf * BM + r] = mx;
       ptx::tc_fence_before();
       __syncwarp();
@@ -445,25 +439,30 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
       const float m_use = m_new == -INFINITY ? 0.0f : m_new;
       const float corr = exp2f(m_run - m_use);   // 0 while nothing has been attended to
       m_run = m_new;
-      float sum = 0.0f;
-#pragma unroll
-      for (int c = 0; c < HK; ++c) {
-        s[c] = exp2f(s[c] - m_use);
-        sum += s[c];
-      }
-      l_run = l_run * corr + sum;
       if (t > 0) add_output(corr);   // the previous tile's PV (complete before S was issued), before its scale is left behind
-#pragma unroll
+      float sum = 0.0f;
+#pragma unroll 1
       for (int c0 = 0; c0 < HK; c0 += 16) {
+        float e[16];
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          const float4 x = row[c0 / 4 + c];
+          e[4 * c] = ptx::ex2_approx(x.x - m_use);
+          e[4 * c + 1] = ptx::ex2_approx(x.y - m_use);
+          e[4 * c + 2] = ptx::ex2_approx(x.z - m_use);
+          e[4 * c + 3] = ptx::ex2_approx(x.w - m_use);
+          sum += (e[4 * c] + e[4 * c + 1]) + (e[4 * c + 2] + e[4 * c + 3]);
+        }
         uint32_t lo[kPlanes][4], hi[kPlanes][4];
-        split_eight(&s[c0], lo);
-        split_eight(&s[c0 + 8], hi);
+        split_eight(e, lo);
+        split_eight(e + 8, hi);
 #pragma unroll
         for (int q = 0; q < kPlanes; ++q) {
           const uint32_t w[8] = {lo[q][0], lo[q][1], lo[q][2], lo[q][3], hi[q][0], hi[q][1], hi[q][2], hi[q][3]};
           ptx::tmem_st8(t_p + (uint32_t)(q * (BN / 2) + c0 / 2), w);
         }
       }
+      l_run = l_run * corr + sum;
       ptx::tmem_wait_st();
       ptx::tc_fence_before();
       __syncwarp();
@@ -482,17 +481,21 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
         const float inv = 1.0f / (l_run + xsum[(1 - hf) * BM + r]);
         const long long at = ((long long)b * L + i) * ((long long)H * D) + (long long)h * D + hf * OW;
 #pragma unroll
-        for (int c = 0; c < OW; c += 4) {
+        for (int c = 0; c < OW; c += 8) {
           const float f[4] = {o[c] * inv, o[c + 1] * inv, o[c + 2] * inv, o[c + 3] * inv};
+          const float g[4] = {o[c + 4] * inv, o[c + 5] * inv, o[c + 6] * inv, o[c + 7] * inv};
           if (out_planes) {
-            uint2 w[kPlanes];
-            split3x4(f, w);
+            uint2 lo[kPlanes], hi[kPlanes];
+            split3x4(f, lo);
+            split3x4(g, hi);
             const long long plane = (long long)p.batch * L * H * D;
 #pragma unroll
             for (int q = 0; q < kPlanes; ++q)
-              *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + q * plane + at + c) = w[q];
+              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + q * plane + at + c) = make_uint4(lo[q].x, lo[q].y, hi[q].x, hi[q].y);
           } else {
-            *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at + c) = make_float4(f[0], f[1], f[2], f[3]);
+            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at + c);
+            dst[0] = make_float4(f[0], f[1], f[2], f[3]);
+            dst[1] = make_float4(g[0], g[1], g[2], g[3]);
           }
         }
       }
