@@ -1,4 +1,5 @@
-// FP32 fused disentangled attention on the tensor cores.
+// FP32 fused disentangled attention on the tensor cores, position scores from memory: head dim 128, modules without position
+// terms, and sequences whose slot table does not fit beside attention_f32_rel.cu's tiles (3409 positions on).
 //
 // Q, K and V come as three bf16 planes each whose sum is the fp32 value (linear_f32.cu: the QKV projection writes them), the
 // position scores C2P / P2C as fp32 [B,H,L,ld].  Semantics of kernel.py:137-345 in fp32 (the reference's strict mode):

@@ -15,11 +15,15 @@
 // memory (pitch 132: neither the diagonal writes nor the row reads meet in a bank), C2P first, P2C added to it.  The same warps
 // then run the softmax, two threads per query row.
 //
-// What bounds a tile at d = 64: 24 MMAs of 128 x 64 a piece, 33 cycles each with Q as the operand (it lives in tensor memory:
-// shared memory has no room for it, and a tensor-memory operand is read faster), 49 with K; 8 pieces, S and PV make 11 k
-// cycles, and 3.5 k of softmax follow the last piece.
-// One CTA per (batch, head, 128-query tile).  Warps 0-7 convert and softmax, 8-9 gather table pieces and V (8 also issues K's
-// TMA loads), 10 issues the MMAs and owns tensor memory: S (128 columns; P's three planes, 192, take its place), O 64, Q 96,
+// What bounds a tile at d = 64, 21 k cycles: its eight pieces, 1.3 (C2P) and 1.6 k (P2C) each: 24 MMAs of 128 x 64, 33 cycles each
+// with Q as the operand (it lives in tensor memory: shared memory has no room for it, and a tensor-memory operand is read
+// faster), 49 with K, and the issuer's waits; the conversion of a P2C piece, 1.2 k, and its gathering, 1.1 k, lie beside it.
+// The softmax, 4.5 k, and PV, 2.6 k, follow.  An item starts and ends with 2 k and 3 k.  A second issuer with every other piece
+// hides the waits, but then the conversions set the same pace.
+// us with the projection, three launches / this one: 8 x 12 heads x 128 x d 64 68 / 41, 8 x 24 x 256 361 / 219, 4 x 12 x 512 221 / 148,
+// 2 x 12 x 1024 316 / 239, 1 x 12 x 64 36 / 27; d 32 8 x 24 x 256 261 / 111.
+// One CTA per (batch, head, 128-query tile).  Warps 0-7 convert and softmax, 8-9 gather table pieces and V, 10 loads Q and K,
+// issues the MMAs and owns tensor memory: S (128 columns; P's three planes, 192, take its place), O 64, Q 96,
 // two accumulators of 64.
 #include "f32_planes.cuh"
 #include "tcgen05_ptx.cuh"
@@ -49,7 +53,7 @@ struct Shape {
 
 struct Barriers {
   uint64_t full[kStages], empty[kStages], acc_full[2], acc_empty[2];
-  uint64_t q_full, k_full, k_empty, s_full, p_full, o_full, pair[4], compute;
+  uint64_t q_load, q_full, k_full, s_full, p_full, o_full, pair[4], compute;
   uint32_t tmem_base;
   int abort_flag;
 };
@@ -57,7 +61,7 @@ static_assert(sizeof(Barriers) <= 256, "barrier block too large");
 
 template <int D>
 __global__ void __launch_bounds__(kThreads, 1)
-attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAttnParams p, const __nv_bfloat16* __restrict__ pos_key,
+attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_constant__ CUtensorMap tmap_k, const DflAttnParams p, const __nv_bfloat16* __restrict__ pos_key,
                          const __nv_bfloat16* __restrict__ pos_query, const int n_active, const int out_planes, int* status_word) {
   using T = Shape<D>;
   constexpr int HK = BN / 2, OW = D / 2;   // keys and output columns per softmax thread
@@ -82,9 +86,9 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
       ptx::mbar_init(&bars->acc_full[a], 1);
       ptx::mbar_init(&bars->acc_empty[a], kComputeWarps);
     }
+    ptx::mbar_init(&bars->q_load, 1);
     ptx::mbar_init(&bars->q_full, kComputeWarps);
     ptx::mbar_init(&bars->k_full, 1);
-    ptx::mbar_init(&bars->k_empty, 1);
     ptx::mbar_init(&bars->s_full, 1);
     ptx::mbar_init(&bars->p_full, kComputeWarps);
     ptx::mbar_init(&bars->o_full, 1);
@@ -97,17 +101,6 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
     ptx::tmem_alloc(&bars->tmem_base, kTmemCols);
     ptx::tmem_relinquish();
   }
-  // lut and mask, like the tables, were there before the projection that precedes this launch
-  for (int e = threadIdx.x; e < 2 * L - 1; e += kThreads) {
-    int slot = p.lut[e];   // entries outside the table (not a table of the builder) are clamped
-    slot = slot < 0 ? 0 : (slot >= n_active ? n_active - 1 : slot);
-    lut_s[e] = (uint16_t)slot;
-  }
-  for (int w = warp; w < n_kt * BN / 32; w += kThreads / 32) {
-    const int j = w * 32 + lane;
-    const uint32_t bits = __ballot_sync(0xffffffffu, j < L && mask_keep(p.mask, p.mask_elem_size, (long long)b * L + j));
-    if (lane == 0) keep_s[w] = bits;
-  }
   ptx::tc_fence_before();
   __syncthreads();
   ptx::tc_fence_after();
@@ -119,9 +112,19 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
   auto first_piece = [&] { return (BM - (L - i0 < BM ? L - i0 : BM)) / kPiece; };
   auto last_piece = [&](int t) { return (BM - 2 + (L - t * BN < BN ? L - t * BN : BN)) / kPiece; };
   auto value_pieces = [&](int t) { return L - t * BN > kPiece ? 2 : 1; };
+  // C2P pieces of tile t whose MMAs run before the PV of the tile ahead of it, while the compute warps are in its softmax: as many
+  // as there are accumulators (K, which P2C needs, is loaded later)
+  auto early_pieces = [&](int t) { return !has_c2p || t == 0 || t == n_kt ? 0 : (last_piece(t) > first_piece() ? 2 : 1); };
 
   if (warp >= kLoadWarp && warp < kLoadWarp + kLoadWarps) {
     const int tid = (warp - kLoadWarp) * 32 + lane;
+#pragma unroll 8
+    for (int e = tid; e < 2 * L - 1; e += kLoadWarps * 32) {   // like the tables, there before the projection ahead of this launch
+      int slot = p.lut[e];   // entries outside the table (not a table of the builder) are clamped
+      slot = slot < 0 ? 0 : (slot >= n_active ? n_active - 1 : slot);
+      lut_s[e] = (uint16_t)slot;
+    }
+    asm volatile("bar.sync 1, 64;" ::: "memory");   // the two gathering warps
     const uint32_t ring = ptx::smem_u32(smem + T::offRing);
     uint32_t issued = 0, signalled = 0;
     bool ok = true;
@@ -159,51 +162,29 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
       ptx::cp_async_wait_group<2>();
       if (issued > 2 && issued - 2 > signalled) signal_to(issued - 2);
     };
-    auto load_keys = [&](int t) {
-      if (warp == kLoadWarp && lane == 0) {
-        ptx::mbar_arrive_expect_tx(&bars->k_full, (uint32_t)T::kK);
-        for (int q = 0; q < kPlanes; ++q)
-          ptx::tma_load_3d(smem + T::offK + q * T::kKPlane, &tmap_k, &bars->k_full, 0, t * BN, q * BH + bh);
-      }
-      __syncwarp();
-    };
-    bool have_keys = false;   // Q, K and V are the predecessor's
-    auto need_keys = [&] {
-      if (!have_keys) {
-        wait_for_predecessor();
-        load_keys(0);
-        have_keys = true;
-      }
+    auto table_piece = [&](int t, int term, int pi) {
+      const __nv_bfloat16* table = term == 0 ? pos_key : pos_query;
+      const int e0 = i0 - t * BN + L - 1 + BM - 1 - pi * kPiece;   // lut index of the piece's first row; rows count down
+      piece(table + (long long)h * n_active * D, (long long)H * n_active * D, [&](int row, bool&) {
+        int e = e0 - row;   // distances that no pair inside the sequence has: any row will do
+        e = e < 0 ? 0 : (e > 2 * L - 2 ? 2 * L - 2 : e);
+        return (int)lut_s[e];
+      });
     };
     for (int t = 0; t < n_kt && ok; ++t) {
       const int p0 = first_piece(), p1 = last_piece(t);
       for (int term = 0; term < 2; ++term) {
-        const __nv_bfloat16* table = term == 0 ? pos_key : pos_query;
-        if (!table) continue;
-        for (int pi = p0; pi <= p1 && ok; ++pi) {
-          const int e0 = i0 - t * BN + L - 1 + BM - 1 - pi * kPiece;   // lut index of the piece's first row; rows count down
-          piece(table + (long long)h * n_active * D, (long long)H * n_active * D, [&](int row, bool&) {
-            int e = e0 - row;   // distances that no pair inside the sequence has: any row will do
-            e = e < 0 ? 0 : (e > 2 * L - 2 ? 2 * L - 2 : e);
-            return (int)lut_s[e];
-          });
-          if (!have_keys && (issued == kStages || pi == p1)) need_keys();
-        }
+        if (!(term == 0 ? has_c2p : has_p2c)) continue;
+        for (int pi = p0 + (term == 0 ? early_pieces(t) : 0); pi <= p1 && ok; ++pi) table_piece(t, term, pi);
       }
-      need_keys();
+      for (int pi = p0; pi < p0 + early_pieces(t + 1) && ok; ++pi) table_piece(t + 1, 0, pi);
+      if (t == 0) wait_for_predecessor();   // V is the predecessor's
       for (int v = 0; v < value_pieces(t) && ok; ++v) {
         const int j0 = t * BN + v * kPiece;
         piece(reinterpret_cast<const __nv_bfloat16*>(p.v) + (long long)bh * L * D, (long long)BH * L * D, [&](int row, bool& valid) {
           valid = j0 + row < L;
           return valid ? j0 + row : 0;
         });
-      }
-      if (t + 1 < n_kt && ok) {
-        if (!__all_sync(0xffffffffu, ptx::mbar_try_wait(&bars->k_empty, (uint32_t)t & 1u))) {
-          drain();
-          ok = wait(&bars->k_empty, (uint32_t)t & 1u, kCode + 72);
-        }
-        if (ok) load_keys(t + 1);
       }
     }
     drain();
@@ -212,73 +193,90 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
     constexpr uint32_t idesc_rel = ptx::make_idesc_f16(1, BM, kPiece, 0, 0), idesc_qk = ptx::make_idesc_f16(1, BM, BN, 0, 0);
     constexpr uint32_t idesc_pv = ptx::make_idesc_f16(1, BM, D, 0, 1);
     constexpr int kSteps = D / 16, kVSteps = kPiece / 16;
-    // plane products, smallest first: (2,0) (1,1) (0,2) (1,0) (0,1) (0,0), two bits each; rolled, see the softmax
-    auto pa = [](int q) { return (0x46u >> (2 * q)) & 3u; };
-    auto pb = [](int q) { return (0x124u >> (2 * q)) & 3u; };
+    constexpr int pa[6] = {2, 1, 0, 1, 0, 0}, pb[6] = {0, 1, 2, 0, 1, 0};   // plane products, smallest first
     const uint64_t kd = ptx::make_smem_desc(ptx::smem_u32(smem + T::offK), 16, sbo, mode);
     const uint64_t rd = ptx::make_smem_desc(ptx::smem_u32(smem + T::offRing), 16, sbo, mode);
     const uint64_t vd = ptx::make_smem_desc(ptx::smem_u32(smem + T::offRing), T::kPiecePlane, sbo, mode);
     uint32_t pc = 0, ac = 0;   // pieces taken from the ring, accumulators filled
-    bool ok = true;
+    auto load = [&](int off, const CUtensorMap* map, uint64_t* bar, int row) {   // 128 rows of each plane
+      if (lane == 0) {
+        ptx::mbar_arrive_expect_tx(bar, (uint32_t)T::kK);
+        for (int q = 0; q < kPlanes; ++q) ptx::tma_load_3d(smem + off + q * T::kKPlane, map, bar, 0, row, q * BH + bh);
+      }
+      __syncwarp();
+    };
+    wait_for_predecessor();
+    load(T::offRel, &tmap_q, &bars->q_load, i0);   // Q passes through the score tile's place on its way to tensor memory
+    load(T::offK, &tmap_k, &bars->k_full, 0);
+    auto mma_piece = [&](int term) -> bool {
+      const uint32_t s = pc % kStages, a = ac & 1u;
+      if (!wait(&bars->full[s], (pc / kStages) & 1u, kCode + 75) || !wait(&bars->acc_empty[a], ((ac >> 1) & 1u) ^ 1u, kCode + 76)) return false;
+      ptx::tc_fence_after();
+      const uint32_t d_tmem = tmem_base + COL_ACC + a * kPiece;
+      const uint64_t bd = rd + (uint64_t)((s * T::kStage) >> 4);
+      if (term == 0) {
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+#pragma unroll
+          for (int k = 0; k < kSteps; ++k)
+            ptx::umma_ts_f16_warp(d_tmem, tmem_base + COL_Q + (uint32_t)(pa[q] * (D / 2) + k * 8),
+                                  bd + (uint64_t)((pb[q] * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
+      } else {
+#pragma unroll
+        for (int q = 0; q < 6; ++q)
+#pragma unroll
+          for (int k = 0; k < kSteps; ++k)
+            ptx::umma_ss_f16_warp(d_tmem, kd + (uint64_t)((pa[q] * T::kKPlane + k * 32) >> 4),
+                                  bd + (uint64_t)((pb[q] * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
+      }
+      ptx::umma_commit_warp(&bars->empty[s]);
+      ptx::umma_commit_warp(&bars->acc_full[a]);
+      ++pc;
+      ++ac;
+      return true;
+    };
+    bool ok = wait(&bars->q_full, 0, kCode + 73);
     for (int t = 0; t < n_kt && ok; ++t) {
-      const int p0 = first_piece(), p1 = last_piece(t);
-      for (int term = 0; term < 2 && ok; ++term) {
-        if (!(term == 0 ? has_c2p : has_p2c)) continue;
-        ok = term == 0 ? wait(&bars->q_full, 0, kCode + 73) : wait(&bars->k_full, (uint32_t)t & 1u, kCode + 74);
+      const int n_pieces = last_piece(t) - first_piece() + 1, early = early_pieces(t), next_early = early_pieces(t + 1);
+      // C2P, P2C, S, then the next tile's first C2P pieces
+      const int c2p_end = has_c2p ? n_pieces - early : 0, p2c_end = c2p_end + (has_p2c ? n_pieces : 0);
 #pragma unroll 1
-        for (int pi = p0; pi <= p1 && ok; ++pi, ++pc, ++ac) {
-          const uint32_t s = pc % kStages, a = ac & 1u;
-          ok = wait(&bars->full[s], (pc / kStages) & 1u, kCode + 75) && wait(&bars->acc_empty[a], ((ac >> 1) & 1u) ^ 1u, kCode + 76);
-          if (!ok) break;
-          ptx::tc_fence_after();
-          const uint32_t d_tmem = tmem_base + COL_ACC + a * kPiece;
-          const uint64_t bd = rd + (uint64_t)((s * T::kStage) >> 4);
-          if (term == 0) {
-#pragma unroll 1
-            for (int q = 0; q < 6; ++q)
-#pragma unroll
-              for (int k = 0; k < kSteps; ++k)
-                ptx::umma_ts_f16_warp(d_tmem, tmem_base + COL_Q + (uint32_t)(pa(q) * (D / 2) + k * 8),
-                                      bd + (uint64_t)((pb(q) * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
-          } else {
-#pragma unroll 1
-            for (int q = 0; q < 6; ++q)
-#pragma unroll
-              for (int k = 0; k < kSteps; ++k)
-                ptx::umma_ss_f16_warp(d_tmem, kd + (uint64_t)((pa(q) * T::kKPlane + k * 32) >> 4),
-                                      bd + (uint64_t)((pb(q) * T::kPiecePlane + k * 32) >> 4), idesc_rel, q != 0 || k != 0 ? 1u : 0u);
-          }
-          ptx::umma_commit_warp(&bars->empty[s]);
-          ptx::umma_commit_warp(&bars->acc_full[a]);
-        }
+      for (int n = 0; n < p2c_end && ok; ++n) {
+        if (n == c2p_end) ok = wait(&bars->k_full, (uint32_t)t & 1u, kCode + 74);
+        ok = ok && mma_piece(n < c2p_end ? 0 : 1);
       }
       // S takes the place of the previous tile's P, which PV has read by then
-      ok = ok && wait(&bars->q_full, 0, kCode + 77) && wait(&bars->k_full, (uint32_t)t & 1u, kCode + 78) &&
+      ok = ok && wait(&bars->k_full, (uint32_t)t & 1u, kCode + 78) &&
            (t == 0 || wait(&bars->o_full, (uint32_t)(t - 1) & 1u, kCode + 79));
       if (!ok) break;
       ptx::tc_fence_after();
-#pragma unroll 1
+#pragma unroll
       for (int q = 0; q < 6; ++q)
 #pragma unroll
         for (int k = 0; k < kSteps; ++k)
-          ptx::umma_ts_f16_warp(tmem_base + COL_SP, tmem_base + COL_Q + (uint32_t)(pa(q) * (D / 2) + k * 8),
-                                kd + (uint64_t)((pb(q) * T::kKPlane + k * 32) >> 4), idesc_qk, q != 0 || k != 0 ? 1u : 0u);
-      ptx::umma_commit_warp(&bars->k_empty);
+          ptx::umma_ts_f16_warp(tmem_base + COL_SP, tmem_base + COL_Q + (uint32_t)(pa[q] * (D / 2) + k * 8),
+                                kd + (uint64_t)((pb[q] * T::kKPlane + k * 32) >> 4), idesc_qk, q != 0 || k != 0 ? 1u : 0u);
       ptx::umma_commit_warp(&bars->s_full);
+#pragma unroll 1
+      for (int n = 0; n < next_early && ok; ++n) ok = mma_piece(0);
       const int n_v = value_pieces(t);
-      ok = wait(&bars->p_full, (uint32_t)t & 1u, kCode + 80);
+      ok = ok && wait(&bars->p_full, (uint32_t)t & 1u, kCode + 80);   // ... and S is complete: K's place is free
+      if (ok && t + 1 < n_kt) load(T::offK, &tmap_k, &bars->k_full, (t + 1) * BN);
       for (int v = 0; v < n_v && ok; ++v) ok = wait(&bars->full[(pc + v) % kStages], ((pc + v) / kStages) & 1u, kCode + 81);
       if (!ok) break;
       ptx::tc_fence_after();
-#pragma unroll 1
+      uint64_t v_stage[2];
+#pragma unroll
+      for (int v = 0; v < 2; ++v) v_stage[v] = vd + (uint64_t)((((pc + v) % kStages) * T::kStage) >> 4);
+#pragma unroll
       for (int q = 0; q < 6; ++q)
-#pragma unroll 1
-        for (int v = 0; v < n_v; ++v) {
-          const uint32_t a = tmem_base + COL_SP + (uint32_t)(pa(q) * (BN / 2) + v * (kPiece / 2));
-          const uint64_t bq = vd + (uint64_t)((((pc + v) % kStages) * T::kStage + pb(q) * T::kPiecePlane) >> 4);
+#pragma unroll
+        for (int v = 0; v < 2; ++v) {
+          if (v >= n_v) continue;
 #pragma unroll
           for (int k = 0; k < kVSteps; ++k)
-            ptx::umma_ts_f16_warp(tmem_base + COL_O, a + (uint32_t)(k * 8), bq + (uint64_t)((k * 16 * T::kRowBytes) >> 4), idesc_pv,
+            ptx::umma_ts_f16_warp(tmem_base + COL_O, tmem_base + COL_SP + (uint32_t)(pa[q] * (BN / 2) + v * (kPiece / 2) + k * 8),
+                                  v_stage[v] + (uint64_t)((pb[q] * T::kPiecePlane + k * 16 * T::kRowBytes) >> 4), idesc_pv,
                                   q != 0 || v != 0 || k != 0 ? 1u : 0u);
         }
       for (int v = 0; v < n_v; ++v, ++pc) ptx::umma_commit_warp(&bars->empty[pc % kStages]);
@@ -294,37 +292,42 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
     const uint32_t t_o = tmem_base + lanes + COL_O + hf * OW, t_acc = tmem_base + lanes + COL_ACC + hf * 32;
     float* xmax = reinterpret_cast<float*>(smem + T::offMax);
     float* rel = reinterpret_cast<float*>(smem + T::offRel);
+    for (int w = warp; w < n_kt * BN / 32; w += kComputeWarps) {   // (a tile's scores are never ready before all warps are here)
+      const int j = w * 32 + lane;
+      const uint32_t bits = __ballot_sync(0xffffffffu, j < L && mask_keep(p.mask, p.mask_elem_size, (long long)b * L + j));
+      if (lane == 0) keep_s[w] = bits;
+    }
     wait_for_predecessor();
-    {   // this thread's half of its query row, all planes, into tensor memory
-      const __nv_bfloat16* q_row = reinterpret_cast<const __nv_bfloat16*>(p.q) + ((long long)bh * L + (row_ok ? i : 0)) * D + hf * OW;
-      uint32_t words[kPlanes][OW / 2];
-#pragma unroll
-      for (int q = 0; q < kPlanes; ++q)
-#pragma unroll
-        for (int c = 0; c < OW / 8; ++c) {
-          const uint4 v = row_ok ? *reinterpret_cast<const uint4*>(q_row + (long long)q * BH * L * D + c * 8) : make_uint4(0u, 0u, 0u, 0u);
-          words[q][4 * c] = v.x;
-          words[q][4 * c + 1] = v.y;
-          words[q][4 * c + 2] = v.z;
-          words[q][4 * c + 3] = v.w;
-        }
+    release_successor();
+    bool ok = wait(&bars->q_load, 0, kCode + 90);
+    {   // this thread's half of its query row, all planes, into tensor memory (a row read by its own thread from global memory:
+        // 3.9 k cycles before the first MMA instead of 2 k)
+      const unsigned char* q_row = smem + T::offRel + r * T::kRowBytes;
+      const int swizzle = T::kRowBytes == 128 ? r & 7 : (r >> 1) & 3;
 #pragma unroll
       for (int q = 0; q < kPlanes; ++q) {
+        uint32_t words[OW / 2];
+#pragma unroll
+        for (int c = 0; c < OW / 8; ++c) {
+          const uint4 v = *reinterpret_cast<const uint4*>(q_row + q * T::kKPlane + (((hf * (OW / 8) + c) ^ swizzle) << 4));
+          words[4 * c] = v.x;
+          words[4 * c + 1] = v.y;
+          words[4 * c + 2] = v.z;
+          words[4 * c + 3] = v.w;
+        }
         const uint32_t at = tmem_base + lanes + COL_Q + (uint32_t)(q * (D / 2) + hf * (OW / 2));
-        if constexpr (D == 64) ptx::tmem_st16(at, words[q]);
-        else ptx::tmem_st8(at, words[q]);
+        if constexpr (D == 64) ptx::tmem_st16(at, words);
+        else ptx::tmem_st8(at, words);
       }
       ptx::tmem_wait_st();
       ptx::tc_fence_before();
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->q_full);
     }
-    release_successor();
     float o[OW];
 #pragma unroll
     for (int c = 0; c < OW; ++c) o[c] = 0.0f;
     float m_run = -INFINITY, l_run = 0.0f;
-    bool ok = true;
     uint32_t ac = 0, syncs = 0;
     auto sync_compute = [&](int code) {   // the eight warps; bounded, unlike a named barrier
       __syncwarp();
@@ -468,35 +471,40 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_k, const DflAt
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->p_full);
     }
-    if (ok) ok = wait(&bars->o_full, (uint32_t)(n_kt - 1) & 1u, kCode + 88);
     if (ok) {
-      ptx::tc_fence_after();
-      add_output(1.0f);
       float* xsum = xmax + (n_kt & 1) * 2 * BM;   // the parity the last tile did not use
       xsum[hf * BM + r] = l_run;
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&bars->pair[quarter]);
       ok = wait(&bars->pair[quarter], (uint32_t)n_kt & 1u, kCode + 89);
-      if (ok && row_ok) {
-        const float inv = 1.0f / (l_run + xsum[(1 - hf) * BM + r]);
-        const long long at = ((long long)b * L + i) * ((long long)H * D) + (long long)h * D + hf * OW;
+      const float inv = 1.0f / (l_run + xsum[(1 - hf) * BM + r]);
+      ok = ok && wait(&bars->o_full, (uint32_t)(n_kt - 1) & 1u, kCode + 88);
+      ptx::tc_fence_after();
+      add_output(inv);
+      // through the rows in shared memory, so that D / 4 lanes store a row
 #pragma unroll
-        for (int c = 0; c < OW; c += 8) {
-          const float f[4] = {o[c] * inv, o[c + 1] * inv, o[c + 2] * inv, o[c + 3] * inv};
-          const float g[4] = {o[c + 4] * inv, o[c + 5] * inv, o[c + 6] * inv, o[c + 7] * inv};
-          if (out_planes) {
-            uint2 lo[kPlanes], hi[kPlanes];
-            split3x4(f, lo);
-            split3x4(g, hi);
-            const long long plane = (long long)p.batch * L * H * D;
+      for (int c = 0; c < OW; c += 4)
+        *reinterpret_cast<float4*>(rel + r * kPitch + hf * OW + c) = make_float4(o[c], o[c + 1], o[c + 2], o[c + 3]);
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&bars->pair[quarter]);
+      ok = wait(&bars->pair[quarter], (uint32_t)(n_kt + 1) & 1u, kCode + 91) && ok;
+      constexpr int kLanes = D / 4, kRowsAtOnce = 32 / kLanes;
+      const int c = lane % kLanes * 4;
+#pragma unroll 4
+      for (int it = 0; it < 16 / kRowsAtOnce; ++it) {
+        const int row = quarter * 32 + hf * 16 + it * kRowsAtOnce + lane / kLanes;
+        if (!ok || i0 + row >= L) continue;
+        const float4 x = *reinterpret_cast<const float4*>(rel + row * kPitch + c);
+        const float f[4] = {x.x, x.y, x.z, x.w};
+        const long long at = ((long long)b * L + i0 + row) * ((long long)H * D) + (long long)h * D + c;
+        if (out_planes) {
+          uint2 w[kPlanes];
+          split3x4(f, w);
+          const long long plane = (long long)p.batch * L * H * D;
 #pragma unroll
-            for (int q = 0; q < kPlanes; ++q)
-              *reinterpret_cast<uint4*>(reinterpret_cast<__nv_bfloat16*>(p.out) + q * plane + at + c) = make_uint4(lo[q].x, lo[q].y, hi[q].x, hi[q].y);
-          } else {
-            float4* dst = reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at + c);
-            dst[0] = make_float4(f[0], f[1], f[2], f[3]);
-            dst[1] = make_float4(g[0], g[1], g[2], g[3]);
-          }
+          for (int q = 0; q < kPlanes; ++q) *reinterpret_cast<uint2*>(reinterpret_cast<__nv_bfloat16*>(p.out) + q * plane + at) = w[q];
+        } else {
+          *reinterpret_cast<float4*>(reinterpret_cast<float*>(p.out) + at) = x;
         }
       }
     }
@@ -517,8 +525,9 @@ int launch_d(const DflAttnParams& p, const void* pos_key, const void* pos_query,
   using T = Shape<D>;
   const int L = p.seq_len, BH = p.batch * p.heads;
   const uint64_t row = (uint64_t)D * 2, seq = (uint64_t)L * row;
-  CUtensorMap tk;
-  int rc = encode_tensor_map_3d(&tk, p.k, D, L, (uint64_t)kPlanes * BH, row, seq, D, BN, T::kRowBytes);
+  CUtensorMap tq, tk;
+  int rc = encode_tensor_map_3d(&tq, p.q, D, L, (uint64_t)kPlanes * BH, row, seq, D, BM, T::kRowBytes);
+  if (rc == DFL_OK) rc = encode_tensor_map_3d(&tk, p.k, D, L, (uint64_t)kPlanes * BH, row, seq, D, BN, T::kRowBytes);
   if (rc != DFL_OK) return rc;
   auto kernel = attention_f32_rel_kernel<D>;
   static KernelDeviceConfig config;   // per instantiation
@@ -534,7 +543,7 @@ int launch_d(const DflAttnParams& p, const void* pos_key, const void* pos_query,
   const long long items = (long long)((L + BM - 1) / BM) * BH;
   if (items > 0x7fffffff) return fail(DFL_ERR_TOO_LARGE, "too many query tiles");
   cudaError_t e = launch_after_predecessor(kernel, dim3((unsigned)items), dim3(kThreads), (size_t)(smem < floor_smem ? floor_smem : smem),
-                                           stream, tk, p, reinterpret_cast<const __nv_bfloat16*>(pos_key),
+                                           stream, tq, tk, p, reinterpret_cast<const __nv_bfloat16*>(pos_key),
                                            reinterpret_cast<const __nv_bfloat16*>(pos_query), n_active, out_planes, status_word);
   if (e != cudaSuccess) return fail(DFL_ERR_LAUNCH, "attention_f32_rel_kernel: %s", cudaGetErrorString(e));
   return check_launch("attention_f32_rel_kernel");
