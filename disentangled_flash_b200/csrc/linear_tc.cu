@@ -291,39 +291,39 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
   };
 
   if (warp == kTmaWarp) {
-    // ---------------------------------------------------------- TMA producer (both CTAs)
-    if (lane == 0) {
-      uint32_t it = 0;
-      bool ok = true;
-      for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
-        int m0, n0, z;
-        tile_coords(tile, m0, n0, z);
-        // k-steps: num_kb = taps x (k-blocks per tap); a plain GEMM has one tap with no row shift
-        const int taps = CONV && g.taps > 1 ? g.taps : 1;
-        const int kb_per_tap = CONV ? num_kb / taps : num_kb;
-        const int w_batch = z % g.w_mod;
-        int tap = 0, kb = 0;
-        for (int step = 0; step < num_kb; ++step, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
-          ok = ptx::mbar_wait(&empty_bar[s], ph ^ 1u, abort_flag, g.status, kWaits + 11);
-          if (!ok) break;
-          if (rank == 0) ptx::mbar_arrive_expect_tx(&full_bar[s], 2u * load_bytes);
-          const uint32_t leader_full = ptx::map_to_cta(ptx::smem_u32(&full_bar[s]), 0);
-          unsigned char* a = smem + s * kPairStageBytes;
-          // rows above the first or below the last row of X_z are filled with zeros by the load
-          if constexpr (CONV) {
-            ptx::tma_load_3d_pair(a, &tmap_x, leader_full, kb * BK, m0 + (int)rank * TM + tap - (taps >> 1), z);
-            ptx::tma_load_3d_pair(a + kTileA, &tmap_w, leader_full, kb * BK, n0 + (int)rank * (bn / 2),
-                                  taps > 1 ? tap : w_batch);
-            if (++kb == kb_per_tap) {
-              kb = 0;
-              ++tap;
-            }
-          } else {
-            ptx::tma_load_3d_pair(a, &tmap_x, leader_full, step * BK, m0 + (int)rank * TM, z);
-            ptx::tma_load_3d_pair(a + kTileA, &tmap_w, leader_full, step * BK, n0 + (int)rank * (bn / 2), w_batch);
+    // ---------------------------------------------------------- TMA producer (both CTAs; the whole warp, converged)
+    const uint32_t ring_addr = ptx::smem_u32(smem), full_addr = ptx::smem_u32(full_bar), leader_full = ptx::map_to_cta(full_addr, 0);
+    const int taps = CONV && g.taps > 1 ? g.taps : 1;
+    int s = 0;
+    uint32_t ph = 1;   // phase of empty_bar[s] to wait for (the first round passes)
+    bool ok = true;
+    for (int tile = pair; tile < num_tiles && ok; tile += num_pairs) {
+      int m0, n0, z;
+      tile_coords(tile, m0, n0, z);
+      // k-steps: num_kb = taps x (k-blocks per tap); a plain GEMM has one tap with no row shift
+      const int kb_per_tap = CONV ? num_kb / taps : num_kb;
+      const int w_batch = z % g.w_mod, x_row = m0 + (int)rank * TM, w_row = n0 + (int)rank * (bn / 2);
+      int tap = 0, kb = 0;
+      for (int step = 0; step < num_kb; ++step) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&empty_bar[s], ph, abort_flag, g.status, kWaits + 11));
+        if (!ok) break;
+        if (rank == 0) ptx::mbar_arrive_expect_tx_warp(full_addr + 8u * s, 2u * load_bytes);
+        const uint32_t a = ring_addr + (uint32_t)s * kPairStageBytes, bar = leader_full + 8u * s;
+        // rows above the first or below the last row of X_z are filled with zeros by the load
+        if constexpr (CONV) {
+          ptx::tma_load_3d_pair_warp(a, &tmap_x, bar, kb * BK, x_row + tap - (taps >> 1), z);
+          ptx::tma_load_3d_pair_warp(a + kTileA, &tmap_w, bar, kb * BK, w_row, taps > 1 ? tap : w_batch);
+          if (++kb == kb_per_tap) {
+            kb = 0;
+            ++tap;
           }
+        } else {
+          ptx::tma_load_3d_pair_warp(a, &tmap_x, bar, step * BK, x_row, z);
+          ptx::tma_load_3d_pair_warp(a + kTileA, &tmap_w, bar, step * BK, w_row, w_batch);
+        }
+        if (++s == STAGES) {
+          s = 0;
+          ph ^= 1u;
         }
       }
     }
@@ -334,7 +334,8 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(BK * 2);
       const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(smem), 16, 8 * BK * 2, mode);
       const uint64_t bdesc0 = ptx::make_smem_desc(ptx::smem_u32(smem + kTileA), 16, 8 * BK * 2, mode);
-      uint32_t it = 0;
+      int s = 0;
+      uint32_t ph = 0;
       bool ok = true;
       int lt = 0;
       for (int tile = pair; tile < num_tiles && ok; tile += num_pairs, ++lt) {
@@ -343,9 +344,7 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
         if (!ok) break;
         ptx::tc_fence_after();
         const uint32_t d_tmem = tmem_base + acc * TN;
-        for (int kb = 0; kb < num_kb; ++kb, ++it) {
-          const int s = it % STAGES;
-          const uint32_t ph = (it / STAGES) & 1u;
+        for (int kb = 0; kb < num_kb; ++kb) {
           ok = __all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 12));
           if (!ok) break;
           ptx::tc_fence_after();
@@ -355,6 +354,10 @@ gemm_tc_pair_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_con
           for (int k = 0; k < BK / 16; ++k)
             ptx::umma_ss_f16_pair_warp(d_tmem, adesc + 2 * k, bdesc + 2 * k, idesc, (kb | k) != 0 ? 1u : 0u);
           ptx::umma_commit_pair_warp(&empty_bar[s]);  // frees the stage in both CTAs
+          if (++s == STAGES) {
+            s = 0;
+            ph ^= 1u;
+          }
         }
         if (!ok) break;
         ptx::umma_commit_pair_warp(&tmem_full_bar[acc]);  // accumulator complete, both CTAs' epilogues may read

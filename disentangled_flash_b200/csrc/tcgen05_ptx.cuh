@@ -299,12 +299,14 @@ __device__ __forceinline__ void mbar_arrive_peer(uint32_t cluster_addr) {
 }
 // TMA load into this CTA's shared memory whose completion bytes are reported to a barrier given by its cluster
 // address (the pair leader's barrier).
-__device__ __forceinline__ void tma_load_3d_pair(void* smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr,
-                                                 int x, int y, int z) {
+// Issued by one elected lane of a converged warp.
+__device__ __forceinline__ void tma_load_3d_pair_warp(uint32_t smem_dst, const CUtensorMap* map, uint32_t bar_cluster_addr, int x, int y,
+                                                      int z) {
   asm volatile(
-      "cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
-      " [%0], [%1, {%3, %4, %5}], [%2];"
-      ::"r"(smem_u32(smem_dst)), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
+      "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
+      "@q cp.async.bulk.tensor.3d.cta_group::2.shared::cluster.global.mbarrier::complete_tx::bytes"
+      " [%0], [%1, {%3, %4, %5}], [%2];\n\t}"
+      ::"r"(smem_dst), "l"(reinterpret_cast<uint64_t>(map)), "r"(bar_cluster_addr), "r"(x), "r"(y), "r"(z)
       : "memory");
 }
 __device__ __forceinline__ void tmem_alloc_pair(uint32_t* smem_holder, uint32_t ncols) {
