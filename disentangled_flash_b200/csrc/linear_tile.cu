@@ -247,41 +247,44 @@ gemm_tile_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_consta
     }
   } else if (warp == kMmaWarp) {
     // ------------------------------------------------------------ MMA issuer (of a pair: the leader's)
-    if (half == 0) {   // the whole warp, converged: see umma_ss_f16_warp
+    if (half == 0 && ptx::elect_one()) {   // one lane, see umma_ss_f16_words
       const uint32_t idesc = ptx::make_idesc_f16(__is_same(T, __nv_bfloat16) ? 1 : 0, PAIR ? 2 * kRows : kRows, a.bn, 0, 0);
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(BK * 2);
-      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(ring), 16, 8 * BK * 2, mode);
-      const uint64_t bdesc0 = ptx::make_smem_desc(ptx::smem_u32(ring) + a_bytes, 16, 8 * BK * 2, mode);
+      const uint64_t desc0 = ptx::make_smem_desc(ptx::smem_u32(ring), 16, 8 * BK * 2, mode);
+      const uint32_t first = (uint32_t)desc0, upper = (uint32_t)(desc0 >> 32);
+      // in descriptor units: from X to W of a stage, from a stage to the next, and from a piece to the next
+      const uint32_t to_w = a_bytes >> 4, stage_next = stage_bytes >> 4, x_next = a.x_piece >> 4, w_next = (uint32_t)(w_rows * BK * 2) >> 4;
+      auto issue = [&](uint32_t ad, uint32_t bd, uint32_t accumulate) {   // one piece
+#pragma unroll
+        for (int k = 0; k < BK / 16; ++k)
+          ptx::umma_ss_f16_words<PAIR>(tmem_base, ad + 2 * k, bd + 2 * k, upper, idesc, k != 0 ? 1u : accumulate);
+      };
+      const int n_kb = kb_end - kb_begin;
       int s = 0;
-      uint32_t ph = 0;
-      bool ok = true;
-      for (int kb = kb_begin; kb < kb_end; ++kb) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 22));
+      uint32_t ph = 0, desc = first;
+      // The next k-block's barrier is looked at between the MMAs of this one: a wait answered only after the last of them leaves the
+      // tensor pipe idle.
+      bool landed = false, ok = true;
+      for (int i = 0; i < n_kb; ++i) {
+        ok = landed || ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 22);
         if (!ok) break;
         ptx::tc_fence_after();
-        const uint64_t adesc = adesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
-        const uint64_t bdesc = bdesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
-        for (int p = 0; p < a.pieces; ++p) {
-          const uint64_t ad = adesc + (uint64_t)((uint32_t)p * (a.x_piece >> 4)), bd = bdesc + (uint64_t)((uint32_t)p * (uint32_t)(w_rows * BK * 2 >> 4));
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint32_t acc = kb != kb_begin || p != 0 || k != 0 ? 1u : 0u;
-            if (PAIR) ptx::umma_ss_f16_pair_warp(tmem_base, ad + 2 * k, bd + 2 * k, idesc, acc);
-            else ptx::umma_ss_f16_warp(tmem_base, ad + 2 * k, bd + 2 * k, idesc, acc);
-          }
-        }
-        if (PAIR) ptx::umma_commit_pair_warp(&empty_bar[s], leader);
-        else ptx::umma_commit_warp(&empty_bar[s]);
+        uint64_t* done = &empty_bar[s];
+        const uint32_t ad = desc, bd = desc + to_w;
+        desc += stage_next;
         if (++s == a.stages) {
           s = 0;
           ph ^= 1u;
+          desc = first;
         }
+        issue(ad, bd, i != 0 ? 1u : 0u);
+        landed = i + 1 < n_kb && ptx::mbar_test(&full_bar[s], ph);
+        if (a.pieces == 2) issue(ad + x_next, bd + w_next, 1u);
+        ptx::umma_commit_one<PAIR>(done, leader);
       }
-      if (ok) {
-        if (PAIR) ptx::umma_commit_pair_warp(acc_bar, leader);
-        else ptx::umma_commit_warp(acc_bar);
-      }
+      if (ok) ptx::umma_commit_one<PAIR>(acc_bar, leader);
     }
+    __syncwarp();
   } else {
     // -------------------------------------------------------------- epilogue
     const int quarter = warp & 3;

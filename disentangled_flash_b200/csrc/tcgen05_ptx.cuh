@@ -273,11 +273,9 @@ __device__ __forceinline__ void umma_commit(uint64_t* bar) {
 // ----------------------------------------------- CTA pairs (cta_group::2) ---
 // Two CTAs of a cluster work on one MMA: each holds half of the rows of A, half of the rows of B and half of the
 // accumulator lanes; the CTA of cluster rank 0 issues the MMAs and owns the barriers the loads report to.
-__device__ __forceinline__ uint32_t cluster_ctarank() {
-  uint32_t r;
-  asm volatile("mov.u32 %0, %%cluster_ctarank;" : "=r"(r));
-  return r;
-}
+// (The intrinsic and not inline assembly: the compiler then knows that it is the same in all lanes, and what depends on it may stay in
+// uniform registers.)
+__device__ __forceinline__ uint32_t cluster_ctarank() { return __clusterRelativeBlockRank(); }
 // Address of `smem_addr` (a shared::cta address of this CTA) as seen in CTA `rank` of the cluster.
 __device__ __forceinline__ uint32_t map_to_cta(uint32_t smem_addr, uint32_t rank) {
   uint32_t r;
@@ -363,6 +361,40 @@ __device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar, uint32_t le
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
       ::"r"(smem_u32(bar)), "h"(both)
       : "memory");
+}
+
+// For a loop that one elected lane runs alone, waits, MMAs and commits together: what it issues costs less than the elections and
+// votes of a converged warp (gemm_tile_kernel, 128 x 32 to 256 x 96 tiles: 60 cycles an MMA in the forms above, 36 here, with the
+// descriptors as words: the upper one is the same for A and B).
+__device__ __forceinline__ bool elect_one() {
+  uint32_t r;
+  asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
+  return r != 0;
+}
+template <bool PAIR>
+__device__ __forceinline__ void umma_ss_f16_words(uint32_t d_tmem, uint32_t a_desc, uint32_t b_desc, uint32_t upper, uint32_t idesc,
+                                                  uint32_t accumulate) {
+  if (PAIR)
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::2.kind::f16 [%0], a, b, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_desc), "r"(b_desc), "r"(upper), "r"(idesc), "r"(accumulate)
+        : "memory");
+  else
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t.reg .b64 a, b;\n\tsetp.ne.b32 p, %5, 0;\n\tmov.b64 a, {%1, %3};\n\tmov.b64 b, {%2, %3};\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], a, b, %4, p;\n\t}"
+        ::"r"(d_tmem), "r"(a_desc), "r"(b_desc), "r"(upper), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+template <bool PAIR>
+__device__ __forceinline__ void umma_commit_one(uint64_t* bar, uint32_t leader) {
+  if (PAIR)
+    asm volatile("tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;"
+                 ::"r"(smem_u32(bar)), "h"((uint16_t)(3u << leader))
+                 : "memory");
+  else
+    asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(smem_u32(bar)) : "memory");
 }
 
 // TMEM <-> registers: each thread of a warp owns one lane (row); N consecutive 32-bit columns.
