@@ -19,8 +19,28 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& a, __nv_bfloat16&
   c = __float2bfloat16_rn(infinite ? x : r1 - __bfloat162float(b));
 }
 
-// Four elements of one row as packed plane words.
+// Four elements of one row as packed plane words.  The looks at infinities, and at what rounding would make one, are left out where
+// the sum of the magnitudes says that there are none (a NaN fails the comparison).
 __device__ __forceinline__ void split3x4(const float (&f)[4], uint2 (&out)[kPlanes]) {
+  if ((fabsf(f[0]) + fabsf(f[1])) + (fabsf(f[2]) + fabsf(f[3])) < 3.0e38f) {
+    uint32_t w[kPlanes][2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const float a = f[2 * j], b = f[2 * j + 1];
+      const __nv_bfloat162 h0 = __floats2bfloat162_rn(a, b);
+      const float2 f0 = __bfloat1622float2(h0);
+      const float ra = a - f0.x, rb = b - f0.y;
+      const __nv_bfloat162 h1 = __floats2bfloat162_rn(ra, rb);
+      const float2 f1 = __bfloat1622float2(h1);
+      const __nv_bfloat162 h2 = __floats2bfloat162_rn(ra - f1.x, rb - f1.y);
+      w[0][j] = *reinterpret_cast<const uint32_t*>(&h0);
+      w[1][j] = *reinterpret_cast<const uint32_t*>(&h1);
+      w[2][j] = *reinterpret_cast<const uint32_t*>(&h2);
+    }
+#pragma unroll
+    for (int q = 0; q < kPlanes; ++q) out[q] = make_uint2(w[q][0], w[q][1]);
+    return;
+  }
   __nv_bfloat16 p[kPlanes][4];
 #pragma unroll
   for (int j = 0; j < 4; ++j) split3(f[j], p[0][j], p[1][j], p[2][j]);

@@ -33,7 +33,7 @@ constexpr int kWaits = kWaitsGemmF32;
 
 struct F32Args {
   int split, stages, num_kb, tiles_m, tiles_n;
-  uint32_t ring_bytes, recv_bytes;
+  uint32_t ring_bytes;   // operand ring; behind it the receive buffer of a split inner product
 };
 
 // planes[q][i] of x[i]; HBM bound (4 bytes in, 6 out).
@@ -110,65 +110,70 @@ __global__ void __launch_bounds__(256, 3) refresh_planes_kernel(const DflPlaneSo
   }
 }
 
-// 32 finished columns [n, n+32) of the warp's 32 rows: bias, activation, then through the staging buffer so that eight
-// lanes store one row segment; row-major or head-major, in fp32 or as bf16 planes.
-__device__ __forceinline__ void emit32(const GemmDesc& g, const float (&acc)[32], const float* bias, float* stage, int row0,
-                                       int rows_live, int z, int n, int ncols, int lane) {
-  float f[32];
-#pragma unroll
-  for (int v = 0; v < 8; ++v) {
-    const float4 b = *reinterpret_cast<const float4*>(bias + 4 * v);
-    f[4 * v] = acc[4 * v] + b.x;
-    f[4 * v + 1] = acc[4 * v + 1] + b.y;
-    f[4 * v + 2] = acc[4 * v + 2] + b.z;
-    f[4 * v + 3] = acc[4 * v + 3] + b.w;
-  }
-  __syncwarp();
-#pragma unroll
-  for (int v = 0; v < 8; ++v)
-    *reinterpret_cast<float4*>(stage + lane * 32 + ((v ^ (lane & 7)) << 2)) = make_float4(f[4 * v], f[4 * v + 1], f[4 * v + 2], f[4 * v + 3]);
-  __syncwarp();
-  int which = 0, h = 0, dd = 0;
-  if (g.head_split) {
-    const int hd = g.heads * g.head_dim;
-    which = n / hd;
-    const int rem = n - which * hd;
-    h = rem / g.head_dim;
-    dd = rem - h * g.head_dim;
-  }
-  const int v = lane & 7;
+// The finished sums of the warp's 32 rows (first output row m0, `rows_live` of them inside the output) and its chunks of 32 columns
+// within [begin, end) of the tile, from shared memory, so that eight lanes store one row segment: bias, activation, row-major or
+// head-major, in fp32 or as bf16 planes.  `sums`: the warp's first row at the tile's column `begin`, `pitch` bytes from row to row.
+// Two rows at a time in one rolled loop: with a row at a time, its place divided out again for every chunk, and infinities looked
+// for element by element, a tile of 128 columns took 10.8 k cycles here, after 18.4 k of MMAs (1024 x 2304 x 768).
+template <int NCH>
+__device__ __forceinline__ void store_sums(const GemmDesc& g, const unsigned char* sums, uint32_t pitch, const float* bias, int m0,
+                                           int rows_live, int z, int n0, int ncols, int begin, int end, int side, int lane) {
+  const int v = lane & 7, hd = g.heads * g.head_dim;
+  const long long plane = g.head_split ? (long long)g.M * hd : (long long)g.M * g.ldc;   // elements of one plane of an output
 #pragma unroll 1
-  for (int it = 0; it < 8; ++it) {
-    const int r = it * 4 + (lane >> 3);
-    float4 val = *reinterpret_cast<const float4*>(stage + r * 32 + ((v ^ (r & 7)) << 2));
-    if (r >= rows_live || n + 4 * v >= ncols) continue;
-    if (g.activation == DFL_ACT_GELU) {
-      val.x = gelu_erf_exact(val.x);
-      val.y = gelu_erf_exact(val.y);
-      val.z = gelu_erf_exact(val.z);
-      val.w = gelu_erf_exact(val.w);
-    }
-    const int m = row0 + r;
-    void* base = g.out[0];
-    long long at, plane;   // element offset, and elements of one plane of this output
-    if (g.head_split) {
-      const int b = m / g.rows_per_seq, l = m - b * g.rows_per_seq;
-      base = which == 0 ? g.out[0] : (which == 1 ? g.out[1] : g.out[2]);
-      at = (((long long)b * g.heads + h) * g.rows_per_seq + l) * g.head_dim + dd + 4 * v;
-      plane = (long long)g.M * g.heads * g.head_dim;
-    } else {
-      at = (long long)z * g.stride_c + (long long)m * g.ldc + n + 4 * v;
-      plane = (long long)g.M * g.ldc;
-    }
-    if (g.out_planes) {
-      const float s4[4] = {val.x, val.y, val.z, val.w};
-      uint2 out[kPlanes];
-      split3x4(s4, out);
-      __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(base) + at;
+  for (int it = 0; it < 8; it += 2) {
+    long long place[2];   // element offset of the row
 #pragma unroll
-      for (int q = 0; q < kPlanes; ++q) *reinterpret_cast<uint2*>(dst + q * plane) = out[q];
-    } else {
-      *reinterpret_cast<float4*>(reinterpret_cast<float*>(base) + at) = val;
+    for (int u = 0; u < 2; ++u) {
+      const int m = m0 + (it + u) * 4 + (lane >> 3);
+      if (g.head_split) {
+        const int b = m / g.rows_per_seq, l = m - b * g.rows_per_seq;
+        place[u] = ((long long)b * g.heads * g.rows_per_seq + l) * g.head_dim;
+      } else {
+        place[u] = (long long)z * g.stride_c + (long long)m * g.ldc;
+      }
+    }
+#pragma unroll 1
+    for (int i = 0; i < NCH; ++i) {
+      const int c = 64 * i + 32 * side, n = n0 + c;
+      if (c < begin || c >= end || n >= ncols) continue;   // warp-uniform
+      void* out = g.out[0];
+      long long column = n;
+      if (g.head_split) {
+        const int which = n / hd, rem = n - which * hd, h = rem / g.head_dim;
+        out = which == 0 ? g.out[0] : (which == 1 ? g.out[1] : g.out[2]);
+        column = (long long)h * g.rows_per_seq * g.head_dim + (rem - h * g.head_dim);
+      }
+      const float4 b4 = *reinterpret_cast<const float4*>(bias + c + 4 * v);
+      float f[2][4];
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        const float4 x = *reinterpret_cast<const float4*>(sums + (uint32_t)((it + u) * 4 + (lane >> 3)) * pitch + (uint32_t)(c - begin + 4 * v) * 4u);
+        f[u][0] = x.x + b4.x;
+        f[u][1] = x.y + b4.y;
+        f[u][2] = x.z + b4.z;
+        f[u][3] = x.w + b4.w;
+      }
+      if (g.activation == DFL_ACT_GELU) {
+#pragma unroll
+        for (int u = 0; u < 2; ++u)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) f[u][j] = gelu_erf_exact(f[u][j]);
+      }
+#pragma unroll
+      for (int u = 0; u < 2; ++u) {
+        uint2 w[kPlanes];
+        if (g.out_planes) split3x4(f[u], w);
+        if ((it + u) * 4 + (lane >> 3) >= rows_live || n + 4 * v >= ncols) continue;
+        const long long at = place[u] + column + 4 * v;
+        if (g.out_planes) {
+          __nv_bfloat16* dst = reinterpret_cast<__nv_bfloat16*>(out) + at;
+#pragma unroll
+          for (int q = 0; q < kPlanes; ++q) *reinterpret_cast<uint2*>(dst + q * plane) = w[q];
+        } else {
+          *reinterpret_cast<float4*>(reinterpret_cast<float*>(out) + at) = make_float4(f[u][0], f[u][1], f[u][2], f[u][3]);
+        }
+      }
     }
   }
 }
@@ -268,45 +273,47 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       }
     }
   } else if (warp == kMmaWarp) {
-    if (half == 0) {
+    if (half == 0 && ptx::elect_one()) {   // one lane, see umma_ss_f16_words
       constexpr uint32_t idesc = ptx::make_idesc_f16(1, PAIR ? 2 * kRows : kRows, bn, 0, 0);
       constexpr uint32_t mode = ptx::swizzle_mode_for_row_bytes(BK * 2);
-      const uint64_t adesc0 = ptx::make_smem_desc(ptx::smem_u32(ring), 16, 8 * BK * 2, mode);
-      const uint64_t bdesc0 = ptx::make_smem_desc(ptx::smem_u32(ring) + a_bytes, 16, 8 * BK * 2, mode);
+      const uint64_t desc0 = ptx::make_smem_desc(ptx::smem_u32(ring), 16, 8 * BK * 2, mode);
+      const uint32_t first = (uint32_t)desc0, upper = (uint32_t)(desc0 >> 32);
+      // The next k-block's two barriers are looked at between the products of this one: answered only after the last of them, they
+      // leave the tensor pipe idle for 340 cycles of a k-block of 1.6 k (128 columns) or 3.1 k (256).
+      bool landed = false, free = false;
       int s = 0;
-      uint32_t ph = 0;
+      uint32_t ph = 0, desc = first;
       for (int i = 0; i < n_kb; ++i) {
         const int acc = i & 1;
-        bool ok = ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 42);
-        ok = ok && ptx::mbar_wait(&acc_empty[acc], ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, g.status, kWaits + 44);
-        if (!__all_sync(0xffffffffu, ok)) break;
+        if (!landed && !ptx::mbar_wait(&full_bar[s], ph, abort_flag, g.status, kWaits + 42)) break;
+        if (!free && !ptx::mbar_wait(&acc_empty[acc], ((uint32_t)(i >> 1) & 1u) ^ 1u, abort_flag, g.status, kWaits + 44)) break;
         ptx::tc_fence_after();
-        const uint64_t ad = adesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4)), bd = bdesc0 + (uint64_t)((uint32_t)s * (stage_bytes >> 4));
-        const uint32_t d_tmem = tmem_base + (uint32_t)(acc * bn);
+        const uint32_t ad = desc, bd = desc + (a_bytes >> 4), d_tmem = tmem_base + (uint32_t)(acc * bn);
+        uint64_t* done = &empty_bar[s];
+        desc += stage_bytes >> 4;
+        if (++s == a.stages) {
+          s = 0;
+          ph ^= 1u;
+          desc = first;
+        }
         // (plane of X, plane of W), smallest products first
         constexpr int px[6] = {2, 1, 0, 1, 0, 0}, pw[6] = {0, 1, 2, 0, 1, 0};
 #pragma unroll
         for (int q = 0; q < 6; ++q) {
-#pragma unroll
-          for (int k = 0; k < BK / 16; ++k) {
-            const uint64_t aq = ad + (uint64_t)(px[q] * (kPlaneA >> 4) + 2 * k), bq = bd + (uint64_t)(pw[q] * (plane_w >> 4) + 2 * k);
-            if (PAIR) ptx::umma_ss_f16_pair_warp(d_tmem, aq, bq, idesc, q != 0 || k != 0 ? 1u : 0u);
-            else ptx::umma_ss_f16_warp(d_tmem, aq, bq, idesc, q != 0 || k != 0 ? 1u : 0u);
+          if (q == 4) {
+            landed = i + 1 < n_kb && ptx::mbar_test(&full_bar[s], ph);
+            free = ptx::mbar_test(&acc_empty[acc ^ 1], ((uint32_t)((i + 1) >> 1) & 1u) ^ 1u);
           }
+#pragma unroll
+          for (int k = 0; k < BK / 16; ++k)
+            ptx::umma_ss_f16_words<PAIR>(d_tmem, ad + (uint32_t)(px[q] * (kPlaneA >> 4) + 2 * k), bd + (uint32_t)(pw[q] * (plane_w >> 4) + 2 * k),
+                                         upper, idesc, q != 0 || k != 0 ? 1u : 0u);
         }
-        if (PAIR) {
-          ptx::umma_commit_pair_warp(&empty_bar[s], leader);
-          ptx::umma_commit_pair_warp(&acc_full[acc], leader);
-        } else {
-          ptx::umma_commit_warp(&empty_bar[s]);
-          ptx::umma_commit_warp(&acc_full[acc]);
-        }
-        if (++s == a.stages) {
-          s = 0;
-          ph ^= 1u;
-        }
+        ptx::umma_commit_one<PAIR>(done, leader);
+        ptx::umma_commit_one<PAIR>(&acc_full[acc], leader);
       }
     }
+    __syncwarp();
   } else {
     const int quarter = warp & 3, side = warp >> 2;   // this warp's chunks: columns 64 * i + 32 * side
     const uint32_t taddr = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(side * 32);
@@ -345,20 +352,24 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
         else ptx::mbar_arrive(&acc_empty[acc]);
       }
     }
-    float* stage = reinterpret_cast<float*>(ring + (a.split == 1 ? 0u : a.ring_bytes + a.recv_bytes)) + warp * 1024;
     int rows_live = out_rows - quarter * 32;
     if (!ready) rows_live = 0;
+    const int r = quarter * 32 + lane, m0 = row0 + quarter * 32;
     if (a.split == 1) {
-      // the staging buffers lie in the operand ring: every warp's last block is complete, so every MMA has read it
+      // the sums go where the operands were: every warp's last block is complete, so every MMA has read them
       asm volatile("bar.sync 1, 256;" ::: "memory");
+      constexpr uint32_t pitch = bn * 4 + 16;
 #pragma unroll
       for (int i = 0; i < NCH; ++i) {
-        const int c = 64 * i + 32 * side;
-        if (n0 + c < ncols) emit32(g, sum[i], bias_s + c, stage, row0 + quarter * 32, rows_live, z, n0 + c, ncols, lane);
+        float4* row = reinterpret_cast<float4*>(ring + (uint32_t)r * pitch) + (64 * i + 32 * side) / 4;
+#pragma unroll
+        for (int j = 0; j < 8; ++j) row[j] = make_float4(sum[i][4 * j], sum[i][4 * j + 1], sum[i][4 * j + 2], sum[i][4 * j + 3]);
       }
+      __syncwarp();
+      store_sums<NCH>(g, ring + (uint32_t)(quarter * 32) * pitch, pitch, bias_s, m0, rows_live, z, n0, ncols, 0, bn, side, lane);
     } else {
       // Exchange as in gemm_tile_kernel: part p finishes columns [p * unit, (p + 1) * unit), unit a multiple of 32.
-      const int unit = bn / a.split, r = quarter * 32 + lane;
+      const int unit = bn / a.split;
       const uint32_t pitch = (uint32_t)(unit * 4 + 16), slot_bytes = (uint32_t)kRows * pitch;
       asm volatile("bar.sync 1, 256;" ::: "memory");   // every warp has added its last block: the ring is idle
 #pragma unroll
@@ -386,23 +397,26 @@ gemm_f32_kernel(const __grid_constant__ CUtensorMap tmap_x, const __grid_constan
       }
       __syncwarp();
       if (!__all_sync(0xffffffffu, ptx::mbar_wait(recv_bar, 0, abort_flag, g.status, kWaits + 45))) rows_live = 0;
-      const unsigned char* recv = ring + a.ring_bytes + (uint32_t)r * pitch;
+      unsigned char* recv = ring + a.ring_bytes;   // the first sender's slot takes the finished sums
 #pragma unroll
       for (int i = 0; i < NCH; ++i) {
         const int c = 64 * i + 32 * side;
-        if (c / unit != part || n0 + c >= ncols) continue;   // warp-uniform
-        if (r < out_rows) {
-          for (int p = 0; p < a.split - 1; ++p) {
-            const float4* src = reinterpret_cast<const float4*>(recv + (uint32_t)p * slot_bytes) + (c - part * unit) / 4;
+        if (c / unit != part || r >= out_rows) continue;
+        float4* own = reinterpret_cast<float4*>(recv + (uint32_t)r * pitch) + (c - part * unit) / 4;
+        for (int p = 0; p < a.split - 1; ++p) {
+          const float4* src = reinterpret_cast<const float4*>(reinterpret_cast<const unsigned char*>(own) + (uint32_t)p * slot_bytes);
 #pragma unroll
-            for (int j = 0; j < 8; ++j) {
-              const float4 s4 = src[j];
-              sum[i][4 * j] += s4.x; sum[i][4 * j + 1] += s4.y; sum[i][4 * j + 2] += s4.z; sum[i][4 * j + 3] += s4.w;
-            }
+          for (int j = 0; j < 8; ++j) {
+            const float4 s4 = src[j];
+            sum[i][4 * j] += s4.x; sum[i][4 * j + 1] += s4.y; sum[i][4 * j + 2] += s4.z; sum[i][4 * j + 3] += s4.w;
           }
         }
-        emit32(g, sum[i], bias_s + c, stage, row0 + quarter * 32, rows_live, z, n0 + c, ncols, lane);
+#pragma unroll
+        for (int j = 0; j < 8; ++j) own[j] = make_float4(sum[i][4 * j], sum[i][4 * j + 1], sum[i][4 * j + 2], sum[i][4 * j + 3]);
       }
+      __syncwarp();
+      store_sums<NCH>(g, recv + (uint32_t)(quarter * 32) * pitch, pitch, bias_s, m0, rows_live, z, n0, ncols, part * unit,
+                      (part + 1) * unit, side, lane);
     }
   }
 
@@ -439,16 +453,15 @@ int launch_plan(const GemmDesc& g, int split, cudaStream_t stream) {
   static KernelDeviceConfig config;   // per template instantiation
   rc = configure_kernel(config, kernel, kMaxSmem, nullptr, "gemm_f32_kernel");
   if (rc != DFL_OK) return rc;
-  const int recv = split > 1 ? (split - 1) * kRows * (bn / split * 4 + 16) : 0, staging = 8 * 4096;
+  const int recv = split > 1 ? (split - 1) * kRows * (bn / split * 4 + 16) : 0;
   const int kb_cta = (a.num_kb + split - 1) / split;
-  a.stages = (kMaxSmem - 3072 - (split > 1 ? recv + staging : 0)) / stage;
+  a.stages = (kMaxSmem - 3072 - recv) / stage;
   if (a.stages > kb_cta) a.stages = kb_cta;
   if (a.stages > kMaxStages) a.stages = kMaxStages;
   if (a.stages < 1) return fail(DFL_ERR_UNSUPPORTED, "gemm_f32: %d columns in %d parts do not fit", bn, split);
-  const int need = split > 1 ? recv : staging;
+  const int need = split > 1 ? recv : kRows * (bn * 4 + 16);   // parked shares, or the finished sums, where the operands were
   a.ring_bytes = (uint32_t)(a.stages * stage > need ? a.stages * stage : need);
-  a.recv_bytes = (uint32_t)recv;
-  const int smem = 3072 + (int)a.ring_bytes + (split > 1 ? recv + staging : 0);
+  const int smem = 3072 + (int)a.ring_bytes + recv;
   const int cluster = split * (PAIR ? 2 : 1);
   const long long ctas = (long long)a.tiles_n * a.tiles_m * g.batch * cluster;
   if (ctas > 0x7fffffff) return fail(DFL_ERR_TOO_LARGE, "gemm_f32: too many tiles");
