@@ -364,11 +364,12 @@ def workload_config(args, note: str | None = None):
 
 
 def executed_tile_fraction(mask: torch.Tensor, bm: int = 128, bn: int = 128) -> float:
-    """Fraction of (query tile, key tile) pairs the fused attention kernel actually computes for this mask.
+    """Fraction of (query tile, key tile) pairs with probabilities to compute for this mask.
 
-    Mirrors the kernel's rule (128 x 128 tiles): a query tile whose in-range rows are all padding takes the
-    mean-of-V path (no tile); a query tile with no padded row walks only the key tiles between the first and the
-    last kept key; a mixed query tile walks every key tile (padded rows attend to all L keys).
+    128 x 128 tiles: a query tile whose in-range rows are all padding is the mean of V (no tile); a query tile with
+    no padded row has the key tiles between the first and the last kept key; a mixed query tile counts every key tile
+    (padded rows attend to all L keys), although the kernel takes the padded rows' share of the tiles without a kept
+    key from a column sum of V.
     """
 
     batch, length = mask.shape

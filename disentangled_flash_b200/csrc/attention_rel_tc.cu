@@ -139,11 +139,9 @@ struct RLayout {
   static constexpr int offEye = offStg + kStgs * STG_BYTES;
   static constexpr int offBar = offEye + EYE_BYTES;
   static constexpr int kBarBytes = 512;
-  // exchange area: [2 parities][2 halves][BM] row maxima (row sums at the end of an item, partial sums of the mean-of-V
-  // path), then the [D] column mean of V
+  // exchange area: [2 parities][2 halves][BM] row maxima (row sums at the end of an item, partial column sums of V)
   static constexpr int offXmax = offBar + kBarBytes;
-  static constexpr int offMeanV = offXmax + (D > 64 ? 8 * D * 4 : 2 * 2 * BM * 4);
-  static constexpr int offItem = offMeanV + 256;
+  static constexpr int offItem = offXmax + (D > 64 ? 8 * D * 4 : 2 * 2 * BM * 4);
   static constexpr int kItemBytes = 304;
   static constexpr int total = offItem + kItemSlots * kItemBytes;
   static_assert(offStg % 16 == 0 && offBar % 16 == 0 && offItem % 16 == 0, "alignment");
@@ -153,7 +151,8 @@ struct RLayout {
 // What the loader warp publishes per item.
 struct ItemSlot {
   int t_begin, t_end;   // key tiles [t_begin, t_end) are processed
-  int any_kept;         // 0: every query row of the tile is padding -> mean-of-V path, no pipeline work
+  int any_kept;         // 0: every query row of the tile is padding -> mean-of-V path, no pipeline work; 2: padded rows beside
+                        // kept ones, and key tiles that are not walked
   int bh, h, i0;        // batch*heads + head, head, first query row
   int out_rows;         // rows of the sequence the output holds, from out_row0 on: [B,L,H*d], or packed rows (see
   long long out_row0;   // DflAttnRelParams.out_row_base)
@@ -291,12 +290,13 @@ __device__ __forceinline__ void kept_bits(const DflAttnRelParams& p, int b, int 
 }
 
 // Key tiles before the first and after the last kept key contribute nothing to a kept query row (their
-// probabilities are exactly zero) and are skipped; a padded query row attends uniformly to all L keys, so a query
-// tile that contains one walks every key tile.  A tile of padded rows only is the column mean of V (any_kept false).
+// probabilities are exactly zero) and are skipped.  A padded query row attends uniformly to all L keys: where a tile has both
+// kinds of rows (fold), the softmax threads add the column sums of V over the skipped keys to its padded rows.  A tile of padded
+// rows only is the column mean of V (any_kept false).
 // Warp-collective: lane l holds the kept-key words l (kb_lo) and l + 32 (kb_hi) of the batch row.
 struct TileRange {
   int t_begin, t_end;
-  bool any_kept;
+  bool any_kept, fold;
 };
 __device__ __forceinline__ TileRange tile_range(uint32_t kb_lo, uint32_t kb_hi, int i0, int L, int lane) {
   const int n_kt = (L + BK - 1) / BK;
@@ -311,12 +311,13 @@ __device__ __forceinline__ TileRange tile_range(uint32_t kb_lo, uint32_t kb_hi, 
   const uint32_t full = rows_here >= 32 ? 0xffffffffu : (rows_here <= 0 ? 0u : ((1u << rows_here) - 1u));
   const bool any_kept = __ballot_sync(0xffffffffu, in_q && kb != 0u) != 0u;
   const bool any_padded = __ballot_sync(0xffffffffu, in_q && (kb & full) != full) != 0u;
-  TileRange r{0, n_kt, any_kept};
-  if (!any_padded && (nz_lo | nz_hi) != 0u) {
+  TileRange r{0, n_kt, any_kept, false};
+  if ((nz_lo | nz_hi) != 0u) {
     const int first = nz_lo ? __ffs(nz_lo) - 1 : 32 + __ffs(nz_hi) - 1;
     const int last = nz_hi ? 32 + 31 - __clz(nz_hi) : 31 - __clz(nz_lo);
     r.t_begin = first >> 2;
     r.t_end = (last >> 2) + 1;
+    r.fold = any_kept && any_padded && (r.t_begin > 0 || r.t_end < n_kt);
   }
   return r;
 }
@@ -459,79 +460,21 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
       if (!ok) break;
       const ItemSlot* sl = &slots[slot];
       const int t_begin = sl->t_begin, n = sl->t_end - sl->t_begin;
-      const bool any_kept = sl->any_kept != 0;
+      const int kind = sl->any_kept;
+      const bool any_kept = kind != 0;
       const int bh = sl->bh, h = sl->h;
       const int i0 = sl->i0;
       const long long out_row0 = sl->out_row0;
       const int out_rows = sl->out_rows;
       if (!any_kept && out_rows <= i0) {
         // a tile of padded positions that the packed output does not hold: nothing to compute, nothing to store
-      } else if (!any_kept) {
-        // Every query row of this tile is padding: each attends uniformly to all L keys, so every output row is
-        // the column mean of V.  No score, no softmax: one pass over V by the 256 softmax threads.
-        // 16-byte loads, every thread sums 8 columns over a stride of rows; the row groups of a warp are folded with
-        // shuffles and the eight warps through shared memory (the row-exchange words are idle during such an item).
-        float* part = xchg;                                          // [8 warps][D] partial sums
-        T* mean = reinterpret_cast<T*>(smem + LO::offMeanV);         // [D]
-        constexpr int kChunks = D / 8;             // 16-byte chunks per row of V
-        constexpr int kRowStep = 256 / kChunks;    // rows covered by the 256 threads at once
-        const int tid = threadIdx.x, chunk = tid % kChunks, rgrp = tid / kChunks;
-        const uint4* V4 = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + (long long)bh * L * D);
-        float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
-#pragma unroll 2
-        for (int row = rgrp; row < L; row += kRowStep) {
-          const uint4 raw = __ldg(V4 + (long long)row * kChunks + chunk);
-          const T* e = reinterpret_cast<const T*>(&raw);
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] += Elem<T>::to_f(e[j]);
-        }
-#pragma unroll
-        for (int o = kChunks; o < 32; o <<= 1) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
-        }
-        // every warp has read its partner's row sums of the item before
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->xbar);
-        ok = wwait(&bars->xbar, 0u, 34);
-        if (!ok) break;
-        if (lane < kChunks) {
-#pragma unroll
-          for (int j = 0; j < 8; ++j) part[warp * D + lane * 8 + j] = acc[j];
-        }
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->xbar);
-        ok = wwait(&bars->xbar, 1u, 36);
-        if (!ok) break;
-        if (tid < D) {
-          float total = 0.0f;
-#pragma unroll
-          for (int w = 0; w < kSoftmaxWarps; ++w) total += part[w * D + tid];
-          mean[tid] = Elem<T>::from_f(total / (float)L);
-        }
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->xbar);
-        ok = wwait(&bars->xbar, 0u, 35);
-        if (!ok) break;
-        const int rows = out_rows - i0 < BM ? out_rows - i0 : BM;
-        constexpr int kVec = D / 8;  // 16-byte chunks per output row
-        const uint4 mine = *reinterpret_cast<const uint4*>(mean + (tid % kVec) * 8);
-        T* out = reinterpret_cast<T*>(p.out) + (out_row0 + i0) * ((long long)H * D) + (long long)h * D;
-        for (int e = tid; e < rows * kVec; e += 256) {
-          const int rr = e / kVec, v = e - rr * kVec;
-          *reinterpret_cast<uint4*>(out + (long long)rr * H * D + v * 8) = mine;
-        }
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&bars->xbar);   // the exchange words are free again
-        ok = wwait(&bars->xbar, 1u, 37);
-        if (!ok) break;
       } else {
         const int i = i0 + r;
         const bool row_ok = i < L;
         const bool q_keep = row_ok && ((sl->kbits[i >> 5] >> (i & 31)) & 1u) != 0u;
         float m_run = -INFINITY, l_run = 0.0f;
 
-        for (int u = 0; u < n && ok; ++u) {
+        for (int u = 0; u < n && any_kept && ok; ++u) {
           const int t = t_begin + u;
           const uint32_t kb0 = sl->kbits[4 * t + 2 * hf], kb1 = sl->kbits[4 * t + 2 * hf + 1];
           const int n_in = L - t * BK - hf * 64;   // in-range keys among this thread's 64 (may be <= 0 or >= 64)
@@ -670,56 +613,142 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (!ok) break;
 
         // ---- row sums, the item's last PV, then normalise and store this thread's half of the output columns
-        const uint32_t sum_phase = (c_t + c_i) & 1u;
-        float* xs = xchg + sum_phase * (2 * BM);
-        xs[hf * BM + r] = l_run;
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(pair2);
-        ok = wwait(pair2, sum_phase, 49);
-        ++c_i;
-        if (!ok) break;
-        const float inv = 1.0f / (l_run + xs[(1 - hf) * BM + r]);
-        ok = wwait(&bars->o_ready, (c_t & 1u) ^ 1u, 48);   // the item's last PV: c_t - 1 completed before it
-        if (!ok) break;
-        ptx::tc_fence_after();
-        // Lanes of one row each would touch 32 cache lines per store (1900 cycles an item).  The kGroup lanes of a group
-        // transpose their 16-byte chunks instead: lane c of the group ends up with chunk c of every row of the group, and a
-        // store covers whole segments.
-        constexpr int OC = OW < 32 ? OW : 32;   // columns at a time
-        constexpr int kGroup = OC / 8;
-        const int row0 = i0 + (r & ~(kGroup - 1)), rows = min(L, out_rows) - row0;
-        T* out = reinterpret_cast<T*>(p.out) + (out_row0 + row0) * ((long long)H * D) + (long long)h * D + hf * OW + (lane & (kGroup - 1)) * 8;
+        float total = 0.0f;
+        if (any_kept) {
+          const uint32_t sum_phase = (c_t + c_i) & 1u;
+          float* xs = xchg + sum_phase * (2 * BM);
+          xs[hf * BM + r] = l_run;
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(pair2);
+          ok = wwait(pair2, sum_phase, 49);
+          ++c_i;
+          if (!ok) break;
+          total = l_run + xs[(1 - hf) * BM + r];
+        }
+        if (kind != 1) {
+          // Padded query rows attend uniformly to all L keys.  Where every row of the tile is one, the outputs are the column mean
+          // of V: no score, no softmax.  Beside kept rows their weight is one on every key (their scores are zero, so is their
+          // maximum), and the keys of the tiles that were not walked are a column sum of V added to the accumulator: 1.5 k cycles
+          // where a tile takes 5.4 k.  Lengths uniform in [256, 512], us: 32 x 12 heads x 512 x d 64 122 -> 118, 16 x 8 x 512 x d 128
+          // 78 -> 74.5.  16-byte loads, every thread sums 8 columns over a stride of rows; the row groups of a warp are folded with
+          // shuffles and the eight warps through shared memory (the row-exchange words, idle from here to the next item).
+          constexpr int kChunks = D / 8;             // 16-byte chunks per row of V
+          constexpr int kRowStep = 256 / kChunks;    // rows covered by the 256 threads at once
+          const int tid = threadIdx.x, chunk = tid % kChunks;
+          const int before = any_kept ? t_begin * BK : L, after = min(L, (t_begin + n) * BK), skipped = any_kept ? before + L - after : L;
+          const uint4* V4 = reinterpret_cast<const uint4*>(reinterpret_cast<const T*>(p.v) + (long long)bh * L * D);
+          float acc[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
+#pragma unroll 2
+          for (int x = tid / kChunks; x < skipped; x += kRowStep) {
+            const int row = x < before ? x : x - before + after;
+            const uint4 raw = __ldg(V4 + (long long)row * kChunks + chunk);
+            const T* e = reinterpret_cast<const T*>(&raw);
 #pragma unroll
-        for (int c0 = 0; c0 < OW; c0 += OC) {
-          uint32_t o[OC];
-          attn::tmem_ld_n(t_o + c0, o);
-          ptx::tmem_wait_ld();
-          if (c0 + OC == OW) {   // the accumulator is in registers: the next item's first PV may overwrite it
-            ptx::tc_fence_before();
-            __syncwarp();
-            if (lane == 0) ptx::mbar_arrive(&bars->o_free);
+            for (int j = 0; j < 8; ++j) acc[j] += Elem<T>::to_f(e[j]);
           }
-          uint32_t w[kGroup][4];
 #pragma unroll
-          for (int x = 0; x < OC / 2; ++x)
-            w[x / 4][x % 4] = Pack2<T>::pack(__uint_as_float(o[2 * x]) * inv, __uint_as_float(o[2 * x + 1]) * inv);
+          for (int o = kChunks; o < 32; o <<= 1) {
 #pragma unroll
-          for (int bit = 1; bit < kGroup; bit <<= 1) {
-            const bool upper = (lane & bit) != 0;
+            for (int j = 0; j < 8; ++j) acc[j] += __shfl_xor_sync(0xffffffffu, acc[j], o);
+          }
+          // every warp has read its partner's row sums of the item before
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->xbar);
+          ok = wwait(&bars->xbar, 0u, 34);
+          if (!ok) break;
+          if (lane < kChunks) {
 #pragma unroll
-            for (int c = 0; c < kGroup; ++c) {
-              if (c & bit) continue;
+            for (int j = 0; j < 8; ++j) xchg[warp * D + lane * 8 + j] = acc[j];
+          }
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->xbar);
+          ok = wwait(&bars->xbar, 1u, 36);
+          if (!ok) break;
+          if (tid < D) {
+            float column = 0.0f;
 #pragma unroll
-              for (int x = 0; x < 4; ++x) {   // the lower lane keeps chunk c and takes the partner's, the upper one chunk c + bit
-                const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? w[c][x] : w[c | bit][x], bit);
-                if (upper) w[c][x] = got;
-                else w[c | bit][x] = got;
+            for (int w = 0; w < kSoftmaxWarps; ++w) column += xchg[w * D + tid];
+            xchg[tid] = column;   // no other thread reads this word of the partial sums
+          }
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->xbar);
+          ok = wwait(&bars->xbar, 0u, 35);
+          if (!ok) break;
+          if (!any_kept) {
+            const int rows = out_rows - i0 < BM ? out_rows - i0 : BM;
+            float mean[8];
+#pragma unroll
+            for (int j = 0; j < 8; ++j) mean[j] = xchg[chunk * 8 + j] / (float)L;
+            const uint4 mine = make_uint4(Pack2<T>::pack(mean[0], mean[1]), Pack2<T>::pack(mean[2], mean[3]),
+                                          Pack2<T>::pack(mean[4], mean[5]), Pack2<T>::pack(mean[6], mean[7]));
+            T* out = reinterpret_cast<T*>(p.out) + (out_row0 + i0) * ((long long)H * D) + (long long)h * D;
+            for (int e = tid; e < rows * kChunks; e += 256)
+              *reinterpret_cast<uint4*>(out + (long long)(e / kChunks) * H * D + chunk * 8) = mine;
+          } else {
+            ok = wwait(&bars->o_ready, (c_t & 1u) ^ 1u, 50);   // the item's last PV
+            if (!ok) break;
+            ptx::tc_fence_after();
+            if (!q_keep) total += (float)skipped;
+#pragma unroll 1
+            for (int c0 = 0; c0 < OW; c0 += 16) {
+              uint32_t o[16];
+              ptx::tmem_ld16(t_o + c0, o);
+              ptx::tmem_wait_ld();
+#pragma unroll
+              for (int x = 0; x < 16; ++x) o[x] = __float_as_uint(__uint_as_float(o[x]) + (q_keep ? 0.0f : xchg[hf * OW + c0 + x]));
+              ptx::tmem_st16(t_o + c0, o);
+            }
+            ptx::tmem_wait_st();
+          }
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&bars->xbar);   // the exchange words are free again
+          ok = wwait(&bars->xbar, 1u, 37);
+          if (!ok) break;
+        }
+        if (any_kept) {
+          const float inv = 1.0f / total;
+          ok = wwait(&bars->o_ready, (c_t & 1u) ^ 1u, 48);   // the item's last PV: c_t - 1 completed before it
+          if (!ok) break;
+          ptx::tc_fence_after();
+          // Lanes of one row each would touch 32 cache lines per store (1900 cycles an item).  The kGroup lanes of a group
+          // transpose their 16-byte chunks instead: lane c of the group ends up with chunk c of every row of the group, and a
+          // store covers whole segments.
+          constexpr int OC = OW < 32 ? OW : 32;   // columns at a time
+          constexpr int kGroup = OC / 8;
+          const int row0 = i0 + (r & ~(kGroup - 1)), rows = min(L, out_rows) - row0;
+          T* out = reinterpret_cast<T*>(p.out) + (out_row0 + row0) * ((long long)H * D) + (long long)h * D + hf * OW + (lane & (kGroup - 1)) * 8;
+#pragma unroll
+          for (int c0 = 0; c0 < OW; c0 += OC) {
+            uint32_t o[OC];
+            attn::tmem_ld_n(t_o + c0, o);
+            ptx::tmem_wait_ld();
+            if (c0 + OC == OW) {   // the accumulator is in registers: the next item's first PV may overwrite it
+              ptx::tc_fence_before();
+              __syncwarp();
+              if (lane == 0) ptx::mbar_arrive(&bars->o_free);
+            }
+            uint32_t w[kGroup][4];
+#pragma unroll
+            for (int x = 0; x < OC / 2; ++x)
+              w[x / 4][x % 4] = Pack2<T>::pack(__uint_as_float(o[2 * x]) * inv, __uint_as_float(o[2 * x + 1]) * inv);
+#pragma unroll
+            for (int bit = 1; bit < kGroup; bit <<= 1) {
+              const bool upper = (lane & bit) != 0;
+#pragma unroll
+              for (int c = 0; c < kGroup; ++c) {
+                if (c & bit) continue;
+#pragma unroll
+                for (int x = 0; x < 4; ++x) {   // the lower lane keeps chunk c and takes the partner's, the upper one chunk c + bit
+                  const uint32_t got = __shfl_xor_sync(0xffffffffu, upper ? w[c][x] : w[c | bit][x], bit);
+                  if (upper) w[c][x] = got;
+                  else w[c | bit][x] = got;
+                }
               }
             }
-          }
 #pragma unroll
-          for (int c = 0; c < kGroup; ++c)
-            if (c < rows) *reinterpret_cast<uint4*>(out + (long long)c * H * D + c0) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+            for (int c = 0; c < kGroup; ++c)
+              if (c < rows) *reinterpret_cast<uint4*>(out + (long long)c * H * D + c0) = make_uint4(w[c][0], w[c][1], w[c][2], w[c][3]);
+          }
         }
       }
       __syncwarp();
@@ -939,7 +968,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
         if (lane == 0) {
           sl->t_begin = range.t_begin;
           sl->t_end = range.t_end;
-          sl->any_kept = range.any_kept ? 1 : 0;
+          sl->any_kept = range.fold ? 2 : (range.any_kept ? 1 : 0);
           sl->bh = bh;
           sl->h = bh - b * H;
           sl->out_row0 = p.out_row_base ? (long long)p.out_row_base[b] : (long long)b * L;
