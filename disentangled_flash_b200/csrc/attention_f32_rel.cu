@@ -1,6 +1,7 @@
 // FP32 fused disentangled attention with the position scores computed in the kernel (head dims 32 and 64).
 //
 //   S[i,j] = q_i.k_j + q_i.pos_key[s] + k_j.pos_query[s],  s = lut[i-j+L-1];  scale, mask, softmax, P V as in attention_f32.cu
+// (the score products of kernel.py:574-585 and the kernel of kernel.py:137-345, both in the reference's strict FP32)
 // Every product is the six plane products of linear_f32.cu, smallest first, and no tensor-core accumulator holds more than one
 // 64-deep block, so the scores are what the score GEMMs and attention_f32_kernel give, but for the order of their two sums.
 //

@@ -471,6 +471,8 @@ int launch_pair(const GemmDesc& g, int bn, cudaStream_t stream) {
 // load is still charged as 128 rows where a tile has fewer.  Against every plan at 172 sizes (32 to 16384 rows, N and K of hidden
 // 768, 1024 and 1536), tiles loading the rows they have, the choice is 1.1 % above the best one on average (1.3 % at row counts
 // that do not fill their tiles), within 5 % at 162 of them, and 26 % at worst (1024 x 1536 x 6144: 24.6 against 19.5 us).
+// (Measured while an MMA of a narrow tile cost 60 cycles to issue; it costs 36 now, and the drain of a pair's tile is shorter.  The
+// plans were not compared again.)
 constexpr double kSmIngest = 83.0;      // operand bytes per cycle and SM ...
 constexpr double kSharedIngest = 0.46;  // ... and how much slower when every SM pulls
 constexpr double kDrain64 = 1460.0;     // draining 64 accumulator columns of a tile that nothing overlaps
