@@ -210,10 +210,10 @@ __device__ __forceinline__ float tanh_fast(float x) {
 // GELU, 0.5 x (1 + erf(x / sqrt 2)), for the GEMM epilogues.
 // Exact form (strict FP32 kernels): the CUDA library's erff.
 __device__ __forceinline__ float gelu_erf_exact(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-// Fast form of one value (16-bit outputs stored by single threads; gelu_erf_pair is the form of two): erf by the rational approximation 7.1.26 of Abramowitz & Stegun,
-// erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z), z >= 0, absolute error below 1.5e-7 - three
-// orders of magnitude under the rounding step of an FP16 or BF16 output - with one approximate reciprocal and one
-// approximate exp2 (relative error ~1e-7 each).
+// Fast form of one value, where single threads store 16-bit outputs (gelu_erf_pair is the form of two): erf by the rational
+// approximation 7.1.26 of Abramowitz & Stegun, erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z), z >= 0, absolute error
+// below 1.5e-7 - three orders of magnitude under the rounding step of an FP16 or BF16 output - with one approximate
+// reciprocal and one approximate exp2 (relative error ~1e-7 each).
 __device__ __forceinline__ float gelu_erf_fast(float x) {
   // gelu(x) = max(x, 0) - |x| * q(t) * exp(-z^2),  z = |x| / sqrt 2,  q(t) = 0.5 (a1 t + ... + a5 t^5).
   // With w = z * sqrt(log2 e): exp(-z^2) = exp2(-w^2) and 1 + p z = 1 + (p / sqrt(log2 e)) w.
@@ -246,8 +246,8 @@ __device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, un
 // error's weight in the result (Lawson's iteration on least squares; its leading coefficient is negative, so p keeps falling
 // beyond the fit).  Absolute error below 2.5e-7 (gelu_erf_fast: 3.3e-7), and relative to the result 4e-4 at worst in the
 // negative tail down to -4.5 (9e-4).  One special-function instruction an element where gelu_erf_fast has two, which bound
-// the epilogue (16 lanes a cycle and SM): 16384 x 3072 x 768 fp16 77.5 -> 72.9 us
-// (65 without an activation), 12288 rows 61.8 -> 55.0, 512 x 6144 x 1536 13.3 -> 12.7.
+// the epilogue (16 lanes a cycle and SM): 16384 x 3072 x 768 fp16 77.5 -> 72.9 us (65 without an activation), 12288 rows 61.8 ->
+// 55.0, 512 x 6144 x 1536 13.3 -> 12.7.  On single values, without the packed multiply-adds, 2 to 3 % slower.
 __device__ __forceinline__ void gelu_erf_pair(float& a, float& b) {
   const float na = -fabsf(a), nb = -fabsf(b);   // the polynomial is in -t: odd coefficients change their sign
   const unsigned long long t = pack_f32x2(na, nb);

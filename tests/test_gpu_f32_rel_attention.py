@@ -61,8 +61,6 @@ def test_against_fp64(d, terms, length):
 
 def test_long_sequences_and_the_kernels_that_read_scores_agree():
     """The longest table that fits shared memory (head dim 64), and the next length, which the score GEMMs serve."""
-    from disentangled_flash_b200 import attention as attn
-
     heads, d, buckets = 4, 64, 256
     outs = []
     for length in (3400, 3600):
