@@ -210,10 +210,11 @@ __device__ __forceinline__ float tanh_fast(float x) {
 // GELU, 0.5 x (1 + erf(x / sqrt 2)), for the GEMM epilogues.
 // Exact form (strict FP32 kernels): the CUDA library's erff.
 __device__ __forceinline__ float gelu_erf_exact(float x) { return 0.5f * x * (1.0f + erff(x * 0.70710678118654752f)); }
-// Fast form of one value, where single threads store 16-bit outputs (gelu_erf_pair is the form of two): erf by the rational
-// approximation 7.1.26 of Abramowitz & Stegun, erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z), z >= 0, absolute error
-// below 1.5e-7 - three orders of magnitude under the rounding step of an FP16 or BF16 output - with one approximate
-// reciprocal and one approximate exp2 (relative error ~1e-7 each).
+// Form for BF16 outputs: erf by the rational approximation 7.1.26 of Abramowitz & Stegun,
+// erf(z) = 1 - (a1 t + ... + a5 t^5) exp(-z^2), t = 1 / (1 + p z), z >= 0, absolute error below 1.5e-7, with one approximate
+// reciprocal and one approximate exp2 (relative error ~1e-7 each).  Its error stays small beside the result far into the negative
+// tail, whose results BF16's exponent range holds: 1.6e-3 of the result at -5, 6.5e-3 at -7, 1.5e-2 at -9 (gelu_erf_pair: 3.3e-3,
+// 0.3, 1).
 __device__ __forceinline__ float gelu_erf_fast(float x) {
   // gelu(x) = max(x, 0) - |x| * q(t) * exp(-z^2),  z = |x| / sqrt 2,  q(t) = 0.5 (a1 t + ... + a5 t^5).
   // With w = z * sqrt(log2 e): exp(-z^2) = exp2(-w^2) and 1 + p z = 1 + (p / sqrt(log2 e)) w.
@@ -240,14 +241,15 @@ __device__ __forceinline__ unsigned long long fma_f32x2(unsigned long long a, un
   asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
   return r;
 }
-// GELU of two values, for the epilogues of the 16-bit GEMMs:
+// GELU of two values, for FP16 outputs:
 //   gelu(x) = max(x, 0) - |x| Phi(-|x|),   Phi(-t) = 2^p(t),  t >= 0,
 // p the degree-8 polynomial that fits log2(erfc(t / sqrt 2) / 2) on [0, 6.5] with the weight t Phi(-t), that is, with the
 // error's weight in the result (Lawson's iteration on least squares; its leading coefficient is negative, so p keeps falling
 // beyond the fit).  Absolute error below 2.5e-7 (gelu_erf_fast: 3.3e-7), and relative to the result 4e-4 at worst in the
-// negative tail down to -4.5 (9e-4).  One special-function instruction an element where gelu_erf_fast has two, which bound
-// the epilogue (16 lanes a cycle and SM): 16384 x 3072 x 768 fp16 77.5 -> 72.9 us (65 without an activation), 12288 rows 61.8 ->
-// 55.0, 512 x 6144 x 1536 13.3 -> 12.7.  On single values, without the packed multiply-adds, 2 to 3 % slower.
+// negative tail down to -4.5 (9e-4).  Below -4.5 the error relative to the result grows (4.9e-2 at -6); in absolute terms it is below
+// 7e-9 there, a tenth of the step between FP16's smallest numbers.  One special-function instruction an element where gelu_erf_fast
+// has two, which bound the epilogue (16 lanes a cycle and SM): 16384 x 3072 x 768 fp16 77.5 -> 72.9 us (65 without an activation),
+// 12288 rows 61.8 -> 55.0, 512 x 6144 x 1536 13.3 -> 12.7.  On single values, without the packed multiply-adds, 2 to 3 % slower.
 __device__ __forceinline__ void gelu_erf_pair(float& a, float& b) {
   const float na = -fabsf(a), nb = -fabsf(b);   // the polynomial is in -t: odd coefficients change their sign
   const unsigned long long t = pack_f32x2(na, nb);
@@ -266,6 +268,16 @@ __device__ __forceinline__ void gelu_erf_pair(float& a, float& b) {
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(eb) : "f"(pb));
   const unsigned long long g = fma_f32x2(t, pack_f32x2(ea, eb), pack_f32x2(fmaxf(a, 0.0f), fmaxf(b, 0.0f)));
   asm("mov.b64 {%0, %1}, %2;" : "=f"(a), "=f"(b) : "l"(g));
+}
+// GELU of two values that are rounded to T next.
+template <typename T>
+__device__ __forceinline__ void gelu_pair(float& a, float& b) {
+  if constexpr (__is_same(T, __half)) {
+    gelu_erf_pair(a, b);
+  } else {
+    a = gelu_erf_fast(a);
+    b = gelu_erf_fast(b);
+  }
 }
 int launch_gemm_simt(const GemmDesc& g, cudaStream_t stream);
 int launch_gemm_tc(const GemmDesc& g, cudaStream_t stream);

@@ -87,7 +87,7 @@ __device__ __forceinline__ void emit(const GemmDesc& g, const float (&acc)[NC], 
   }
   if (g.activation == DFL_ACT_GELU) {
 #pragma unroll
-    for (int j = 0; j < NC; j += 2) gelu_erf_pair(f[j], f[j + 1]);
+    for (int j = 0; j < NC; j += 2) gelu_pair<T>(f[j], f[j + 1]);
   } else if (CONV && g.activation == DFL_ACT_TANH) {
 #pragma unroll
     for (int j = 0; j < NC; ++j) f[j] = tanh_fast(f[j]);
