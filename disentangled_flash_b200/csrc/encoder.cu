@@ -89,6 +89,9 @@ int validate(const DflEncoderParams& p) {
     if (!aligned16(p.outs[l])) return fail(DFL_ERR_ALIGNMENT, "outs[%d] not 16-byte aligned", l);
     if (!(y.attn_norm_eps >= 0.0f) || !(y.ffn_norm_eps >= 0.0f)) return fail(DFL_ERR_BAD_ARG, "eps must be non-negative");
     if ((!y.rel_key && !y.rel_query) != two_call(p)) return fail(DFL_ERR_BAD_ARG, "layers with and without rel tables");
+    // the F32 kernel gathers rows of these tables by the slots of lut, clamped to [0, n_active)
+    if (two_call(p) && (y.pos_key || y.pos_query) && (!p.lut || p.n_active < 1))
+      return fail(DFL_ERR_BAD_ARG, "layer %d: position tables without a LUT or with n_active %d", l, p.n_active);
   }
   if (p.attention_only && (p.n_layers != 1 || p.packed_rows > 0 || p.conv_w))
     return fail(DFL_ERR_BAD_ARG, "attention_only takes one layer of padded rows");
