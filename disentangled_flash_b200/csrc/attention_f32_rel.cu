@@ -444,6 +444,7 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
       const float corr = exp2f(m_run - m_use);   // 0 while nothing has been attended to
       m_run = m_new;
       if (t > 0) add_output(corr);   // the previous tile's PV (complete before S was issued), before its scale is left behind
+      // (exp2f: ex2.approx.ftz makes zeros of probabilities below 2^-126, and takes 2 % less at d 32, 0.5 % at d 64)
       float sum = 0.0f;
 #pragma unroll 1
       for (int c0 = 0; c0 < HK; c0 += 16) {
@@ -451,10 +452,10 @@ attention_f32_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __gri
 #pragma unroll
         for (int c = 0; c < 4; ++c) {
           const float4 x = row[c0 / 4 + c];
-          e[4 * c] = ptx::ex2_approx(x.x - m_use);
-          e[4 * c + 1] = ptx::ex2_approx(x.y - m_use);
-          e[4 * c + 2] = ptx::ex2_approx(x.z - m_use);
-          e[4 * c + 3] = ptx::ex2_approx(x.w - m_use);
+          e[4 * c] = exp2f(x.x - m_use);
+          e[4 * c + 1] = exp2f(x.y - m_use);
+          e[4 * c + 2] = exp2f(x.z - m_use);
+          e[4 * c + 3] = exp2f(x.w - m_use);
           sum += (e[4 * c] + e[4 * c + 1]) + (e[4 * c + 2] + e[4 * c + 3]);
         }
         uint32_t lo[kPlanes][4], hi[kPlanes][4];
