@@ -38,7 +38,7 @@ namespace {
 constexpr int BM = 128, BN = 128, kPiece = 64, kStages = 4;
 constexpr int kComputeWarps = 8, kLoadWarp = 8, kLoadWarps = 2, kMmaWarp = 10, kThreads = 352;
 constexpr int kMaxSmem = 232448;
-constexpr int kCode = kWaitsAttentionF32;
+constexpr int kCode = kWaitsAttentionF32Rel;
 constexpr int COL_SP = 0, COL_O = 192, COL_Q = 256, COL_ACC = 384, kTmemCols = 512;
 constexpr int kPitch = 132;   // floats per row of the score tile
 

@@ -40,7 +40,7 @@ inline int check_launch(const char* what) {
 // of these.
 enum WaitCodes {
   kWaitsAttention = 100, kWaitsGemmPair = 200, kWaitsGemmTile = 300, kWaitsAttentionRel = 400, kWaitsGemmF32 = 500,
-  kWaitsAttentionF32 = 600
+  kWaitsAttentionF32 = 600, kWaitsAttentionF32Rel = kWaitsAttentionF32 + 100
 };
 inline const char* kernel_of_wait(int code) {
   switch (code / 100 * 100) {
@@ -50,6 +50,7 @@ inline const char* kernel_of_wait(int code) {
     case kWaitsAttentionRel: return "attention_rel_kernel";
     case kWaitsGemmF32: return "gemm_f32_kernel";
     case kWaitsAttentionF32: return "attention_f32_kernel";
+    case kWaitsAttentionF32Rel: return "attention_f32_rel_kernel";
   }
   return code == 99 ? "the self test" : "unknown";
 }
