@@ -363,13 +363,14 @@ def workload_config(args, note: str | None = None):
     return cfg
 
 
-def executed_tile_fraction(mask: torch.Tensor, bm: int = 128, bn: int = 128) -> float:
+def executed_tile_fraction(mask: torch.Tensor, bm: int = 128, bn: int = 128, folded: bool = False) -> float:
     """Fraction of (query tile, key tile) pairs with probabilities to compute for this mask.
 
     128 x 128 tiles: a query tile whose in-range rows are all padding is the mean of V (no tile); a query tile with
     no padded row has the key tiles between the first and the last kept key; a mixed query tile counts every key tile
-    (padded rows attend to all L keys), although the kernel takes the padded rows' share of the tiles without a kept
-    key from a column sum of V.
+    (padded rows attend to all L keys).  ``folded``: the tiles that the relative-table attention kernel walks.  It takes
+    the padded rows' share of the tiles outside the kept keys from a column sum of V, so that a mixed query tile has the
+    same key tiles as one without a padded row.
     """
 
     batch, length = mask.shape
@@ -384,7 +385,7 @@ def executed_tile_fraction(mask: torch.Tensor, bm: int = 128, bn: int = 128) -> 
             rows = row[q * bm:(q + 1) * bm]
             if not rows.any():
                 continue
-            done += n_k if not rows.all() else last - first + 1
+            done += last - first + 1 if folded or rows.all() else n_k
     return done / float(batch * n_q * n_k)
 
 
@@ -591,12 +592,12 @@ def run_v3_base(args, ctx: GpuContext) -> None:
 
     # Roofline of the dominant kernel: the fused attention forward (tensor-core bound by design).
     # Only work the kernel does not skip is counted (key tiles outside the kept range and fully padded
-    # query tiles are skipped; see executed_tile_fraction).
+    # query tiles are skipped; see executed_tile_fraction).  The column sums of V that stand in for skipped tiles are not.
     B, H, L, d = args.batch, g["heads"], seq_len, g["head_dim"]
     n_active = int(encoder._active_plans[0].active_slots.numel())
     in_kernel_scores = observer.kernel_name == "dfl_attention_rel_fwd"
     used = [host_mask[i % len(host_mask)] for i in range(args.steps)]
-    executed = statistics.mean(executed_tile_fraction(m) for m in used) if in_kernel_scores else 1.0
+    executed = statistics.mean(executed_tile_fraction(m, folded=True) for m in used) if in_kernel_scores else 1.0
     flops_attn = 4.0 * B * H * L * L * d * executed  # QK^T + PV over the executed tiles
     # with the relative scores computed in-kernel, their non-redundant GEMM work (2 terms, A active slots)
     # is part of the launch, in the same proportion; window MMAs executed beyond that are not counted
