@@ -1,5 +1,6 @@
 // FP32 fused disentangled attention on the tensor cores, position scores from memory: head dim 128, modules without position
-// terms, and sequences whose slot table does not fit beside attention_f32_rel.cu's tiles (3409 positions on).
+// terms, and at head dim 64 sequences whose slot table does not fit beside attention_f32_rel.cu's tiles (3409 positions on; at
+// head dim 32 every length fits).
 //
 // Q, K and V come as three bf16 planes each whose sum is the fp32 value (linear_f32.cu: the QKV projection writes them), the
 // position scores C2P / P2C as fp32 [B,H,L,ld].  Semantics of kernel.py:137-345 in fp32 (the reference's strict mode):
