@@ -149,7 +149,7 @@ __device__ __forceinline__ void drain_accumulator(const GemmDesc& g, const CUten
       ptx::tmem_ld32(taddr + (uint32_t)c0, r);
       ptx::tmem_wait_ld();
       if (!ready || m >= g.M) continue;
-      store_chunk<T>(g, r, m, n, z, ncols, hd, bias);
+      store_chunk<T>(g, r, m, n, hd, bias);   // head-major: see tiled_store_ok
     }
     release();
     return;

@@ -323,7 +323,7 @@ __device__ __forceinline__ void tmem_dealloc_pair(uint32_t taddr, uint32_t ncols
 // one elected lane issues (the same lane every time, so that a commit covers the MMAs before it).  A branch on the lane
 // around the plain forms keeps the operands out of the uniform registers the instruction reads, and moving them there
 // costs more than a narrow MMA runs: M=128 SS N=32 / 64 / 128 measured 41 / 49 / 65 cycles per MMA in this form, 57 /
-// 57 / 65 in the other; with A in TMEM 18 / 33 / 65 against 54 / 54 / 65.
+// 57 / 65 in the other; with A in TMEM 18 / 33 / 65 against 54 / 54 / 65 (MMAs back to back, no waits between them).
 __device__ __forceinline__ void umma_ss_f16_warp(uint32_t d_tmem, uint64_t a_desc, uint64_t b_desc, uint32_t idesc,
                                                  uint32_t accumulate) {
   asm volatile(
@@ -354,18 +354,17 @@ __device__ __forceinline__ void umma_commit_warp(uint64_t* bar) {
       "@q tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];\n\t}" ::"r"(smem_u32(bar))
       : "memory");
 }
-__device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar, uint32_t leader = 0) {
-  const uint16_t both = (uint16_t)(3u << leader);
+__device__ __forceinline__ void umma_commit_pair_warp(uint64_t* bar) {   // on both CTAs' barriers, of a cluster that is one pair
   asm volatile(
       "{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\t"
       "@q tcgen05.commit.cta_group::2.mbarrier::arrive::one.shared::cluster.multicast::cluster.b64 [%0], %1;\n\t}"
-      ::"r"(smem_u32(bar)), "h"(both)
+      ::"r"(smem_u32(bar)), "h"((uint16_t)3)
       : "memory");
 }
 
 // For a loop that one elected lane runs alone, waits, MMAs and commits together: what it issues costs less than the elections and
-// votes of a converged warp (gemm_tile_kernel, 128 x 32 to 256 x 96 tiles: 60 cycles an MMA in the forms above, 36 here, with the
-// descriptors as words: the upper one is the same for A and B).
+// votes of a converged warp (gemm_tile_kernel, 128 x 32 to 256 x 96 tiles, a wait and a commit every eight MMAs counted in: 60 cycles
+// an MMA in the forms above, 36 here, with the descriptors as words: the upper one is the same for A and B).
 __device__ __forceinline__ bool elect_one() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred q;\n\telect.sync _|q, 0xffffffff;\n\tselp.u32 %0, 1, 0, q;\n\t}" : "=r"(r));
