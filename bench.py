@@ -64,9 +64,9 @@ WORKLOAD = dict(name="deberta-v3-base-encoder", geometry="v3-base", batch=32, se
 MIXED = dict(name="deberta-v3-large-mixed-buckets", geometry="v3-large", buckets={128: 171, 256: 171, 512: 170})
 FALLBACK_PEAKS = dict(hbm_gbs=6650.0, bf16_tflops=1590.0, bf16_tflops_sustained=1400.0)
 # DRAM bytes of one dfl_attention_rel_fwd launch per sequence of the default workload (12 heads, L=512, d=64, FP16,
-# valid lengths U[256,512]): dram__bytes_read.sum + dram__bytes_write.sum of an ncu capture of the launch inside the
-# workload (81.1 MB read + 12.5 MB written at B=32), per sequence.
-ATTN_DRAM_BYTES_PER_SEQUENCE = (81.146624e6 + 12.506368e6) / 32
+# valid lengths U[256,512]): dram__bytes_read.sum + dram__bytes_write.sum of ncu captures of two launches inside the
+# workload with two layers (78.2 + 11.3 and 75.6 + 7.9 MB read + written at B=32), their mean, per sequence.
+ATTN_DRAM_BYTES_PER_SEQUENCE = (76.903808e6 + 9.612928e6) / 32
 
 
 def make_config(geometry: str, layers: int | None = None):

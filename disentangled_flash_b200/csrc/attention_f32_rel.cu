@@ -21,8 +21,9 @@
 // faster), 49 with K, and the issuer's waits; the conversion of a P2C piece, 1.2 k, and its gathering, 1.1 k, lie beside it.
 // The softmax, 4.5 k, and PV, 2.6 k, follow.  An item starts and ends with 2 k and 3 k.  A second issuer with every other piece
 // hides the waits, but then the conversions set the same pace.
-// us with the projection, three launches / this one: 8 x 12 heads x 128 x d 64 68 / 41, 8 x 24 x 256 361 / 219, 4 x 12 x 512 221 / 148,
-// 2 x 12 x 1024 316 / 239, 1 x 12 x 64 36 / 27; d 32 8 x 24 x 256 261 / 111.
+// us with the projection, three launches / this one: 8 x 12 heads x 128 x d 64 65 / 40, 8 x 24 x 256 352 / 213, 4 x 12 x 512 217 / 146,
+// 2 x 12 x 1024 308 / 239, 1 x 12 x 64 34 / 26, 1 x 12 x 3400 1221 / 1037; d 32 8 x 24 x 256 257 / 110, 1 x 24 x 8192 9633 / 7079.  At no
+// length from 16 to 8192, with one term or two, 1 to 170 sequences, were the three launches faster.
 // One CTA per (batch, head, 128-query tile).  Warps 0-7 convert and softmax, 8-9 gather table pieces and V, 10 loads Q and K,
 // issues the MMAs and owns tensor memory: S (128 columns; P's three planes, 192, take its place), O 64, Q 96,
 // two accumulators of 64.

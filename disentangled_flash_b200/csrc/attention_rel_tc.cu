@@ -172,7 +172,7 @@ struct RBarriers {
   uint64_t c2p_ready, ring_release; // C2P rows of a tile: converters -> softmax -> converters
   uint64_t pair2[4];                // the two warps of a lane quarter: row maximum (row sum) posted
   uint64_t item_full[kItemSlots], item_empty[kItemSlots];
-  uint64_t xbar;                    // the eight softmax warps (mean-of-V path)
+  uint64_t xbar;                    // the eight softmax warps (column sums of V, for padded query rows)
   uint32_t tmem_base;
 };
 static_assert(sizeof(RBarriers) <= 512, "barrier block too large");
@@ -449,7 +449,7 @@ attention_rel_kernel(const __grid_constant__ CUtensorMap tmap_q, const __grid_co
     uint64_t* pair2 = &bars->pair2[q4];
     // Two running counts give every barrier phase of this role: c_t = key tiles started (all items), c_i = items with
     // kept rows finished.  Per tile one phase each of s_full, c2p_ready and o_ready, per tile and per item one of pair2;
-    // an item of padded rows only uses xbar exactly four times.
+    // an item that takes column sums of V (padded rows only, or beside kept ones) uses xbar exactly four times.
     uint32_t c_t = 0, c_i = 0;
     bool ok = true;
 

@@ -8,8 +8,8 @@
 namespace dfl {
 
 // Epilogue of one accumulator chunk of a head-major output whose rows cannot leave as whole boxes: 32 consecutive columns [n, n+32) of
-// output row m, as fp32 bit patterns in r.  Adds the bias, rounds to T and stores 32 (or 16) bytes at a time.  (With
-// the branches of row-major outputs and of GELU, which no launch reached, the operator at 16 x 24 heads x 256 x d 32 took 56.0 us, 52.8 without.)
+// output row m, as fp32 bit patterns in r.  Adds the bias, rounds to T and stores 32 (or 16) bytes at a time.  (With branches for
+// row-major outputs and GELU, which no launch reached, the operator at 16 x 24 heads x 256 x d 32 took 56.0 us; 52.8 without.)
 template <typename T>
 __device__ __forceinline__ void store_chunk(const GemmDesc& g, const uint32_t (&r)[32], int m, int n, int hd, const T* bias) {
   const int which = n / hd, rem = n - which * hd;

@@ -114,7 +114,9 @@ __global__ void __launch_bounds__(256, 3) refresh_planes_kernel(const DflPlaneSo
 // within [begin, end) of the tile, from shared memory, so that eight lanes store one row segment: bias, activation, row-major or
 // head-major, in fp32 or as bf16 planes.  `sums`: the warp's first row at the tile's column `begin`, `pitch` bytes from row to row.
 // Two rows at a time in one rolled loop: with a row at a time, its place divided out again for every chunk, and infinities looked
-// for element by element, a tile of 128 columns took 10.8 k cycles here, after 18.4 k of MMAs (1024 x 2304 x 768).
+// for element by element, a tile of 128 columns took 10.8 k cycles here, after 18.4 k of MMAs (1024 x 2304 x 768).  The kernels of 192 and
+// 256 columns hold their sums in registers around it and spill a little more for it: 60 / 136 and 68 / 156 bytes stored / loaded (12 / 4
+// and 44 / 72 before).
 template <int NCH>
 __device__ __forceinline__ void store_sums(const GemmDesc& g, const unsigned char* sums, uint32_t pitch, const float* bias, int m0,
                                            int rows_live, int z, int n0, int ncols, int begin, int end, int side, int lane) {
@@ -477,7 +479,8 @@ int launch_plan(const GemmDesc& g, int split, cudaStream_t stream) {
 }
 
 // Tile, pair and split by the same considerations as choose_gemm (linear_tc.cu), with six MMAs per product: nearly every
-// size is bound by the MMA rate times the waves over the SMs.
+// size is bound by the MMA rate times the waves over the SMs.  (The cycles of an MMA and of a tile's end were measured while a
+// converged warp issued the MMAs and finished tiles left a row at a time; the plans were not compared again.)
 struct F32Choice {
   int pair, nch, split;
 };
